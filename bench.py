@@ -59,10 +59,10 @@ def alg_bytes_per_cell_step(phase, s_pd, s_all, n_acoustic=7):
         "small_step_prep": 3 * (16 + 13),
         "calc_p_rho_0": 3 * (7 + 3),
         "calc_coef_w": 3 * (2 + 3),
-        "advance_uv": n_acoustic * (14 + 2),
-        "advance_mu_t": n_acoustic * (9 + 3),
+        "advance_uv": n_acoustic * (14 + 4),         # with sumflux's ru_m, rv_m
+        "advance_mu_t": n_acoustic * (10 + 4),       # with sumflux's ww_m
         "advance_w": n_acoustic * (17 + 3),
-        "sumflux_calc_p_rho": n_acoustic * (13 + 6),
+        "sumflux_calc_p_rho": n_acoustic * (6 + 3),  # calc_p_rho alone
         "small_step_finish": 3 * (13 + 6),
         "rk_update_scalar_pd": 2 * s_pd,
         # stages 1-2: read q (+ q_old at stage 2), write new q (+ q_old at stage 1),

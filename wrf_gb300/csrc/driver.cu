@@ -126,9 +126,9 @@ struct Ensemble {
   std::vector<WrfGpuDomainDesc> descs;
   std::vector<Mem> hm;                 // host copies of the member descriptors
   Mem* d_mems = nullptr;
-  int *d_bs2 = nullptr, *d_bs3 = nullptr, *d_bs_st = nullptr, *d_bs_tm = nullptr;
+  int *d_bs2 = nullptr, *d_bs3 = nullptr, *d_bs_st = nullptr, *d_bs_tm = nullptr, *d_bs_rw = nullptr;
   int* d_bs_pr = nullptr;  // mass tiles x pairs of species (the scalar transport)
-  int nb2 = 0, nb3 = 0, nb_st = 0, nb_tm = 0, nb_pr = 0;
+  int nb2 = 0, nb3 = 0, nb_st = 0, nb_tm = 0, nb_pr = 0, nb_rw = 0;
   // edge strips of members with open lateral boundaries (strip columns x
   // levels): the tendencies and the 5th/3rd-order transport, the PD
   // transport, and its limiter factors (one wider, halo included)
@@ -138,6 +138,7 @@ struct Ensemble {
   bool capturing = false;
   int capture_swaps = 0;               // species-buffer swaps in one captured step
   int nsp_max = 0, ns_max = 0, nlev_max = 0;
+  bool col_step = false;  // the acoustic step's mass columns go through k_advance_col (col_max_segments)
   bool damp3 = false;  // some member uses damp_opt = 3
   bool diff6 = false;  // some member stores diffusion tendencies (diff_6th_opt != 0 or diff_opt = 1)
   bool damp2 = false;  // some member uses damp_opt = 2 (Rayleigh damping toward the base state)
@@ -180,6 +181,7 @@ struct Ensemble {
   TileLaunch LP() const { return TileLaunch{d_mems, d_bs_pr, nmem}; }  // tiles x species pairs
   TileLaunch LST() const { return TileLaunch{d_mems, d_bs_st, nmem}; }  // staggered-extent tiles
   TileLaunch LTM() const { return TileLaunch{d_mems, d_bs_tm, nmem}; }  // mass-extent tiles
+  TileLaunch LRW() const { return TileLaunch{d_mems, d_bs_rw, nmem}; }  // row segments of 32 mass columns
   StripLaunch LS3() const { return StripLaunch{d_mems, d_bs_s3, nmem, STRIP_W_TEND, 0}; }
   StripLaunch LS4() const { return StripLaunch{d_mems, d_bs_s4, nmem, STRIP_W_PD, 0}; }
   StripLaunch LS5() const { return StripLaunch{d_mems, d_bs_s5, nmem, STRIP_W_PD + 1, 1}; }
@@ -638,6 +640,7 @@ struct Ensemble {
     if (d_bs_pr) cudaFree(d_bs_pr);
     if (d_bs_st) cudaFree(d_bs_st);
     if (d_bs_tm) cudaFree(d_bs_tm);
+    if (d_bs_rw) cudaFree(d_bs_rw);
     if (d_bs_s3) cudaFree(d_bs_s3);
     if (d_bs_s4) cudaFree(d_bs_s4);
     if (d_bs_s5) cudaFree(d_bs_s5);
@@ -698,7 +701,7 @@ struct Ensemble {
     CK(cudaMalloc(&d_cfl, sizeof(float) * 2 * n));
     CK(cudaMemsetAsync(d_cfl, 0, sizeof(float) * 2 * n, stream));
     std::vector<float*> scr(n);
-    std::vector<int> bs2(n + 1, 0), bs3(n + 1, 0), bst(n + 1, 0), btm(n + 1, 0), bpr(n + 1, 0), bs_s3(n + 1, 0),
+    std::vector<int> bs2(n + 1, 0), bs3(n + 1, 0), bst(n + 1, 0), btm(n + 1, 0), brw(n + 1, 0), bpr(n + 1, 0), bs_s3(n + 1, 0),
         bs_s4(n + 1, 0), bs_s5(n + 1, 0);
     for (int m = 0; m < n; ++m) {
       const WrfGpuDomainDesc& d = ds[m];
@@ -750,6 +753,7 @@ struct Ensemble {
       bpr[m + 1] = bpr[m] + tiles_x(M) * tiles_y(M) * blocks_per_tile(M.nsp, TILE_PER_PAIR);
       bst[m + 1] = bst[m] + tiles_x(M, true) * tiles_y(M, true);
       btm[m + 1] = btm[m] + tiles_x(M) * tiles_y(M);
+      brw[m + 1] = brw[m] + tiles_x(M) * (std::min(M.jte, M.jde - 1) - M.jts + 1);
       auto strip_blocks = [&](int w, int h) {
         const int nc = strip_cols(M.ide, M.jde, M.cf.open_xs, M.cf.open_ys, w, h);
         return (nc * (M.kme - M.kms + 1) + STRIP_THREADS - 1) / STRIP_THREADS;
@@ -759,7 +763,9 @@ struct Ensemble {
       bs_s4[m + 1] = bs_s4[m] + strip_blocks(STRIP_W_PD, 0);
       bs_s5[m + 1] = bs_s5[m] + strip_blocks(STRIP_W_PD + 1, 1);
     }
-    nb2 = bs2[n]; nb3 = bs3[n]; nb_st = bst[n]; nb_tm = btm[n]; nb_pr = bpr[n];
+    nb2 = bs2[n]; nb3 = bs3[n]; nb_st = bst[n]; nb_tm = btm[n]; nb_pr = bpr[n]; nb_rw = brw[n];
+    col_step = nb_rw <= col_max_segments(fp64, damp3);
+    if (fp64) tune[TU_AMUT] = 1;  // three blocks per SM (kernels.h)
     nb_s3 = bs_s3[n]; nb_s4 = bs_s4[n]; nb_s5 = bs_s5[n];
     {  // tensor maps of every 3-D buffer: halo and tile boxes
       int rc = get_tensor_map_encoder();
@@ -800,7 +806,7 @@ struct Ensemble {
     CK(cudaMemcpyAsync(d_bs_st, bst.data(), sizeof(int) * (n + 1), cudaMemcpyHostToDevice, stream));
     CK(cudaMalloc(&d_bs_tm, sizeof(int) * (n + 1)));
     CK(cudaMemcpyAsync(d_bs_tm, btm.data(), sizeof(int) * (n + 1), cudaMemcpyHostToDevice, stream));
-    for (auto& pr : {std::make_pair(&d_bs_s3, &bs_s3), std::make_pair(&d_bs_s4, &bs_s4),
+    for (auto& pr : {std::make_pair(&d_bs_rw, &brw), std::make_pair(&d_bs_s3, &bs_s3), std::make_pair(&d_bs_s4, &bs_s4),
                      std::make_pair(&d_bs_s5, &bs_s5)}) {
       CK(cudaMalloc(pr.first, sizeof(int) * (n + 1)));
       CK(cudaMemcpyAsync(*pr.first, pr.second->data(), sizeof(int) * (n + 1), cudaMemcpyHostToDevice, stream));
@@ -920,13 +926,17 @@ struct Ensemble {
       for (int it = 1; it <= nsmall_max; ++it) {
         StepArgs ai{rk_step, it, 0, 0};
         mark(PH_AUV); launch_advance_uv_col(LST(), nb_st, rk_step, it, stream, tune[TU_AUV]);
-        mark(PH_AMUT); launch_advance_mu_t_col(LTM(), nb_tm, rk_step, it, fp64, stream, tune[TU_AMUT]);
-        mark(PH_AW); launch_advance_w_col(LTM(), nb_tm, rk_step, it, fp64, stream, tune[TU_AW], damp3);
-        mark(PH_SUMF); launch_sumflux_p_rho_col(LST(), nb_st, rk_step, it, stream, tune[TU_SUMF]);
+        // advance_mu_t and sumflux's ww_m, advance_w, calc_p_rho
+        if (col_step) {
+          mark(PH_AW); launch_advance_col(LRW(), nb_rw, nlev_max, rk_step, it, fp64, stream, damp3);
+        } else {
+          mark(PH_AMUT); launch_advance_mu_t_col(LTM(), nb_tm, rk_step, it, fp64, stream, tune[TU_AMUT]);
+          mark(PH_AW); launch_advance_w_col(LTM(), nb_tm, rk_step, it, fp64, stream, tune[TU_AW], damp3);
+          mark(PH_SUMF); launch_calc_p_rho_col(LTM(), nb_tm, ai, stream, TUNE_PARAM[TU_SUMF][tune[TU_SUMF]]);
+        }
         // the fills of solve_em.F:1659-1716 (ph_2, al, p, muts, mu_2, mudf) are
-        // the producers' own halo stores (MassImages): advance_mu_t,
-        // advance_w and calc_p_rho write each halo image with its interior
-        // point, and nothing in the acoustic step reads these halos before
+        // the producers' own halo stores (MassImages): they write each halo
+        // image with its interior point, and nothing in the acoustic step reads these halos before
         // the next step's advance_uv; open boundaries' copies are the fill's
         if (any_open) {
           JobList j;

@@ -1,144 +1,33 @@
-// Column-marching forms of the acoustic-step kernels used by the fused
-// solver (the routine kernels of k_small.cu stay for routine-level calls).
+// Column forms of the acoustic-step kernels used by the fused solver (the
+// routine kernels of k_small.cu stay for routine-level calls):
 //
-// A block owns a TX x TY tile of columns and each thread marches its column
-// up k.  The inputs of level k+1 are loaded into registers before level k
-// is computed and stored, so every thread keeps a whole level of loads in
-// flight instead of waiting behind its own stores (the stores may alias the
-// loads as far as the compiler knows).  The per-point arithmetic is the
-// reference's, in its order: results are bit-identical to k_small.cu.
+//   k_advance_uv_col    advance_uv (module_small_step_em.F:654-967) and the
+//                       ru_m, rv_m sums of sumflux (:1473-1633)
+//   k_advance_mu_t_col  advance_mu_t (:969-1175) and the ww_m sum
+//   k_advance_w_col     advance_w (:1178-1469)
+//   k_advance_col       the last two and calc_p_rho (:438-568) in one pass, for
+//                       domains whose columns alone do not fill the GPU
 //
-//   k_sumflux_p_rho_col  sumflux (module_small_step_em.F:1473-1633) on the
-//                        u, v and w points of the column + calc_p_rho
-//                        (:438-568) on its mass points; tiles cover the
-//                        staggered extents so the u point i = ide and the v
-//                        point j = jde are included.
+// The per-point arithmetic is the reference's, in its order: results are
+// bit-identical to k_small.cu.
 #include "common.cuh"
 #include "kernels.h"
 #include "ffmath.h"
+#include "pair.cuh"
 
 namespace wrfgpu {
 
-namespace {
-struct SFLevel {
-  float rum, rvm, wwm;      // accumulated mass fluxes (0 at the first iteration)
-  float u, v, ww;           // current u, v, omega
-  float us, vs, ww1;        // linear parts (last iteration only)
-  float ph1, alt, t2, t1, c2a, pm1;  // calc_p_rho inputs (ph at k+1)
-};
-}  // namespace
-
-// One block per (staggered tile, chunk of levels: gridDim.y chunks); the
-// levels are independent but for ph(k), carried from the level below within
-// a chunk and read at a chunk's first level.
-template <int MINB>
-__global__ void __launch_bounds__(TX* TY, MINB) k_sumflux_p_rho_col(TileLaunch L, int rk_step, int iteration) {
-  const TilePos tp = tile_pos(L, false, true);
-  const Mem& m = block_member(L.mem, tp.m);
-  const Stage st = stage_of(m, rk_step);
-  if (iteration > st.nsmall) return;  // members with fewer acoustic steps
-  const int i = tp.i0 + threadIdx.x, j = tp.j0 + threadIdx.y;
-  if (i > m.ite || j > m.jte) return;
-  const int ns = st.nsmall;
-  const bool first = iteration == 1, last = iteration == ns;
-  const int mini = min(m.ide - 1, m.ite), minj = min(m.jde - 1, m.jte), mink = min(m.kde - 1, m.kte);
-  const int kts = m.kts, kte = m.kte;
-  const bool ucol = j <= minj, vcol = i <= mini, mcol = ucol && vcol;
-  MassImages img;  // the halo images of al and p (mass columns)
-  img.init(m, i, j);
-  F3 ru_m = f3(m, WRFGPU_RU_M), rv_m = f3(m, WRFGPU_RV_M), ww_m = f3(m, WRFGPU_WW_M);
-  F3 u2 = f3(m, WRFGPU_U_2), v2 = f3(m, WRFGPU_V_2), ww = f3(m, WRFGPU_WW), us = f3(m, WRFGPU_U_SAVE),
-     vs = f3(m, WRFGPU_V_SAVE), ww1 = f3(m, WRFGPU_WW1);
-  F3 al = f3(m, WRFGPU_AL), p = f3(m, WRFGPU_P), ph = f3(m, WRFGPU_PH_2), alt = f3(m, WRFGPU_ALT),
-     t_2 = f3(m, WRFGPU_T_2), t_1 = f3(m, WRFGPU_T_SAVE), c2a = f3(m, WRFGPU_C2A), pm1 = f3(m, WRFGPU_PM1);
-  F1 c1h = f1(m, WRFGPU_C1H), c2h = f1(m, WRFGPU_C2H), rdnw = f1(m, WRFGPU_RDNW);
-  float muu = 0.f, muv = 0.f, msfuy = 1.f, msfvx_inv = 1.f, muij = 0.f, mutij = 0.f;
-  if (last && ucol) { muu = f2(m, WRFGPU_MUU).ro(i, j); msfuy = f2(m, WRFGPU_MSFUY).ro(i, j); }
-  if (last && vcol) { muv = f2(m, WRFGPU_MUV).ro(i, j); msfvx_inv = f2(m, WRFGPU_MSFVX_INV).ro(i, j); }
-  if (mcol) { muij = f2(m, WRFGPU_MU_2).ro(i, j); mutij = f2(m, WRFGPU_MUTS).ro(i, j); }
-  const float smdiv = m.smdiv;
-
-  auto load = [&](int k, SFLevel& v) {
-    const bool ru_acc = ucol && k <= mink, rv_acc = vcol && k <= mink, mass = mcol && k <= mink;
-    v.rum = (!first && ru_acc) ? ru_m(i, k, j) : 0.f;
-    v.rvm = (!first && rv_acc) ? rv_m(i, k, j) : 0.f;
-    v.wwm = (!first && mcol) ? ww_m(i, k, j) : 0.f;
-    v.u = ru_acc ? u2.ro(i, k, j) : 0.f;
-    v.v = rv_acc ? v2.ro(i, k, j) : 0.f;
-    v.ww = mcol ? ww.ro(i, k, j) : 0.f;
-    v.us = (last && ru_acc) ? us.ro(i, k, j) : 0.f;
-    v.vs = (last && rv_acc) ? vs.ro(i, k, j) : 0.f;
-    v.ww1 = (last && mcol) ? ww1.ro(i, k, j) : 0.f;
-    if (mass) {
-      v.ph1 = ph.ro(i, k + 1, j);
-      v.alt = alt.ro(i, k, j); v.t2 = t_2.ro(i, k, j); v.t1 = t_1.ro(i, k, j); v.c2a = c2a.ro(i, k, j);
-      v.pm1 = pm1(i, k, j);
-    } else {
-      v.ph1 = v.alt = v.t2 = v.t1 = v.c2a = v.pm1 = 0.f;
-    }
-  };
-  const int per = (kte - kts + 1 + (int)gridDim.y - 1) / (int)gridDim.y;
-  const int k0 = kts + (int)blockIdx.y * per, k1 = min(kte, k0 + per - 1);
-  if (k0 > k1) return;
-  SFLevel cur, nxt;
-  load(k0, cur);
-  float ph_k = mcol ? ph.ro(i, k0, j) : 0.f;
-  for (int k = k0; k <= k1; ++k) {
-    if (k + 1 <= k1) load(k + 1, nxt);
-    const bool ru_acc = ucol && k <= mink, rv_acc = vcol && k <= mink;
-    // sumflux
-    float rum = cur.rum, rvm = cur.rvm, wwm = cur.wwm;
-    if (ru_acc) {
-      rum = rum + cur.u;
-      if (last) rum = rum / float(ns) + (c1h(k) * muu + c2h(k)) * cur.us / msfuy;
-    }
-    if (rv_acc) {
-      rvm = rvm + cur.v;
-      if (last) rvm = rvm / float(ns) + (c1h(k) * muv + c2h(k)) * cur.vs * msfvx_inv;
-    }
-    if (mcol) {
-      wwm = wwm + cur.ww;
-      if (last) wwm = wwm / float(ns) + cur.ww1;
-    }
-    if (first || ru_acc) ru_m(i, k, j) = rum;
-    if (first || rv_acc) rv_m(i, k, j) = rvm;
-    if (first || mcol) ww_m(i, k, j) = wwm;
-    // calc_p_rho on the mass point
-    if (mcol && k <= mink) {
-      const float a = cur.alt, t1 = cur.t1;
-      float alv = -1.f / (c1h(k) * mutij + c2h(k)) * (a * (c1h(k) * muij) + rdnw(k) * (cur.ph1 - ph_k));
-      img.store([&](int ii, int jj) { al(ii, k, jj) = alv; });
-      float pv = cur.c2a * (a * (cur.t2 - (c1h(k) * muij) * t1) / ((c1h(k) * mutij + c2h(k)) * (T0 + t1)) - alv);
-      if (iteration == 0) {
-        pm1(i, k, j) = pv;
-      } else {
-        const float ptmp = pv;
-        pv = pv + smdiv * (pv - cur.pm1);
-        pm1(i, k, j) = ptmp;
-      }
-      img.store([&](int ii, int jj) { p(ii, k, jj) = pv; });
-      ph_k = cur.ph1;
-    }
-    cur = nxt;
-  }
-}
-
-// variant parameter: 10 x blocks per SM + level chunks
-void launch_sumflux_p_rho_col(const TileLaunch& L, int nblocks, int rk_step, int iteration, cudaStream_t s, int var) {
-  const int p = TUNE_PARAM[TU_SUMF][var], chunks = p % 10;
-  if (p / 10 == 4) k_sumflux_p_rho_col<4><<<dim3(nblocks, chunks), dim3(TX, TY), 0, s>>>(L, rk_step, iteration);
-  else k_sumflux_p_rho_col<3><<<dim3(nblocks, chunks), dim3(TX, TY), 0, s>>>(L, rk_step, iteration);
-}
-
 // ---------------------------------------------------------------------------
 // advance_uv (module_small_step_em.F:654-967) on the u and v points of the
-// column, plus sumflux's accumulation of ru_m / rv_m left to
-// k_sumflux_p_rho_col.  Horizontal neighbours i-1 (u) and j-1 (v) are read
+// column, and sumflux's sums of ru_m and rv_m there: the new u and v are in
+// registers, so the sums cost one read and one write of ru_m and rv_m (in a
+// kernel of their own they read u and v again).  Horizontal neighbours i-1 (u) and j-1 (v) are read
 // directly (L1); p and ph of level k are kept from the previous level.
 // ---------------------------------------------------------------------------
 namespace {
 struct UVLevel {
   float u, rut, cqu, v, rvt, cqv;  // own u / v point
+  float rum, rvm, us, vs;          // accumulated mass fluxes (0 at the first iteration), linear parts (last one only)
   float p1, ph1, pb, php, alt, al;           // (i, j):   p, ph at k+1; the rest at k
   float p1x, ph1x, pbx, phpx, altx, alx;     // (i-1, j)
   float p1y, ph1y, pby, phpy, alty, aly;     // (i, j-1)
@@ -172,7 +61,13 @@ __global__ void __launch_bounds__(TX* TY, MINB) k_advance_uv_col(TileLaunch L, i
   const bool u_pg = upt && i >= i_start_up && i <= i_end_up;
   const bool vpt = j >= j_start_v_tend && j <= j_end_v_tend && i >= i_start && i <= i_end;
   const bool v_pg = vpt && j >= j_start_vp && j <= j_end_vp;
-  if (!upt && !vpt) return;
+  // sumflux: the points whose u (v) is summed; at the first iteration every
+  // point of the staggered tile starts from zero
+  const bool ucol = j <= min(m.jde - 1, m.jte), vcol = i <= min(m.ide - 1, m.ite);
+  const bool first = iteration == 1, last = iteration == st.nsmall;
+  const float fns = float(st.nsmall);
+  F3 ru_m = f3(m, WRFGPU_RU_M), rv_m = f3(m, WRFGPU_RV_M), ww_m = f3(m, WRFGPU_WW_M);
+  F3 usv = f3(m, WRFGPU_U_SAVE), vsv = f3(m, WRFGPU_V_SAVE);
   F3 p = f3(m, WRFGPU_P), pb = f3(m, WRFGPU_PB), ph = f3(m, WRFGPU_PH_2), php = f3(m, WRFGPU_PHP),
      alt = f3(m, WRFGPU_ALT), al = f3(m, WRFGPU_AL);
   F3 u = f3(m, WRFGPU_U_2), ru_tend = f3(m, WRFGPU_RU_TEND), cqu = f3(m, WRFGPU_CQU);
@@ -206,12 +101,19 @@ __global__ void __launch_bounds__(TX* TY, MINB) k_advance_uv_col(TileLaunch L, i
       mu_i = MU.ro(i, j); mu_jm = MU.ro(i, j - 1);
     }
   }
+  float muu_s = 0.f, muv_s = 0.f, msfuy_s = 1.f, mxi_s = 1.f;
+  if (last && ucol) { muu_s = f2(m, WRFGPU_MUU).ro(i, j); msfuy_s = f2(m, WRFGPU_MSFUY).ro(i, j); }
+  if (last && vcol) { muv_s = f2(m, WRFGPU_MUV).ro(i, j); mxi_s = f2(m, WRFGPU_MSFVX_INV).ro(i, j); }
   const bool need_x = u_pg, need_y = v_pg, need_c = u_pg || v_pg;
   auto load = [&](int k, UVLevel& d) {
-    d.u = upt ? u(i, k, j) : 0.f;
+    d.rum = (!first && ucol) ? ru_m(i, k, j) : 0.f;
+    d.rvm = (!first && vcol) ? rv_m(i, k, j) : 0.f;
+    d.us = (last && ucol) ? usv.ro(i, k, j) : 0.f;
+    d.vs = (last && vcol) ? vsv.ro(i, k, j) : 0.f;
+    d.u = ucol ? u(i, k, j) : 0.f;
     d.rut = u_tend ? ru_tend.ro(i, k, j) : 0.f;
     d.cqu = u_pg ? cqu.ro(i, k, j) : 0.f;
-    d.v = vpt ? v(i, k, j) : 0.f;
+    d.v = vcol ? v(i, k, j) : 0.f;
     d.rvt = vpt ? rv_tend.ro(i, k, j) : 0.f;
     d.cqv = v_pg ? cqv.ro(i, k, j) : 0.f;
     const bool top = k + 1 <= kde - 1;  // p exists up to kde-1
@@ -262,14 +164,13 @@ __global__ void __launch_bounds__(TX* TY, MINB) k_advance_uv_col(TileLaunch L, i
       dpn_v_top = .5f * (cf1 * (p.ro(i, kde - 1, j - 1) + p.ro(i, kde - 1, j)) + cf2 * (p.ro(i, kde - 2, j - 1) + p.ro(i, kde - 2, j)) +
                          cf3 * (p.ro(i, kde - 3, j - 1) + p.ro(i, kde - 3, j)));
   }
-  UVLevel cur, nxt;
-  load(k0, cur);
   for (int k = k0; k <= k1; ++k) {
-    if (k + 1 <= k1) load(k + 1, nxt);
+    UVLevel cur;  // a level's inputs go out together
+    load(k, cur);
     const int kk = k + 1;
     // u
+    float uv = cur.u;
     if (upt) {
-      float uv = cur.u;
       if (u_tend) uv = uv + dts * cur.rut;
       float dpn_hi = 0.f;
       if (u_pg) {
@@ -285,8 +186,9 @@ __global__ void __launch_bounds__(TX* TY, MINB) k_advance_uv_col(TileLaunch L, i
       u(i, k, j) = uv;
     }
     // v
+    float vv = cur.v;
     if (vpt) {
-      float vv = cur.v + dts * cur.rvt;
+      vv = vv + dts * cur.rvt;
       if (v_pg) {
         const float dpn_hi = (kk == kde) ? dpn_v_top : .5f * (fnm(kk) * (cur.p1 + cur.p1y) + fnp(kk) * (p0 + p0y));
         float dpxy = va * (c1h(k) * muv + c2h(k)) *
@@ -299,8 +201,26 @@ __global__ void __launch_bounds__(TX* TY, MINB) k_advance_uv_col(TileLaunch L, i
       }
       v(i, k, j) = vv;
     }
+    // sumflux
+    float rum = cur.rum, rvm = cur.rvm;
+    if (ucol) {
+      rum = rum + uv;
+      if (last) rum = rum / fns + (c1h(k) * muu_s + c2h(k)) * cur.us / msfuy_s;
+    }
+    if (vcol) {
+      rvm = rvm + vv;
+      if (last) rvm = rvm / fns + (c1h(k) * muv_s + c2h(k)) * cur.vs * mxi_s;
+    }
+    if (first || ucol) ru_m(i, k, j) = rum;
+    if (first || vcol) rv_m(i, k, j) = rvm;
+    if (first && !(ucol && vcol)) ww_m(i, k, j) = 0.f;
     p0 = cur.p1; ph0 = cur.ph1; p0x = cur.p1x; ph0x = cur.ph1x; p0y = cur.p1y; ph0y = cur.ph1y;
-    cur = nxt;
+  }
+  if (first && k1 == k_end) {  // level kde holds no mass flux but ww_m of the mass columns
+    const int kt = k_end + 1;
+    ru_m(i, kt, j) = 0.f;
+    rv_m(i, kt, j) = 0.f;
+    if (!(ucol && vcol)) ww_m(i, kt, j) = 0.f;
   }
 }
 
@@ -311,13 +231,12 @@ void launch_advance_uv_col(const TileLaunch& L, int nblocks, int rk_step, int it
   else k_advance_uv_col<3><<<dim3(nblocks, chunks), dim3(TX, TY), 0, s>>>(L, rk_step, iteration);
 }
 
-
-
 // ---------------------------------------------------------------------------
 // advance_mu_t (module_small_step_em.F:969-1175), one thread per mass column:
 // pass 1 the column divergence (kept per level) and its sum, then mu, and
-// pass 2 omega by upward recursion and theta.  RC: accumulation type of the
-// column sum and the recursion (float: the reference; double: mixed form).
+// pass 2 omega by upward recursion, theta and sumflux's sum of ww_m (:1473-1633).
+// RC: accumulation type of the column sum and the recursion (float: the
+// reference; double: mixed form).
 // ---------------------------------------------------------------------------
 constexpr int KCOL = 129;  // column scratch (kde <= 128)
 
@@ -374,9 +293,12 @@ __global__ void __launch_bounds__(TX* TY, MINB) k_advance_mu_t_col(TileLaunch L,
   const float my = msfty.ro(i, j), mx = msftx.ro(i, j);
   const RC rmy = rcp_rc<RC>((RC)my);  // mixed form only
   // pass 2: omega (recursion one level ahead of theta) and theta
-  struct D2 { float ww1, t, ft, t1, t1xm, t1xp, t1ym, t1yp, u0, u1, v0, v1; };
+  F3 ww_m = f3(m, WRFGPU_WW_M);
+  const bool first = iteration == 1, last = iteration == st.nsmall;
+  const float fns = float(st.nsmall);
+  struct D2 { float ww1, wwm, t, ft, t1, t1xm, t1xp, t1ym, t1yp, u0, u1, v0, v1; };
   auto load2 = [&](int k, D2& d) {
-    d.ww1 = ww_1.ro(i, k, j); d.t = t(i, k, j); d.ft = ft.ro(i, k, j);
+    d.ww1 = ww_1.ro(i, k, j); d.wwm = first ? 0.f : ww_m(i, k, j); d.t = t(i, k, j); d.ft = ft.ro(i, k, j);
     d.t1 = t_1.ro(i, k, j); d.t1xm = t_1.ro(i - 1, k, j); d.t1xp = t_1.ro(i + 1, k, j);
     d.t1ym = t_1.ro(i, k, j - 1); d.t1yp = t_1.ro(i, k, j + 1);
     d.u0 = u.ro(i, k, j); d.u1 = u.ro(i + 1, k, j); d.v0 = v.ro(i, k, j); d.v1 = v.ro(i, k, j + 1);
@@ -403,6 +325,11 @@ __global__ void __launch_bounds__(TX* TY, MINB) k_advance_mu_t_col(TileLaunch L,
       wwf_kp1 = (float)wwk - nxt.ww1;
     }
     ww(i, k, j) = wwf_k;
+    {
+      float wwm = cur.wwm + wwf_k;
+      if (last) wwm = wwm / fns + cur.ww1;
+      ww_m(i, k, j) = wwm;
+    }
     // theta of level k
     const float tv = cur.t;
     t_ave(i, k, j) = tv;
@@ -416,6 +343,11 @@ __global__ void __launch_bounds__(TX* TY, MINB) k_advance_mu_t_col(TileLaunch L,
     wdtn_lo = wdtn_hi;
     wwf_k = wwf_kp1;
     cur = nxt;
+  }
+  {  // level kde, whose omega stays
+    float wwm = (first ? 0.f : ww_m(i, kde, j)) + ww.ro(i, kde, j);
+    if (last) wwm = wwm / fns + ww_1.ro(i, kde, j);
+    ww_m(i, kde, j) = wwm;
   }
 }
 
@@ -720,6 +652,556 @@ void launch_advance_w_col(const TileLaunch& L, int nblocks, int rk_step, int ite
   const int minb = TUNE_PARAM[TU_AW][var];
   if (damp) launch_advance_w_var<true>(L, nblocks, rk_step, iteration, fp64, s, minb);
   else launch_advance_w_var<false>(L, nblocks, rk_step, iteration, fp64, s, minb);
+}
+
+// ---------------------------------------------------------------------------
+// advance_mu_t, advance_w, the ww_m sum of sumflux and calc_p_rho on one row
+// segment of 32 mass columns per block.  None of the four reads what another
+// column's four write, so once u and v have advanced they are one pass over
+// the column.
+//
+// Two columns per lane (8-byte accesses, packed adds), so 16 lanes hold the
+// segment and every half warp takes its own contiguous chunk of levels; the
+// column's intermediate values live in shared memory.  Only what the
+// reference sums or recurs level after level stays serial: the divergence sum
+// and the omega recursion are one add per level and are walked by every half
+// warp for itself (FP64 form: by warp 0, one lane per column), the tridiagonal
+// elimination and back substitution by warp 0.  Everything else — the
+// divergence, theta, the right-hand sides, the geopotential, p and al — runs
+// with all levels in flight.  A march of one thread per column took 1.1 to 2
+// us per level (barrier, loads and divisions in one chain) whatever the
+// domain's size, and left a narrow domain's other SMs idle.
+//
+// RC: type of the column sums and recursions (float: the reference; double:
+// the mixed form).
+// ---------------------------------------------------------------------------
+constexpr int COL_MAXW = 16;  // warps per block
+
+template <typename RC> struct alignas(2 * sizeof(RC)) Pair { RC x, y; };
+
+// Shared memory: level tables, then columns [kde + 1][32] of type RC (four:
+// the sum's terms, then c2a alt t_2ave, then w; and a, alpha, gamma, before
+// them the omega recursion's) and float (two: dv, then rhs; theta's part of p).
+template <typename RC> constexpr size_t col_smem(int nlev) {
+  return (size_t)(nlev + 2) * (2 * sizeof(float4) + 32 * (2 * sizeof(float) + 4 * sizeof(RC))) +
+         2 * COL_MAXW * 32 * sizeof(float);
+}
+
+template <typename RC, bool DAMP>
+__global__ void __launch_bounds__(32 * COL_MAXW, 1) k_advance_col(TileLaunch L, int rk_step, int iteration) {
+  extern __shared__ __align__(128) unsigned char smem[];
+  constexpr bool fp64 = sizeof(RC) == 8;
+  using P = Pair<RC>;
+  const int mi = find_member(L.block_start, L.nmem, blockIdx.x);
+  const Mem& m = block_member(L.mem, mi);
+  const Stage st = stage_of(m, rk_step);
+  if (iteration > st.nsmall) return;  // members with fewer acoustic steps
+  const int tid = threadIdx.x, hw = tid >> 4, c = (tid & 15) * 2;  // half warp, first column
+  const int lb = (int)blockIdx.x - __ldg(L.block_start + mi), ntx = tiles_x(m);
+  const int i0 = m.its + (lb % ntx) * 32, j = m.jts + lb / ntx;
+  const int i_end = min(m.ite, m.ide - 1);
+  // every lane takes part in the block's barriers; only columns of the domain
+  // store (a lane past them works on the segment's first pair; a pair's
+  // second column may be the first halo column)
+  const bool act = i0 + c <= i_end, act2 = i0 + c + 1 <= i_end;
+  const int i = act ? i0 + c : i0;
+  const int k_end = m.kte - 1, kde = m.kde, nlev = m.kme - m.kms + 1;
+  const bool first = iteration == 1, last = iteration == st.nsmall;
+  const float dts = st.dts_rk, epssm = m.epssm, rdx = m.rdx, rdy = m.rdy;
+  // this half warp's levels (a short column leaves the last half warps without)
+  const int nh = min((int)blockDim.x >> 4, nlev);
+  const int per = (k_end + nh - 1) / nh, ka = 1 + hw * per, kb = min(k_end, ka + per - 1);
+  const bool some = ka <= kb, top = some && kb == k_end;  // top: this half warp also owns level kde
+
+  const int NC = (nlev + 2) * 32;
+  // level tables: {c1h, c2h, c1f, c2f}, {dnw, rdnw, fnm, fnp} (the column kernels'
+  // 1-D coefficients, one 16-byte shared load instead of four global ones each)
+  float4* tA = reinterpret_cast<float4*>(smem);
+  float4* tB = tA + nlev + 2;
+  RC* sW = reinterpret_cast<RC*>(tB + nlev + 2);
+  RC* sA = sW + NC;
+  RC* sAL = sA + NC;
+  RC* sGA = sAL + NC;
+  float* sR = reinterpret_cast<float*>(sGA + NC);
+  float* sQ = sR + NC;
+  float* sX = sQ + NC;  // c2a alt t_2ave of each half warp's last level
+  auto at = [&](int k) { return k * 32 + c; };
+  auto rd = [&](const RC* s, int k) -> P { return *reinterpret_cast<const P*>(s + at(k)); };
+  auto wr = [&](RC* s, int k, RC a, RC b) { *reinterpret_cast<P*>(s + at(k)) = P{a, b}; };
+  auto rdf = [&](const float* s, int k) -> float2 { return *reinterpret_cast<const float2*>(s + at(k)); };
+  auto wrf = [&](float* s, int k, float2 v) { *reinterpret_cast<float2*>(s + at(k)) = v; };
+  auto gro = [&](const F3& a, int ii, int k, int jj) { return __ldg(reinterpret_cast<const float2*>(a.p + a.off(ii, k, jj))); };
+  auto g = [&](const F3& a, int k) { return *reinterpret_cast<const float2*>(a.p + a.off(i, k, j)); };
+  auto put = [&](const F3& a, int k, float2 v) {
+    if (act2) *reinterpret_cast<float2*>(a.p + a.off(i, k, j)) = v;
+    else if (act) a.p[a.off(i, k, j)] = v.x;
+  };
+  auto g2 = [&](int f, int ii, int jj) { const F2 a = f2(m, f); return make_float2(a.ro(ii, jj), a.ro(ii + 1, jj)); };
+  auto mul = [](float2 a, float2 b) { return make_float2(a.x * b.x, a.y * b.y); };
+  auto div = [](float2 a, float2 b) { return make_float2(a.x / b.x, a.y / b.y); };
+  // s1 x + s2
+  auto lin = [](float s1, float2 x, float s2) { return add2(muls(s1, x), bc2(s2)); };
+
+  F3 ww = f3(m, WRFGPU_WW), ww_1 = f3(m, WRFGPU_WW1), u = f3(m, WRFGPU_U_2), v = f3(m, WRFGPU_V_2),
+     t = f3(m, WRFGPU_T_2), t_1 = f3(m, WRFGPU_T_SAVE);
+  const F1 rdn = f1(m, WRFGPU_RDN);
+  {
+    F1 c1h = f1(m, WRFGPU_C1H), c2h = f1(m, WRFGPU_C2H), c1f = f1(m, WRFGPU_C1F), c2f = f1(m, WRFGPU_C2F),
+       dnw = f1(m, WRFGPU_DNW), fnm = f1(m, WRFGPU_FNM), fnp = f1(m, WRFGPU_FNP), rdnw = f1(m, WRFGPU_RDNW);
+    for (int k = 1 + tid; k <= kde; k += blockDim.x) {
+      tA[k] = make_float4(c1h(k), c2h(k), c1f(k), c2f(k));
+      tB[k] = make_float4(dnw(k), rdnw(k), fnm(k), fnp(k));
+    }
+  }
+  const float2 my = g2(WRFGPU_MSFTY, i, j), mx = g2(WRFGPU_MSFTX, i, j);
+  const float2 mu_tend = g2(WRFGPU_MU_TEND, i, j), mutij = g2(WRFGPU_MUT, i, j);
+  // read by every half warp before the first barrier, written by one after it
+  const float2 mu_old = make_float2(f2(m, WRFGPU_MU_2)(i, j), f2(m, WRFGPU_MU_2)(i + 1, j)), ww_bot = g(ww, 1);
+  __syncthreads();  // the level tables
+
+  // ---- advance_mu_t: the column divergence
+  const bool one_y = __all_sync(~0u, my.x == 1.f && my.y == 1.f);  // x / 1 = x: no map factor, no division
+  {
+    F3 u_1 = f3(m, WRFGPU_U_SAVE), v_1 = f3(m, WRFGPU_V_SAVE);
+    const float2 mxy = mul(mx, my);
+    const float2 muv0 = g2(WRFGPU_MUV, i, j), muv1 = g2(WRFGPU_MUV, i, j + 1), muu0 = g2(WRFGPU_MUU, i, j),
+                 muu1 = g2(WRFGPU_MUU, i + 1, j);
+    const float2 vi0 = g2(WRFGPU_MSFVX_INV, i, j), vi1 = g2(WRFGPU_MSFVX_INV, i, j + 1), uy0 = g2(WRFGPU_MSFUY, i, j),
+                 uy1 = g2(WRFGPU_MSFUY, i + 1, j);
+    const bool one_u = __all_sync(~0u, uy0.x == 1.f && uy0.y == 1.f && uy1.y == 1.f);
+#pragma unroll 2
+    for (int k = ka; k <= kb; ++k) {
+      const float2 v0 = gro(v, i, k, j), v1 = gro(v, i, k, j + 1), vo0 = gro(v_1, i, k, j), vo1 = gro(v_1, i, k, j + 1);
+      const float2 u0 = gro(u, i, k, j), uo0 = gro(u_1, i, k, j);
+      const float2 u1 = make_float2(u0.y, u.ro(i + 2, k, j)), uo1 = make_float2(uo0.y, u_1.ro(i + 2, k, j));
+      const float4 ta = tA[k];
+      float2 q0 = mul(lin(ta.x, muu0, ta.y), uo0), q1 = mul(lin(ta.x, muu1, ta.y), uo1);
+      if (!one_u) { q0 = div(q0, uy0); q1 = div(q1, uy1); }
+      const float2 dv =
+          mul(mxy, add2(muls(rdy, sub2(add2(v1, mul(mul(lin(ta.x, muv1, ta.y), vo1), vi1)),
+                                       add2(v0, mul(mul(lin(ta.x, muv0, ta.y), vo0), vi0)))),
+                        muls(rdx, sub2(add2(u1, q1), add2(u0, q0)))));
+      wrf(sR, k, dv);
+      const float dnw = tB[k].x;
+      // FP64: the product is exact, so adding it is the fused multiply-add of the mixed form
+      wr(sW, k, (RC)dnw * (RC)dv.x, (RC)dnw * (RC)dv.y);
+    }
+  }
+  __syncthreads();
+  // its sum in k order, and the omega recursion: the FP32 form leaves the
+  // recursion's terms in sAL, the FP64 form omega itself
+  P dmdt{RC(0.), RC(0.)};
+  if constexpr (fp64) {
+    // the conversions and products are formed by all warps, so that one FP64
+    // operation per level is left in each chain (it waits about 110 cycles
+    // for its predecessor)
+    if (tid < 32) {
+      RC s = RC(0.);
+#pragma unroll 8
+      for (int k = 1; k <= k_end; ++k) s = s + sW[k * 32 + tid];
+      sGA[32 + tid] = s;
+    }
+    __syncthreads();
+    dmdt = rd(sGA, 1);
+    const P rmy{rcp_rc<RC>((RC)my.x), rcp_rc<RC>((RC)my.y)};
+    const P dm{dmdt.x + (RC)mu_tend.x, dmdt.y + (RC)mu_tend.y};
+    for (int k = ka; k <= kb; ++k) {
+      const RC c1 = (RC)tA[k].x, dn = (RC)tB[k].x;
+      const float2 dv = rdf(sR, k);
+      wr(sA, k, -fma(c1, dm.x, (RC)dv.x), -fma(c1, dm.y, (RC)dv.y));
+      wr(sW, k, dn * rmy.x, dn * rmy.y);
+    }
+    if (hw == 0) wr(sAL, 1, (RC)ww_bot.x, (RC)ww_bot.y);
+    __syncthreads();
+    if (tid < 32) {
+      RC wwk = sAL[32 + tid];
+#pragma unroll 4
+      for (int k = 1; k < k_end; ++k) {
+        wwk = fma(sA[k * 32 + tid], sW[k * 32 + tid], wwk);
+        sAL[(k + 1) * 32 + tid] = wwk;
+      }
+    }
+  } else {
+    float2 s = bc2(0.f);
+#pragma unroll 8
+    for (int k = 1; k <= k_end; ++k) s = add2(s, rdf(sW, k));
+    dmdt = P{s.x, s.y};
+    for (int k = ka; k <= kb; ++k) {
+      const float c1 = tA[k].x;
+      float2 tt = muls(tB[k].x, add2(add2(muls(c1, s), rdf(sR, k)), muls(c1, mu_tend)));
+      if (!one_y) tt = div(tt, my);
+      wrf(sAL, k, tt);
+    }
+  }
+  __syncthreads();
+  float2 mu, mudf;
+  mu.x = (float)((RC)mu_old.x + (RC)dts * (dmdt.x + (RC)mu_tend.x));
+  mu.y = (float)((RC)mu_old.y + (RC)dts * (dmdt.y + (RC)mu_tend.y));
+  mudf.x = (float)(dmdt.x + (RC)mu_tend.x);
+  mudf.y = (float)(dmdt.y + (RC)mu_tend.y);
+  const float2 mts = add2(mutij, mu);
+  const float2 mua = muls(.5f, add2(muls(1.f + epssm, mu), muls(1.f - epssm, mu_old)));
+  MassImages im0, im1;  // the halo images of mu, mudf, muts, ph, p and al
+  im0.init(m, i, j);
+  im1.init(m, i + 1, j);
+  const bool img = im0.any || im1.any || !act2;
+  // v into field a at level k and its halo images
+  auto put_img = [&](const F3& a, int k, float2 val) {
+    if (!img) {
+      *reinterpret_cast<float2*>(a.p + a.off(i, k, j)) = val;
+      return;
+    }
+    if (act) im0.store([&](int ii, int jj) { a.p[a.off(ii, k, jj)] = val.x; });
+    if (act2) im1.store([&](int ii, int jj) { a.p[a.off(ii, k, jj)] = val.y; });
+  };
+  if (hw == 0) {
+    F2 MU = f2(m, WRFGPU_MU_2), MUDF = f2(m, WRFGPU_MUDF), MUTS = f2(m, WRFGPU_MUTS), MUAVE = f2(m, WRFGPU_MUAVE);
+    if (act) {
+      im0.store([&](int ii, int jj) { MU(ii, jj) = mu.x; MUDF(ii, jj) = mudf.x; MUTS(ii, jj) = mts.x; });
+      MUAVE(i, j) = mua.x;
+    }
+    if (act2) {
+      im1.store([&](int ii, int jj) { MU(ii, jj) = mu.y; MUDF(ii, jj) = mudf.y; MUTS(ii, jj) = mts.y; });
+      MUAVE(i + 1, j) = mua.y;
+    }
+  }
+
+  // ---- theta and ww_m; then per level what advance_w and calc_p_rho take
+  // from theta, and advance_w's rhs
+  F3 ph = f3(m, WRFGPU_PH_2), w = f3(m, WRFGPU_W_2), c2a = f3(m, WRFGPU_C2A), alt = f3(m, WRFGPU_ALT);
+  const bool adv2 = m.cf.phi_adv_z == 2;
+  float2 x_top = bc2(0.f);  // 2 rdnw c2a alt t_2ave of level k_end, for the lid's w
+  if (some) {
+    F3 ww_m = f3(m, WRFGPU_WW_M), ft = f3(m, WRFGPU_T_TEND), pht = f3(m, WRFGPU_PH_TEND), ph1 = f3(m, WRFGPU_PH_SAVE),
+       phb = f3(m, WRFGPU_PHB), t_2ave = f3(m, WRFGPU_T_2SAVE);
+    const float fns = float(st.nsmall);
+    const bool keep_tave = last && rk_step == 3;  // t_2ave as the large step leaves it
+    const float2 mydts = muls(dts, my);  // my dts = dts my
+    // omega before the linear part is taken off, at levels ka - 1 and ka
+    float2 wr_m = bc2(0.f), wrr = ww_bot;
+    if constexpr (fp64) {
+      const P a = rd(sAL, max(ka - 1, 1)), b = rd(sAL, ka);
+      wr_m = make_float2((float)a.x, (float)a.y);
+      wrr = make_float2((float)b.x, (float)b.y);
+    } else {
+#pragma unroll 8
+      for (int k = 2; k <= ka; ++k) { wr_m = wrr; wrr = sub2(wrr, rdf(sAL, k - 1)); }
+    }
+    float2 ww1_k = gro(ww_1, i, ka, j), ww_k = sub2(wrr, ww1_k);
+    float2 t1_k = gro(t_1, i, ka, j), ph1_k = gro(ph1, i, ka, j), phb_k = gro(phb, i, ka, j);
+    float2 wdtn_lo = bc2(0.f), wd_k = bc2(0.f);
+    if (ka > 1) {
+      const float4 tb = tB[ka];
+      const float2 ww_km = sub2(wr_m, gro(ww_1, i, ka - 1, j));
+      wdtn_lo = mul(ww_k, add2(muls(tb.z, t1_k), muls(tb.w, gro(t_1, i, ka - 1, j))));
+      const float2 dphi = sub2(add2(sub2(ph1_k, gro(ph1, i, ka - 1, j)), phb_k), gro(phb, i, ka - 1, j));
+      const float rd_m = tB[ka - 1].y;
+      if (adv2) wd_k = muls(rd_m, dphi);
+      else wd_k = mul(muls(rd_m, muls(.5f, add2(ww_k, ww_km))), dphi);
+    }
+    const float2 ww_top = top ? gro(ww, i, kde, j) : bc2(0.f);
+    float2 x = bc2(0.f);
+    for (int k = ka; k <= kb; ++k) {
+      const bool in = k < k_end;
+      const float2 ww1_n = (in || last) ? gro(ww_1, i, k + 1, j) : bc2(0.f);
+      const float2 c_t = g(t, k), c_ft = gro(ft, i, k, j), t1_n = in ? gro(t_1, i, k + 1, j) : bc2(0.f);
+      const float2 ym = gro(t_1, i, k, j - 1), yp = gro(t_1, i, k, j + 1);
+      const float2 xm = make_float2(t_1.ro(i - 1, k, j), t1_k.x), xp = make_float2(t1_k.y, t_1.ro(i + 2, k, j));
+      const float2 u0 = gro(u, i, k, j), u1 = make_float2(u0.y, u.ro(i + 2, k, j));
+      const float2 v0 = gro(v, i, k, j), v1 = gro(v, i, k, j + 1);
+      const float2 c_alt = gro(alt, i, k, j), c_c2a = gro(c2a, i, k, j), c_ph = g(ph, k);
+      const float2 ph1_n = gro(ph1, i, k + 1, j), phb_n = gro(phb, i, k + 1, j);
+      const float2 c_pht = gro(pht, i, k, j), c_w = g(w, k);
+      const float2 c_wwm = first ? bc2(0.f) : g(ww_m, k);
+      const float4 ta = tA[k], tb = tB[k], tn = tB[k + 1];
+      // omega of the level above: wwf for theta (zero at the lid), ww for phi
+      float2 wwf_n = bc2(0.f), ww_n = ww_top;
+      if (in) {
+        if constexpr (fp64) {
+          const P b = rd(sAL, k + 1);
+          wrr = make_float2((float)b.x, (float)b.y);
+        } else {
+          wrr = sub2(wrr, rdf(sAL, k));
+        }
+        wwf_n = sub2(wrr, ww1_n);
+        ww_n = wwf_n;
+      }
+      if (last || k == 1) put(ww, k, ww_k);
+      {  // sumflux
+        float2 wwm = add2(c_wwm, ww_k);
+        if (last) wwm = add2(div(wwm, bc2(fns)), ww1_k);
+        put(ww_m, k, wwm);
+      }
+      // theta
+      const float2 wdtn_hi = in ? mul(wwf_n, add2(muls(tn.z, t1_n), muls(tn.w, t1_k))) : bc2(0.f);
+      float2 tt = add2(c_t, mul(mydts, c_ft));
+      tt = sub2(tt, mul(mydts,
+                        add2(mul(mx, add2(muls(.5f * rdy, sub2(mul(v1, add2(yp, t1_k)), mul(v0, add2(t1_k, ym)))),
+                                          muls(.5f * rdx, sub2(mul(u1, add2(xp, t1_k)), mul(u0, add2(t1_k, xm)))))),
+                             muls(tb.y, sub2(wdtn_hi, wdtn_lo)))));
+      put(t, k, tt);
+      wdtn_lo = wdtn_hi;
+      // t_2ave, and theta's part of p
+      const float2 mth = mul(lin(ta.x, mts, ta.y), add2(bc2(T0), t1_k));
+      float2 tav = muls(.5f, add2(muls(1.f + epssm, tt), muls(1.f - epssm, c_t)));
+      tav = div(add2(tav, muls(T0, muls(ta.x, mua))), mth);
+      if (keep_tave) put(t_2ave, k, tav);
+      x = mul(mul(c_c2a, c_alt), tav);
+      wr(sW, k, (RC)x.x, (RC)x.y);
+      if (k == k_end) x_top = mul(mul(muls(2.f * tb.y, c_c2a), c_alt), tav);
+      wrf(sQ, k, div(mul(c_alt, sub2(tt, mul(muls(ta.x, mu), t1_k))), mth));
+      // rhs
+      const float2 dphi = sub2(add2(sub2(ph1_n, ph1_k), phb_n), phb_k);
+      float2 wd_hi;
+      if (adv2) wd_hi = muls(tb.y, dphi);
+      else wd_hi = mul(muls(tb.y, muls(.5f, add2(ww_n, ww_k))), dphi);
+      float2 r = bc2(0.f);
+      if (k >= 2) {
+        r = muls(dts, add2(c_pht, muls(.5f * G * (1.f - epssm), c_w)));
+        const float2 wdi = add2(muls(tb.z, wd_hi), muls(tb.w, wd_k));
+        if (adv2) r = sub2(r, mul(muls(dts, ww_k), wdi));
+        else r = sub2(r, muls(dts, wdi));
+        r = add2(c_ph, div(mul(my, r), lin(ta.z, mutij, ta.w)));
+      }
+      wrf(sR, k, r);
+      wd_k = wd_hi; ww_k = ww_n; ww1_k = ww1_n; t1_k = t1_n; ph1_k = ph1_n; phb_k = phb_n;
+    }
+    *reinterpret_cast<float2*>(sX + hw * 32 + c) = x;
+    if (top) {  // level kde: rhs without omega; ww_m
+      float2 wwm = add2(first ? bc2(0.f) : g(ww_m, kde), ww_top);
+      if (last) wwm = add2(div(wwm, bc2(fns)), ww1_k);
+      put(ww_m, kde, wwm);
+      const float4 ta = tA[kde];
+      const float2 rr = muls(dts, add2(gro(pht, i, kde, j), muls(.5f * G * (1.f - epssm), g(w, kde))));
+      float2 r = add2(g(ph, kde), div(mul(my, rr), lin(ta.z, mutij, ta.w)));
+      if (m.cf.top_lid) r = bc2(0.f);
+      wrf(sR, kde, r);
+    }
+  }
+  __syncthreads();
+
+  // ---- advance_w: explicit w of every level, and the elimination's coefficients
+  const float eps1 = 1.f + epssm, eps0 = 1.f - epssm;
+  float2 w1 = bc2(0.f);
+  if (hw == 0) {  // surface w
+    F2 ht = f2(m, WRFGPU_HT);
+    const float cf1 = m.cf1, cf2 = m.cf2, cf3 = m.cf3;
+    auto surf = [&](int I, int J, float myc, float mxc) {
+      return (myc * .5f * rdy *
+                  ((ht.ro(I, J + 1) - ht.ro(I, J)) * (cf1 * v.ro(I, 1, J + 1) + cf2 * v.ro(I, 2, J + 1) + cf3 * v.ro(I, 3, J + 1)) +
+                   (ht.ro(I, J) - ht.ro(I, J - 1)) * (cf1 * v.ro(I, 1, J) + cf2 * v.ro(I, 2, J) + cf3 * v.ro(I, 3, J))) +
+              mxc * .5f * rdx *
+                  ((ht.ro(I + 1, J) - ht.ro(I, J)) * (cf1 * u.ro(I + 1, 1, J) + cf2 * u.ro(I + 1, 2, J) + cf3 * u.ro(I + 1, 3, J)) +
+                   (ht.ro(I, J) - ht.ro(I - 1, J)) * (cf1 * u.ro(I, 1, J) + cf2 * u.ro(I, 2, J) + cf3 * u.ro(I, 3, J))));
+    };
+    w1 = make_float2(surf(i, j, my.x, mx.x), surf(i + 1, j, my.y, mx.y));
+    put(w, 1, w1);  // level 1 of w is not read in this kernel after the last barrier
+  }
+  if (some) {
+    F3 rwt = f3(m, WRFGPU_RW_TEND), cqw = f3(m, WRFGPU_CQW);
+    auto coef = [&](int q, int k) -> P {
+      if constexpr (fp64) {
+        const double2 d = __ldg(reinterpret_cast<const double2*>(&d3(m, m.wd[q])(i, k, j)));
+        return P{d.x, d.y};
+      } else {
+        const float2 d = gro(f3(m, q == 0 ? WRFGPU_A : q == 1 ? WRFGPU_ALPHA : WRFGPU_GAMMA), i, k, j);
+        return P{d.x, d.y};
+      }
+    };
+    const float2 msft_inv = div(bc2(1.f), my);
+    // level k's term of the vertical difference, from levels k and k+1
+    auto dz = [&](int k, float2 c2ak, float2 r_0, float2 r_p, float2 ph_0, float2 ph_p) {
+      const float4 ta = tA[k];
+      return mul(div(muls(tB[k].y, c2ak), lin(ta.x, mutij, ta.y)),
+                 add2(muls(eps1, sub2(r_p, r_0)), muls(eps0, sub2(ph_p, ph_0))));
+    };
+    float2 r_k = rdf(sR, ka), ph_k = g(ph, ka);
+    float2 dz_m = bc2(0.f), x_m = bc2(0.f), c_c2a = bc2(0.f);
+    if (ka > 1) {
+      dz_m = dz(ka - 1, gro(c2a, i, ka - 1, j), rdf(sR, ka - 1), r_k, g(ph, ka - 1), ph_k);
+      x_m = *reinterpret_cast<const float2*>(sX + (hw - 1) * 32 + c);
+    }
+    float2 r_m = bc2(0.f), ph_m = bc2(0.f);
+    for (int k = ka; k <= kb; ++k) {
+      c_c2a = gro(c2a, i, k, j);
+      const float2 ph_p = g(ph, k + 1), r_p = rdf(sR, k + 1);
+      const P xr = rd(sW, k);
+      const float2 x = make_float2((float)xr.x, (float)xr.y);
+      const float2 c_w = g(w, k), c_rwt = gro(rwt, i, k, j), c_cqw = gro(cqw, i, k, j);
+      const P ca = coef(0, k), cal = coef(1, k), cga = coef(2, k);
+      const float2 dz_k = dz(k, c_c2a, r_k, r_p, ph_k, ph_p);
+      if (k >= 2) {
+        const float rdnk = rdn(k);
+        const float2 wk = add2(add2(add2(c_w, muls(dts, c_rwt)),
+                                    mul(mul(msft_inv, c_cqw), muls(+.5f * dts * G * rdnk, sub2(dz_k, dz_m)))),
+                               mul(muls(dts * G, msft_inv), sub2(muls(rdnk, sub2(x, x_m)), muls(tA[k].z, mua))));
+        wr(sW, k, (RC)wk.x, (RC)wk.y);
+        wr(sA, k, ca.x, ca.y);
+        wr(sAL, k, cal.x, cal.y);
+        wr(sGA, k, cga.x, cga.y);
+      }
+      dz_m = dz_k; x_m = x; r_m = r_k; ph_m = ph_k; r_k = r_p; ph_k = ph_p;
+    }
+    if (hw == 0) wr(sW, 1, (RC)w1.x, (RC)w1.y);
+    if (top) {
+      const int k = kde;
+      const float r = tB[k - 1].y;
+      const float4 tm = tA[k - 1];
+      const float2 q = muls(r * r, div(bc2(-.5f * dts * G), lin(tm.x, mutij, tm.y)));
+      const float2 a = mul(mul(muls(2.f, q), c_c2a),
+                           add2(muls(eps1, sub2(r_k, r_m)), muls(eps0, sub2(ph_k, ph_m))));
+      float2 wk = add2(add2(g(w, k), muls(dts, gro(rwt, i, k, j))),
+                       mul(msft_inv, sub2(a, muls(dts * G, add2(x_top, muls(tA[k].z, mua))))));
+      if (m.cf.top_lid) wk = bc2(0.f);
+      const P ca = coef(0, k), cal = coef(1, k);
+      wr(sW, k, (RC)wk.x, (RC)wk.y);
+      wr(sA, k, ca.x, ca.y);
+      wr(sAL, k, cal.x, cal.y);
+    }
+  }
+  __syncthreads();
+  // ---- the tridiagonal solve, one lane per column; a batch of levels is read
+  // ahead of its recursion
+  if (tid < 32) {
+    constexpr int Q = fp64 ? 4 : 8;
+    RC wk = sW[32 + tid], b[Q], a[Q], al[Q];
+    auto up = [&](int kq) {
+#pragma unroll
+      for (int q = 0; q < Q; ++q) {
+        const int o = min(kq + q, kde) * 32 + tid;
+        b[q] = sW[o]; a[q] = sA[o]; al[q] = sAL[o];
+      }
+    };
+    up(2);
+    for (int kq = 2; kq <= kde; kq += Q) {
+      RC r[Q], cb[Q], ca[Q], cal[Q];
+#pragma unroll
+      for (int q = 0; q < Q; ++q) { cb[q] = b[q]; ca[q] = a[q]; cal[q] = al[q]; }
+      up(kq + Q);
+#pragma unroll
+      for (int q = 0; q < Q; ++q) {
+        if constexpr (fp64) wk = fma(-ca[q], wk, cb[q]) * cal[q];  // mixed form: one FP64 fma
+        else wk = (cb[q] - ca[q] * wk) * cal[q];
+        r[q] = wk;
+      }
+#pragma unroll
+      for (int q = 0; q < Q; ++q)
+        if (kq + q <= kde) sW[(kq + q) * 32 + tid] = r[q];
+    }
+    wk = sW[kde * 32 + tid];
+    auto down = [&](int kq) {
+#pragma unroll
+      for (int q = 0; q < Q; ++q) {
+        const int o = max(kq - q, 2) * 32 + tid;
+        b[q] = sW[o]; a[q] = sGA[o];
+      }
+    };
+    down(k_end);
+    for (int kq = k_end; kq >= 2; kq -= Q) {
+      RC r[Q], cb[Q], ca[Q];
+#pragma unroll
+      for (int q = 0; q < Q; ++q) { cb[q] = b[q]; ca[q] = a[q]; }
+      down(kq - Q);
+#pragma unroll
+      for (int q = 0; q < Q; ++q) {
+        if constexpr (fp64) wk = fma(-ca[q], wk, cb[q]);
+        else wk = cb[q] - ca[q] * wk;
+        r[q] = wk;
+      }
+#pragma unroll
+      for (int q = 0; q < Q; ++q)
+        if (kq - q >= 2) sW[(kq - q) * 32 + tid] = r[q];
+    }
+  }
+  __syncthreads();
+  if (!some || !act) return;
+
+  // ---- damp_opt = 3 (module_small_step_em.F:1445-1458): after the back
+  // substitution, w relaxes toward w_save in the top zdamp metres with
+  // weight dampmag sin^2(pi/2 (h - hbot) / zdamp); the geopotential then
+  // takes the damped w.  The recursion itself ran on the undamped values.
+  // DAMP: compiled in only when some member uses it (the launcher's choice)
+  const bool damp3 = DAMP && m.cf.damp_opt == 3;
+  const F3 w_save = f3(m, WRFGPU_W_SAVE), ph_1 = f3(m, WRFGPU_PH_SAVE), phb = f3(m, WRFGPU_PHB);
+  const float hdepth = m.cf.zdamp, dampmag = dts * m.cf.dampcoef;
+  float2 hbot = bc2(0.f);
+  if (damp3) {
+    const float2 h = add2(gro(ph_1, i, kde, j), gro(phb, i, kde, j));
+    hbot = make_float2(h.x / G - hdepth, h.y / G - hdepth);
+  }
+  auto damped = [&](float wk, float h, float hb, float mass, float ws) -> float {
+    const float hk = h / G;
+    float dampwt = 0.f;
+    if (hk >= hb) {
+      const float sn = wrfgpu_ff::sinf_cr(.5f * PI_F * (hk - hb) / hdepth);
+      dampwt = dampmag * sn * sn;
+    }
+    return (wk - dampwt * mass * ws) / (1.f + dampwt);
+  };
+  auto new_w = [&](int k) -> float2 {
+    const P r = rd(sW, k);
+    float2 wk = make_float2((float)r.x, (float)r.y);
+    if (damp3) {
+      const float2 h = add2(gro(ph_1, i, k, j), gro(phb, i, k, j)), ws = gro(w_save, i, k, j);
+      const float2 mass = lin(tA[k].z, mutij, tA[k].w);
+      wk = make_float2(damped(wk.x, h.x, hbot.x, mass.x, ws.x), damped(wk.y, h.y, hbot.y, mass.y, ws.y));
+    }
+    return wk;
+  };
+  const float2 pc = muls(eps1, muls(G, muls(dts, muls(.5f, my))));  // my .5 dts g (1 + epssm), left to right
+  auto new_ph = [&](int k, float2 wst) {
+    const float4 ta = tA[k];
+    return add2(rdf(sR, k), div(mul(pc, wst), lin(ta.z, mts, ta.w)));
+  };
+  // ---- w, the geopotential, and calc_p_rho between two of its levels
+  F3 al = f3(m, WRFGPU_AL), p = f3(m, WRFGPU_P), pm1 = f3(m, WRFGPU_PM1);
+  const float smdiv = m.smdiv;
+  float2 ph_k;
+  if (ka == 1) {
+    ph_k = g(ph, 1);
+  } else {
+    const float2 wst = new_w(ka);
+    put(w, ka, wst);
+    ph_k = new_ph(ka, wst);
+    put_img(ph, ka, ph_k);
+  }
+  for (int k = ka; k <= kb; ++k) {
+    const float2 a = gro(alt, i, k, j), c_c2a = gro(c2a, i, k, j), c_pm1 = g(pm1, k);
+    const int kn = k + 1;
+    const float2 wst = new_w(kn), ph_n = new_ph(kn, wst);
+    if (kn <= kb || kn == kde) {  // else the next half warp's own level
+      put(w, kn, wst);
+      put_img(ph, kn, ph_n);
+    }
+    const float4 ta = tA[k];
+    const float2 alv = mul(div(bc2(-1.f), lin(ta.x, mts, ta.y)),
+                           add2(mul(a, muls(ta.x, mu)), muls(tB[k].y, sub2(ph_n, ph_k))));
+    put_img(al, k, alv);
+    const float2 pn = mul(c_c2a, sub2(rdf(sQ, k), alv));
+    put(pm1, k, pn);
+    put_img(p, k, add2(pn, muls(smdiv, sub2(pn, c_pm1))));
+    ph_k = ph_n;
+  }
+}
+
+void launch_advance_col(const TileLaunch& L, int nblocks, int nlev_max, int rk_step, int iteration, bool fp64,
+                        cudaStream_t s, bool damp) {
+  static bool attr = false;
+  if (!attr) {
+    const int f = (int)col_smem<float>(128), d = (int)col_smem<double>(128);
+    cudaFuncSetAttribute(k_advance_col<float, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, f);
+    cudaFuncSetAttribute(k_advance_col<float, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, f);
+    cudaFuncSetAttribute(k_advance_col<double, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, d);
+    cudaFuncSetAttribute(k_advance_col<double, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, d);
+    attr = true;
+  }
+  const size_t sm = fp64 ? col_smem<double>(nlev_max) : col_smem<float>(nlev_max);
+  // two blocks of 8 warps per SM; 16 warps where shared memory leaves room for one block
+  const int threads = 32 * (sm > 113 * 1024 ? COL_MAXW : COL_MAXW / 2);
+  if (fp64 && damp) k_advance_col<double, true><<<nblocks, threads, sm, s>>>(L, rk_step, iteration);
+  else if (fp64) k_advance_col<double, false><<<nblocks, threads, sm, s>>>(L, rk_step, iteration);
+  else if (damp) k_advance_col<float, true><<<nblocks, threads, sm, s>>>(L, rk_step, iteration);
+  else k_advance_col<float, false><<<nblocks, threads, sm, s>>>(L, rk_step, iteration);
 }
 
 }  // namespace wrfgpu

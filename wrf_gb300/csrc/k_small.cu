@@ -170,10 +170,13 @@ __global__ void __launch_bounds__(BX* BY) k_calc_p_rho(Launch L, int step) {
 
 // Column form over mass tiles x level chunks: the levels of a chunk are
 // independent, so their loads go out four levels at a time; the arithmetic
-// of each point is calc_p_rho_point's.
-__global__ void __launch_bounds__(TX* TY) k_calc_p_rho_col(TileLaunch L, int step) {
+// of each point is calc_p_rho_point's.  ACOUSTIC: an acoustic step's
+// (step >= 1), whose halo fill is this kernel's own stores (MassImages).
+template <bool ACOUSTIC>
+__global__ void __launch_bounds__(TX* TY, ACOUSTIC ? 4 : 1) k_calc_p_rho_col(TileLaunch L, int rk_step, int step) {
   const TilePos tp = tile_pos(L, false, false);
   const Mem& m = block_member(L.mem, tp.m);
+  if (ACOUSTIC && step > stage_of(m, rk_step).nsmall) return;  // members with fewer acoustic steps
   const int i = tp.i0 + threadIdx.x, j = tp.j0 + threadIdx.y;
   if (i > min(m.ite, m.ide - 1) || j > min(m.jte, m.jde - 1)) return;
   int c0, c1;
@@ -182,6 +185,12 @@ __global__ void __launch_bounds__(TX* TY) k_calc_p_rho_col(TileLaunch L, int ste
      t_2 = f3(m, WRFGPU_T_2), t_1 = f3(m, WRFGPU_T_SAVE), c2a = f3(m, WRFGPU_C2A), pm1 = f3(m, WRFGPU_PM1);
   F1 c1h = f1(m, WRFGPU_C1H), c2h = f1(m, WRFGPU_C2H), rdnw = f1(m, WRFGPU_RDNW);
   const float muij = f2(m, WRFGPU_MU_2).ro(i, j), mutij = f2(m, WRFGPU_MUTS).ro(i, j), smdiv = m.smdiv;
+  MassImages img;
+  if (ACOUSTIC) img.init(m, i, j);
+  auto put = [&](const F3& a, int k, float v) {
+    if (ACOUSTIC) img.store([&](int ii, int jj) { a(ii, k, jj) = v; });
+    else a(i, k, j) = v;
+  };
   struct LP { float a, t1, t2, c2a, ph0, ph1, pm1; };
   chunked_levels<4, LP>(
       c0, c1,
@@ -191,16 +200,16 @@ __global__ void __launch_bounds__(TX* TY) k_calc_p_rho_col(TileLaunch L, int ste
       },
       [&](int k, const LP& d) {
         const float alv = -1.f / (c1h(k) * mutij + c2h(k)) * (d.a * (c1h(k) * muij) + rdnw(k) * (d.ph1 - d.ph0));
-        al(i, k, j) = alv;
+        put(al, k, alv);
         float pv = d.c2a * (d.a * (d.t2 - (c1h(k) * muij) * d.t1) / ((c1h(k) * mutij + c2h(k)) * (T0 + d.t1)) - alv);
-        if (step == 0) {
+        if (!ACOUSTIC && step == 0) {
           pm1(i, k, j) = pv;
         } else {
           const float ptmp = pv;
           pv = pv + smdiv * (pv - d.pm1);
           pm1(i, k, j) = ptmp;
         }
-        p(i, k, j) = pv;
+        put(p, k, pv);
       });
 }
 
@@ -734,8 +743,9 @@ void launch_small_step_prep(const Launch& L2, int nb2, const TileLaunch& LST, in
 void launch_calc_p_rho(const Launch& L, int nb, StepArgs a, cudaStream_t s) {
   k_calc_p_rho<<<nb, dim3(BX, BY), 0, s>>>(L, a.iteration);
 }
-void launch_calc_p_rho_col(const TileLaunch& L, int nb, StepArgs a, cudaStream_t s) {
-  k_calc_p_rho_col<<<dim3(nb, 4), dim3(TX, TY), 0, s>>>(L, a.iteration);
+void launch_calc_p_rho_col(const TileLaunch& L, int nb, StepArgs a, cudaStream_t s, int chunks) {
+  if (a.iteration > 0) k_calc_p_rho_col<true><<<dim3(nb, chunks), dim3(TX, TY), 0, s>>>(L, a.rk_step, a.iteration);
+  else k_calc_p_rho_col<false><<<dim3(nb, chunks), dim3(TX, TY), 0, s>>>(L, a.rk_step, 0);
 }
 void launch_calc_coef_w_col(const TileLaunch& L, int nb, StepArgs a, bool fp64, cudaStream_t s) {
   if (fp64) k_calc_coef_w_col<double><<<nb, dim3(TX, TY), 0, s>>>(L, a.rk_step);

@@ -46,10 +46,14 @@ enum Tune { TU_PD = 0, TU_ADV, TU_AW, TU_AUV, TU_SUMF, TU_PREP, TU_SSF, TU_SSP, 
             TU_CPRP, TU_AMUT, NTUNE };
 constexpr int TUNE_MAXVAR = 4;
 constexpr int TUNE_NVAR[NTUNE] = {2, 3, 3, 4, 4, 2, 2, 4, 4, 3, 4, 4, 4, 4};
-constexpr int TUNE_DEFAULT[NTUNE] = {1, 1, 1, 0, 0, 1, 1, 2, 2, 1, 0, 0, 2, 0};
-// the parameter each variant stands for: blocks per SM, level chunks, or
-// (advance_uv, sumflux, rk_tend_u, rk_tend_v) 10 x blocks per SM + level chunks
-constexpr int TUNE_PARAM[NTUNE][TUNE_MAXVAR] = {{1, 2, 0, 0}, {2, 3, 4, 0}, {2, 3, 4, 0}, {32, 42, 34, 44}, {32, 42, 34, 44},
+// (defaults measured on 512x512x80 and up: advance_mu_t 278 us with four blocks
+// per SM against 393 with two, advance_w 340 against 388; the FP64 form of
+// advance_mu_t is best with three, 524 against 571 us on the 16-member ensemble)
+constexpr int TUNE_DEFAULT[NTUNE] = {1, 1, 2, 1, 2, 1, 1, 2, 2, 1, 0, 0, 2, 2};
+// the parameter each variant stands for: blocks per SM, level chunks
+// (sumflux: of calc_p_rho), or (advance_uv, rk_tend_u, rk_tend_v) 10 x blocks
+// per SM + level chunks
+constexpr int TUNE_PARAM[NTUNE][TUNE_MAXVAR] = {{1, 2, 0, 0}, {2, 3, 4, 0}, {2, 3, 4, 0}, {32, 42, 34, 44}, {1, 2, 4, 8},
                                                 {3, 8, 0, 0}, {4, 8, 0, 0}, {1, 2, 4, 8}, {2, 4, 8, 16}, {2, 3, 4, 0},
                                                 {32, 42, 34, 44}, {32, 42, 34, 44}, {1, 2, 4, 8}, {2, 3, 4, 5}};
 
@@ -106,7 +110,8 @@ void launch_unpack_species(const Mem* mems, int member, int s, const float* src,
                            cudaStream_t st);
 void launch_pack_species(const Mem* mems, int member, int s, float* dst, int cols, int rows, int pitch,
                          cudaStream_t st);
-void launch_calc_p_rho_col(const TileLaunch& L, int nblocks, StepArgs a, cudaStream_t s);        // mass tiles
+// mass tiles x level chunks; iteration 0: step 0 of the stage, else the acoustic step (halo images stored)
+void launch_calc_p_rho_col(const TileLaunch& L, int nblocks, StepArgs a, cudaStream_t s, int chunks = 4);
 // sct: some member stores the species' sixth-order diffusion tendency sc_tend
 void launch_update_scalar_pd_col(const TileLaunch& L, int nblocks, StepArgs a, cudaStream_t s, bool sct = false);  // mass tiles
 void launch_calc_p_rho_phi_col(const TileLaunch& L, int nblocks, cudaStream_t s, int var = TUNE_DEFAULT[TU_CPRP]);  // mass tiles
@@ -124,16 +129,29 @@ void launch_scalar_pd_update(const TileLaunch& L, int nblocks, int nlev_max, int
                              int var = TUNE_DEFAULT[TU_PD]);
 void launch_swap_species(Mem* d_mems, int nmem, cudaStream_t s);
 
-// column-marching acoustic kernels (k_acoustic_col.cu): one block per tile
-// of the staggered extents
-void launch_sumflux_p_rho_col(const TileLaunch& L, int nblocks, int rk_step, int iteration, cudaStream_t s,
-                              int var = TUNE_DEFAULT[TU_SUMF]);
+// the acoustic step (k_acoustic_col.cu): one block per tile of the staggered
+// extents, then either one block per row segment of 32 mass columns
+// (advance_mu_t, advance_w, sumflux's ww_m, calc_p_rho) or one thread per
+// mass column (advance_mu_t and ww_m, then advance_w), then calc_p_rho
 void launch_advance_uv_col(const TileLaunch& L, int nblocks, int rk_step, int iteration, cudaStream_t s,
                            int var = TUNE_DEFAULT[TU_AUV]);
-// one block per tile of mass columns
+// The largest number of row segments (all members) that k_advance_col takes.
+// Its time grows with the number of blocks from the start; the three marching
+// kernels take about 1.5 us per level until their 256-column tiles fill the
+// GPU.  Measured on GB300, ms per large step, column kernel against marches:
+// FP32  41x41x41 (82 segments) 0.15 / 0.80, 100x70x30 (280) 0.13 / 0.64,
+// 190x161x60 (966) 0.77 / 1.33, 256x256x80 (2048) 1.70 / 1.99, 24 small members
+// (about 2900) 2.23 / 2.30, 512x512x80 (8192) 6.30 / 5.67, 1024x1024x96 (32768)
+// 29.0 / 24.9; FP64 columns (whose chains wait about 110 cycles per operation)
+// 75x90x128 (270) 1.12 / 3.11, 16 members of up to 256x256x80 (about 14000)
+// 17.5 / 9.3; with damp_opt = 3 (whose FP64 sine sits in few of the block's warps)
+// 160x144x64 (720) 1.88 / 1.82.
+constexpr int col_max_segments(bool fp64, bool damp) { return damp ? 500 : fp64 ? 1000 : 3000; }
+// damp: some member uses damp_opt = 3 (compiles the damping into the kernel)
+void launch_advance_col(const TileLaunch& L, int nblocks, int nlev_max, int rk_step, int iteration, bool fp64,
+                        cudaStream_t s, bool damp = false);
 void launch_advance_mu_t_col(const TileLaunch& L, int nblocks, int rk_step, int iteration, bool fp64, cudaStream_t s,
                              int var = TUNE_DEFAULT[TU_AMUT]);
-// damp: some member uses damp_opt = 3 (compiles the damping into the kernel)
 void launch_advance_w_col(const TileLaunch& L, int nblocks, int rk_step, int iteration, bool fp64, cudaStream_t s,
                           int var = TUNE_DEFAULT[TU_AW], bool damp = false);
 
