@@ -6,6 +6,11 @@ and the tallest column, odd widths (whose last pair of columns is half
 inside), and a domain on each side of the size rule.  The FP64 column form
 is compared between the two: a member alone takes one of them, in an ensemble
 above the rule the other, and the fields agree bit for bit.
+
+The same domains cover the level chunks of the other column kernels (one
+level in the last chunk, chunks that a short member leaves empty) and the
+row-segment forms of rk_step_prep and calc_coef_w on both sides of their
+size rules.
 """
 import pytest
 
@@ -20,7 +25,7 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("nx,ny,kde", [(31, 9, 14), (32, 8, 15), (33, 10, 17), (64, 9, 33), (65, 8, 128),
-                                       (12, 3011, 14), (33, 1510, 16)])
+                                       (12, 3011, 14), (33, 1510, 16), (31, 950, 14), (40, 1255, 15)])
 def test_column_forms_bitwise(gpulib, nx, ny, kde):
     case = cases.small_case(nx=nx, ny=ny, kde=kde, n_scalar=1, seed=nx + kde)
     od = OracleDomain(case, "f32")
@@ -60,3 +65,17 @@ def test_fp64_column_forms_agree(gpulib, kde):
     for nm in STATE_FIELDS:
         fid = abi.FIELD_ID[nm]
         assert (alone.get(0, fid) == both.get(0, fid)).all(), nm
+
+
+def test_level_chunks_of_uneven_members(gpulib):
+    """One launch cuts every member's levels into the tallest member's chunks:
+    members of 14, 43 and 128 levels, plain, each equal to its own run."""
+    three = [cases.small_case(nx=20 + q, ny=9 + q, kde=kde, n_scalar=2, seed=q) for q, kde in enumerate((14, 43, 128))]
+    ens = G.Ensemble.from_cases(three)
+    ens.step(2)
+    ens.sync()
+    for q, case in enumerate(three):
+        od = OracleDomain(case, "f32")
+        od.step(2)
+        bad = _bitwise_diffs(case, ens, od, member=q)
+        assert not bad, "\n".join(bad)

@@ -234,6 +234,7 @@ struct Launch {
   const int* block_start;    // [nmem+1] prefix over blocks of this launch kind
   int nmem;
   int kind;                  // 2: column blocks (i,j); 3: point blocks (i,j,k)
+  int nlev = 0;              // levels of the tallest member (host: the launchers' level chunks)
 };
 
 struct BlockPos {
@@ -450,6 +451,14 @@ struct MassImages {
   }
 };
 
+// Level chunk of this block (gridDim.y chunks of k0..k1; k0 > k1: none left).
+struct Chunk { int k0, k1; };
+__device__ __forceinline__ Chunk level_chunk_of(int kts, int ktf) {
+  const int per = (ktf - kts + 1 + (int)gridDim.y - 1) / (int)gridDim.y;
+  const int k0 = kts + (int)blockIdx.y * per;
+  return Chunk{k0, min(ktf, k0 + per - 1)};
+}
+
 // Edge-strip launches of members with open boundaries (open_adv.cuh):
 // blocks of STRIP_THREADS over each member's strip points.
 constexpr int STRIP_THREADS = 256;
@@ -465,7 +474,25 @@ struct TileLaunch {
   const Mem* mem;
   const int* block_start;  // [nmem+1] prefix over tiles x per_tile
   int nmem;
+  int nlev = 0;            // levels of the tallest member (host: the launchers' level chunks)
 };
+
+// Level chunks (gridDim.y) of a column kernel of nblocks tiles, `resident` of
+// whose blocks the GPU holds at a time: the count from `base` on with the
+// fewest level times, waves x (levels per chunk + 2).  A chunk forms its first
+// level's carried values afresh and waits for its first loads, about two
+// levels' time, and none is shorter than `minlev` levels.  Tiles that fill the
+// GPU several times over keep `base`.
+inline int level_chunks(int nblocks, int nlev, int base, int minlev, int resident = 4 * 152) {
+  int best = base;
+  double cost = 0.;
+  for (int c = base; c <= (nlev / minlev > base ? nlev / minlev : base); ++c) {
+    const int waves = (int)(((long long)nblocks * c + resident - 1) / resident);
+    const double t = waves * ((nlev + c - 1) / c + 2.0);
+    if (c == base || t < cost) { best = c; cost = t; }
+  }
+  return best;
+}
 
 struct TilePos {
   int m;       // member

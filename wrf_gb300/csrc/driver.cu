@@ -126,9 +126,9 @@ struct Ensemble {
   std::vector<WrfGpuDomainDesc> descs;
   std::vector<Mem> hm;                 // host copies of the member descriptors
   Mem* d_mems = nullptr;
-  int *d_bs2 = nullptr, *d_bs3 = nullptr, *d_bs_st = nullptr, *d_bs_tm = nullptr, *d_bs_rw = nullptr;
+  int *d_bs2 = nullptr, *d_bs3 = nullptr, *d_bs_st = nullptr, *d_bs_tm = nullptr, *d_bs_rw = nullptr, *d_bs_rs = nullptr;
   int* d_bs_pr = nullptr;  // mass tiles x pairs of species (the scalar transport)
-  int nb2 = 0, nb3 = 0, nb_st = 0, nb_tm = 0, nb_pr = 0, nb_rw = 0;
+  int nb2 = 0, nb3 = 0, nb_st = 0, nb_tm = 0, nb_pr = 0, nb_rw = 0, nb_rs = 0;
   // edge strips of members with open lateral boundaries (strip columns x
   // levels): the tendencies and the 5th/3rd-order transport, the PD
   // transport, and its limiter factors (one wider, halo included)
@@ -176,12 +176,13 @@ struct Ensemble {
     prof->push_back({ph, e});
   }
 
-  Launch L2() const { return Launch{d_mems, d_bs2, nmem, 2}; }
+  Launch L2() const { return Launch{d_mems, d_bs2, nmem, 2, nlev_max}; }
   Launch L3() const { return Launch{d_mems, d_bs3, nmem, 3}; }
-  TileLaunch LP() const { return TileLaunch{d_mems, d_bs_pr, nmem}; }  // tiles x species pairs
-  TileLaunch LST() const { return TileLaunch{d_mems, d_bs_st, nmem}; }  // staggered-extent tiles
-  TileLaunch LTM() const { return TileLaunch{d_mems, d_bs_tm, nmem}; }  // mass-extent tiles
-  TileLaunch LRW() const { return TileLaunch{d_mems, d_bs_rw, nmem}; }  // row segments of 32 mass columns
+  TileLaunch LP() const { return TileLaunch{d_mems, d_bs_pr, nmem, nlev_max}; }  // tiles x species pairs
+  TileLaunch LST() const { return TileLaunch{d_mems, d_bs_st, nmem, nlev_max}; }  // staggered-extent tiles
+  TileLaunch LTM() const { return TileLaunch{d_mems, d_bs_tm, nmem, nlev_max}; }  // mass-extent tiles
+  TileLaunch LRW() const { return TileLaunch{d_mems, d_bs_rw, nmem, nlev_max}; }  // row segments of 32 mass columns
+  TileLaunch LRS() const { return TileLaunch{d_mems, d_bs_rs, nmem, nlev_max}; }  // row segments of the staggered columns, rows jts-1 .. jte
   StripLaunch LS3() const { return StripLaunch{d_mems, d_bs_s3, nmem, STRIP_W_TEND, 0}; }
   StripLaunch LS4() const { return StripLaunch{d_mems, d_bs_s4, nmem, STRIP_W_PD, 0}; }
   StripLaunch LS5() const { return StripLaunch{d_mems, d_bs_s5, nmem, STRIP_W_PD + 1, 1}; }
@@ -641,6 +642,7 @@ struct Ensemble {
     if (d_bs_st) cudaFree(d_bs_st);
     if (d_bs_tm) cudaFree(d_bs_tm);
     if (d_bs_rw) cudaFree(d_bs_rw);
+    if (d_bs_rs) cudaFree(d_bs_rs);
     if (d_bs_s3) cudaFree(d_bs_s3);
     if (d_bs_s4) cudaFree(d_bs_s4);
     if (d_bs_s5) cudaFree(d_bs_s5);
@@ -701,7 +703,7 @@ struct Ensemble {
     CK(cudaMalloc(&d_cfl, sizeof(float) * 2 * n));
     CK(cudaMemsetAsync(d_cfl, 0, sizeof(float) * 2 * n, stream));
     std::vector<float*> scr(n);
-    std::vector<int> bs2(n + 1, 0), bs3(n + 1, 0), bst(n + 1, 0), btm(n + 1, 0), brw(n + 1, 0), bpr(n + 1, 0), bs_s3(n + 1, 0),
+    std::vector<int> bs2(n + 1, 0), bs3(n + 1, 0), bst(n + 1, 0), btm(n + 1, 0), brw(n + 1, 0), brs(n + 1, 0), bpr(n + 1, 0), bs_s3(n + 1, 0),
         bs_s4(n + 1, 0), bs_s5(n + 1, 0);
     for (int m = 0; m < n; ++m) {
       const WrfGpuDomainDesc& d = ds[m];
@@ -754,6 +756,7 @@ struct Ensemble {
       bst[m + 1] = bst[m] + tiles_x(M, true) * tiles_y(M, true);
       btm[m + 1] = btm[m] + tiles_x(M) * tiles_y(M);
       brw[m + 1] = brw[m] + tiles_x(M) * (std::min(M.jte, M.jde - 1) - M.jts + 1);
+      brs[m + 1] = brs[m] + tiles_x(M, true) * (M.jte - M.jts + 2);
       auto strip_blocks = [&](int w, int h) {
         const int nc = strip_cols(M.ide, M.jde, M.cf.open_xs, M.cf.open_ys, w, h);
         return (nc * (M.kme - M.kms + 1) + STRIP_THREADS - 1) / STRIP_THREADS;
@@ -763,7 +766,7 @@ struct Ensemble {
       bs_s4[m + 1] = bs_s4[m] + strip_blocks(STRIP_W_PD, 0);
       bs_s5[m + 1] = bs_s5[m] + strip_blocks(STRIP_W_PD + 1, 1);
     }
-    nb2 = bs2[n]; nb3 = bs3[n]; nb_st = bst[n]; nb_tm = btm[n]; nb_pr = bpr[n]; nb_rw = brw[n];
+    nb2 = bs2[n]; nb3 = bs3[n]; nb_st = bst[n]; nb_tm = btm[n]; nb_pr = bpr[n]; nb_rw = brw[n]; nb_rs = brs[n];
     col_step = nb_rw <= col_max_segments(fp64, damp3);
     if (fp64) tune[TU_AMUT] = 1;  // three blocks per SM (kernels.h)
     nb_s3 = bs_s3[n]; nb_s4 = bs_s4[n]; nb_s5 = bs_s5[n];
@@ -806,7 +809,7 @@ struct Ensemble {
     CK(cudaMemcpyAsync(d_bs_st, bst.data(), sizeof(int) * (n + 1), cudaMemcpyHostToDevice, stream));
     CK(cudaMalloc(&d_bs_tm, sizeof(int) * (n + 1)));
     CK(cudaMemcpyAsync(d_bs_tm, btm.data(), sizeof(int) * (n + 1), cudaMemcpyHostToDevice, stream));
-    for (auto& pr : {std::make_pair(&d_bs_rw, &brw), std::make_pair(&d_bs_s3, &bs_s3), std::make_pair(&d_bs_s4, &bs_s4),
+    for (auto& pr : {std::make_pair(&d_bs_rw, &brw), std::make_pair(&d_bs_rs, &brs), std::make_pair(&d_bs_s3, &bs_s3), std::make_pair(&d_bs_s4, &bs_s4),
                      std::make_pair(&d_bs_s5, &bs_s5)}) {
       CK(cudaMalloc(pr.first, sizeof(int) * (n + 1)));
       CK(cudaMemcpyAsync(*pr.first, pr.second->data(), sizeof(int) * (n + 1), cudaMemcpyHostToDevice, stream));
@@ -821,7 +824,13 @@ struct Ensemble {
         CK(cudaMemcpy(hm[m].f2[f - WRFGPU_F2D_BASE], ones.data(), n2[m] * 4, cudaMemcpyHostToDevice));
     }
     CK(cudaStreamSynchronize(stream));
-    halo_blocks = std::max(8, std::min(256, (int)(n3[0] / 20000)));
+    // fill blocks per job and member: one x unit or two y units per thread of the
+    // largest member (k_fill_halo)
+    halo_blocks = 8;
+    for (int m = 0; m < n; ++m) {
+      const int x = (int)(nk_[m] * nj_[m] / 256), y = (int)(nk_[m] * ((ni_[m] + 127) / 128));
+      halo_blocks = std::max(halo_blocks, std::min(256, std::max(x, y) / 2));
+    }
     return WRFGPU_OK;
   }
 
@@ -883,7 +892,8 @@ struct Ensemble {
     for (int rk_step = 1; rk_step <= 3; ++rk_step) {
       StepArgs a{rk_step, 0, 0, 0};
       mark(PH_PREP);
-      launch_rk_step_prep(l2, nb2, stream, tune[TU_PREP]);
+      if (nb_rs <= PREP_ROW_MAX) launch_rk_step_prep_row(LRS(), nb_rs, stream);
+      else launch_rk_step_prep(l2, nb2, stream, tune[TU_PREP]);
       {  // rk_phys_bc_dry_1 + al, ph_2 (solve_em.F:726-754)
         JobList j;
         j.f3(WRFGPU_RU, 'u'); j.f3(WRFGPU_RV, 'v'); j.f3(WRFGPU_RW, 'w'); j.f3(WRFGPU_WW, 'w');
@@ -913,7 +923,8 @@ struct Ensemble {
       // small_step_prep, calc_p_rho(step 0), calc_coef_w (solve_em.F:1089-1140)
       mark(PH_SSP); launch_small_step_prep(l2, nb2, LST(), nb_st, a, stream, tune[TU_SSP]);
       mark(PH_CPR0); launch_calc_p_rho_col(LTM(), nb_tm, StepArgs{rk_step, 0, 0, 0}, stream);
-      mark(PH_COEFW); launch_calc_coef_w_col(LTM(), nb_tm, a, fp64, stream);
+      mark(PH_COEFW); if (!fp64 && nb_rw <= COEF_ROW_MAX) launch_calc_coef_w_row(LRW(), nb_rw, a, stream);
+      else launch_calc_coef_w_col(LTM(), nb_tm, a, fp64, stream);
       {  // solve_em.F:1176-1264
         JobList j;
         j.f3(WRFGPU_RU_TEND, 'u'); j.f3(WRFGPU_RV_TEND, 'v'); j.f3(WRFGPU_PH_2, 'w'); j.f3(WRFGPU_AL, 'p');

@@ -226,7 +226,7 @@ __global__ void __launch_bounds__(TX* TY, MINB) k_advance_uv_col(TileLaunch L, i
 
 // variant parameter: 10 x blocks per SM + level chunks
 void launch_advance_uv_col(const TileLaunch& L, int nblocks, int rk_step, int iteration, cudaStream_t s, int var) {
-  const int p = TUNE_PARAM[TU_AUV][var], chunks = p % 10;
+  const int p = TUNE_PARAM[TU_AUV][var], chunks = level_chunks(nblocks, L.nlev, p % 10, 2);
   if (p / 10 == 4) k_advance_uv_col<4><<<dim3(nblocks, chunks), dim3(TX, TY), 0, s>>>(L, rk_step, iteration);
   else k_advance_uv_col<3><<<dim3(nblocks, chunks), dim3(TX, TY), 0, s>>>(L, rk_step, iteration);
 }

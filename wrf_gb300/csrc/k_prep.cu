@@ -149,6 +149,128 @@ __global__ void __launch_bounds__(BX* BY, MINB) k_rk_step_prep(Launch L) {
   }
 }
 
+// The same on a row segment of 32 columns per block, the levels in contiguous
+// chunks over the block's warps: the point-wise fields and the column
+// divergence of a chunk, then (one barrier later) its divergence sum and the
+// omega recursion up to the chunk from shared memory, one add per level,
+// walked by every warp for itself in k order.
+constexpr int PREP_WARPS = 8;
+__global__ void __launch_bounds__(32 * PREP_WARPS) k_rk_step_prep_row(TileLaunch L) {
+  extern __shared__ float s_dv[];  // [kte + 1][32]
+  const int mi = find_member(L.block_start, L.nmem, blockIdx.x);
+  const Mem& m = block_member(L.mem, mi);
+  const int ln = threadIdx.x & 31, wp = threadIdx.x >> 5;
+  const int lb = (int)blockIdx.x - __ldg(L.block_start + mi), ntx = tiles_x(m, true);
+  const int i = m.its + (lb % ntx) * 32 + ln, j = m.jts - 1 + lb / ntx;
+  const int itf_m = min(m.ite, m.ide - 1), jtf_m = min(m.jte, m.jde - 1), ktf = min(m.kte, m.kde - 1);
+  const int kts = m.kts, kte = m.kte;
+  const bool px = m.cf.periodic_x, py = m.cf.periodic_y;
+  const float rdx = m.rdx, rdy = m.rdy;
+  F2 MU = f2(m, WRFGPU_MU_2), MUB = f2(m, WRFGPU_MUB);
+  const bool row_t = j >= m.jts && j <= jtf_m, at_u = row_t && i <= m.ite, at_t = row_t && i <= itf_m,
+             at_v = j >= m.jts && i <= itf_m;
+  // calculate_full, calc_mu_uv
+  float mut_ij = 0.f, muu_ij = 0.f, muv_ij = 0.f;
+  if (i <= itf_m && j <= jtf_m) {
+    mut_ij = MUB.ro(i, j) + MU.ro(i, j);
+    F2 MUT = f2(m, WRFGPU_MUT);
+    if (wp == 0) {
+      MUT(i, j) = mut_ij;
+      if (i == m.its) MUT(i - 1, j) = MUB.ro(i - 1, j) + MU.ro(i - 1, j);
+    }
+  }
+  if (at_u) {
+    const bool lo = i == m.ids && m.its == m.ids, hi = i == m.ide && m.ite == m.ide;
+    const int ia = hi ? i - 1 : i, im = lo ? (px ? i - 1 : i) : hi ? (px ? i : i - 1) : i - 1;
+    muu_ij = 0.5f * (MU.ro(ia, j) + MU.ro(im, j) + MUB.ro(ia, j) + MUB.ro(im, j));
+    if (wp == 0) f2(m, WRFGPU_MUU)(i, j) = muu_ij;
+  }
+  if (at_v) {
+    const bool lo = j == m.jds && m.jts == m.jds, hi = j == m.jde && m.jte == m.jde;
+    const int ja = hi ? j - 1 : j, jm = lo ? (py ? j - 1 : j) : hi ? (py ? j : j - 1) : j - 1;
+    muv_ij = 0.5f * (MU.ro(i, ja) + MU.ro(i, jm) + MUB.ro(i, ja) + MUB.ro(i, jm));
+    if (wp == 0) f2(m, WRFGPU_MUV)(i, j) = muv_ij;
+  }
+  if (j < m.jts) return;  // block-uniform: the row below the domain has its column mass only
+  const int per = (ktf - kts + 1 + PREP_WARPS - 1) / PREP_WARPS, ka = kts + wp * per, kb = min(ktf, ka + per - 1);
+  F3 u = f3(m, WRFGPU_U_2), v = f3(m, WRFGPU_V_2), w = f3(m, WRFGPU_W_2), ph = f3(m, WRFGPU_PH_2);
+  F3 ru = f3(m, WRFGPU_RU), rv = f3(m, WRFGPU_RV), rw = f3(m, WRFGPU_RW), ww = f3(m, WRFGPU_WW);
+  F3 php = f3(m, WRFGPU_PHP), alt = f3(m, WRFGPU_ALT), phb = f3(m, WRFGPU_PHB), al = f3(m, WRFGPU_AL),
+     alb = f3(m, WRFGPU_ALB);
+  F3 cqu = f3(m, WRFGPU_CQU), cqv = f3(m, WRFGPU_CQV), cqw = f3(m, WRFGPU_CQW), qv = f3p(m, m.q[0]);
+  F1 c1h = f1(m, WRFGPU_C1H), c2h = f1(m, WRFGPU_C2H), c1f = f1(m, WRFGPU_C1F), c2f = f1(m, WRFGPU_C2F),
+     dnw = f1(m, WRFGPU_DNW);
+  const float uy0 = at_u ? f2(m, WRFGPU_MSFUY).ro(i, j) : 1.f, vi0 = at_v ? f2(m, WRFGPU_MSFVX_INV).ro(i, j) : 1.f;
+  float muu0 = 0.f, muu1 = 0.f, muv0 = 0.f, muv1 = 0.f, mx = 0.f, my = 1.f, uy1 = 1.f, vi1 = 1.f;
+  if (at_t) {
+    muu0 = 0.5f * (MU.ro(i, j) + MUB.ro(i, j) + MU.ro(i - 1, j) + MUB.ro(i - 1, j));
+    muu1 = 0.5f * (MU.ro(i + 1, j) + MUB.ro(i + 1, j) + MU.ro(i, j) + MUB.ro(i, j));
+    muv0 = 0.5f * (MU.ro(i, j) + MUB.ro(i, j) + MU.ro(i, j - 1) + MUB.ro(i, j - 1));
+    muv1 = 0.5f * (MU.ro(i, j + 1) + MUB.ro(i, j + 1) + MU.ro(i, j) + MUB.ro(i, j));
+    mx = f2(m, WRFGPU_MSFTX).ro(i, j); my = f2(m, WRFGPU_MSFTY).ro(i, j);
+    uy1 = f2(m, WRFGPU_MSFUY).ro(i + 1, j); vi1 = f2(m, WRFGPU_MSFVX_INV).ro(i, j + 1);
+  }
+  struct LV { float u, v, q, qi, qj, qk, u1, v1, w, al, alb, phb0, phb1, ph0, ph1; };
+  chunked_levels<2, LV>(
+      ka, kb,
+      [&](int k, LV& d) {
+        d.u = at_u ? u.ro(i, k, j) : 0.f;
+        d.v = at_v ? v.ro(i, k, j) : 0.f;
+        d.q = at_u || at_v ? qv.ro(i, k, j) : 0.f;
+        d.qi = at_u ? qv.ro(i - 1, k, j) : 0.f;
+        d.qj = at_v ? qv.ro(i, k, j - 1) : 0.f;
+        if (at_t) {
+          d.qk = k > kts ? qv.ro(i, k - 1, j) : 0.f;
+          d.u1 = u.ro(i + 1, k, j); d.v1 = v.ro(i, k, j + 1); d.w = w.ro(i, k, j);
+          d.al = al.ro(i, k, j); d.alb = alb.ro(i, k, j);
+          d.phb0 = phb.ro(i, k, j); d.phb1 = phb.ro(i, k + 1, j); d.ph0 = ph.ro(i, k, j); d.ph1 = ph.ro(i, k + 1, j);
+        }
+      },
+      [&](int k, const LV& d) {
+        const float h1 = c1h(k), h2 = c2h(k);
+        if (at_u) {  // couple_momentum, calc_cq
+          ru(i, k, j) = d.u * (h1 * muu_ij + h2) / uy0;
+          const float qtot = 0.f + d.q + d.qi;
+          cqu(i, k, j) = 1.f / (1.f + 0.5f * qtot);
+        }
+        if (at_v) {
+          rv(i, k, j) = d.v * (h1 * muv_ij + h2) * vi0;
+          const float qtot = 0.f + d.q + d.qj;
+          cqv(i, k, j) = 1.f / (1.f + 0.5f * qtot);
+        }
+        if (at_t) {  // calc_ww_cp's divergence; rw, cqw, alt, php
+          s_dv[k * 32 + ln] = mx * dnw(k) *
+                              (rdx * ((h1 * muu1 + h2) * d.u1 / uy1 - (h1 * muu0 + h2) * d.u / uy0) +
+                               rdy * ((h1 * muv1 + h2) * d.v1 * vi1 - (h1 * muv0 + h2) * d.v * vi0));
+          rw(i, k, j) = d.w * (c1f(k) * mut_ij + c2f(k)) / my;
+          if (k >= kts + 1) {
+            const float qtot = 0.f + d.q + d.qk;
+            cqw(i, k, j) = 0.5f * qtot;
+          }
+          alt(i, k, j) = d.al + d.alb;
+          php(i, k, j) = 0.5f * (d.phb0 + d.phb1 + d.ph0 + d.ph1);
+        }
+      });
+  if (at_t && kb == ktf && ka <= kb)
+    for (int k = ktf + 1; k <= kte; ++k) rw(i, k, j) = w.ro(i, k, j) * (c1f(k) * mut_ij + c2f(k)) / my;
+  __syncthreads();
+  if (at_u && wp == 0) { ww(i, 1, j) = 0.f; ww(i, kte, j) = 0.f; }
+  if (at_t && ka <= kb) {
+    float dmdt = 0.f, wwk = 0.f;
+#pragma unroll 8
+    for (int k = kts; k <= ktf; ++k) dmdt = dmdt + s_dv[k * 32 + ln];
+#pragma unroll 4
+    for (int k = 2; k <= kb; ++k) {
+      wwk = wwk - dnw(k - 1) * c1h(k - 1) * dmdt - s_dv[(k - 1) * 32 + ln];
+      if (k >= ka) ww(i, k, j) = wwk;
+    }
+  }
+}
+
+void launch_rk_step_prep_row(const TileLaunch& L, int nblocks, cudaStream_t s) {
+  k_rk_step_prep_row<<<nblocks, 32 * PREP_WARPS, (L.nlev + 2) * 32 * sizeof(float), s>>>(L);
+}
+
 void launch_rk_step_prep(const Launch& L, int nblocks, cudaStream_t s, int var) {
   // 3 blocks of 128 threads per SM leave the register count free (88);
   // 8 hold it to 64 for twice the resident warps

@@ -457,14 +457,15 @@ __global__ void __launch_bounds__(TX* TY, 4) k_cfl_check_col(TileLaunch L) {
 
 // ------------------------------------------------------------ launchers
 void launch_cfl_check_col(const TileLaunch& L, int nb, cudaStream_t s, int var) {
-  k_cfl_check_col<<<dim3(nb, TUNE_PARAM[TU_CFL][var]), dim3(TX, TY), 0, s>>>(L);
+  k_cfl_check_col<<<dim3(nb, level_chunks(nb, L.nlev, TUNE_PARAM[TU_CFL][var], 2)), dim3(TX, TY), 0, s>>>(L);
 }
 void launch_update_scalar_pd(const Launch& L, int nb, StepArgs a, cudaStream_t s) {
   k_update_scalar_pd<<<nb, dim3(BX, BY), 0, s>>>(L, a.rk_step);
 }
 void launch_update_scalar_pd_col(const TileLaunch& L, int nb, StepArgs a, cudaStream_t s, bool sct) {
-  if (sct) k_update_scalar_pd_col<true><<<dim3(nb, 4), dim3(TX, TY), 0, s>>>(L, a.rk_step);
-  else k_update_scalar_pd_col<false><<<dim3(nb, 4), dim3(TX, TY), 0, s>>>(L, a.rk_step);
+  const dim3 grid(nb, level_chunks(nb, L.nlev, 4, 2));
+  if (sct) k_update_scalar_pd_col<true><<<grid, dim3(TX, TY), 0, s>>>(L, a.rk_step);
+  else k_update_scalar_pd_col<false><<<grid, dim3(TX, TY), 0, s>>>(L, a.rk_step);
 }
 void launch_advect_scalar(const Launch& L, int nb, StepArgs a, cudaStream_t s) {
   k_advect_scalar<<<nb, dim3(BX, BY), 0, s>>>(L, a.species, a.rk_step, a.flags);
@@ -481,7 +482,7 @@ void launch_update_scalar(const Launch& L, int nb, StepArgs a, cudaStream_t s) {
 }
 void launch_calc_p_rho_phi(const Launch& L, int nb, cudaStream_t s) { k_calc_p_rho_phi<<<nb, dim3(BX, BY), 0, s>>>(L); }
 void launch_calc_p_rho_phi_col(const TileLaunch& L, int nb, cudaStream_t s, int var) {
-  k_calc_p_rho_phi_col<<<dim3(nb, TUNE_PARAM[TU_CPRP][var]), dim3(TX, TY), 0, s>>>(L);
+  k_calc_p_rho_phi_col<<<dim3(nb, level_chunks(nb, L.nlev, TUNE_PARAM[TU_CPRP][var], 2)), dim3(TX, TY), 0, s>>>(L);
 }
 void launch_set_w_surface(const Launch& L, int nb, cudaStream_t s) { k_set_w_surface<<<nb, dim3(BX, BY), 0, s>>>(L); }
 

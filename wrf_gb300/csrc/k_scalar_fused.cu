@@ -99,13 +99,16 @@ __global__ void __launch_bounds__(TX* TY, MINB) k_scalar_adv_update(TileLaunch L
   const int i0 = tp.i0, j0 = tp.j0;
   const int itf = min(m.ite, m.ide - 1), jtf = min(m.jte, m.jde - 1), ktf = min(m.kte, m.kde - 1);
   const int kts = m.kts, kte = m.kte, kme = m.kme;
+  const Chunk ch = level_chunk_of(kts, ktf);
+  const int k0 = ch.k0, k1 = ch.k1;  // this block's levels
+  if (k0 > k1) return;
 
   PlaneRing<ADV_NPL, ADV_RING> ring;
   ring.buf = (float*)smem;
   float2* fx_base = reinterpret_cast<float2*>(ring.buf + ADV_RING * ADV_NPL * HPLANE);  // [2][TY][TX+1]
   float2* fy_base = fx_base + 2 * TY * (TX + 1);                                      // [2][TY+1][TX]
   ring.bar = reinterpret_cast<uint64_t*>(fy_base + 2 * (TY + 1) * TX);
-  ring.kts = kts;
+  ring.kts = k0;
   const CUtensorMap* maps[ADV_NPL] = {tmap_of(m, m.qmap[sp.s0], BOX_HALO), tmap_of(m, m.qmap[sp.s1], BOX_HALO),
                                       tmap_of(m, WRFGPU_RU_M, BOX_HALO), tmap_of(m, WRFGPU_RV_M, BOX_HALO)};
   const int x0 = i0 - TMA_HALO - m.ims, z0 = j0 - TMA_HALO - m.jms;
@@ -115,7 +118,7 @@ __global__ void __launch_bounds__(TX* TY, MINB) k_scalar_adv_update(TileLaunch L
   }
   __syncthreads();
   if (tid == 0)
-    for (int d = 0; d < ADV_RING - 1 && kts + d <= ktf; ++d) ring.issue(kts + d, maps, x0, z0, m.kms);
+    for (int d = 0; d < ADV_RING - 1 && k0 + d <= k1; ++d) ring.issue(k0 + d, maps, x0, z0, m.kms);
 
   const int i = i0 + tx, j = j0 + ty;
   const bool own = i <= itf && j <= jtf;
@@ -138,17 +141,23 @@ __global__ void __launch_bounds__(TX* TY, MINB) k_scalar_adv_update(TileLaunch L
     msfty = f2(m, WRFGPU_MSFTY)(i, j);
     muold = f2(m, WRFGPU_MU_1)(i, j) + f2(m, WRFGPU_MUB)(i, j);
     munew = f2(m, WRFGPU_MU_2)(i, j) + f2(m, WRFGPU_MUB)(i, j);
-    w0 = ld2(fa, fb, i, kts, j);
-    wp1 = ld2(fa, fb, i, kts + 1, j);
-    wp2 = (kts + 2 <= kme) ? ld2(fa, fb, i, kts + 2, j) : bc2(0.f);
-    old_k = rk_step == 1 ? bc2(0.f) : ld2(olda, oldb, i, kts, j);
-    rom_k1 = rom(i, kts + 1, j);
+    if (k0 > kts) wm1 = ld2(fa, fb, i, k0 - 1, j);
+    w0 = ld2(fa, fb, i, k0, j);
+    wp1 = ld2(fa, fb, i, k0 + 1, j);
+    wp2 = (k0 + 2 <= kme) ? ld2(fa, fb, i, k0 + 2, j) : bc2(0.f);
+    old_k = rk_step == 1 ? bc2(0.f) : ld2(olda, oldb, i, k0, j);
+    rom_k1 = rom(i, k0 + 1, j);
   }
   const float rdx = m.rdx, rdy = m.rdy;
-  float2 vf_lo = bc2(0.f);  // vf(kts) = 0
+  float2 vf_lo = bc2(0.f);  // vf(k0), formed as level k0 - 1 forms its upper face; vf(kts) = 0
+  if (own && k0 > kts) {
+    const float vel = rom(i, k0, j);
+    if (k0 == kts + 1 || k0 == ktf) vf_lo = muls(vel, add2(muls(fzm(k0), w0), muls(fzp(k0), wm1)));
+    else vf_lo = muls(vel, flux3_2(ld2(fa, fb, i, k0 - 2, j), wm1, w0, wp1, -vel));
+  }
   bool ok = true;
-  for (int k = kts; k <= ktf; ++k) {
-    if (tid == 0 && k + ADV_RING - 1 <= ktf) ring.issue(k + ADV_RING - 1, maps, x0, z0, m.kms);
+  for (int k = k0; k <= k1; ++k) {
+    if (tid == 0 && k + ADV_RING - 1 <= k1) ring.issue(k + ADV_RING - 1, maps, x0, z0, m.kms);
     ok = ring.wait(k) && ok;
     const int sl = ring.slot_of(k);
     const float* QA = ring.plane(sl, 0);
@@ -246,10 +255,10 @@ __global__ void __launch_bounds__(BX* BY) k_pd_courant(Launch L, int rk_step) {
   const float xdx = 2.f / (msy(i, j) + msy(i - 1, j)) / rdx;
   const float ydy = 2.f / (msx(i, j) + msx(i, j - 1)) / rdy;
   const float xdxt = xdx / dt, ydyt = ydy / dt;
-  const int klast = max(ktf, m.kde - 1);
+  const Chunk ch = level_chunk_of(m.kts, max(ktf, m.kde - 1));
   struct V { float u, v, w; };
   chunked_levels<4, V>(
-      m.kts, klast,
+      ch.k0, ch.k1,
       [&](int k, V& d) {
         d.u = k <= ktf ? ru.ro(i, k, j) : 0.f;
         d.v = k <= ktf ? rv.ro(i, k, j) : 0.f;
@@ -349,6 +358,11 @@ __global__ void __launch_bounds__(PD_THREADS, MINB) k_scalar_pd_update(TileLaunc
   const int i0 = tp.i0, j0 = tp.j0;
   const int itf = min(m.ite, m.ide - 1), jtf = min(m.jte, m.jde - 1), ktf = min(m.kte, m.kde - 1);
   const int kts = m.kts, kme = m.kme;
+  // this block's levels; its first iteration is one level below them (whose
+  // limiter factor the first level's lower z face takes), its last one above
+  const Chunk ch = level_chunk_of(kts, ktf);
+  const int k0 = ch.k0, k1 = ch.k1, L0 = max(kts, k0 - 1), L1 = min(ktf, k1 + 1);
+  if (k0 > k1) return;
   const Stage st = stage_of(m, rk_step);
   const float dt = st.dt_rk, rdx = m.rdx, rdy = m.rdy;
 
@@ -363,7 +377,7 @@ __global__ void __launch_bounds__(PD_THREADS, MINB) k_scalar_pd_update(TileLaunc
   const int nlev = m.kme - m.kms + 1;
   LevelConst* sLV = reinterpret_cast<LevelConst*>(p);  // [k - kms]
   ring.bar = reinterpret_cast<uint64_t*>(sLV + nlev);
-  ring.kts = kts;
+  ring.kts = L0;
   const CUtensorMap* maps[PD_NPL] = {tmap_of(m, m.qmap[s0], BOX_HALO), tmap_of(m, m.qmap[s1], BOX_HALO),
                                      tmap_of(m, WRFGPU_N3D + 3 * s0 + 1, BOX_HALO),
                                      tmap_of(m, WRFGPU_N3D + 3 * s1 + 1, BOX_HALO),
@@ -377,7 +391,7 @@ __global__ void __launch_bounds__(PD_THREADS, MINB) k_scalar_pd_update(TileLaunc
   }
   __syncthreads();
   if (tid == 0)
-    for (int d = 0; d < PD_RING - 1 && kts + d <= ktf; ++d) ring.issue(kts + d, maps, x0, z0, m.kms);
+    for (int d = 0; d < PD_RING - 1 && L0 + d <= L1; ++d) ring.issue(L0 + d, maps, x0, z0, m.kms);
 
   const F3 fa = f3p(m, m.q[s0]), fb = f3p(m, m.q[s1]), foa = f3p(m, m.qo[s0]), fob = f3p(m, m.qo[s1]);
   const F3 outa = f3p(m, m.qa[s0]), outb = f3p(m, m.qa[s1]), rom = f3(m, WRFGPU_WW_M);
@@ -443,13 +457,24 @@ __global__ void __launch_bounds__(PD_THREADS, MINB) k_scalar_pd_update(TileLaunc
   if (c.valid) {
     c.mut = mut2(c.i, c.j); c.mub = mub2(c.i, c.j); c.mu_old = mu1(c.i, c.j);
     c.mx = msx2(c.i, c.j); c.my = msy2(c.i, c.j);
-    // window for L = kts (f(L-1) unused: face kts+1 is second order); z face kts = 0
-    c.f0 = ld2(fa, fb, c.i, kts, c.j);
-    c.fp1 = ld2(fa, fb, c.i, kts + 1, c.j);
-    c.fp2 = (kts + 2 <= kme) ? ld2(fa, fb, c.i, kts + 2, c.j) : bc2(0.f);
-    c.fo0 = ld2(foa, fob, c.i, kts, c.j);
-    c.fop1 = ld2(foa, fob, c.i, kts + 1, c.j);
-    c.romp1 = rom(c.i, kts + 1, c.j);
+    // window for L = L0 (at kts f(L-1) is unused: face kts+1 is second order) and
+    // z face L0, formed as level L0 - 1 forms its upper face (z face kts = 0)
+    c.f0 = ld2(fa, fb, c.i, L0, c.j);
+    c.fp1 = ld2(fa, fb, c.i, L0 + 1, c.j);
+    c.fo0 = ld2(foa, fob, c.i, L0, c.j);
+    if (L0 > kts) {
+      c.fm1 = ld2(fa, fb, c.i, L0 - 1, c.j);
+      ZCell d = c;  // the window one level down
+      d.fm1 = L0 - 2 >= kts ? ld2(fa, fb, c.i, L0 - 2, c.j) : bc2(0.f);
+      d.f0 = c.fm1; d.fp1 = c.f0; d.fp2 = c.fp1;
+      d.fo0 = ld2(foa, fob, c.i, L0 - 1, c.j);
+      d.fop1 = c.fo0;
+      d.romp1 = rom(c.i, L0, c.j);
+      zface(d, L0, sLV[L0 - m.kms], crza.ro(c.i, L0, c.j), lfza.ro(c.i, L0, c.j), kts, m.kde, ktf, &c.hz0, &c.lz0);
+    }
+    c.fp2 = (L0 + 2 <= kme) ? ld2(fa, fb, c.i, L0 + 2, c.j) : bc2(0.f);
+    c.fop1 = ld2(foa, fob, c.i, L0 + 1, c.j);
+    c.romp1 = rom(c.i, L0 + 1, c.j);
   }
   // interior cells of the region are the tile's cells: they also update
   const int i = c.i, j = c.j;
@@ -473,7 +498,7 @@ __global__ void __launch_bounds__(PD_THREADS, MINB) k_scalar_pd_update(TileLaunc
     *lf = zin ? lfza.ro(c.i, lv + 1, c.j) : 0.f;
   };
   float crz_n, lfz_n;
-  zcourant(kts, &crz_n, &lfz_n);
+  zcourant(L0, &crz_n, &lfz_n);
 
   // One barrier per level.  Iteration Lv: faces of level Lv (face slot Lv % 3)
   // and the z face Lv+1 of the own cell; barrier; limiter factor of level Lv
@@ -485,12 +510,12 @@ __global__ void __launch_bounds__(PD_THREADS, MINB) k_scalar_pd_update(TileLaunc
   // this barrier; factor slot (Lv+1) & 1 holds level Lv-1, read before the
   // next one; the ring slot of level Lv+3 (issued after this barrier) held
   // level Lv, read before it.
-  for (int Lv = kts; Lv <= ktf + 1; ++Lv) {
+  for (int Lv = L0; Lv <= k1 + 1; ++Lv) {
     const int slot = Lv & 1;
     float c1k = 0.f, c2k = 0.f, rdzwk = 0.f;
     if (Lv <= ktf) {
       const float crz = crz_n, lfz = lfz_n;
-      if (tid == 0 && Lv + PD_RING - 1 <= ktf) ring.issue(Lv + PD_RING - 1, maps, x0, z0, m.kms);
+      if (tid == 0 && Lv + PD_RING - 1 <= L1) ring.issue(Lv + PD_RING - 1, maps, x0, z0, m.kms);
       const float4 tl = sLV[Lv - m.kms].a;
       c1k = tl.x; c2k = tl.y; rdzwk = tl.z;
       ok = ring.wait(Lv) && ok;
@@ -564,7 +589,7 @@ __global__ void __launch_bounds__(PD_THREADS, MINB) k_scalar_pd_update(TileLaunc
     }
     // ---- divergence + update of level k = Lv - 1
     const int k = Lv - 1;
-    if (k >= kts && own) {
+    if (k >= k0 && own) {
       const int fs = k % PD_FSLOT;
       const float2* XH = sXH + fs * P::XN; const float2* XL = sXL + fs * P::XN;
       const float2* YH = sYH + fs * P::YN; const float2* YL = sYL + fs * P::YN;
@@ -660,10 +685,11 @@ void launch_scalar_adv_update(const TileLaunch& L, int nblocks, int rk_step, cud
     attr = true;
   }
   const int minb = TUNE_PARAM[TU_ADV][var];
-  if (sct) k_scalar_adv_update<3, true><<<nblocks, dim3(TX, TY), ADV_SMEM, s>>>(L, rk_step, pairs);
-  else if (minb == 2) k_scalar_adv_update<2, false><<<nblocks, dim3(TX, TY), ADV_SMEM, s>>>(L, rk_step, pairs);
-  else if (minb == 3) k_scalar_adv_update<3, false><<<nblocks, dim3(TX, TY), ADV_SMEM, s>>>(L, rk_step, pairs);
-  else k_scalar_adv_update<4, false><<<nblocks, dim3(TX, TY), ADV_SMEM, s>>>(L, rk_step, pairs);
+  const dim3 grid(nblocks, level_chunks(nblocks, L.nlev, 1, 4, 3 * 152));
+  if (sct) k_scalar_adv_update<3, true><<<grid, dim3(TX, TY), ADV_SMEM, s>>>(L, rk_step, pairs);
+  else if (minb == 2) k_scalar_adv_update<2, false><<<grid, dim3(TX, TY), ADV_SMEM, s>>>(L, rk_step, pairs);
+  else if (minb == 3) k_scalar_adv_update<3, false><<<grid, dim3(TX, TY), ADV_SMEM, s>>>(L, rk_step, pairs);
+  else k_scalar_adv_update<4, false><<<grid, dim3(TX, TY), ADV_SMEM, s>>>(L, rk_step, pairs);
 }
 void launch_scalar_pd_update(const TileLaunch& L, int nblocks, int nlev_max, int rk_step, cudaStream_t s, int var) {
   static size_t attr = 0;
@@ -673,11 +699,13 @@ void launch_scalar_pd_update(const TileLaunch& L, int nblocks, int nlev_max, int
     set_smem(k_scalar_pd_update<2>, bytes);
     attr = bytes;
   }
-  if (TUNE_PARAM[TU_PD][var] == 1) k_scalar_pd_update<1><<<nblocks, PD_THREADS, bytes, s>>>(L, rk_step);
-  else k_scalar_pd_update<2><<<nblocks, PD_THREADS, bytes, s>>>(L, rk_step);
+  // a chunk computes two levels more than it writes
+  const dim3 grid(nblocks, level_chunks(nblocks, L.nlev, 1, 6, 2 * 152));
+  if (TUNE_PARAM[TU_PD][var] == 1) k_scalar_pd_update<1><<<grid, PD_THREADS, bytes, s>>>(L, rk_step);
+  else k_scalar_pd_update<2><<<grid, PD_THREADS, bytes, s>>>(L, rk_step);
 }
 void launch_pd_courant(const Launch& L2, int nblocks, int rk_step, cudaStream_t s) {
-  k_pd_courant<<<nblocks, dim3(BX, BY), 0, s>>>(L2, rk_step);
+  k_pd_courant<<<dim3(nblocks, level_chunks(nblocks, L2.nlev, 1, 4, 8 * 152)), dim3(BX, BY), 0, s>>>(L2, rk_step);
 }
 void launch_swap_species(Mem* d_mems, int nmem, cudaStream_t s) {
   k_swap_species<<<(nmem + 63) / 64, 64, 0, s>>>(d_mems, nmem);

@@ -314,6 +314,81 @@ __global__ void __launch_bounds__(TX* TY) k_calc_coef_w_col(TileLaunch L, int rk
   coef_w_column<RC>(m, i, j, rk_step);
 }
 
+// The same on a row segment of 32 mass columns per block: a, b and c of all
+// levels by all warps into shared memory, the recursion (a division per level,
+// each waiting for the one below) by one warp, alpha and gamma stored by all.
+constexpr int COEF_WARPS = 8;
+__global__ void __launch_bounds__(32 * COEF_WARPS) k_calc_coef_w_row(TileLaunch L, int rk_step) {
+  extern __shared__ float s_coef[];  // alpha, gamma, a, b, c: [kde + 1][32] each
+  const int mi = find_member(L.block_start, L.nmem, blockIdx.x);
+  const Mem& m = block_member(L.mem, mi);
+  const int ln = threadIdx.x & 31, wp = threadIdx.x >> 5;
+  const int lb = (int)blockIdx.x - __ldg(L.block_start + mi), ntx = tiles_x(m);
+  const int i0 = m.its + (lb % ntx) * 32 + ln, j = m.jts + lb / ntx;
+  const bool act = i0 <= min(m.ite, m.ide - 1);
+  const int i = act ? i0 : m.its;
+  const Stage st = stage_of(m, rk_step);
+  const int kde = m.kde, nc = (m.kme - m.kms + 2) * 32;
+  float *sAL = s_coef, *sGA = sAL + nc, *sA = sGA + nc, *sB = sA + nc, *sC = sB + nc;
+  F3 cqw = f3(m, WRFGPU_CQW), c2a = f3(m, WRFGPU_C2A);
+  F1 c1h = f1(m, WRFGPU_C1H), c2h = f1(m, WRFGPU_C2H), c1f = f1(m, WRFGPU_C1F), c2f = f1(m, WRFGPU_C2F),
+     rdn = f1(m, WRFGPU_RDN), rdnw = f1(m, WRFGPU_RDNW);
+  const float MUT = f2(m, WRFGPU_MUT).ro(i, j);
+  const float lid_flag = m.cf.top_lid ? 0.f : 1.f;
+  const float tt = (.5f * st.dts_rk * G * (1.f + m.epssm));
+  const float cof = tt * tt;
+  const F3 A = f3(m, WRFGPU_A), AL = f3(m, WRFGPU_ALPHA), GA = f3(m, WRFGPU_GAMMA);
+#pragma unroll 2
+  for (int k = 2 + wp; k <= kde - 1; k += COEF_WARPS) {
+    const float q = cqw.ro(i, k, j), ck = c2a.ro(i, k, j), cm = c2a.ro(i, k - 1, j);
+    const int kl = k - 1;
+    float a_k = 0.f;
+    if (k >= 3)
+      a_k = -q * cof * rdn(k) * rdnw(k - 1) * cm / ((c1h(kl) * MUT + c2h(kl)) * (c1f(kl) * MUT + c2f(kl)));
+    sA[k * 32 + ln] = a_k;
+    sB[k * 32 + ln] = 1.f + q * cof * rdn(k) *
+                                (rdnw(k) * ck / ((c1h(k) * MUT + c2h(k)) * (c1f(k) * MUT + c2f(k))) +
+                                 rdnw(k - 1) * cm / ((c1h(k - 1) * MUT + c2h(k - 1)) * (c1f(k) * MUT + c2f(k))));
+    sC[k * 32 + ln] = -q * cof * rdn(k) * rdnw(k) * ck / ((c1h(k) * MUT + c2h(k)) * (c1f(k + 1) * MUT + c2f(k + 1)));
+    if (act) A(i, k, j) = a_k;
+  }
+  if (wp == COEF_WARPS - 1) {  // the lid
+    const int kl = kde - 1;
+    const float r = rdnw(kl), ct = c2a.ro(i, kl, j);
+    const float a_top = -2.f * cof * (r * r) * ct * lid_flag / ((c1h(kl) * MUT + c2h(kl)) * (c1f(kl) * MUT + c2f(kl)));
+    sA[kde * 32 + ln] = a_top;
+    sB[kde * 32 + ln] = 1.f + 2.f * cof * (r * r) * ct / ((c1h(kl) * MUT + c2h(kl)) * (c1f(kde) * MUT + c2f(kde)));
+    sC[kde * 32 + ln] = 0.f;
+    if (act) A(i, kde, j) = a_top;
+  }
+  __syncthreads();
+  if (wp == 0) {
+    float gprev = 0.f;
+    sGA[32 + ln] = gprev;
+#pragma unroll 4
+    for (int k = 2; k <= kde; ++k) {
+      const float al = 1.f / (sB[k * 32 + ln] - sA[k * 32 + ln] * gprev);
+      sAL[k * 32 + ln] = al;
+      gprev = sC[k * 32 + ln] * al;
+      sGA[k * 32 + ln] = gprev;
+    }
+  }
+  __syncthreads();
+  if (!act) return;
+  for (int k = 1 + wp; k <= kde; k += COEF_WARPS) {
+    if (k >= 2) AL(i, k, j) = sAL[k * 32 + ln];
+    GA(i, k, j) = sGA[k * 32 + ln];
+  }
+}
+void launch_calc_coef_w_row(const TileLaunch& L, int nb, StepArgs a, cudaStream_t s) {
+  static bool attr = false;
+  if (!attr) {
+    cudaFuncSetAttribute(k_calc_coef_w_row, cudaFuncAttributeMaxDynamicSharedMemorySize, 129 * 32 * 20);
+    attr = true;
+  }
+  k_calc_coef_w_row<<<nb, 32 * COEF_WARPS, (size_t)(L.nlev + 1) * 32 * 20, s>>>(L, a.rk_step);
+}
+
 // ------------------------------------------------------------ advance_uv
 __global__ void __launch_bounds__(BX* BY) k_advance_uv(Launch L, int rk_step, int iteration) {
   BlockPos bp = block_pos(L);
@@ -676,29 +751,33 @@ __global__ void __launch_bounds__(BX* BY, MINB) k_small_step_finish(Launch L, in
     if (i == m.ids && m.its == m.ids) { int im = px ? i - 1 : i; muus = 0.5f * (MU(i, j) + MU(im, j)); }
     else if (i == m.ide && m.ite == m.ide) { int im = px ? i : i - 1; muus = 0.5f * (MU(i - 1, j) + MU(im, j)); }
     else muus = 0.5f * (MU(i, j) + MU(i - 1, j));
-    MUU(i, j) = muus;
+    if (blockIdx.y == 0) MUU(i, j) = muus;
   }
   if (vpt && calc_mus) {
     if (j == m.jds && m.jts == m.jds) { int jm = py ? j - 1 : j; muvs = 0.5f * (MU(i, j) + MU(i, jm)); }
     else if (j == m.jde && m.jte == m.jde) { int jm = py ? j : j - 1; muvs = 0.5f * (MU(i, j - 1) + MU(i, jm)); }
     else muvs = 0.5f * (MU(i, j) + MU(i, j - 1));
-    MUV(i, j) = muvs;
+    if (blockIdx.y == 0) MUV(i, j) = muvs;
   }
   F1 c1h = f1(m, WRFGPU_C1H), c2h = f1(m, WRFGPU_C2H), c1f = f1(m, WRFGPU_C1F), c2f = f1(m, WRFGPU_C2F);
   // levels are independent: inputs of a chunk of levels are loaded first
+  // (gridDim.y blocks share the levels; level kde goes to the last)
+  const Chunk ch = level_chunk_of(m.kds, m.kde - 1);
+  const int k0 = ch.k0, k1 = ch.k1;
+  if (k0 > k1) return;
   struct L2 { float x, s; };
   if (vpt) {
     F3 v_2 = f3(m, WRFGPU_V_2), v_save = f3(m, WRFGPU_V_SAVE);
     const float muv = f2(m, WRFGPU_MUV).ro(i, j), mx = f2(m, WRFGPU_MSFVX).ro(i, j);
     chunked_levels<8, L2>(
-        m.kds, m.kde - 1, [&](int k, L2& d) { d.x = v_2(i, k, j); d.s = v_save.ro(i, k, j); },
+        k0, k1, [&](int k, L2& d) { d.x = v_2(i, k, j); d.s = v_save.ro(i, k, j); },
         [&](int k, const L2& d) { v_2(i, k, j) = (mx * d.x + d.s * (c1h(k) * muv + c2h(k))) / (c1h(k) * muvs + c2h(k)); });
   }
   if (upt) {
     F3 u_2 = f3(m, WRFGPU_U_2), u_save = f3(m, WRFGPU_U_SAVE);
     const float muu = f2(m, WRFGPU_MUU).ro(i, j), my = f2(m, WRFGPU_MSFUY).ro(i, j);
     chunked_levels<8, L2>(
-        m.kds, m.kde - 1, [&](int k, L2& d) { d.x = u_2(i, k, j); d.s = u_save.ro(i, k, j); },
+        k0, k1, [&](int k, L2& d) { d.x = u_2(i, k, j); d.s = u_save.ro(i, k, j); },
         [&](int k, const L2& d) { u_2(i, k, j) = (my * d.x + d.s * (c1h(k) * muu + c2h(k))) / (c1h(k) * muus + c2h(k)); });
   }
   if (upt && vpt) {
@@ -709,7 +788,7 @@ __global__ void __launch_bounds__(BX* BY, MINB) k_small_step_finish(Launch L, in
     const bool last = rk_step >= m.cf.rk_ord;
     struct LW { float w, ws, p, ps, ww, ww1, t, ts, hd; };
     chunked_levels<6, LW>(
-        m.kds, m.kde,
+        k0, k1 == m.kde - 1 ? m.kde : k1,
         [&](int k, LW& d) {
           d.w = w_2(i, k, j); d.ws = w_save.ro(i, k, j); d.p = ph_2(i, k, j); d.ps = ph_save.ro(i, k, j);
           d.ww = ww(i, k, j); d.ww1 = ww1.ro(i, k, j);
@@ -730,7 +809,7 @@ __global__ void __launch_bounds__(BX* BY, MINB) k_small_step_finish(Launch L, in
           }
         });
     F2 mu_2 = f2(m, WRFGPU_MU_2);
-    mu_2(i, j) = mu_2(i, j) + f2(m, WRFGPU_MU_SAVE)(i, j);
+    if (blockIdx.y == 0) mu_2(i, j) = mu_2(i, j) + f2(m, WRFGPU_MU_SAVE)(i, j);
   }
 }
 
@@ -738,12 +817,13 @@ __global__ void __launch_bounds__(BX* BY, MINB) k_small_step_finish(Launch L, in
 void launch_small_step_prep(const Launch& L2, int nb2, const TileLaunch& LST, int nb_st, StepArgs a, cudaStream_t s,
                             int var) {
   k_small_step_prep_2d<<<nb2, dim3(BX, BY), 0, s>>>(L2, a.rk_step);
-  k_small_step_prep_3d<<<dim3(nb_st, TUNE_PARAM[TU_SSP][var]), dim3(TX, TY), 0, s>>>(LST, a.rk_step);
+  k_small_step_prep_3d<<<dim3(nb_st, level_chunks(nb_st, LST.nlev, TUNE_PARAM[TU_SSP][var], 2)), dim3(TX, TY), 0, s>>>(LST, a.rk_step);
 }
 void launch_calc_p_rho(const Launch& L, int nb, StepArgs a, cudaStream_t s) {
   k_calc_p_rho<<<nb, dim3(BX, BY), 0, s>>>(L, a.iteration);
 }
 void launch_calc_p_rho_col(const TileLaunch& L, int nb, StepArgs a, cudaStream_t s, int chunks) {
+  chunks = level_chunks(nb, L.nlev, chunks, 2);
   if (a.iteration > 0) k_calc_p_rho_col<true><<<dim3(nb, chunks), dim3(TX, TY), 0, s>>>(L, a.rk_step, a.iteration);
   else k_calc_p_rho_col<false><<<dim3(nb, chunks), dim3(TX, TY), 0, s>>>(L, a.rk_step, 0);
 }
@@ -772,8 +852,9 @@ void launch_sumflux_p_rho(const Launch& L, int nb, StepArgs a, bool do_p_rho, cu
 void launch_sumflux(const Launch& L, int nb, StepArgs a, cudaStream_t s) { launch_sumflux_p_rho(L, nb, a, false, s); }
 void launch_small_step_finish(const Launch& L, int nb, StepArgs a, cudaStream_t s, int var, bool calc_mus) {
   // 4 blocks of 128 threads per SM leave the registers free (~80); 8 hold them to 64
-  if (var == 0) k_small_step_finish<4><<<nb, dim3(BX, BY), 0, s>>>(L, a.rk_step, calc_mus);
-  else k_small_step_finish<8><<<nb, dim3(BX, BY), 0, s>>>(L, a.rk_step, calc_mus);
+  const dim3 grid(nb, level_chunks(nb, L.nlev, 1, 4, 8 * 152));
+  if (var == 0) k_small_step_finish<4><<<grid, dim3(BX, BY), 0, s>>>(L, a.rk_step, calc_mus);
+  else k_small_step_finish<8><<<grid, dim3(BX, BY), 0, s>>>(L, a.rk_step, calc_mus);
 }
 
 }  // namespace wrfgpu

@@ -58,14 +58,6 @@ __device__ __forceinline__ void tile_faces(const float* Q, float* FX, float* FY,
   if (ty == TY - 2) yface(TY, tx);
 }
 
-// Level chunk of this block (gridDim.y chunks of kts..ktf).
-struct Chunk { int k0, k1; };
-__device__ __forceinline__ Chunk level_chunk_of(int kts, int ktf) {
-  const int per = (ktf - kts + 1 + (int)gridDim.y - 1) / (int)gridDim.y;
-  const int k0 = kts + (int)blockIdx.y * per;
-  return Chunk{k0, min(ktf, k0 + per - 1)};
-}
-
 // ---------------------------------------------------------------- ru_tend
 // A level's point inputs of the u (v) tendency beyond the staged planes, with
 // the sums and differences of the two columns formed as the reference's
@@ -462,10 +454,10 @@ __global__ void __launch_bounds__(TX* TY, MINB) k_tend_v_col(TileLaunch L) {
 // advect_w (module_advect_em.F:4364-6064), pg_buoy_w, coriolis and curvature
 // (module_big_step_utilities_em.F) on the w levels.  pg_buoy_w overwrites
 // cqw(k) with 1/(1+cqw(k)) after the k = kde point has read the original
-// cqw(kde-1), so each column is walked in order by one thread (no level
-// chunks).  The face velocities interpolate ru, rv between levels k and k-1
-// (k-1 and k-2 at the top), so the ring keeps the two levels below the
-// current one: after the barrier of level k the slot of level k-3 is free.
+// cqw(kde-1), so the last level chunk holds both.  The face velocities
+// interpolate ru, rv between levels k and k-1 (k-1 and k-2 at the top), so
+// the ring starts one level below the chunk and keeps the two levels below
+// the current one: after the barrier of level k the slot of level k-3 is free.
 constexpr int W_RING = 6;
 using HaloRingW = LevelRing<3, W_RING, HALO_W, HALO_H>;
 constexpr size_t TENDW_SMEM = HaloRingW::SMEM + 2 * (FXN + FYN) * 4;
@@ -483,9 +475,12 @@ __global__ void __launch_bounds__(TX* TY, MINB) k_tend_w_col(TileLaunch L) {
   const int itf = min(m.ite, m.ide - 1), jtf = min(m.jte, m.jde - 1), ktf = min(kte, kde - 1);
   const bool inside = i <= m.ite && j <= m.jte;
   const bool acc = inside && i <= itf && j <= jtf;
-  if ((FL & TF_ZERO) && inside && !acc)
+  if ((FL & TF_ZERO) && inside && !acc && blockIdx.y == 0)
     for (int k = kts; k <= kte; ++k) tend(i, k, j) = 0.f;
-  if (!(tp.i0 <= itf && tp.j0 <= jtf)) return;  // block-uniform
+  Chunk ch = level_chunk_of(kts, ktf);
+  if (ch.k0 <= ktf && ch.k1 == ktf) ch.k1 = kte;
+  const int k0 = ch.k0, k1 = ch.k1, kf = max(kts, k0 - 1);  // this block's levels; first staged level
+  if (!(tp.i0 <= itf && tp.j0 <= jtf) || k0 > k1) return;  // block-uniform
   // next to an open boundary rw_tend has been formed by the edge-strip
   // kernel (k_tend.cu) from the cqw this kernel overwrites: keep it
   const bool keep = !((m.cf.open_xs || m.cf.open_ys) && in_open_strip(m, i, j, STRIP_W_TEND));
@@ -495,7 +490,7 @@ __global__ void __launch_bounds__(TX* TY, MINB) k_tend_w_col(TileLaunch L) {
            c1f = f1(m, WRFGPU_C1F), c2f = f1(m, WRFGPU_C2F);
   const float rdx = m.rdx, rdy = m.rdy;
   HaloRingW ring;
-  ring.init(smem, kts);
+  ring.init(smem, kf);
   float* FXb = (float*)(smem + HaloRingW::SMEM);
   float* FYb = FXb + 2 * FXN;
   const CUtensorMap* maps[3] = {tmap_of(m, WRFGPU_W_2, BOX_HALO), tmap_of(m, WRFGPU_RU, BOX_HALO),
@@ -507,7 +502,7 @@ __global__ void __launch_bounds__(TX* TY, MINB) k_tend_w_col(TileLaunch L) {
   }
   __syncthreads();
   if (tid == 0)
-    for (int d = 0; d < W_RING - 3 && kts + d <= kte; ++d) ring.issue(kts + d, maps, x0, z0, m.kms);
+    for (int k = kf; k <= min(k0 + W_RING - 4, k1); ++k) ring.issue(k, maps, x0, z0, m.kms);
   auto vf = [&](int kk) -> float {
     if (kk == kts + 1 || kk == ktf + 1) return 0.25f * (rom(i, kk, j) + rom(i, kk - 1, j)) * (w(i, kk, j) + w(i, kk - 1, j));
     float vel = 0.5f * (rom(i, kk, j) + rom(i, kk - 1, j));
@@ -530,9 +525,9 @@ __global__ void __launch_bounds__(TX* TY, MINB) k_tend_w_col(TileLaunch L) {
     }
     ratio05 = ratio * 0.5f;
     if (FL & TF_PG) { muf_c = f2(m, WRFGPU_MU_2)(i, j); mub_c = f2(m, WRFGPU_MUB)(i, j); }
-    cqw_top = cqw(i, kde - 1, j);  // read before the k = kde-1 overwrite below
+    if (k1 == kte) cqw_top = cqw(i, kde - 1, j);  // read before the k = kde-1 overwrite below
     // the vertical flux of face k+1 is the lower face of level k+1
-    vf_lo = kts + 1 <= ktf + 1 ? vf(kts + 1) : 0.f;
+    vf_lo = vf(max(k0, kts + 1));
   }
   // levels k-1 (and k-2) of the mass fluxes at the own point and its +i / +j
   // neighbours, and of u, v, p, carried down the column; w(k-1 .. k+1) and
@@ -542,13 +537,24 @@ __global__ void __launch_bounds__(TX* TY, MINB) k_tend_w_col(TileLaunch L) {
   float wkm1 = 0.f, wk0 = 0.f, wkp1 = 0.f, romk = 0.f;
   const int kme = m.kme;
   if (acc) {
-    wk0 = w(i, kts, j);
-    wkp1 = kts + 1 <= kme ? w(i, kts + 1, j) : 0.f;
-    romk = rom(i, kts, j);
+    if (k0 > kts) wkm1 = w(i, k0 - 1, j);
+    wk0 = w(i, k0, j);
+    wkp1 = k0 + 1 <= kme ? w(i, k0 + 1, j) : 0.f;
+    romk = rom(i, k0, j);
   }
   const int o = (ty + TMA_HALO) * HALO_W + tx + TMA_HALO;
   bool ok = true;
-  for (int k = kts; k <= kte; ++k) {
+  if (k0 > kts) {  // what level k0 takes from the level below
+    if (acc) {
+      if (FL & TF_CURV) { u0m = u(i, k0 - 1, j); u1m = u(i + 1, k0 - 1, j); v0m = v(i, k0 - 1, j); v1m = v(i, k0 - 1, j + 1); }
+      if (FL & TF_PG) pkm = p(i, k0 - 1, j);
+    }
+    ok = ring.wait(kf) && ok;
+    const float* RU = ring.plane(kf, 1);
+    const float* RV = ring.plane(kf, 2);
+    ru0m = RU[o]; ru1m = RU[o + 1]; rv0m = RV[o]; rv1m = RV[o + HALO_W];
+  }
+  for (int k = k0; k <= k1; ++k) {
     // the level's global inputs, loaded together before the face work and
     // the level barrier so that their latency overlaps them
     float u0 = 0.f, u1 = 0.f, v0 = 0.f, v1 = 0.f, pk = 0.f, cqk = 0.f, romk1 = 0.f, wk2 = 0.f, t = 0.f;
@@ -585,7 +591,7 @@ __global__ void __launch_bounds__(TX* TY, MINB) k_tend_w_col(TileLaunch L) {
       }
     }
     __syncthreads();
-    if (tid == 0 && k - 3 + W_RING <= kte) ring.issue(k - 3 + W_RING, maps, x0, z0, m.kms);
+    if (tid == 0 && k - 3 + W_RING <= k1) ring.issue(k - 3 + W_RING, maps, x0, z0, m.kms);
     if (!acc) continue;
     const float ru0 = RUk[o], ru1 = RUk[o + 1], rv0 = RVk[o], rv1 = RVk[o + HALO_W];
     if (adv) {
@@ -665,7 +671,9 @@ __global__ void __launch_bounds__(TX* TY, MINB) k_tend_t_col(TileLaunch L) {
   const int kts = m.kts, kte = m.kte, kme = m.kme;
   const int itf = min(m.ite, m.ide - 1), jtf = min(m.jte, m.jde - 1), ktf = min(kte, m.kde - 1);
   const bool inside = i <= m.ite && j <= m.jte;
-  if ((FL & TF_ZERO) && inside) {
+  const Chunk ch = level_chunk_of(kts, ktf);
+  const int k0 = ch.k0, k1 = ch.k1;
+  if ((FL & TF_ZERO) && inside && blockIdx.y == 0) {
     const bool ie = i == m.ide, je = j == m.jde;
     const F3 us = f3(m, WRFGPU_U_SAVE), vs = f3(m, WRFGPU_V_SAVE), ts = f3(m, WRFGPU_T_SAVE),
              ws = f3(m, WRFGPU_W_SAVE), phs = f3(m, WRFGPU_PH_SAVE);
@@ -679,13 +687,13 @@ __global__ void __launch_bounds__(TX* TY, MINB) k_tend_t_col(TileLaunch L) {
     if (ie || je) f2(m, WRFGPU_MU_SAVE)(i, j) = 0.f;
   }
   const bool acc = inside && i <= itf && j <= jtf;
-  if ((FL & TF_ZERO) && inside && !acc)
+  if ((FL & TF_ZERO) && inside && !acc && blockIdx.y == 0)
     for (int k = kts; k <= kte; ++k) tend(i, k, j) = 0.f;
-  if (tp.i0 <= itf && tp.j0 <= jtf) {  // block-uniform
+  if (tp.i0 <= itf && tp.j0 <= jtf && k0 <= k1) {  // block-uniform
     const F3 fld = f3(m, WRFGPU_T_2), rom = f3(m, WRFGPU_WW);
     const F1 fzm = f1(m, WRFGPU_FNM), fzp = f1(m, WRFGPU_FNP), rdzw = f1(m, WRFGPU_RDNW);
     HaloRing ring;
-    ring.init(smem, kts);
+    ring.init(smem, k0);
     float* FXb = (float*)(smem + HaloRing::SMEM);
     float* FYb = FXb + 2 * FXN;
     const CUtensorMap* maps[3] = {tmap_of(m, WRFGPU_T_2, BOX_HALO), tmap_of(m, WRFGPU_RU, BOX_HALO),
@@ -697,16 +705,22 @@ __global__ void __launch_bounds__(TX* TY, MINB) k_tend_t_col(TileLaunch L) {
     }
     __syncthreads();
     if (tid == 0)
-      for (int d = 0; d < TEND_RING - 1 && kts + d <= ktf; ++d) ring.issue(kts + d, maps, x0, z0, m.kms);
+      for (int d = 0; d < TEND_RING - 1 && k0 + d <= k1; ++d) ring.issue(k0 + d, maps, x0, z0, m.kms);
     float mrdy = 0.f, mrdx = 0.f, fm1 = 0.f, f0 = 0.f, fp1 = 0.f, fp2 = 0.f;
     if (acc) {
       const float msftx_c = f2(m, WRFGPU_MSFTX)(i, j);
       mrdy = msftx_c * m.rdy; mrdx = msftx_c * m.rdx;
-      f0 = fld(i, kts, j); fp1 = fld(i, kts + 1, j); fp2 = (kts + 2 <= kme) ? fld(i, kts + 2, j) : 0.f;
+      if (k0 > kts) fm1 = fld(i, k0 - 1, j);
+      f0 = fld(i, k0, j); fp1 = fld(i, k0 + 1, j); fp2 = (k0 + 2 <= kme) ? fld(i, k0 + 2, j) : 0.f;
     }
-    float vf_lo = 0.f;  // vf(kts) = 0
+    float vf_lo = 0.f;  // vf(k0), formed as level k0 - 1 forms its upper face; vf(kts) = 0
+    if (acc && k0 > kts) {
+      const float vel = rom(i, k0, j);
+      if (k0 == kts + 1 || k0 == ktf) vf_lo = vel * (fzm(k0) * f0 + fzp(k0) * fm1);
+      else vf_lo = vel * flux3(fld(i, k0 - 2, j), fm1, f0, fp1, -vel);
+    }
     bool ok = true;
-    for (int k = kts; k <= ktf; ++k) {
+    for (int k = k0; k <= k1; ++k) {
       // the level's own-column loads, issued before the face work and the
       // barrier so that their latency overlaps them
       float fp3 = 0.f, romk1 = 0.f;
@@ -722,7 +736,7 @@ __global__ void __launch_bounds__(TX* TY, MINB) k_tend_t_col(TileLaunch L) {
       float* FY = FYb + (k & 1) * FYN;
       tile_faces(T, FX, FY, [&](int q) { return RU[q]; }, [&](int q) { return RV[q]; }, tx, ty);
       __syncthreads();
-      if (tid == 0 && k + TEND_RING - 1 <= ktf) ring.issue(k + TEND_RING - 1, maps, x0, z0, m.kms);
+      if (tid == 0 && k + TEND_RING - 1 <= k1) ring.issue(k + TEND_RING - 1, maps, x0, z0, m.kms);
       if (!acc) continue;
       if (k + 2 <= kme) { prefetch_l2(&rom(i, k + 2, j)); prefetch_l2(&tend(i, k + 2, j)); }
       float t = (FL & TF_ZERO) ? 0.f : tend(i, k, j);
@@ -743,7 +757,7 @@ __global__ void __launch_bounds__(TX* TY, MINB) k_tend_t_col(TileLaunch L) {
     }
     if (!ok && tid == 0) raise_err(m, ERR_TIMEOUT);
   }
-  if ((FL & TF_ZERO) && acc)
+  if ((FL & TF_ZERO) && acc && blockIdx.y == 0)
     for (int k = ktf + 1; k <= kte; ++k) tend(i, k, j) = 0.f;
 }
 
@@ -767,13 +781,14 @@ __global__ void __launch_bounds__(TX* TY, 4) k_tend_ph_col(TileLaunch L) {
   const int itf = min(m.ite, m.ide - 1), jtf = min(m.jte, m.jde - 1);
   const bool inside = i <= m.ite && j <= m.jte;
   const bool acc = inside && i <= itf && j <= jtf;
-  if (inside && !acc)
+  if (inside && !acc && blockIdx.y == 0)
     for (int k = kts; k <= kte; ++k) tend(i, k, j) = 0.f;
   if (!(tp.i0 <= itf && tp.j0 <= jtf)) return;  // block-uniform
-  if (acc)
+  if (acc && blockIdx.y == 0)
     for (int k = kts; k <= min(kte, 1); ++k) tend(i, k, j) = 0.f;
-  const int ks = max(kts, 2);
-  if (ks > kte) return;
+  const Chunk ch = level_chunk_of(max(kts, 2), kte);
+  const int ks = ch.k0, ke = ch.k1;  // this block's levels
+  if (ks > ke) return;
   const F3 u = f3(m, WRFGPU_U_2), v = f3(m, WRFGPU_V_2), ww = f3(m, WRFGPU_WW), ph = f3(m, WRFGPU_PH_2),
            phb = f3(m, WRFGPU_PHB), w = f3(m, WRFGPU_W_2);
   const F1 c1f = f1(m, WRFGPU_C1F), c2f = f1(m, WRFGPU_C2F), fnm = f1(m, WRFGPU_FNM), fnp = f1(m, WRFGPU_FNP),
@@ -788,7 +803,7 @@ __global__ void __launch_bounds__(TX* TY, 4) k_tend_ph_col(TileLaunch L) {
   }
   __syncthreads();
   if (tid == 0)
-    for (int d = 0; d < PH_RING - 1 && ks + d <= kte; ++d) ring.issue(ks + d, maps, x0, z0, m.kms);
+    for (int d = 0; d < PH_RING - 1 && ks + d <= ke; ++d) ring.issue(ks + d, maps, x0, z0, m.kms);
   // column constants
   float mut_c = 0.f, msfty_c = 0.f, muv1 = 0.f, muv0 = 0.f, muu1 = 0.f, muu0 = 0.f, mvy1 = 0.f, mvy0 = 0.f;
   float mux1 = 0.f, mux0 = 0.f, cy4 = 0.f, cx4 = 0.f, cy2 = 0.f, cx2 = 0.f;
@@ -810,13 +825,16 @@ __global__ void __launch_bounds__(TX* TY, 4) k_tend_ph_col(TileLaunch L) {
     mux1 = f2(m, WRFGPU_MSFUX)(i + 1, j); mux0 = f2(m, WRFGPU_MSFUX)(i, j);
     cy4 = 0.25f * m.rdy / msfty_c; cx4 = 0.25f * m.rdx / msfty_c;
     cy2 = 0.5f * m.rdy / msfty_c; cx2 = 0.5f * m.rdx / msfty_c;
-    u0m = u(i, 1, j); u1m = u(i + 1, 1, j); v0m = v(i, 1, j); v1m = v(i, 1, j + 1);  // level k-1 = 1
-    wd_lo = (2 <= kte - 1) ? wdwn(2) : 0.f;  // wdwn(k) at k = 2
+    u0m = u(i, ks - 1, j); u1m = u(i + 1, ks - 1, j); v0m = v(i, ks - 1, j); v1m = v(i, ks - 1, j + 1);
+    if (ks == kte) {  // the top level extrapolates from the two below it
+      u0mm = u(i, ks - 2, j); u1mm = u(i + 1, ks - 2, j); v0mm = v(i, ks - 2, j); v1mm = v(i, ks - 2, j + 1);
+    }
+    wd_lo = (ks <= kte - 1) ? wdwn(ks) : 0.f;  // wdwn(k) at k = ks
     ph_c = ph(i, ks, j); phb_c = phb(i, ks, j); ww_c = ww(i, ks, j);
   }
   const int o = (ty + TMA_HALO) * HALO_W + tx + TMA_HALO;
   bool ok = true;
-  for (int k = ks; k <= kte; ++k) {
+  for (int k = ks; k <= ke; ++k) {
     // the level's global inputs, loaded together before the barrier so that
     // their latency overlaps it
     float ph_n = 0.f, phb_n = 0.f, ww_n = 0.f, u0 = 0.f, u1 = 0.f, v0 = 0.f, v1 = 0.f, wk = 0.f;
@@ -828,7 +846,7 @@ __global__ void __launch_bounds__(TX* TY, 4) k_tend_ph_col(TileLaunch L) {
       if (m.cf.non_hydrostatic) wk = w(i, k, j);
     }
     __syncthreads();  // every thread is done with level k-1's slot
-    if (tid == 0 && k + PH_RING - 1 <= kte) ring.issue(k + PH_RING - 1, maps, x0, z0, m.kms);
+    if (tid == 0 && k + PH_RING - 1 <= ke) ring.issue(k + PH_RING - 1, maps, x0, z0, m.kms);
     ok = ring.wait(k) && ok;
     if (!acc) continue;
     const float* PH = ring.plane(k, 0);
@@ -878,17 +896,20 @@ __global__ void __launch_bounds__(TX* TY, 4) k_tend_ph_col(TileLaunch L) {
   if (!ok && tid == 0) raise_err(m, ERR_TIMEOUT);
 }
 
+// The shortest level chunk of the staged tendencies.
+constexpr int TEND_MINLEV = 4;
+
 // variant parameter: 10 x blocks per SM + level chunks
 void launch_tend_u_col(const TileLaunch& L, int nb, int flags, cudaStream_t s, int var) {
   const int p = TUNE_PARAM[TU_TENDU][var];
-  const dim3 grid(nb, p % 10);
+  const dim3 grid(nb, level_chunks(nb, L.nlev, p % 10, TEND_MINLEV));
   if (flags != TF_ALL) return;
   if (p / 10 == 4) k_tend_u_col<TF_ALL, 4><<<grid, dim3(TX, TY), TEND_SMEM, s>>>(L);
   else k_tend_u_col<TF_ALL, 3><<<grid, dim3(TX, TY), TEND_SMEM, s>>>(L);
 }
 void launch_tend_v_col(const TileLaunch& L, int nb, int flags, cudaStream_t s, int var) {
   const int p = TUNE_PARAM[TU_TENDV][var];
-  const dim3 grid(nb, p % 10);
+  const dim3 grid(nb, level_chunks(nb, L.nlev, p % 10, TEND_MINLEV));
   if (flags != TF_ALL) return;
   if (p / 10 == 4) k_tend_v_col<TF_ALL, 4><<<grid, dim3(TX, TY), TEND_SMEM, s>>>(L);
   else k_tend_v_col<TF_ALL, 3><<<grid, dim3(TX, TY), TEND_SMEM, s>>>(L);
@@ -902,15 +923,16 @@ void launch_tend_w_col(const TileLaunch& L, int nb, int var, cudaStream_t s) {
     attr = true;
   }
   const int minb = TUNE_PARAM[TU_TENDW][var];
-  if (minb == 2) k_tend_w_col<TF_ALL, 2><<<nb, dim3(TX, TY), TENDW_SMEM, s>>>(L);
-  else if (minb == 3) k_tend_w_col<TF_ALL, 3><<<nb, dim3(TX, TY), TENDW_SMEM, s>>>(L);
-  else k_tend_w_col<TF_ALL, 4><<<nb, dim3(TX, TY), TENDW_SMEM, s>>>(L);
+  const dim3 grid(nb, level_chunks(nb, L.nlev, 1, TEND_MINLEV));
+  if (minb == 2) k_tend_w_col<TF_ALL, 2><<<grid, dim3(TX, TY), TENDW_SMEM, s>>>(L);
+  else if (minb == 3) k_tend_w_col<TF_ALL, 3><<<grid, dim3(TX, TY), TENDW_SMEM, s>>>(L);
+  else k_tend_w_col<TF_ALL, 4><<<grid, dim3(TX, TY), TENDW_SMEM, s>>>(L);
 }
 void launch_tend_t_col(const TileLaunch& L, int nb, int flags, cudaStream_t s) {
-  if (flags == (TF_ZERO | TF_ADV)) k_tend_t_col<TF_ZERO | TF_ADV, 4><<<nb, dim3(TX, TY), TEND_SMEM, s>>>(L);
+  if (flags == (TF_ZERO | TF_ADV)) k_tend_t_col<TF_ZERO | TF_ADV, 4><<<dim3(nb, level_chunks(nb, L.nlev, 1, TEND_MINLEV)), dim3(TX, TY), TEND_SMEM, s>>>(L);
 }
 void launch_tend_ph_col(const TileLaunch& L, int nb, int flags, cudaStream_t s) {
-  if (flags == (TF_ZERO | TF_ADV)) k_tend_ph_col<TF_ZERO | TF_ADV><<<nb, dim3(TX, TY), PhRing::SMEM, s>>>(L);
+  if (flags == (TF_ZERO | TF_ADV)) k_tend_ph_col<TF_ZERO | TF_ADV><<<dim3(nb, level_chunks(nb, L.nlev, 1, TEND_MINLEV)), dim3(TX, TY), PhRing::SMEM, s>>>(L);
 }
 
 }  // namespace wrfgpu

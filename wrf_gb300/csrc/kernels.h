@@ -49,7 +49,7 @@ constexpr int TUNE_NVAR[NTUNE] = {2, 3, 3, 4, 4, 2, 2, 4, 4, 3, 4, 4, 4, 4};
 // (defaults measured on 512x512x80 and up: advance_mu_t 278 us with four blocks
 // per SM against 393 with two, advance_w 340 against 388; the FP64 form of
 // advance_mu_t is best with three, 524 against 571 us on the 16-member ensemble)
-constexpr int TUNE_DEFAULT[NTUNE] = {1, 1, 2, 1, 2, 1, 1, 2, 2, 1, 0, 0, 2, 2};
+constexpr int TUNE_DEFAULT[NTUNE] = {1, 1, 2, 1, 2, 1, 0, 2, 2, 1, 3, 3, 2, 2};
 // the parameter each variant stands for: blocks per SM, level chunks
 // (sumflux: of calc_p_rho), or (advance_uv, rk_tend_u, rk_tend_v) 10 x blocks
 // per SM + level chunks
@@ -58,6 +58,12 @@ constexpr int TUNE_PARAM[NTUNE][TUNE_MAXVAR] = {{1, 2, 0, 0}, {2, 3, 4, 0}, {2, 
                                                 {32, 42, 34, 44}, {32, 42, 34, 44}, {1, 2, 4, 8}, {2, 3, 4, 5}};
 
 void launch_rk_step_prep(const Launch& L, int nblocks, cudaStream_t s, int var = TUNE_DEFAULT[TU_PREP]);
+// one block per row segment of 32 columns (rows jts-1 .. jte), levels over its
+// warps; taken up to PREP_ROW_MAX segments.  ms per step, this form against the
+// column march: 41x41x41 (84 segments) 0.038 / 0.147, 190x161x60 (972) 0.17 / 0.28,
+// 256x256x80 (2322) 0.39 / 0.45, 24 small members (about 3000) 0.49 / 0.44.
+constexpr int PREP_ROW_MAX = 2500;
+void launch_rk_step_prep_row(const TileLaunch& L, int nblocks, cudaStream_t s);
 void launch_fill_halo(const Mem* d_mems, int nmem, const HaloJobs& jobs, int blocks_per_job, cudaStream_t s);
 
 // rk_tendency
@@ -87,6 +93,12 @@ void launch_small_step_prep(const Launch& L2, int nb2, const TileLaunch& LST, in
 void launch_calc_p_rho(const Launch& L3, int nblocks, StepArgs a, cudaStream_t s);
 void launch_calc_coef_w(const Launch& L2, int nblocks, StepArgs a, bool fp64, cudaStream_t s);
 void launch_calc_coef_w_col(const TileLaunch& L, int nblocks, StepArgs a, bool fp64, cudaStream_t s);  // mass tiles
+// mass row segments, FP32, up to COEF_ROW_MAX of them (its recursion runs in one
+// warp of a block): 41x41x41 (82) 0.037 / 0.083, 160x144x64 (720) 0.099 / 0.139,
+// 190x161x60 (966) 0.129 / 0.132, 256x256x80 (2048) 0.27 / 0.19; FP64 75x90x128
+// (270) 0.43 / 0.40
+constexpr int COEF_ROW_MAX = 900;
+void launch_calc_coef_w_row(const TileLaunch& L, int nblocks, StepArgs a, cudaStream_t s);
 void launch_advance_uv(const Launch& L3, int nblocks, StepArgs a, cudaStream_t s);
 void launch_advance_mu_t(const Launch& L2, int nblocks, StepArgs a, bool fp64, cudaStream_t s);
 void launch_advance_w(const Launch& L2, int nblocks, StepArgs a, bool fp64, cudaStream_t s);
