@@ -129,13 +129,11 @@ int wrfgpu_advect_scalar_pd(const float *field, const float *field_old, float *t
  * layout and meaning as above, unused arguments dropped; tendency
  * accumulates), enqueued on `stream` (a cudaStream_t, NULL = default stream)
  * without allocating device memory.  For callers whose state is already on
- * the GPU and that cannot allocate there.  The limiter-factor scratch is a
- * fixed static device array: the memory shape may hold at most 8 Mi points
- * (WRFGPU_E_SIZE otherwise).  Options a device domain does not accept
- * return WRFGPU_E_ARG.  The first call on a device (or after its context
- * was re-created) does a one-time setup and should come before any stream
- * capture; calls that overlap in time race on the shared scratch.  The
- * kernels have no device-side failure: the return code is the whole status. */
+ * the GPU and that cannot allocate there.  The memory shape may hold at most
+ * 8 Mi points (WRFGPU_E_SIZE otherwise).  Options a device domain does not
+ * accept return WRFGPU_E_ARG.  One kernel launch with no state of its own:
+ * calls on different streams or threads do not disturb one another.  The
+ * kernel has no device-side failure: the return code is the whole status. */
 int wrfgpu_advect_scalar_pd_noalloc(const float *field, const float *field_old, float *tendency,
                                     const float *ru, const float *rv, const float *rom, const float *c1,
                                     const float *c2, const float *mut, const float *mub, const float *mu_old,

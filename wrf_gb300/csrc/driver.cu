@@ -1144,10 +1144,10 @@ struct Ensemble {
       case 119: launch_small_step_finish(l2, nb2, a, stream, TUNE_DEFAULT[TU_SSF], false); break;  // muus, muvs given
       case 20: launch_update_scalar_pd(l3, nb3, a, stream); break;
       case 21: launch_advect_scalar(l3, nb3, StepArgs{rk_step, 0, species, 0}, stream); break;
-      case 22: launch_advect_scalar_pd2(l3, nb3, StepArgs{rk_step, 0, species, 2}, d_pd_scratch, stream); break;
+      case 22: launch_advect_scalar_pd(LTM(), nb_tm, species, rk_step, false, stream); break;
       // accumulating forms (tendency += ...) for the routine-level C ABI
       case 121: launch_advect_scalar(l3, nb3, StepArgs{rk_step, 0, species, 4}, stream); break;
-      case 122: launch_advect_scalar_pd2(l3, nb3, StepArgs{rk_step, 0, species, 6}, d_pd_scratch, stream); break;
+      case 122: launch_advect_scalar_pd(LTM(), nb_tm, species, rk_step, true, stream); break;
       case 23: launch_update_scalar(l3, nb3, a, stream); break;
       // routine-level C ABI forms of the scalar updates (sc_tend in H_DIABATIC)
       // and of rk_scalar_tend's sixth-order diffusion of one species

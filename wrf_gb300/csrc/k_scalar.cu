@@ -113,44 +113,273 @@ __global__ void __launch_bounds__(BX* BY) k_advect_scalar(Launch L, int species,
   tend(i, k, j) = adv_scalar_point(m, a, accum ? tend(i, k, j) : 0.f, i, j, k);
 }
 
-// ------------------------------------------------------------ advect_scalar_pd (open_adv.cuh)
-// Pass 1: limiter scale of each cell of the tile + 1-cell halo (-1: not limited).
-// mode 0: only members whose species uses the positive-definite scheme; mode 2: always.
-__global__ void __launch_bounds__(BX* BY) k_pd_scale(Launch L, int species, int rk_step, int mode, float* const* scratch) {
-  BlockPos bp = block_pos(L);
-  const Mem& m = block_member(L.mem, bp.m);
-  if (!bp.valid) return;
-  if (species >= m.nsp) return;
-  if ((mode & 3) == 0 && !pd_applies(m, species, rk_step)) return;
-  const int i = bp.i, j = bp.j, k = bp.k;
-  const int itf = min(m.ite, m.ide - 1), jtf = min(m.jte, m.jde - 1), ktf = min(m.kte, m.kde - 1);
-  if (i < m.its - 1 || i > itf + 1 || j < m.jts - 1 || j > jtf + 1 || k < m.kts || k > ktf) return;
-  const Stage st = stage_of(m, rk_step);
-  const PDCtx c = pd_ctx(m, species, st.dt_rk);
-  f3p(m, scratch[bp.m])(i, k, j) = pd_scale_cell(m, c, i, k, j);
-}
+// ------------------------------------------------------------ advect_scalar_pd
+// One species' limited transport into advect_tend, for the routine-level
+// entry points: one block per (32 x 8 tile of mass columns, chunk of levels),
+// marching up k.  The four input planes of a level (scalar, old scalar, ru, rv:
+// the tile and a 4-point halo) arrive by cp.async, three levels ahead — the
+// caller's arrays have any pitch and alignment, which a tensor map does not
+// take.  Every face flux of the limiter region (tile + 1) is formed once, by
+// one thread, into shared memory; the vertical ones stay in registers; one
+// barrier per level (the face slots and factor slots are those of
+// k_scalar_pd_update, k_scalar_fused.cu, which documents their reuse).  Two
+// passes over points formed each flux two (limiter, divergence) times two
+// (the face's two cells) times, with its two divisions, from global memory:
+// a call on 231 x 180 x 64 took 384 us, with this form 137 us.  Issue-bound.
+//
+// The arithmetic is open_adv.cuh's point functions', term for term.
+struct PdrPlanes {
+  static constexpr int HW = TX + 8, HH = TY + 8, HN = HW * HH;  // staged plane, origin (i0 - 4, j0 - 4)
+  static constexpr int SW = TX + 2, SH = TY + 2, SN = SW * SH;  // limiter region
+  static constexpr int XW = TX + 3, YW = TX + 2;                // x faces [SH][XW], y faces [SH + 1][YW]
+  static constexpr int XN = XW * SH, YN = YW * (SH + 1);
+  static constexpr int THREADS = SN + SH + YW;  // one per cell, one per face the cells leave out: 384
+  static constexpr int RING = 4, FSLOT = 3;
+  static constexpr int FLOATS = RING * 4 * HN + FSLOT * 2 * (XN + YN) + 2 * SN;
+};
+// Constants of level k: a = {c1, c2, rdzw, dz / dt}, b = {fzm, fzp, dz, 0} (dz of the z face k).
+struct PdrLevel { float4 a, b; };
 
-// Pass 2: divergence of the limited fluxes (z, then x, then y) into advect_tend.
-__global__ void __launch_bounds__(BX* BY) k_pd_tend(Launch L, int species, int rk_step, int mode, float* const* scratch) {
-  BlockPos bp = block_pos(L);
-  const Mem& m = block_member(L.mem, bp.m);
-  if (!bp.valid) return;
-  if (species >= m.nsp) return;
-  const bool accum = (mode & 4) != 0;  // tendency += (routine-level callers)
-  if ((mode & 3) == 0 && !pd_applies(m, species, rk_step)) return;
-  const int i = bp.i, j = bp.j, k = bp.k;
-  F3 tend = f3(m, WRFGPU_ADVECT_TEND);
-  const bool in_zero = i >= m.its && i <= m.ite && j >= m.jts && j <= m.jte && k >= m.kts && k <= m.kte;
-  const int ktf = min(m.kte, m.kde - 1);
-  if (!(mass_pt(m, i, j) && k >= m.kts && k <= ktf)) {
-    if (in_zero && !accum) tend(i, k, j) = 0.f;
-    return;
+__device__ __forceinline__ void pd_tile(const Mem& m, int species, int rk_step, bool accum, int i0, int j0) {
+  using P = PdrPlanes;
+  extern __shared__ __align__(16) float pdr_smem[];
+  const int tid = threadIdx.x;
+  const int itf = min(m.ite, m.ide - 1), jtf = min(m.jte, m.jde - 1), ktf = min(m.kte, m.kde - 1);
+  const int kts = m.kts, kde = m.kde, kme = m.kme;
+  const Chunk ch = level_chunk_of(kts, ktf);
+  const int k0 = ch.k0, k1 = ch.k1, L0 = max(kts, k0 - 1), L1 = min(ktf, k1 + 1);
+  if (k0 > k1) return;  // block-uniform
+  const float dt = stage_of(m, rk_step).dt_rk, rdx = m.rdx, rdy = m.rdy;
+  float* ring = pdr_smem;
+  float* sXH = ring + P::RING * 4 * P::HN;
+  float* sXL = sXH + P::FSLOT * P::XN;
+  float* sYH = sXL + P::FSLOT * P::XN;
+  float* sYL = sYH + P::FSLOT * P::YN;
+  float* sSC = sYL + P::FSLOT * P::YN;
+  PdrLevel* sLV = reinterpret_cast<PdrLevel*>(sSC + 2 * P::SN);  // [k - kts]; SN and the rest are multiples of 4 floats
+  static_assert((P::RING * 4 * P::HN + P::FSLOT * 2 * (P::XN + P::YN) + 2 * P::SN) % 4 == 0, "level table alignment");
+  const F3 f = f3p(m, m.q[species]), fo = f3p(m, m.qo[species]), ru = f3(m, WRFGPU_RU_M), rv = f3(m, WRFGPU_RV_M),
+           rom = f3(m, WRFGPU_WW_M), tend = f3(m, WRFGPU_ADVECT_TEND);
+  const F2 mut2 = f2(m, WRFGPU_MUTS), msx = f2(m, WRFGPU_MSFTX), msy = f2(m, WRFGPU_MSFTY);
+  const F1 c1 = f1(m, WRFGPU_C1H), c2 = f1(m, WRFGPU_C2H), fzm = f1(m, WRFGPU_FNM), fzp = f1(m, WRFGPU_FNP),
+           rdzw = f1(m, WRFGPU_RDNW);
+
+  // this thread's elements of a staged plane (indices clamped to the memory extent)
+  constexpr int EL = (P::HN + P::THREADS - 1) / P::THREADS;
+  int eoff[EL];
+#pragma unroll
+  for (int q = 0; q < EL; ++q) {
+    const int e = min(tid + q * P::THREADS, P::HN - 1);
+    const int ei = min(max(i0 - 4 + e % P::HW, m.ims), m.ime), ej = min(max(j0 - 4 + e / P::HW, m.jms), m.jme);
+    eoff[q] = f.off(ei, m.kms, ej);
   }
-  const Stage st = stage_of(m, rk_step);
-  const PDCtx c = pd_ctx(m, species, st.dt_rk);
-  const F3 sc = f3p(m, scratch[bp.m]);
-  tend(i, k, j) = pd_tend_cell(m, c, i, k, j, accum ? tend(i, k, j) : 0.f,
-                               [&](int ci, int ck, int cj) { return sc(ci, ck, cj); });
+  auto issue = [&](int k) {
+    float* dst = ring + (k % P::RING) * 4 * P::HN;
+    const int lk = (k - m.kms) * f.sk;
+#pragma unroll
+    for (int q = 0; q < EL; ++q) {
+      const int e = tid + q * P::THREADS;
+      if (e < P::HN) {
+        cp_async4(dst + e, f.p + eoff[q] + lk);
+        cp_async4(dst + P::HN + e, fo.p + eoff[q] + lk);
+        cp_async4(dst + 2 * P::HN + e, ru.p + eoff[q] + lk);
+        cp_async4(dst + 3 * P::HN + e, rv.p + eoff[q] + lk);
+      }
+    }
+  };
+  issue(L0);
+  cp_async_commit();
+  if (L0 + 1 <= L1) issue(L0 + 1);
+  cp_async_commit();
+  if (L0 + 2 <= L1) issue(L0 + 2);
+  cp_async_commit();
+  for (int k = kts + tid; k <= ktf; k += P::THREADS) {
+    const float dz = k > kts ? 2.f / (rdzw(k) + rdzw(k - 1)) : 0.f;
+    sLV[k - kts].a = make_float4(c1(k), c2(k), rdzw(k), dz / dt);
+    sLV[k - kts].b = make_float4(fzm(k), fzp(k), dz, 0.f);
+  }
+
+  // this thread's limiter cell and its faces: cells 0..31 of each row on one
+  // warp, the rows' last two cells on the next 20 threads, then the x faces
+  // of column i0 + 33 and the y faces of row j0 + 9
+  const bool has_cell = tid < P::SN;
+  int sx, sy;
+  bool fx = has_cell, fy = has_cell;
+  if (tid < 32 * P::SH) { sy = tid >> 5; sx = tid & 31; }
+  else if (has_cell) { const int q = tid - 32 * P::SH; sy = q >> 1; sx = 32 + (q & 1); }
+  else if (tid < P::SN + P::SH) { sy = tid - P::SN; sx = P::SW; fx = true; }
+  else { sy = P::SH; sx = tid - P::SN - P::SH; fy = true; }
+  const int i = i0 - 1 + sx, j = j0 - 1 + sy;
+  const int xq = sy * P::XW + sx, yq = sy * P::YW + sx;  // left and bottom face
+  const int so = sy * P::SW + sx, o = (sy + 3) * P::HW + sx + 3;  // own point in the factor and staged planes
+  const bool xok = fx && i >= m.its - 1 && i <= itf + 2 && j >= m.jts - 1 && j <= jtf + 1;
+  const bool yok = fy && i >= m.its - 1 && i <= itf + 1 && j >= m.jts - 1 && j <= jtf + 2;
+  const bool cell = has_cell && i >= m.its - 1 && i <= itf + 1 && j >= m.jts - 1 && j <= jtf + 1;
+  const bool own = has_cell && sx >= 1 && sx <= TX && sy >= 1 && sy <= TY && i <= itf && j <= jtf;
+  float mt = 0.f, mt_x = 0.f, mt_y = 0.f, dx = 1.f, dxdt = 1.f, dy = 1.f, dydt = 1.f, mx = 1.f, my = 1.f, mub = 0.f,
+        mu_old = 0.f;
+  int ox = 5, oy = 5;
+  bool quirk = false, limited = false, xdiv = false, ydiv = false;
+  if (xok || yok) { mt = mut2(i, j); mx = msx(i, j); my = msy(i, j); }
+  if (xok) {
+    ox = open_order_mass(i, m.cf.open_xs, m.cf.open_xe, m.ids, m.ide);
+    quirk = ox == 2 && m.cf.open_xs && i == m.ids + 1;
+    mt_x = mut2(i - 1, j);
+    dx = 2.f / (my + msy(i - 1, j)) / rdx;
+    dxdt = dx / dt;
+  }
+  if (yok) {
+    oy = open_order_mass(j, m.cf.open_ys, m.cf.open_ye, m.jds, m.jde);
+    mt_y = mut2(i, j - 1);
+    dy = 2.f / (mx + msx(i, j - 1)) / rdy;
+    dydt = dy / dt;
+  }
+  if (cell) {
+    mub = f2(m, WRFGPU_MUB)(i, j); mu_old = f2(m, WRFGPU_MU_1)(i, j);
+    limited = pd_limited(m, i, j);
+    xdiv = pd_xdiv(m, i); ydiv = pd_ydiv(m, j);
+  }
+  // the column's vertical window: scalar at L-1 .. L+2, old scalar at L, L+1, omega of face L+1
+  float fm1 = 0.f, f0 = 0.f, fp1 = 0.f, fp2 = 0.f, fo0 = 0.f, fop1 = 0.f, romp1 = 0.f;
+  float hz0 = 0.f, lz0 = 0.f, hz1 = 0.f, lz1 = 0.f, hzm = 0.f, lzm = 0.f;  // z faces L, L+1, L-1
+  __syncthreads();  // the level table
+  // z face kk (pd_fz) from the scalars around it and the old scalars on its two sides
+  auto zface = [&](int kk, float q_2, float q_1, float q0, float q1, float o_1, float o0, float vel, float* hi, float* lo) {
+    if (kk == 1 || kk == kde) { *hi = 0.f; *lo = 0.f; return; }
+    const float4 a = sLV[kk - kts].a, b = sLV[kk - kts].b;
+    const float mu = 0.5f * ((a.x * mt + a.y) + (a.x * mt + a.y));
+    const float cr = vel * dt / b.z / mu, lf = mu * a.w;
+    const float l = lf * flux_upwind(o_1, o0, cr);
+    float h;
+    if (kk == kts + 1 || kk == ktf) h = vel * (b.x * q0 + b.y * q_1);
+    else h = vel * pflux3(q_2, q_1, q0, q1, -vel);
+    *lo = l; *hi = h - l;
+  };
+  if (cell) {
+    f0 = f(i, L0, j); fp1 = f(i, L0 + 1, j);
+    fp2 = L0 + 2 <= kme ? f(i, L0 + 2, j) : 0.f;
+    fo0 = fo(i, L0, j); fop1 = fo(i, L0 + 1, j);
+    romp1 = rom(i, L0 + 1, j);
+    if (L0 > kts) {
+      fm1 = f(i, L0 - 1, j);
+      zface(L0, L0 - 2 >= kts ? f(i, L0 - 2, j) : 0.f, fm1, f0, fp1, fo(i, L0 - 1, j), fo0, rom(i, L0, j), &hz0, &lz0);
+    }
+  }
+  float sc_m1 = -1.f, sc_0 = -1.f, sc_p1 = -1.f;  // own column's factors at levels L-2, L-1, L
+  auto lim = [](float h, float sc) { return sc >= 0.f ? sc * h : h; };
+  cp_async_wait<2>();
+  __syncthreads();  // level L0 staged
+  for (int L = L0; L <= k1 + 1; ++L) {
+    float4 a = make_float4(0.f, 0.f, 0.f, 0.f);
+    const int fs = (L % P::FSLOT);
+    float *XH = sXH + fs * P::XN, *XL = sXL + fs * P::XN, *YH = sYH + fs * P::YN, *YL = sYL + fs * P::YN;
+    if (L <= ktf) {
+      a = sLV[L - kts].a;
+      const float* Q = ring + (L % P::RING) * 4 * P::HN;
+      const float *FO = Q + P::HN, *RU = FO + P::HN, *RV = RU + P::HN;
+      const float mk = a.x * mt + a.y;
+      if (xok) {  // pd_fx
+        const float mu = 0.5f * (mk + (a.x * mt_x + a.y));
+        const float r = RU[o];
+        float vel = r, cr;
+        if (quirk) { vel = r / mu; cr = vel * dt / dx; }
+        else cr = vel * dt / dx / mu;
+        const float l = (mu * dxdt) * flux_upwind(FO[o - 1], FO[o], cr);
+        float h;
+        if (ox == 5) h = vel * pflux5(Q[o - 3], Q[o - 2], Q[o - 1], Q[o], Q[o + 1], Q[o + 2], vel);
+        else if (ox == 3) h = vel * pflux3(Q[o - 2], Q[o - 1], Q[o], Q[o + 1], vel);
+        else h = 0.5f * r * (Q[o] + Q[o - 1]);
+        XH[xq] = h - l; XL[xq] = l;
+      }
+      if (yok) {  // pd_fy
+        constexpr int W = P::HW;
+        const float mu = 0.5f * (mk + (a.x * mt_y + a.y));
+        const float vel = RV[o], cr = vel * dt / dy / mu;
+        const float l = (mu * dydt) * flux_upwind(FO[o - W], FO[o], cr);
+        float h;
+        if (oy == 5) h = vel * pflux5(Q[o - 3 * W], Q[o - 2 * W], Q[o - W], Q[o], Q[o + W], Q[o + 2 * W], vel);
+        else if (oy == 3) h = vel * pflux3(Q[o - 2 * W], Q[o - W], Q[o], Q[o + W], vel);
+        else h = 0.5f * vel * (Q[o] + Q[o - W]);
+        YH[yq] = h - l; YL[yq] = l;
+      }
+      if (cell) zface(L + 1, fm1, f0, fp1, fp2, fo0, fop1, romp1, &hz1, &lz1);
+    }
+    cp_async_wait<1>();  // this thread's copies of level L + 1
+    __syncthreads();
+    if (L + 3 <= L1) issue(L + 3);  // into the slot of level L - 1, read before this barrier
+    cp_async_commit();
+    // own inputs of the next level, and of the divergence below
+    float fp3 = 0.f, fop2 = 0.f, romp2 = 0.f, t = 0.f;
+    const int k = L - 1;
+    const bool div = own && k >= k0;
+    if (cell) {
+      fp3 = L + 3 <= kme ? f(i, L + 3, j) : 0.f;
+      fop2 = L + 2 <= kme ? fo(i, L + 2, j) : 0.f;
+      romp2 = L + 2 <= kme ? rom(i, L + 2, j) : 0.f;
+    }
+    if (div && accum) t = tend(i, k, j);
+    if (L <= ktf && cell) {  // pd_scale_cell
+      float sc = -1.f;
+      if (limited) {
+        const float hx0 = XH[xq], hx1 = XH[xq + 1], lx0 = XL[xq], lx1 = XL[xq + 1];
+        const float hy0 = YH[yq], hy1 = YH[yq + P::YW], ly0 = YL[yq], ly1 = YL[yq + P::YW];
+        const float ph_low = ((a.x * mub + a.y) + (a.x * mu_old)) * fo0 -
+                             dt * (mx * my * (rdx * (lx1 - lx0) + rdy * (ly1 - ly0)) + my * a.z * (lz1 - lz0));
+        const float flux_out = dt * ((mx * my) * (rdx * (fmaxf_f(0.f, hx1) - fminf_f(0.f, hx0)) +
+                                                  rdy * (fmaxf_f(0.f, hy1) - fminf_f(0.f, hy0))) +
+                                     my * a.z * (fminf_f(0.f, hz1) - fmaxf_f(0.f, hz0)));
+        if (flux_out > ph_low) sc = fmaxf_f(0.f, ph_low / (flux_out + 1.e-20f));
+      }
+      sSC[(L & 1) * P::SN + so] = sc;
+      sc_p1 = sc;
+    }
+    if (div) {  // pd_tend_cell of level k = L - 1
+      const int ks = k % P::FSLOT;
+      const float *kXH = sXH + ks * P::XN, *kXL = sXL + ks * P::XN, *kYH = sYH + ks * P::YN, *kYL = sYL + ks * P::YN;
+      const float* SC = sSC + (k & 1) * P::SN;
+      t = scalar_radiation(m, f, fo, ru, rv, t, i, j, k);
+      float h0 = hzm, h1 = hz0;
+      if (k > 1) { if (h0 < 0.f) h0 = lim(h0, sc_m1); else if (h0 > 0.f) h0 = lim(h0, sc_0); }
+      if (k + 1 < kde) { if (h1 < 0.f) h1 = lim(h1, sc_0); else if (h1 > 0.f) h1 = lim(h1, sc_p1); }
+      t = t - sLV[k - kts].a.z * (h1 - h0 + lz0 - lzm);
+      if (xdiv) {
+        float g0 = kXH[xq], g1 = kXH[xq + 1];
+        if (g0 > 0.f) g0 = lim(g0, SC[so - 1]); else if (g0 < 0.f) g0 = lim(g0, sc_0);
+        if (g1 > 0.f) g1 = lim(g1, sc_0); else if (g1 < 0.f) g1 = lim(g1, SC[so + 1]);
+        t = t - mx * (rdx * (g1 - g0 + kXL[xq + 1] - kXL[xq]));
+      }
+      if (ydiv) {
+        float g0 = kYH[yq], g1 = kYH[yq + P::YW];
+        if (g0 > 0.f) g0 = lim(g0, SC[so - P::SW]); else if (g0 < 0.f) g0 = lim(g0, sc_0);
+        if (g1 > 0.f) g1 = lim(g1, sc_0); else if (g1 < 0.f) g1 = lim(g1, SC[so + P::SW]);
+        t = t - mx * (rdy * (g1 - g0 + kYL[yq + P::YW] - kYL[yq]));
+      }
+      tend(i, k, j) = t;
+    }
+    sc_m1 = sc_0; sc_0 = sc_p1;
+    hzm = hz0; lzm = lz0; hz0 = hz1; lz0 = lz1;
+    fm1 = f0; f0 = fp1; fp1 = fp2; fp2 = fp3;
+    fo0 = fop1; fop1 = fop2; romp1 = romp2;
+  }
+  if (!accum && own) {  // zero_tend of the tile's points that hold no mass
+    for (int k = k0; k <= (k1 == ktf ? m.kte : k1); ++k) {
+      if (k > ktf) tend(i, k, j) = 0.f;
+      if (i == itf && m.ite > itf) tend(i + 1, k, j) = 0.f;
+      if (j == jtf && m.jte > jtf) tend(i, k, j + 1) = 0.f;
+      if (i == itf && m.ite > itf && j == jtf && m.jte > jtf) tend(i + 1, k, j + 1) = 0.f;
+    }
+  }
+}
+// of one member given by value (the caller's arrays; no table on the device)
+__global__ void __launch_bounds__(PdrPlanes::THREADS, 2) k_pd_tend_member(const __grid_constant__ Mem m, int rk_step, bool accum) {
+  const int ntx = tiles_x(m);
+  pd_tile(m, 0, rk_step, accum, m.its + ((int)blockIdx.x % ntx) * TX, m.jts + ((int)blockIdx.x / ntx) * TY);
+}
+__global__ void __launch_bounds__(PdrPlanes::THREADS, 2) k_pd_tend(TileLaunch L, int species, int rk_step, bool accum) {
+  const TilePos tp = tile_pos(L, TILE_ONE);
+  const Mem& m = block_member(L.mem, tp.m);
+  if (species >= m.nsp) return;
+  pd_tile(m, species, rk_step, accum, tp.i0, tp.j0);
 }
 
 // ------------------------------------------------------------ edge strips
@@ -470,9 +699,23 @@ void launch_update_scalar_pd_col(const TileLaunch& L, int nb, StepArgs a, cudaSt
 void launch_advect_scalar(const Launch& L, int nb, StepArgs a, cudaStream_t s) {
   k_advect_scalar<<<nb, dim3(BX, BY), 0, s>>>(L, a.species, a.rk_step, a.flags);
 }
-void launch_advect_scalar_pd2(const Launch& L, int nb, StepArgs a, float* const* d_scratch, cudaStream_t s) {
-  k_pd_scale<<<nb, dim3(BX, BY), 0, s>>>(L, a.species, a.rk_step, a.flags, d_scratch);
-  k_pd_tend<<<nb, dim3(BX, BY), 0, s>>>(L, a.species, a.rk_step, a.flags, d_scratch);
+// Shared memory of pd_tile; the attribute belongs to the current device's
+// context, so it is set at every launch (a table lookup).
+template <typename K>
+static size_t pdr_smem(K kernel, int nlev) {
+  const size_t n = PdrPlanes::FLOATS * 4 + (size_t)nlev * sizeof(PdrLevel);
+  cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)n);
+  return n;
+}
+// a chunk computes two levels more than it writes; two blocks per SM
+void launch_advect_scalar_pd(const TileLaunch& L, int nb, int species, int rk_step, bool accum, cudaStream_t s) {
+  const dim3 grid(nb, level_chunks(nb, L.nlev, 1, 6, 2 * 152));
+  k_pd_tend<<<grid, PdrPlanes::THREADS, pdr_smem(k_pd_tend, L.nlev), s>>>(L, species, rk_step, accum);
+}
+void launch_advect_scalar_pd_member(const Mem& m, int rk_step, bool accum, cudaStream_t s) {
+  const int nb = tiles_x(m) * tiles_y(m), nlev = m.kme - m.kms + 1;
+  const dim3 grid(nb, level_chunks(nb, nlev, 1, 6, 2 * 152));
+  k_pd_tend_member<<<grid, PdrPlanes::THREADS, pdr_smem(k_pd_tend_member, nlev), s>>>(m, rk_step, accum);
 }
 void launch_update_scalar_routine(const Launch& L, int nb, int rk_step, int pd, cudaStream_t s) {
   k_update_scalar_routine<<<nb, dim3(BX, BY), 0, s>>>(L, rk_step, pd);

@@ -111,7 +111,10 @@ void launch_small_step_finish(const Launch& L2, int nblocks, StepArgs a, cudaStr
 // scalars and diagnosis
 void launch_update_scalar_pd(const Launch& L3, int nblocks, StepArgs a, cudaStream_t s);
 void launch_advect_scalar(const Launch& L3, int nblocks, StepArgs a, cudaStream_t s);
-void launch_advect_scalar_pd2(const Launch& L3, int nblocks, StepArgs a, float* const* d_scratch, cudaStream_t s);
+// advect_scalar_pd of one species into advect_tend (accum: added to it), mass
+// tiles; and of species 0 of one member given by value
+void launch_advect_scalar_pd(const TileLaunch& L, int nblocks, int species, int rk_step, bool accum, cudaStream_t s);
+void launch_advect_scalar_pd_member(const Mem& m, int rk_step, bool accum, cudaStream_t s);
 void launch_update_scalar(const Launch& L3, int nblocks, StepArgs a, cudaStream_t s);
 void launch_update_scalar_routine(const Launch& L3, int nblocks, int rk_step, int pd, cudaStream_t s);
 void launch_calc_p_rho_phi(const Launch& L3, int nblocks, cudaStream_t s);

@@ -6,10 +6,11 @@
 // budgeted up front for the resident state, and cudaMalloc / cudaFree would
 // also synchronize the device under its other streams.  The routine-level
 // entry point wrfgpu_advect_scalar_pd copies host arrays into a cached device
-// domain, which it allocates on first use; this variant runs the same two
-// kernels (limiter factors, then the limited flux divergence; k_scalar.cu) on
-// the caller's pointers and keeps the one scratch array they need, the
-// per-cell limiter factor, in a fixed static device array.
+// domain, which it allocates on first use; this variant runs the same kernel
+// (pd_tile, k_scalar.cu) on the caller's pointers, which reach it in the
+// member descriptor, a kernel parameter; the limiter factors stay in shared
+// memory.  One launch, no device state between calls, no host memory read
+// after the call returns.
 //
 // Limits and rules:
 //   * the memory shape (ime-ims+1)(kme-kms+1)(jme-jms+1) may hold at most
@@ -18,100 +19,17 @@
 //   * the options are those a device domain accepts (periodic x, periodic or
 //     symmetric y, 5th/3rd-order advection, ...): anything else returns
 //     WRFGPU_E_ARG before any device work;
-//   * nothing in the static arrays has to start at zero except the block
-//     prefix's first entry, which the one-time setup writes: the factor pass
-//     writes every factor the divergence pass reads, within the same call;
-//   * the first call on a device (and the first after that device's primary
-//     context was replaced, e.g. after cudaDeviceReset) does the setup —
-//     symbol addresses through cudaGetSymbolAddress and one blocking copy —
-//     so it should come before any stream capture; every call then enqueues
-//     two things on the caller's stream: a one-thread kernel that writes the
-//     member descriptor (passed by value as a kernel parameter, so no host
-//     memory is read after the call returns) and the two PD kernels;
-//   * the two PD kernels have no device-side failure (no bounded wait, no
-//     health check): the return code reports argument and launch errors, and
-//     there is no device status word to read back;
-//   * the static arrays are shared: calls that overlap in time (two host
-//     threads, or two streams without ordering between them) race on them.
-//     Serialize calls on one stream or synchronize between them.
+//   * the kernel has no device-side failure (no bounded wait, no health
+//     check): the return code reports argument and launch errors, and there
+//     is no device status word to read back.
 #include <cstring>
-#include <mutex>
-#include <cudaTypedefs.h>
 #include "common.cuh"
 #include "kernels.h"
 #include "fcall.h"
 #include "../../include/wrfgpu_fortran.h"
 
 namespace wrfgpu {
-namespace {
-
-constexpr long long NOALLOC_MAX_POINTS = 8ll * 1024 * 1024;  // 32 MiB of FP32 factors
-
-static __device__ __align__(256) float g_pd_factor[NOALLOC_MAX_POINTS];
-static __device__ __align__(16) Mem g_member;
-static __device__ int g_block_start[2];
-static __device__ float* g_factor_table[1];
-
-constexpr int MAX_DEVICES = 64;
-struct DeviceSetup {
-  bool done = false;
-  CUcontext ctx = nullptr;  // the context the addresses below belong to
-  float* factor = nullptr;
-  Mem* member = nullptr;
-  int* block_start = nullptr;
-  float** factor_table = nullptr;
-};
-static DeviceSetup g_setup[MAX_DEVICES];
-static std::mutex g_setup_mu;
-
-// cuCtxGetCurrent from the driver (no link against libcuda): a device's
-// static arrays move when its primary context is destroyed and re-created.
-static PFN_cuCtxGetCurrent_v4000 g_ctx_current = nullptr;
-static int current_context(CUcontext* ctx) {
-  if (!g_ctx_current) {
-    void* fn = nullptr;
-    cudaDriverEntryPointQueryResult q;
-    if (cudaGetDriverEntryPointByVersion("cuCtxGetCurrent", &fn, 4000, cudaEnableDefault, &q) != cudaSuccess ||
-        q != cudaDriverEntryPointSuccess || !fn)
-      return WRFGPU_E_CUDA;
-    g_ctx_current = (PFN_cuCtxGetCurrent_v4000)fn;
-  }
-  *ctx = nullptr;
-  return g_ctx_current(ctx) == CUDA_SUCCESS && *ctx ? WRFGPU_OK : WRFGPU_E_CUDA;
-}
-
-// Once per device and context, with that device current: the addresses of
-// the static arrays, and the two table entries the kernels read (no
-// allocation).
-int setup_current_device(DeviceSetup** out) {
-  int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= MAX_DEVICES) return WRFGPU_E_CUDA;
-  // make the device's primary context current (initialised if need be)
-  if (cudaSetDevice(dev) != cudaSuccess) return WRFGPU_E_CUDA;
-  CUcontext ctx = nullptr;
-  if (current_context(&ctx)) return WRFGPU_E_CUDA;
-  std::lock_guard<std::mutex> lock(g_setup_mu);
-  DeviceSetup& s = g_setup[dev];
-  if (!s.done || s.ctx != ctx) {
-    s.done = false;
-    if (cudaGetSymbolAddress((void**)&s.factor, g_pd_factor) != cudaSuccess) return WRFGPU_E_CUDA;
-    if (cudaGetSymbolAddress((void**)&s.member, g_member) != cudaSuccess) return WRFGPU_E_CUDA;
-    if (cudaGetSymbolAddress((void**)&s.block_start, g_block_start) != cudaSuccess) return WRFGPU_E_CUDA;
-    if (cudaGetSymbolAddress((void**)&s.factor_table, g_factor_table) != cudaSuccess) return WRFGPU_E_CUDA;
-    if (cudaMemcpyToSymbol(g_factor_table, &s.factor, sizeof(float*)) != cudaSuccess) return WRFGPU_E_CUDA;
-    const int zero = 0;
-    if (cudaMemcpyToSymbol(g_block_start, &zero, sizeof(int)) != cudaSuccess) return WRFGPU_E_CUDA;
-    s.ctx = ctx;
-    s.done = true;
-  }
-  *out = &s;
-  return WRFGPU_OK;
-}
-
-// The member descriptor, written on the stream from a kernel parameter.
-__global__ void k_noalloc_set_member(Mem M, Mem* dst) { *dst = M; }
-
-}  // namespace
+constexpr long long NOALLOC_MAX_POINTS = 8ll * 1024 * 1024;
 }  // namespace wrfgpu
 
 using namespace wrfgpu;
@@ -147,10 +65,6 @@ extern "C" int wrfgpu_advect_scalar_pd_noalloc(
     if (check_desc(d)) return WRFGPU_E_ARG;
   }
 
-  DeviceSetup* s = nullptr;
-  int rc = setup_current_device(&s);
-  if (rc) return rc;
-
   Mem M;
   std::memset(&M, 0, sizeof(Mem));
   M.ids = *ids; M.ide = *ide; M.jds = *jds; M.jde = *jde; M.kds = *kds; M.kde = *kde;
@@ -178,17 +92,11 @@ extern "C" int wrfgpu_advect_scalar_pd_noalloc(
   M.dt = *dt; M.dtrk_fix = *dt;
   M.rdx = *rdx; M.rdy = *rdy;
   M.cf = *config_flags;
-  M.err = nullptr;  // the PD kernels raise no device status
+  M.err = nullptr;  // the PD kernel raises no device status
 
-  cudaStream_t st = (cudaStream_t)stream;
-  k_noalloc_set_member<<<1, 1, 0, st>>>(M, s->member);
-  if (cudaGetLastError() != cudaSuccess) return WRFGPU_E_CUDA;
-  const int nb = blocks_for(M.ims, M.ime, M.jms, M.jme, (int)nk, 3);
-  const Launch L{s->member, s->block_start, 1, 3};
-  // rk_step 3 (the last stage, where the reference applies the PD scheme);
-  // flags 2 | 4: limiter on regardless of the configuration's scheme, and
-  // the tendency accumulates into the caller's array, as advect_scalar_pd does
-  launch_advect_scalar_pd2(L, nb, StepArgs{3, 0, 0, 6}, s->factor_table, st);
+  // rk_step 3: the last stage, where the reference applies the PD scheme; the
+  // tendency accumulates into the caller's array, as advect_scalar_pd does
+  launch_advect_scalar_pd_member(M, 3, true, (cudaStream_t)stream);
   if (cudaGetLastError() != cudaSuccess) return WRFGPU_E_CUDA;
   return WRFGPU_OK;
 }
