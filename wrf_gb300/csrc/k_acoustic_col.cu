@@ -234,7 +234,10 @@ void launch_advance_uv_col(const TileLaunch& L, int nblocks, int rk_step, int it
 // ---------------------------------------------------------------------------
 // advance_mu_t (module_small_step_em.F:969-1175), one thread per mass column:
 // pass 1 the column divergence (kept per level) and its sum, then mu, and
-// pass 2 omega by upward recursion, theta and sumflux's sum of ww_m (:1473-1633).
+// pass 2 omega by upward recursion, theta, sumflux's sum of ww_m (:1473-1633)
+// and advance_w's t_2ave, whose inputs are at hand here (the old and new
+// theta, the column masses): advance_w then reads one array instead of three
+// and writes none of them back.
 // RC: accumulation type of the column sum and the recursion (float: the
 // reference; double: mixed form).
 // ---------------------------------------------------------------------------
@@ -289,7 +292,8 @@ __global__ void __launch_bounds__(TX* TY, MINB) k_advance_mu_t_col(TileLaunch L,
   MassImages img;
   img.init(m, i, j);
   img.store([&](int ii, int jj) { MU(ii, jj) = mu; MUDF(ii, jj) = mudf; MUTS(ii, jj) = muts; });
-  MUAVE(i, j) = .5f * ((1.f + epssm) * mu + (1.f - epssm) * muave);
+  const float mua = .5f * ((1.f + epssm) * mu + (1.f - epssm) * muave);
+  MUAVE(i, j) = mua;
   const float my = msfty.ro(i, j), mx = msftx.ro(i, j);
   const RC rmy = rcp_rc<RC>((RC)my);  // mixed form only
   // pass 2: omega (recursion one level ahead of theta) and theta
@@ -332,7 +336,6 @@ __global__ void __launch_bounds__(TX* TY, MINB) k_advance_mu_t_col(TileLaunch L,
     }
     // theta of level k
     const float tv = cur.t;
-    t_ave(i, k, j) = tv;
     float tt = tv + my * dts * cur.ft;
     const float wdtn_hi = (k + 1 == kde) ? 0.f : wwf_kp1 * (fnm(k + 1) * (k + 1 <= k_end ? nxt.t1 : 0.f) + fnp(k + 1) * cur.t1);
     tt = tt - dts * my *
@@ -340,6 +343,9 @@ __global__ void __launch_bounds__(TX* TY, MINB) k_advance_mu_t_col(TileLaunch L,
                          .5f * rdx * (cur.u1 * (cur.t1xp + cur.t1) - cur.u0 * (cur.t1 + cur.t1xm))) +
                    rdnw(k) * (wdtn_hi - wdtn_lo));
     t(i, k, j) = tt;
+    float tav = .5f * ((1.f + epssm) * tt + (1.f - epssm) * tv);
+    tav = (tav + (c1h(k) * mua) * T0) / ((c1h(k) * muts + c2h(k)) * (T0 + cur.t1));
+    t_ave(i, k, j) = tav;
     wdtn_lo = wdtn_hi;
     wwf_k = wwf_kp1;
     cur = nxt;
@@ -353,7 +359,7 @@ __global__ void __launch_bounds__(TX* TY, MINB) k_advance_mu_t_col(TileLaunch L,
 
 // ---------------------------------------------------------------------------
 // advance_w (module_small_step_em.F:1178-1469), one thread per mass column.
-// Upward pass: at level L, t_2ave(L), the raw right-hand side of L+1, the
+// Upward pass: at level L, the raw right-hand side of L+1, the
 // omega advection term that completes rhs(L), and the explicit w and forward
 // elimination of level L-1 (which needs rhs(L)); everything the elimination
 // reads from neighbouring levels sits in register windows.  Downward pass:
@@ -362,22 +368,21 @@ __global__ void __launch_bounds__(TX* TY, MINB) k_advance_mu_t_col(TileLaunch L,
 // ---------------------------------------------------------------------------
 // Level inputs of advance_w staged by TMA: plane index of each field in a
 // ring slot (the FP64 a / alpha of the mixed form are read from global
-// memory instead, so that form stages the first 13).
-enum AwPlane { AW_T2 = 0, AW_T2A, AW_T1, AW_PH, AW_W, AW_RWT, AW_CQW, AW_C2A, AW_ALT, AW_PHT, AW_WW, AW_PH1, AW_PHB,
+// memory instead, so that form stages the first 11).
+enum AwPlane { AW_TA = 0, AW_PH, AW_W, AW_RWT, AW_CQW, AW_C2A, AW_ALT, AW_PHT, AW_WW, AW_PH1, AW_PHB,
                AW_A, AW_AL, AW_NPLANE };
-// Ring depth: levels L, L+1 resident and L+2, L+3 in flight; at four
-// blocks per SM (which the shared memory of four slots does not allow) only
-// L+2 is in flight.
-template <typename RC, int NSLOT> struct AwCfg {
+// Ring depth: levels L, L+1 resident and L+2, L+3 in flight (52 KB: four
+// blocks per SM fit).
+constexpr int AW_RING = 4;
+template <typename RC> struct AwCfg {
   static constexpr int NF = sizeof(RC) == 8 ? AW_A : AW_NPLANE;
-  using Ring = TileRing<NF, NSLOT>;
+  using Ring = TileRing<NF, AW_RING>;
 };
 
 template <typename RC, int MINB, bool DAMP>
 __global__ void __launch_bounds__(TX* TY, MINB) k_advance_w_col(TileLaunch L, int rk_step, int iteration) {
-  constexpr int AW_RING = MINB >= 4 ? 3 : 4;
-  using Ring = typename AwCfg<RC, AW_RING>::Ring;
-  constexpr int NF = AwCfg<RC, AW_RING>::NF;
+  using Ring = typename AwCfg<RC>::Ring;
+  constexpr int NF = AwCfg<RC>::NF;
   extern __shared__ __align__(128) unsigned char smem[];
   const TilePos tp = tile_pos(L, false, false);
   const Mem& m = block_member(L.mem, tp.m);
@@ -396,7 +401,7 @@ __global__ void __launch_bounds__(TX* TY, MINB) k_advance_w_col(TileLaunch L, in
   Ring ring;
   ring.init(smem, 1);
   {
-    const int ids[AW_NPLANE] = {WRFGPU_T_2, WRFGPU_T_2SAVE, WRFGPU_T_SAVE, WRFGPU_PH_2, WRFGPU_W_2, WRFGPU_RW_TEND,
+    const int ids[AW_NPLANE] = {WRFGPU_T_2SAVE, WRFGPU_PH_2, WRFGPU_W_2, WRFGPU_RW_TEND,
                                 WRFGPU_CQW, WRFGPU_C2A, WRFGPU_ALT, WRFGPU_PH_TEND, WRFGPU_WW, WRFGPU_PH_SAVE,
                                 WRFGPU_PHB, WRFGPU_A, WRFGPU_ALPHA};
     const CUtensorMap* maps[NF];
@@ -411,7 +416,7 @@ __global__ void __launch_bounds__(TX* TY, MINB) k_advance_w_col(TileLaunch L, in
       for (int k = 1; k <= min(AW_RING - 1, kde); ++k) ring.issue(k, maps, x0, z0, m.kms);
     bool ok = true;
 
-    F3 w = f3(m, WRFGPU_W_2), t_2ave = f3(m, WRFGPU_T_2SAVE), ph = f3(m, WRFGPU_PH_2), u = f3(m, WRFGPU_U_2),
+    F3 w = f3(m, WRFGPU_W_2), ph = f3(m, WRFGPU_PH_2), u = f3(m, WRFGPU_U_2),
        v = f3(m, WRFGPU_V_2);
     F2 ht = f2(m, WRFGPU_HT), msftx = f2(m, WRFGPU_MSFTX), msfty = f2(m, WRFGPU_MSFTY);
     F1 c1h = f1(m, WRFGPU_C1H), c2h = f1(m, WRFGPU_C2H), c1f = f1(m, WRFGPU_C1F), c2f = f1(m, WRFGPU_C2F),
@@ -482,16 +487,12 @@ __global__ void __launch_bounds__(TX* TY, MINB) k_advance_w_col(TileLaunch L, in
       __syncthreads();  // level Lk-1's slot is free
       if (tid == 0 && Lk + AW_RING - 1 <= kde) ring.issue(Lk + AW_RING - 1, maps, x0, z0, m.kms);
       ok = ring.wait(Lk + 1) && ok;
-      const float c_t2 = P(Lk, AW_T2), c_t2a = P(Lk, AW_T2A), c_t1 = P(Lk, AW_T1), c_ph = P(Lk, AW_PH);
+      const float tav = P(Lk, AW_TA), c_ph = P(Lk, AW_PH);
       const float c_w = P(Lk, AW_W), c_rwt = P(Lk, AW_RWT), c_cqw = P(Lk, AW_CQW), c_c2a = P(Lk, AW_C2A),
                   c_alt = P(Lk, AW_ALT);
       const RC c_a = Acoef(Lk), c_al = ALcoef(Lk);
       const float c_pht1 = P(Lk + 1, AW_PHT), c_w1 = P(Lk + 1, AW_W), c_ww1 = P(Lk + 1, AW_WW),
                   c_ph11 = P(Lk + 1, AW_PH1), c_phb1 = P(Lk + 1, AW_PHB);
-      // t_2ave(L)
-      float tav = .5f * ((1.f + epssm) * c_t2 + (1.f - epssm) * c_t2a);
-      tav = (tav + (c1h(Lk) * mua) * T0) / ((c1h(Lk) * mts + c2h(Lk)) * (T0 + c_t1));
-      if (act) t_2ave(i, Lk, j) = tav;
       // raw rhs(L+1), wdwn(L+1)
       const float rr_next = dts * (c_pht1 + .5f * G * (1.f - epssm) * c_w1);
       float wd_hi;
@@ -626,25 +627,24 @@ template <bool DAMP>
 static void launch_advance_w_var(const TileLaunch& L, int nblocks, int rk_step, int iteration, bool fp64,
                                  cudaStream_t s, int minb) {
   static bool attr = false;
-  constexpr size_t S32 = AwCfg<float, 4>::Ring::SMEM, S64 = AwCfg<double, 4>::Ring::SMEM;
-  constexpr size_t S32_3 = AwCfg<float, 3>::Ring::SMEM, S64_3 = AwCfg<double, 3>::Ring::SMEM;
+  constexpr size_t S32 = AwCfg<float>::Ring::SMEM, S64 = AwCfg<double>::Ring::SMEM;
   if (!attr) {
     cudaFuncSetAttribute(k_advance_w_col<float, 2, DAMP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S32);
     cudaFuncSetAttribute(k_advance_w_col<float, 3, DAMP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S32);
-    cudaFuncSetAttribute(k_advance_w_col<float, 4, DAMP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S32_3);
+    cudaFuncSetAttribute(k_advance_w_col<float, 4, DAMP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S32);
     cudaFuncSetAttribute(k_advance_w_col<double, 2, DAMP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S64);
     cudaFuncSetAttribute(k_advance_w_col<double, 3, DAMP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S64);
-    cudaFuncSetAttribute(k_advance_w_col<double, 4, DAMP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S64_3);
+    cudaFuncSetAttribute(k_advance_w_col<double, 4, DAMP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S64);
     attr = true;
   }
   if (fp64) {
     if (minb == 2) k_advance_w_col<double, 2, DAMP><<<nblocks, dim3(TX, TY), S64, s>>>(L, rk_step, iteration);
     else if (minb == 3) k_advance_w_col<double, 3, DAMP><<<nblocks, dim3(TX, TY), S64, s>>>(L, rk_step, iteration);
-    else k_advance_w_col<double, 4, DAMP><<<nblocks, dim3(TX, TY), S64_3, s>>>(L, rk_step, iteration);
+    else k_advance_w_col<double, 4, DAMP><<<nblocks, dim3(TX, TY), S64, s>>>(L, rk_step, iteration);
   } else {
     if (minb == 2) k_advance_w_col<float, 2, DAMP><<<nblocks, dim3(TX, TY), S32, s>>>(L, rk_step, iteration);
     else if (minb == 3) k_advance_w_col<float, 3, DAMP><<<nblocks, dim3(TX, TY), S32, s>>>(L, rk_step, iteration);
-    else k_advance_w_col<float, 4, DAMP><<<nblocks, dim3(TX, TY), S32_3, s>>>(L, rk_step, iteration);
+    else k_advance_w_col<float, 4, DAMP><<<nblocks, dim3(TX, TY), S32, s>>>(L, rk_step, iteration);
   }
 }
 void launch_advance_w_col(const TileLaunch& L, int nblocks, int rk_step, int iteration, bool fp64, cudaStream_t s,
