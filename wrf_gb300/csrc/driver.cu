@@ -141,6 +141,7 @@ struct Ensemble {
   bool col_step = false;  // the acoustic step's mass columns go through k_advance_col (col_max_segments)
   bool damp3 = false;  // some member uses damp_opt = 3
   bool diff6 = false;  // some member stores diffusion tendencies (diff_6th_opt != 0 or diff_opt = 1)
+  bool any_pd = false, all_pd = true;  // some / every species takes the positive-definite scheme at the last stage
   bool damp2 = false;  // some member uses damp_opt = 2 (Rayleigh damping toward the base state)
   std::vector<size_t> n3, n2, n1;      // element counts per member (padded rows)
   std::vector<size_t> ni_, nk_, nj_, pitch_;  // Fortran extents and the padded row pitch
@@ -174,6 +175,27 @@ struct Ensemble {
     cudaEventCreate(&e);
     cudaEventRecord(e, stream);
     prof->push_back({ph, e});
+  }
+
+  // Side branches of a step: kernels that neither read nor write one another's
+  // fields run beside the main stream's and are joined before their results
+  // are used.  A narrow domain's kernels leave most SMs idle, so the step's
+  // length is its longest chain of launches; a wide one gains only the tails.
+  // Not while profiling (the phase marks time the main stream).
+  static constexpr int NSIDE = 3;
+  cudaStream_t side[NSIDE] = {nullptr, nullptr, nullptr};
+  cudaEvent_t ev_side[NSIDE] = {nullptr, nullptr, nullptr}, ev_sfork = nullptr;
+  // the stream of branch b from here on (the main one while profiling)
+  cudaStream_t fork(int b) {
+    if (prof) return stream;
+    cudaEventRecord(ev_sfork, stream);
+    cudaStreamWaitEvent(side[b], ev_sfork, 0);
+    return side[b];
+  }
+  void join(int b) {
+    if (prof) return;
+    cudaEventRecord(ev_side[b], side[b]);
+    cudaStreamWaitEvent(stream, ev_side[b], 0);
   }
 
   Launch L2() const { return Launch{d_mems, d_bs2, nmem, 2, nlev_max}; }
@@ -652,6 +674,11 @@ struct Ensemble {
     if (d_cfl) cudaFree(d_cfl);
     if (ev0) cudaEventDestroy(ev0);
     if (ev1) cudaEventDestroy(ev1);
+    for (int b = 0; b < NSIDE; ++b) {
+      if (side[b]) cudaStreamDestroy(side[b]);
+      if (ev_side[b]) cudaEventDestroy(ev_side[b]);
+    }
+    if (ev_sfork) cudaEventDestroy(ev_sfork);
     if (stream) cudaStreamDestroy(stream);
   }
 
@@ -668,6 +695,11 @@ struct Ensemble {
     CK(cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking));
     CK(cudaEventCreate(&ev0));
     CK(cudaEventCreate(&ev1));
+    for (int b = 0; b < NSIDE; ++b) {
+      CK(cudaStreamCreateWithFlags(&side[b], cudaStreamNonBlocking));
+      CK(cudaEventCreateWithFlags(&ev_side[b], cudaEventDisableTiming));
+    }
+    CK(cudaEventCreateWithFlags(&ev_sfork, cudaEventDisableTiming));
     hm.resize(n); n3.resize(n); n2.resize(n); n1.resize(n);
     ni_.resize(n); nk_.resize(n); nj_.resize(n); pitch_.resize(n);
     // sizes
@@ -750,6 +782,11 @@ struct Ensemble {
       damp3 = damp3 || M.cf.damp_opt == 3;
       diff6 = diff6 || M.cf.diff_6th_opt != 0 || M.cf.diff_opt == 1;
       damp2 = damp2 || M.cf.damp_opt == 2;
+      for (int sp = 0; sp < M.nsp; ++sp) {
+        const bool pd = M.cf.rk_ord == 3 && (sp < M.n_moist ? M.cf.moist_adv_opt : M.cf.scalar_adv_opt) == 1;
+        any_pd = any_pd || pd;
+        all_pd = all_pd && pd;
+      }
       bs2[m + 1] = bs2[m] + blocks_for(M.ims, M.ime, M.jms, M.jme, M.kme - M.kms + 1, 2);
       bs3[m + 1] = bs3[m] + blocks_for(M.ims, M.ime, M.jms, M.jme, M.kme - M.kms + 1, 3);
       bpr[m + 1] = bpr[m] + tiles_x(M) * tiles_y(M) * blocks_per_tile(M.nsp, TILE_PER_PAIR);
@@ -875,13 +912,14 @@ struct Ensemble {
     void f2(int id, char var) { HaloJob j{id, 2, -1, 0, var, {0, 0, 0}}; v.push_back(j); }
     void sp(int s, int old, char var) { HaloJob j{0, 3, s, old, var, {0, 0, 0}}; v.push_back(j); }
   };
-  void fill(const JobList& jl) {
+  void fill(const JobList& jl) { fill(jl, stream); }
+  void fill(const JobList& jl, cudaStream_t st) {
     mark(PH_FILL);
     for (size_t b = 0; b < jl.v.size(); b += MAX_HALO_JOBS) {
       HaloJobs hj;
       hj.n = (int)std::min(jl.v.size() - b, (size_t)MAX_HALO_JOBS);
       for (int q = 0; q < hj.n; ++q) hj.job[q] = jl.v[b + q];
-      launch_fill_halo(d_mems, nmem, hj, halo_blocks, stream);
+      launch_fill_halo(d_mems, nmem, hj, halo_blocks, st);
     }
   }
 
@@ -902,29 +940,40 @@ struct Ensemble {
         j.f3(WRFGPU_AL, 'p'); j.f3(WRFGPU_PH_2, 'w');
         fill(j);
       }
-      // rk_tendency (module_em.F:370-781)
-      mark(PH_TEND_U); launch_tend_u_col(LST(), nb_st, TF_ALL, stream, tune[TU_TENDU]);
-      mark(PH_TEND_V); launch_tend_v_col(LST(), nb_st, TF_ALL, stream, tune[TU_TENDV]);
+      // rk_tendency (module_em.F:370-781): five independent tendencies
+      const cudaStream_t sw = fork(0), sp = fork(1);
+      const bool fdiff = rk_step == 1 && (diff6 || damp2);  // module_em.F:801-944 (stage 1), into arrays of its own
+      if (fdiff) {
+        const cudaStream_t sd = fork(2);
+        mark(PH_DIFF);
+        if (diff6) launch_forward_diff(l3, nb3, 0, sd);
+        if (damp2) launch_rayleigh_damp(l2, nb2, sd);
+      }
       mark(PH_TEND_W);
       // open boundaries: rw_tend next to them from the cqw the tile kernel overwrites
-      if (any_open) launch_strip_tend_w(LS3(), nb_s3, stream);
-      launch_tend_w_col(LST(), nb_st, tune[TU_TENDW], stream);
-      mark(PH_TEND_T); launch_tend_t_col(LST(), nb_st, TF_ZERO | TF_ADV, stream);
-      mark(PH_TEND_PH); launch_tend_ph_col(LST(), nb_st, TF_ZERO | TF_ADV, stream);
+      if (any_open) launch_strip_tend_w(LS3(), nb_s3, sw);
+      launch_tend_w_col(LST(), nb_st, tune[TU_TENDW], sw);
+      if (cfl_check) { mark(PH_CFL); launch_cfl_check_col(LTM(), nb_tm, sw, tune[TU_CFL]); }
+      mark(PH_TEND_T); launch_tend_t_col(LST(), nb_st, TF_ZERO | TF_ADV, sp);
+      mark(PH_TEND_PH); launch_tend_ph_col(LST(), nb_st, TF_ZERO | TF_ADV, sp);
+      mark(PH_TEND_U); launch_tend_u_col(LST(), nb_st, TF_ALL, stream, tune[TU_TENDU]);
+      mark(PH_TEND_V); launch_tend_v_col(LST(), nb_st, TF_ALL, stream, tune[TU_TENDV]);
+      join(0);
+      join(1);
       // open boundaries: the lower-order fluxes and radiation terms next to them
-      if (any_open) launch_strip_tend(LS3(), nb_s3, stream);
-      if (diff6 || damp2) {  // module_em.F:801-944 (stage 1), then rk_addtend_dry (solve_em.F:967)
+      if (any_open) { mark(PH_TEND_PH); launch_strip_tend(LS3(), nb_s3, stream); }
+      if (fdiff) join(2);
+      if (diff6 || damp2) {  // rk_addtend_dry (solve_em.F:967)
         mark(PH_DIFF);
-        if (rk_step == 1 && diff6) launch_forward_diff(l3, nb3, 0, stream);
-        if (rk_step == 1 && damp2) launch_rayleigh_damp(l2, nb2, stream);
         launch_addtend_dry(l3, nb3, stream);
       }
-      if (cfl_check) { mark(PH_CFL); launch_cfl_check_col(LTM(), nb_tm, stream, tune[TU_CFL]); }
       // small_step_prep, calc_p_rho(step 0), calc_coef_w (solve_em.F:1089-1140)
       mark(PH_SSP); launch_small_step_prep(l2, nb2, LST(), nb_st, a, stream, tune[TU_SSP]);
+      const cudaStream_t sc = fork(0);  // the acoustic steps' coefficients beside p and the halo fill
+      mark(PH_COEFW);
+      if (!fp64 && nb_rw <= COEF_ROW_MAX) launch_calc_coef_w_row(LRW(), nb_rw, a, sc);
+      else launch_calc_coef_w_col(LTM(), nb_tm, a, fp64, sc);
       mark(PH_CPR0); launch_calc_p_rho_col(LTM(), nb_tm, StepArgs{rk_step, 0, 0, 0}, stream);
-      mark(PH_COEFW); if (!fp64 && nb_rw <= COEF_ROW_MAX) launch_calc_coef_w_row(LRW(), nb_rw, a, stream);
-      else launch_calc_coef_w_col(LTM(), nb_tm, a, fp64, stream);
       {  // solve_em.F:1176-1264
         JobList j;
         j.f3(WRFGPU_RU_TEND, 'u'); j.f3(WRFGPU_RV_TEND, 'v'); j.f3(WRFGPU_PH_2, 'w'); j.f3(WRFGPU_AL, 'p');
@@ -932,6 +981,7 @@ struct Ensemble {
         j.f2(WRFGPU_MU_1, 't'); j.f2(WRFGPU_MU_2, 't'); j.f2(WRFGPU_MUDF, 't');
         fill(j);
       }
+      join(0);
       int nsmall_max = 0;
       for (int m = 0; m < nmem; ++m) nsmall_max = std::max(nsmall_max, stage_of(hm[m], rk_step).nsmall);
       for (int it = 1; it <= nsmall_max; ++it) {
@@ -956,6 +1006,15 @@ struct Ensemble {
           fill(j);
         }
       }
+      if (rk_step == 3) {
+        // the PD pre-update of the old species (solve_em.F:1770-1790) and their
+        // halos: first read by the PD transport
+        const cudaStream_t su = fork(0);
+        if (any_pd) { mark(PH_USPD); launch_update_scalar_pd_col(LTM(), nb_tm, a, su, diff6); }
+        JobList jo;
+        for (int s = 0; s < nsp_max; ++s) jo.sp(s, 1, 'p');
+        fill(jo, su);
+      }
       mark(PH_SSF); launch_small_step_finish(l2, nb2, a, stream, tune[TU_SSF]);
       if (rk_step == 3) {
         // solve_em.F:1754-1800, and the end-of-step fills of the _2 dry state
@@ -973,10 +1032,7 @@ struct Ensemble {
         fill(j);
         mark(PH_WSURF); launch_set_w_surface(l2, nb2, stream);
         io_dry_out();
-        mark(PH_USPD); launch_update_scalar_pd_col(LTM(), nb_tm, a, stream, diff6);
-        JobList jo;
-        for (int s = 0; s < nsp_max; ++s) jo.sp(s, 1, 'p');
-        fill(jo);
+        join(0);
       }
       // scalar loop (solve_em.F:1815-2160): rk_scalar_tend + rk_update_scalar of every
       // species, fused; the positive-definite scheme at the last stage
@@ -990,9 +1046,11 @@ struct Ensemble {
       } else {
         io_join();  // passive scalars copied in by a host I/O step are read from here on
         if (diff6 && rk_step == 1) { mark(PH_DIFF); launch_forward_diff(l3, nb3, 1, stream); }  // module_em.F:1378-1435
-        mark(PH_ADVS); launch_scalar_adv_update(LP(), nb_pr, rk_step, stream, tune[TU_ADV], diff6);
+        if (rk_step < 3 || !all_pd) {
+          mark(PH_ADVS); launch_scalar_adv_update(LP(), nb_pr, rk_step, stream, tune[TU_ADV], diff6);
+        }
       }
-      if (rk_step == 3) {
+      if (rk_step == 3 && any_pd) {
         mark(PH_PD);
         launch_pd_courant(l2, nb2, rk_step, stream);
         launch_scalar_pd_update(LP(), nb_pr, nlev_max, rk_step, stream, tune[TU_PD]);
