@@ -804,7 +804,7 @@ struct Ensemble {
       bs_s5[m + 1] = bs_s5[m] + strip_blocks(STRIP_W_PD + 1, 1);
     }
     nb2 = bs2[n]; nb3 = bs3[n]; nb_st = bst[n]; nb_tm = btm[n]; nb_pr = bpr[n]; nb_rw = brw[n]; nb_rs = brs[n];
-    col_step = nb_rw <= col_max_segments(fp64, damp3);
+    col_step = nb_rw <= col_max_segments(fp64);
     if (fp64) tune[TU_AMUT] = 1;  // three blocks per SM (kernels.h)
     nb_s3 = bs_s3[n]; nb_s4 = bs_s4[n]; nb_s5 = bs_s5[n];
     {  // tensor maps of every 3-D buffer: halo and tile boxes

@@ -198,12 +198,18 @@ FFM_HD ff ff_exp_t(ff z, int* k) {
 
 // Ziv's rounding test for a normalised float-float v = hi + lo (|lo| <= ulp(hi)/2)
 // known to relative accuracy 1e-13 or better: hi is the correctly rounded value unless
-// |lo| lies within 1e-12 |hi| of half an ulp of hi, or hi is a power of two.
+// |lo| lies within 1e-12 |hi| of half an ulp of hi.  Below a power of two the
+// floats are twice as dense, so there a lo toward zero has half that room
+// (the sine of the damping layer's top, sin(pi/2) = 1 - 1e-15, is such a value).
+// Half an ulp comes from hi's exponent field (|hi| >= 2^-100; smaller ones do not pass).
 FFM_HD bool rounds_safely(ff v) {
-  int e;
-  const float m = frexpf_(fabsf(v.hi), &e);
-  if (m == 0.5f) return false;
-  const float half_ulp = ldexpf_(1.f, e - 25);
+  const uint32_t b = f2u(v.hi) & 0x7FFFFFFFu;
+  if (b < (27u << 23)) return false;
+  const float half_ulp = u2f((b & 0x7F800000u) - (24u << 23));
+  if ((b & 0x007FFFFFu) == 0u) {
+    const bool inward = (v.lo < 0.f) == (v.hi > 0.f);
+    return fabsf(v.lo) < (inward ? 0.5f * half_ulp : half_ulp) - 1e-12f * fabsf(v.hi);
+  }
   return fabsf(fabsf(v.lo) - half_ulp) > 1e-12f * fabsf(v.hi);
 }
 
@@ -230,7 +236,7 @@ FFM_HD float powf_cr(float x, float y) {
       int k = 0;
       ff v = ff_exp_t(z, &k);
       v = fast_two_sum(v.hi, v.lo);
-      if (k > -120 && k < 120 && rounds_safely(v)) return ldexpf_(v.hi, k);
+      if (k > -120 && k < 120 && rounds_safely(v)) return v.hi * u2f((uint32_t)(k + 127) << 23);  // exact
     }
   }
   return (float)::pow((double)x, (double)y);
@@ -277,13 +283,44 @@ FFM_HD dd sin_dd_small(double x) {
   return sum;
 }
 
-// sin(x) for |x| <= 2, correctly rounded to float.  Fast path: the FP64 sine
-// (libm on the host, CUDA's double sin on the device; both within 2 ulp of
-// FP64) rounded once, accepted when it lies farther than 2^-45 of its value
-// from a float rounding boundary; otherwise the double-double series decides
-// (the same code on host and device).  Used by the w Rayleigh damping of
-// advance_w (damp_opt = 3), whose argument lies in [0, pi/2].
+// sin x for a float 0 <= x <= 1.6 as a float pair: the Taylor series to
+// x^19/19!, the terms through x^11 in float-float, the rest (below 4e-8 of
+// the sum) in float.  Relative error below 1e-13.
+FFM_HD ff ff_sin_t(float x) {
+  // 1/n! split into two floats
+  constexpr double R3 = -1. / 6., R5 = 1. / 120., R7 = -1. / 5040., R9 = 1. / 362880., R11 = -1. / 39916800.;
+  constexpr double R13 = 1. / 6227020800., R15 = -1. / 1307674368000., R17 = 1. / 355687428096000.,
+                   R19 = -1. / 121645100408832000.;
+#define WRFGPU_FF(r) ff{(float)(r), (float)((r) - (double)(float)(r))}
+  const ff x2 = two_prod(x, x);
+  const float y = x2.hi;
+  const float t = (float)R13 + y * ((float)R15 + y * ((float)R17 + y * (float)R19));
+  ff v = ff_addf(WRFGPU_FF(R11), y * t);
+  v = ff_add(WRFGPU_FF(R9), ff_mul(x2, v));
+  v = ff_add(WRFGPU_FF(R7), ff_mul(x2, v));
+  v = ff_add(WRFGPU_FF(R5), ff_mul(x2, v));
+  v = ff_add(WRFGPU_FF(R3), ff_mul(x2, v));
+#undef WRFGPU_FF
+  const ff w = ff_mulf(ff_mul(x2, v), x);
+  const ff s = fast_two_sum(x, w.hi);
+  return fast_two_sum(s.hi, s.lo + w.lo);
+}
+
+// sin(x) for |x| <= 2, correctly rounded to float.  Fast path for [0, 1.6]: the
+// float-float series with Ziv's rounding test (FP64 runs at 1/64 of the FP32
+// rate here, and at the damping layer's top the sine's distance to 1 sent every
+// column through the double-double series: the damped column kernel of the
+// acoustic step took 1.88 ms per large step of 160x144x64, now 0.76).  Then the FP64 sine (libm on the host, CUDA's double sin on
+// the device; both within 2 ulp of FP64) rounded once, accepted when it lies
+// farther than 2^-45 of its value from a float rounding boundary; otherwise
+// the double-double series decides (the same code on host and device).  Used
+// by the w Rayleigh damping of advance_w (damp_opt = 3), whose argument lies
+// in [0, pi/2].
 FFM_HD float sinf_cr(float x) {
+  if (x >= 0x1p-30f && x <= 1.6f) {
+    const ff v = ff_sin_t(x);
+    if (rounds_safely(v)) return v.hi;
+  }
   const double d = (double)x;
   const double s = ::sin(d);
   const float f = (float)s;

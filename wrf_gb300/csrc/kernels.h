@@ -159,9 +159,8 @@ void launch_advance_uv_col(const TileLaunch& L, int nblocks, int rk_step, int it
 // (about 2900) 2.23 / 2.30, 512x512x80 (8192) 6.30 / 5.67, 1024x1024x96 (32768)
 // 29.0 / 24.9; FP64 columns (whose chains wait about 110 cycles per operation)
 // 75x90x128 (270) 1.12 / 3.11, 16 members of up to 256x256x80 (about 14000)
-// 17.5 / 9.3; with damp_opt = 3 (whose FP64 sine sits in few of the block's warps)
-// 160x144x64 (720) 1.88 / 1.82.
-constexpr int col_max_segments(bool fp64, bool damp) { return damp ? 500 : fp64 ? 1000 : 3000; }
+// 17.5 / 9.3; with damp_opt = 3 160x144x64 (720) 0.76 / 1.39.
+constexpr int col_max_segments(bool fp64) { return fp64 ? 1000 : 3000; }
 // damp: some member uses damp_opt = 3 (compiles the damping into the kernel)
 void launch_advance_col(const TileLaunch& L, int nblocks, int nlev_max, int rk_step, int iteration, bool fp64,
                         cudaStream_t s, bool damp = false);
