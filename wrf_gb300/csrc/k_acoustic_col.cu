@@ -21,26 +21,23 @@ namespace wrfgpu {
 // advance_uv (module_small_step_em.F:654-967) on the u and v points of the
 // column, and sumflux's sums of ru_m and rv_m there: the new u and v are in
 // registers, so the sums cost one read and one write of ru_m and rv_m (in a
-// kernel of their own they read u and v again).  Horizontal neighbours i-1 (u) and j-1 (v) are read
-// directly (L1); p and ph of level k are kept from the previous level.
+// kernel of their own they read u and v again).
+//
+// A tile of 32 x 8 staggered columns per block, two columns per thread: every
+// field of the pair is one 8-byte load, the pair's left neighbour one scalar
+// load, and the additions are packed (pair.cuh).  With one column per thread
+// each level cost 26 loads per column of which 12 re-read the neighbours.  ms per
+// large step, one column per thread against two: 100x70x30 0.103 / 0.083,
+// 256x256x80 0.72 / 0.67, 512x512x80 2.53 / 2.48, 1024x1024x96 10.95 / 10.81 (18
+// arrays at 4.7 TB/s).  p, ph and dpn of level k are kept from the level below.
 // ---------------------------------------------------------------------------
-namespace {
-struct UVLevel {
-  float u, rut, cqu, v, rvt, cqv;  // own u / v point
-  float rum, rvm, us, vs;          // accumulated mass fluxes (0 at the first iteration), linear parts (last one only)
-  float p1, ph1, pb, php, alt, al;           // (i, j):   p, ph at k+1; the rest at k
-  float p1x, ph1x, pbx, phpx, altx, alx;     // (i-1, j)
-  float p1y, ph1y, pby, phpy, alty, aly;     // (i, j-1)
-};
-}  // namespace
-
 template <int MINB>
-__global__ void __launch_bounds__(TX* TY, MINB) k_advance_uv_col(TileLaunch L, int rk_step, int iteration) {
+__global__ void __launch_bounds__(TX* TY / 2, MINB) k_advance_uv_col(TileLaunch L, int rk_step, int iteration) {
   const TilePos tp = tile_pos(L, false, true);
   const Mem& m = block_member(L.mem, tp.m);
   const Stage st = stage_of(m, rk_step);
   if (iteration > st.nsmall) return;
-  const int i = tp.i0 + threadIdx.x, j = tp.j0 + threadIdx.y;
+  const int i = tp.i0 + 2 * ((int)threadIdx.x & 15), j = tp.j0 + ((int)threadIdx.x >> 4);
   if (i > m.ite || j > m.jte) return;
   const float dts = st.dts_rk;
   const WrfDynConfig& cf = m.cf;
@@ -55,15 +52,24 @@ __global__ void __launch_bounds__(TX* TY, MINB) k_advance_uv_col(TileLaunch L, i
   if (cf.symmetric_xe && m.ite == m.ide) i_end_u_tend = i_end_u_tend - 1;
   if (cf.symmetric_ys && m.jts == m.jds) j_start_v_tend = j_start_v_tend + 1;
   if (cf.symmetric_ye && m.jte == m.jde) j_end_v_tend = j_end_v_tend - 1;
-  const bool upt = j >= j_start && j <= min(m.jte, m.jde - 1) && i >= min(i_start_u_tend, i_start_up) &&
-                   i <= max(i_end_u_tend, i_end_up);
-  const bool u_tend = upt && i >= i_start_u_tend && i <= i_end_u_tend;
-  const bool u_pg = upt && i >= i_start_up && i <= i_end_up;
-  const bool vpt = j >= j_start_v_tend && j <= j_end_v_tend && i >= i_start && i <= i_end;
-  const bool v_pg = vpt && j >= j_start_vp && j <= j_end_vp;
-  // sumflux: the points whose u (v) is summed; at the first iteration every
-  // point of the staggered tile starts from zero
-  const bool ucol = j <= min(m.jde - 1, m.jte), vcol = i <= min(m.ide - 1, m.ite);
+  // what each column of the pair takes part in: u's update, its tendency and
+  // pressure gradient, v's, and the sums (whose points at the first iteration
+  // start from zero over the whole staggered tile)
+  struct Col { bool in, ut, up, u, v, vp, us, vs; };
+  auto col_of = [&](int ii) {
+    Col c;
+    c.in = ii <= m.ite;
+    const bool urow = c.in && j <= min(m.jte, m.jde - 1);
+    c.ut = urow && ii >= i_start_u_tend && ii <= i_end_u_tend;
+    c.up = urow && ii >= i_start_up && ii <= i_end_up;
+    c.u = urow && ii >= min(i_start_u_tend, i_start_up) && ii <= max(i_end_u_tend, i_end_up);
+    c.v = j >= j_start_v_tend && j <= j_end_v_tend && ii <= i_end;
+    c.vp = c.v && j >= j_start_vp && j <= j_end_vp;
+    c.us = urow;
+    c.vs = ii <= i_end;
+    return c;
+  };
+  const Col ca = col_of(i), cb = col_of(i + 1);
   const bool first = iteration == 1, last = iteration == st.nsmall;
   const float fns = float(st.nsmall);
   F3 ru_m = f3(m, WRFGPU_RU_M), rv_m = f3(m, WRFGPU_RV_M), ww_m = f3(m, WRFGPU_WW_M);
@@ -76,159 +82,139 @@ __global__ void __launch_bounds__(TX* TY, MINB) k_advance_uv_col(TileLaunch L, i
      rdnw = f1(m, WRFGPU_RDNW);
   const float rdx = m.rdx, rdy = m.rdy, emdiv = m.emdiv, cf1 = m.cf1, cf2 = m.cf2, cf3 = m.cf3;
   const int kde = m.kde, k_start = m.kts, k_end = m.kte - 1;
-  // per-column factors (the reference's left-to-right products, split where they start)
-  F2 MU = f2(m, WRFGPU_MU_2), MUDF = f2(m, WRFGPU_MUDF);
-  float ua = 0.f, uc = 0.f, mudf_u = 0.f, muu = 0.f, mu_i = 0.f, mu_im = 0.f;
-  float va = 0.f, vc = 0.f, mudf_v = 0.f, muv = 0.f, mu_jm = 0.f;
-  if (u_pg) {
-    const float msfux = f2(m, WRFGPU_MSFUX).ro(i, j), msfuy = f2(m, WRFGPU_MSFUY).ro(i, j);
-    const float dx = 1.f / rdx;
-    mudf_u = -emdiv * dx * (MUDF.ro(i, j) - MUDF.ro(i - 1, j)) / msfuy;
-    ua = (msfux / msfuy) * .5f * rdx;
-    uc = (msfux / msfuy) * rdx;
-    muu = f2(m, WRFGPU_MUU).ro(i, j);
-    mu_i = MU.ro(i, j); mu_im = MU.ro(i - 1, j);
-  }
-  if (vpt) {
-    const float msfvx_inv = f2(m, WRFGPU_MSFVX_INV).ro(i, j);
-    const float dy = 1.f / rdy;
-    mudf_v = -emdiv * dy * (MUDF.ro(i, j) - MUDF.ro(i, j - 1)) * msfvx_inv;
-    if (v_pg) {
-      const float msfvx = f2(m, WRFGPU_MSFVX).ro(i, j), msfvy = f2(m, WRFGPU_MSFVY).ro(i, j);
-      va = (msfvy / msfvx) * .5f * rdy;
-      vc = (msfvy / msfvx) * rdy;
-      muv = f2(m, WRFGPU_MUV).ro(i, j);
-      mu_i = MU.ro(i, j); mu_jm = MU.ro(i, j - 1);
-    }
-  }
-  float muu_s = 0.f, muv_s = 0.f, msfuy_s = 1.f, mxi_s = 1.f;
-  if (last && ucol) { muu_s = f2(m, WRFGPU_MUU).ro(i, j); msfuy_s = f2(m, WRFGPU_MSFUY).ro(i, j); }
-  if (last && vcol) { muv_s = f2(m, WRFGPU_MUV).ro(i, j); mxi_s = f2(m, WRFGPU_MSFVX_INV).ro(i, j); }
-  const bool need_x = u_pg, need_y = v_pg, need_c = u_pg || v_pg;
-  auto load = [&](int k, UVLevel& d) {
-    d.rum = (!first && ucol) ? ru_m(i, k, j) : 0.f;
-    d.rvm = (!first && vcol) ? rv_m(i, k, j) : 0.f;
-    d.us = (last && ucol) ? usv.ro(i, k, j) : 0.f;
-    d.vs = (last && vcol) ? vsv.ro(i, k, j) : 0.f;
-    d.u = ucol ? u(i, k, j) : 0.f;
-    d.rut = u_tend ? ru_tend.ro(i, k, j) : 0.f;
-    d.cqu = u_pg ? cqu.ro(i, k, j) : 0.f;
-    d.v = vcol ? v(i, k, j) : 0.f;
-    d.rvt = vpt ? rv_tend.ro(i, k, j) : 0.f;
-    d.cqv = v_pg ? cqv.ro(i, k, j) : 0.f;
-    const bool top = k + 1 <= kde - 1;  // p exists up to kde-1
-    if (need_c) {
-      d.p1 = top ? p.ro(i, k + 1, j) : 0.f; d.ph1 = ph.ro(i, k + 1, j);
-      d.pb = pb.ro(i, k, j); d.php = php.ro(i, k, j); d.alt = alt.ro(i, k, j); d.al = al.ro(i, k, j);
-    }
-    if (need_x) {
-      d.p1x = top ? p.ro(i - 1, k + 1, j) : 0.f; d.ph1x = ph.ro(i - 1, k + 1, j);
-      d.pbx = pb.ro(i - 1, k, j); d.phpx = php.ro(i - 1, k, j); d.altx = alt.ro(i - 1, k, j); d.alx = al.ro(i - 1, k, j);
-    }
-    if (need_y) {
-      d.p1y = top ? p.ro(i, k + 1, j - 1) : 0.f; d.ph1y = ph.ro(i, k + 1, j - 1);
-      d.pby = pb.ro(i, k, j - 1); d.phpy = php.ro(i, k, j - 1); d.alty = alt.ro(i, k, j - 1); d.aly = al.ro(i, k, j - 1);
-    }
+  auto mul = [](float2 a, float2 b) { return make_float2(a.x * b.x, a.y * b.y); };
+  auto div = [](float2 a, float2 b) { return make_float2(a.x / b.x, a.y / b.y); };
+  auto ro = [&](const F3& a, int k, int jj) { return __ldg(reinterpret_cast<const float2*>(a.p + a.off(i, k, jj))); };
+  auto rw = [&](const F3& a, int k) { return *reinterpret_cast<const float2*>(a.p + a.off(i, k, j)); };
+  // the pair (i - 1, i): its own first column is the pair's
+  auto left = [&](const F3& a, int k, float2 own) { return make_float2(a.ro(i - 1, k, j), own.x); };
+  auto put = [&](const F3& a, int k, float2 val, bool ea, bool eb) {
+    if (ea && eb) *reinterpret_cast<float2*>(a.p + a.off(i, k, j)) = val;
+    else if (ea) a.p[a.off(i, k, j)] = val.x;
+    else if (eb) a.p[a.off(i, k, j) + 1] = val.y;
   };
+  auto sel = [](bool ea, bool eb, float2 t, float2 f) { return make_float2(ea ? t.x : f.x, eb ? t.y : f.y); };
+  auto g2 = [&](int f, int ii, int jj) { const F2 a = f2(m, f); return make_float2(a.ro(ii, jj), a.ro(ii + 1, jj)); };
+  // per-column factors (the reference's left-to-right products, split where they start)
+  const float2 mu_i = g2(WRFGPU_MU_2, i, j), mu_im = make_float2(f2(m, WRFGPU_MU_2).ro(i - 1, j), mu_i.x),
+               mu_jm = g2(WRFGPU_MU_2, i, j - 1);
+  const float2 msfuy = g2(WRFGPU_MSFUY, i, j), mxi = g2(WRFGPU_MSFVX_INV, i, j);
+  const float2 muu = g2(WRFGPU_MUU, i, j), muv = g2(WRFGPU_MUV, i, j);
+  float2 ua, uc, va, vc, mudf_u, mudf_v;
+  {
+    const float2 d = g2(WRFGPU_MUDF, i, j), dl = make_float2(f2(m, WRFGPU_MUDF).ro(i - 1, j), d.x),
+                 dd = g2(WRFGPU_MUDF, i, j - 1);
+    const float dx = 1.f / rdx, dy = 1.f / rdy;
+    mudf_u = div(muls(-emdiv * dx, sub2(d, dl)), msfuy);
+    mudf_v = mul(muls(-emdiv * dy, sub2(d, dd)), mxi);
+    const float2 ru = div(g2(WRFGPU_MSFUX, i, j), msfuy), rv = div(g2(WRFGPU_MSFVY, i, j), g2(WRFGPU_MSFVX, i, j));
+    ua = muls(rdx, muls(.5f, ru));
+    uc = muls(rdx, ru);
+    va = muls(rdy, muls(.5f, rv));
+    vc = muls(rdy, rv);
+  }
+  const bool pg_u = ca.up || cb.up, pg_v = ca.vp || cb.vp;
   // this block's chunk of levels (gridDim.y chunks); the levels are
   // independent but for the carried p, ph and dpn of the level below
   const int per = (k_end - k_start + 1 + (int)gridDim.y - 1) / (int)gridDim.y;
   const int k0 = k_start + (int)blockIdx.y * per, k1 = min(k_end, k0 + per - 1);
   if (k0 > k1) return;
-  // level k0 values of p and ph, and dpn(k0) (dpn(1) has its own formula)
-  float p0 = 0.f, ph0 = 0.f, p0x = 0.f, ph0x = 0.f, p0y = 0.f, ph0y = 0.f, dpn_u = 0.f, dpn_v = 0.f;
-  if (need_c) { p0 = p.ro(i, k0, j); ph0 = ph.ro(i, k0, j); }
-  if (need_x) {
-    p0x = p.ro(i - 1, k0, j); ph0x = ph.ro(i - 1, k0, j);
-    if (k0 == 1)
-      dpn_u = .5f * (cf1 * (p.ro(i, 1, j) + p.ro(i - 1, 1, j)) + cf2 * (p.ro(i, 2, j) + p.ro(i - 1, 2, j)) +
-                     cf3 * (p.ro(i, 3, j) + p.ro(i - 1, 3, j)));
-    else
-      dpn_u = .5f * (fnm(k0) * (p0 + p0x) + fnp(k0) * (p.ro(i, k0 - 1, j) + p.ro(i - 1, k0 - 1, j)));
+  // level k0 values of p and ph, and dpn(k0) (dpn(1) has its own formula);
+  // dpn(kde) is zero unless the lid is rigid.  x: columns i - 1, y: row j - 1
+  auto edge = [&](float a1, int ka, float a2, int kb, float a3, int kc, bool x) {
+    auto both = [&](int k) {
+      const float2 o = ro(p, k, j);
+      return x ? add2(o, left(p, k, o)) : add2(o, ro(p, k, j - 1));
+    };
+    return muls(.5f, add2(add2(muls(a1, both(ka)), muls(a2, both(kb))), muls(a3, both(kc))));
+  };
+  float2 p0 = ro(p, k0, j), ph0 = ro(ph, k0, j), p0x = left(p, k0, p0), ph0x = left(ph, k0, ph0),
+         p0y = ro(p, k0, j - 1), ph0y = ro(ph, k0, j - 1);
+  float2 dpn_u, dpn_v, dpn_u_top = bc2(0.f), dpn_v_top = bc2(0.f);
+  if (k0 == 1) {
+    dpn_u = edge(cf1, 1, cf2, 2, cf3, 3, true);
+    dpn_v = edge(cf1, 1, cf2, 2, cf3, 3, false);
+  } else {
+    const float2 pm = ro(p, k0 - 1, j);
+    dpn_u = muls(.5f, add2(muls(fnm(k0), add2(p0, p0x)), muls(fnp(k0), add2(pm, left(p, k0 - 1, pm)))));
+    dpn_v = muls(.5f, add2(muls(fnm(k0), add2(p0, p0y)), muls(fnp(k0), add2(pm, ro(p, k0 - 1, j - 1)))));
   }
-  if (need_y) {
-    p0y = p.ro(i, k0, j - 1); ph0y = ph.ro(i, k0, j - 1);
-    if (k0 == 1)
-      dpn_v = .5f * (cf1 * (p.ro(i, 1, j) + p.ro(i, 1, j - 1)) + cf2 * (p.ro(i, 2, j) + p.ro(i, 2, j - 1)) +
-                     cf3 * (p.ro(i, 3, j) + p.ro(i, 3, j - 1)));
-    else
-      dpn_v = .5f * (fnm(k0) * (p0 + p0y) + fnp(k0) * (p.ro(i, k0 - 1, j) + p.ro(i, k0 - 1, j - 1)));
-  }
-  // top value of dpn (kde): zero unless the lid is rigid
-  float dpn_u_top = 0.f, dpn_v_top = 0.f;
   if (cf.top_lid) {
-    if (need_x)
-      dpn_u_top = .5f * (cf1 * (p.ro(i - 1, kde - 1, j) + p.ro(i, kde - 1, j)) + cf2 * (p.ro(i - 1, kde - 2, j) + p.ro(i, kde - 2, j)) +
-                         cf3 * (p.ro(i - 1, kde - 3, j) + p.ro(i, kde - 3, j)));
-    if (need_y)
-      dpn_v_top = .5f * (cf1 * (p.ro(i, kde - 1, j - 1) + p.ro(i, kde - 1, j)) + cf2 * (p.ro(i, kde - 2, j - 1) + p.ro(i, kde - 2, j)) +
-                         cf3 * (p.ro(i, kde - 3, j - 1) + p.ro(i, kde - 3, j)));
+    dpn_u_top = edge(cf1, kde - 1, cf2, kde - 2, cf3, kde - 3, true);
+    dpn_v_top = edge(cf1, kde - 1, cf2, kde - 2, cf3, kde - 3, false);
   }
   for (int k = k0; k <= k1; ++k) {
-    UVLevel cur;  // a level's inputs go out together
-    load(k, cur);
     const int kk = k + 1;
+    // a level's inputs go out together
+    const float2 c_u = rw(u, k), c_v = rw(v, k), rut = ro(ru_tend, k, j), rvt = ro(rv_tend, k, j);
+    const float2 c_rum = first ? bc2(0.f) : rw(ru_m, k), c_rvm = first ? bc2(0.f) : rw(rv_m, k);
+    const float2 c_us = last ? ro(usv, k, j) : bc2(0.f), c_vs = last ? ro(vsv, k, j) : bc2(0.f);
+    const float2 c_cqu = ro(cqu, k, j), c_cqv = ro(cqv, k, j);
+    const float2 p1 = ro(p, kk, j), ph1 = ro(ph, kk, j), c_pb = ro(pb, k, j), c_php = ro(php, k, j), c_alt = ro(alt, k, j),
+                 c_al = ro(al, k, j);
+    const float2 p1x = left(p, kk, p1), ph1x = left(ph, kk, ph1), pbx = left(pb, k, c_pb), phpx = left(php, k, c_php),
+                 altx = left(alt, k, c_alt), alx = left(al, k, c_al);
+    const float2 p1y = ro(p, kk, j - 1), ph1y = ro(ph, kk, j - 1), pby = ro(pb, k, j - 1), phpy = ro(php, k, j - 1),
+                 alty = ro(alt, k, j - 1), aly = ro(al, k, j - 1);
+    const float h1 = c1h(k), h2 = c2h(k), rz = rdnw(k);
+    const float zm = kk < kde ? fnm(kk) : 0.f, zp = kk < kde ? fnp(kk) : 0.f;
+    const float2 mh = muls(h1, mu_i);
     // u
-    float uv = cur.u;
-    if (upt) {
-      if (u_tend) uv = uv + dts * cur.rut;
-      float dpn_hi = 0.f;
-      if (u_pg) {
-        dpn_hi = (kk == kde) ? dpn_u_top : .5f * (fnm(kk) * (cur.p1 + cur.p1x) + fnp(kk) * (p0 + p0x));
-        float dpxy = ua * (c1h(k) * muu + c2h(k)) *
-                     (((cur.ph1 - cur.ph1x) + (ph0 - ph0x)) + (cur.alt + cur.altx) * (p0 - p0x) +
-                      (cur.al + cur.alx) * (cur.pb - cur.pbx));
-        dpxy = dpxy + uc * (cur.php - cur.phpx) *
-                          (rdnw(k) * (dpn_hi - dpn_u) - .5f * ((c1h(k) * mu_im) + (c1h(k) * mu_i)));
-        uv = uv - dts * cur.cqu * dpxy + (c1h(k) * mudf_u);
-        dpn_u = dpn_hi;
-      }
-      u(i, k, j) = uv;
+    float2 uv = sel(ca.ut, cb.ut, add2(c_u, muls(dts, rut)), c_u);
+    if (pg_u) {
+      const float2 dpn_hi = kk == kde ? dpn_u_top : muls(.5f, add2(muls(zm, add2(p1, p1x)), muls(zp, add2(p0, p0x))));
+      float2 dpxy = mul(mul(ua, add2(muls(h1, muu), bc2(h2))),
+                        add2(add2(add2(sub2(ph1, ph1x), sub2(ph0, ph0x)), mul(add2(c_alt, altx), sub2(p0, p0x))),
+                             mul(add2(c_al, alx), sub2(c_pb, pbx))));
+      dpxy = add2(dpxy, mul(mul(uc, sub2(c_php, phpx)),
+                            sub2(muls(rz, sub2(dpn_hi, dpn_u)), muls(.5f, add2(muls(h1, mu_im), mh)))));
+      uv = sel(ca.up, cb.up, add2(sub2(uv, mul(muls(dts, c_cqu), dpxy)), muls(h1, mudf_u)), uv);
+      dpn_u = dpn_hi;
     }
+    put(u, k, uv, ca.u, cb.u);
     // v
-    float vv = cur.v;
-    if (vpt) {
-      vv = vv + dts * cur.rvt;
-      if (v_pg) {
-        const float dpn_hi = (kk == kde) ? dpn_v_top : .5f * (fnm(kk) * (cur.p1 + cur.p1y) + fnp(kk) * (p0 + p0y));
-        float dpxy = va * (c1h(k) * muv + c2h(k)) *
-                     (((cur.ph1 - cur.ph1y) + (ph0 - ph0y)) + (cur.alt + cur.alty) * (p0 - p0y) +
-                      (cur.al + cur.aly) * (cur.pb - cur.pby));
-        dpxy = dpxy + vc * (cur.php - cur.phpy) *
-                          (rdnw(k) * (dpn_hi - dpn_v) - .5f * ((c1h(k) * mu_jm) + (c1h(k) * mu_i)));
-        vv = vv - dts * cur.cqv * dpxy + (c1h(k) * mudf_v);
-        dpn_v = dpn_hi;
-      }
-      v(i, k, j) = vv;
+    float2 vv = sel(ca.v, cb.v, add2(c_v, muls(dts, rvt)), c_v);
+    if (pg_v) {
+      const float2 dpn_hi = kk == kde ? dpn_v_top : muls(.5f, add2(muls(zm, add2(p1, p1y)), muls(zp, add2(p0, p0y))));
+      float2 dpxy = mul(mul(va, add2(muls(h1, muv), bc2(h2))),
+                        add2(add2(add2(sub2(ph1, ph1y), sub2(ph0, ph0y)), mul(add2(c_alt, alty), sub2(p0, p0y))),
+                             mul(add2(c_al, aly), sub2(c_pb, pby))));
+      dpxy = add2(dpxy, mul(mul(vc, sub2(c_php, phpy)),
+                            sub2(muls(rz, sub2(dpn_hi, dpn_v)), muls(.5f, add2(muls(h1, mu_jm), mh)))));
+      vv = sel(ca.vp, cb.vp, add2(sub2(vv, mul(muls(dts, c_cqv), dpxy)), muls(h1, mudf_v)), vv);
+      dpn_v = dpn_hi;
     }
+    put(v, k, vv, ca.v, cb.v);
     // sumflux
-    float rum = cur.rum, rvm = cur.rvm;
-    if (ucol) {
-      rum = rum + uv;
-      if (last) rum = rum / fns + (c1h(k) * muu_s + c2h(k)) * cur.us / msfuy_s;
+    float2 rum = add2(c_rum, uv), rvm = add2(c_rvm, vv);
+    if (last) {
+      rum = add2(div(rum, bc2(fns)), div(mul(add2(muls(h1, muu), bc2(h2)), c_us), msfuy));
+      rvm = add2(div(rvm, bc2(fns)), mul(mul(add2(muls(h1, muv), bc2(h2)), c_vs), mxi));
     }
-    if (vcol) {
-      rvm = rvm + vv;
-      if (last) rvm = rvm / fns + (c1h(k) * muv_s + c2h(k)) * cur.vs * mxi_s;
+    if (first) {
+      put(ru_m, k, sel(ca.us, cb.us, rum, bc2(0.f)), ca.in, cb.in);
+      put(rv_m, k, sel(ca.vs, cb.vs, rvm, bc2(0.f)), ca.in, cb.in);
+      put(ww_m, k, bc2(0.f), ca.in && !(ca.us && ca.vs), cb.in && !(cb.us && cb.vs));
+    } else {
+      put(ru_m, k, rum, ca.us, cb.us);
+      put(rv_m, k, rvm, ca.vs, cb.vs);
     }
-    if (first || ucol) ru_m(i, k, j) = rum;
-    if (first || vcol) rv_m(i, k, j) = rvm;
-    if (first && !(ucol && vcol)) ww_m(i, k, j) = 0.f;
-    p0 = cur.p1; ph0 = cur.ph1; p0x = cur.p1x; ph0x = cur.ph1x; p0y = cur.p1y; ph0y = cur.ph1y;
+    p0 = p1; ph0 = ph1; p0x = p1x; ph0x = ph1x; p0y = p1y; ph0y = ph1y;
   }
   if (first && k1 == k_end) {  // level kde holds no mass flux but ww_m of the mass columns
     const int kt = k_end + 1;
-    ru_m(i, kt, j) = 0.f;
-    rv_m(i, kt, j) = 0.f;
-    if (!(ucol && vcol)) ww_m(i, kt, j) = 0.f;
+    put(ru_m, kt, bc2(0.f), ca.in, cb.in);
+    put(rv_m, kt, bc2(0.f), ca.in, cb.in);
+    put(ww_m, kt, bc2(0.f), ca.in && !(ca.us && ca.vs), cb.in && !(cb.us && cb.vs));
   }
 }
 
-// variant parameter: 10 x blocks per SM + level chunks
+// variant parameter: 10 x blocks per SM (of the one-column form's 256 threads) + level chunks
 void launch_advance_uv_col(const TileLaunch& L, int nblocks, int rk_step, int iteration, cudaStream_t s, int var) {
   const int p = TUNE_PARAM[TU_AUV][var], chunks = level_chunks(nblocks, L.nlev, p % 10, 2);
-  if (p / 10 == 4) k_advance_uv_col<4><<<dim3(nblocks, chunks), dim3(TX, TY), 0, s>>>(L, rk_step, iteration);
-  else k_advance_uv_col<3><<<dim3(nblocks, chunks), dim3(TX, TY), 0, s>>>(L, rk_step, iteration);
+  const dim3 grid(nblocks, chunks), block(TX * TY / 2);
+  if (p / 10 == 4) k_advance_uv_col<5><<<grid, block, 0, s>>>(L, rk_step, iteration);
+  else k_advance_uv_col<4><<<grid, block, 0, s>>>(L, rk_step, iteration);
 }
 
 // ---------------------------------------------------------------------------

@@ -49,7 +49,7 @@ constexpr int TUNE_NVAR[NTUNE] = {2, 3, 3, 4, 4, 2, 2, 4, 4, 3, 4, 4, 4, 4};
 // (defaults measured on 512x512x80 and up: advance_mu_t 278 us with four blocks
 // per SM against 393 with two, advance_w 340 against 388; the FP64 form of
 // advance_mu_t is best with three, 524 against 571 us on the 16-member ensemble)
-constexpr int TUNE_DEFAULT[NTUNE] = {1, 1, 2, 1, 2, 1, 0, 2, 2, 1, 3, 3, 2, 2};
+constexpr int TUNE_DEFAULT[NTUNE] = {1, 1, 2, 0, 2, 1, 0, 2, 2, 1, 3, 3, 2, 2};
 // the parameter each variant stands for: blocks per SM, level chunks
 // (sumflux: of calc_p_rho), or (advance_uv, rk_tend_u, rk_tend_v) 10 x blocks
 // per SM + level chunks
