@@ -219,8 +219,9 @@ struct Ensemble {
         std::swap(hm[m].qmap[s], hm[m].qamap[s]);
       }
   }
-  void swap_species() {
-    launch_swap_species(d_mems, nmem, stream);
+  // done: the groups of a last step's transport have been swapped one by one
+  void swap_species(bool done) {
+    if (!done) launch_swap_species(d_mems, nmem, stream);
     host_flip();
     if (capturing) ++capture_swaps;
   }
@@ -249,12 +250,16 @@ struct Ensemble {
   // transport, cross the host link on a second stream while stage 1's
   // dynamics run; everything else (the dry state and the moist species, read
   // from the first kernel on) before the step, and the downloads after it.
+  // fields up to this size are stored to host memory by the pack kernel (2 MB:
+  // 10 us on the link, what a staged copy takes before its first byte)
+  static constexpr size_t DIRECT_OUT_MAX = 2u << 20;
   struct HostIO {
     int member = 0, id = 0;
     int species = -1;        // >= 0: the current value of that species (buffers looked up on the device)
     bool late = false;       // a passive scalar: may arrive while stage 1's dynamics run
     const float* in = nullptr;
     float* out = nullptr;
+    float* out_dev = nullptr;  // small fields: `out` as the device addresses it (written by the pack kernel)
     float* dev = nullptr;    // a fixed field buffer (species < 0)
     size_t count = 0, cols = 0, rows = 0, pitch = 0;
     float* stage = nullptr;  // contiguous device copy
@@ -263,8 +268,11 @@ struct Ensemble {
   };
   std::vector<HostIO> hio;
   cudaStream_t cstream = nullptr;  // downloads of the host I/O step that overlap its kernels
+  cudaStream_t pstream = nullptr;  // packing of the next large download while one crosses the link
   cudaStream_t ustream = nullptr;  // uploads of the host I/O step that overlap its kernels
   std::vector<cudaEvent_t> ev_dn;  // per bound field: its overlapped download is complete
+  std::vector<cudaEvent_t> ev_pk;  // per bound field: it is packed
+  cudaEvent_t ev_pfork = nullptr;
   cudaEvent_t ev_head = nullptr, ev_ojoin2 = nullptr;
   cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
   // [head][prefetch]: head = the previous step's deferred downloads come
@@ -295,12 +303,13 @@ struct Ensemble {
     cudaEventRecord(ev_mfork, stream);
     cudaStreamWaitEvent(cstream, ev_mfork, 0);
     io_moist_done.assign(hio.size(), 0);
+    std::vector<size_t> l;
     for (size_t q = 0; q < hio.size(); ++q)
       if (hio[q].out && hio[q].species >= 0 && !hio[q].late) {
-        copy_out(hio[q], cstream);
-        cudaEventRecord(ev_dn[q], cstream);
+        l.push_back(q);
         io_moist_done[q] = 1;
       }
+    copy_out(l);
     return true;
   }
 
@@ -332,12 +341,43 @@ struct Ensemble {
     return b.species < 0 && (b.id == WRFGPU_U_2 || b.id == WRFGPU_V_2 || b.id == WRFGPU_W_2 ||
                              b.id == WRFGPU_T_2 || b.id == WRFGPU_PH_2 || b.id == WRFGPU_MU_2);
   }
-  void copy_out(const HostIO& b, cudaStream_t st) {
-    if (b.species >= 0)
-      launch_pack_species(d_mems, b.member, b.species, b.stage, (int)b.cols, (int)b.rows, (int)b.pitch, st);
-    else
-      launch_pack_rows(b.dev, b.stage, (int)b.cols, (int)b.rows, (int)b.pitch, st);
-    cudaMemcpyAsync(b.out, b.stage, b.count * 4, cudaMemcpyDeviceToHost, st);
+  // Downloads of the fields `l` on cstream, each marked by its ev_dn.  Small
+  // ones are stored to their host buffers by one pack launch (a pack and a
+  // copy each cost a launch and 5 us of latency per field); large ones go
+  // through their staging buffers and the copy engine, each packed on pstream
+  // while the one before it crosses the link.
+  void copy_out(const std::vector<size_t>& l) {
+    auto job = [&](const HostIO& b, float* dst) {
+      return PackJob{b.dev, dst, b.member, b.species, (int)b.cols, (int)b.rows, (int)b.pitch};
+    };
+    PackJobs pj;
+    pj.n = 0;
+    for (size_t q : l)
+      if (hio[q].out_dev) {
+        pj.job[pj.n++] = job(hio[q], hio[q].out_dev);
+        if (pj.n == MAX_PACK_JOBS) { launch_pack_fields(d_mems, pj, cstream); pj.n = 0; }
+      }
+    launch_pack_fields(d_mems, pj, cstream);
+    for (size_t q : l)
+      if (hio[q].out_dev) cudaEventRecord(ev_dn[q], cstream);
+    bool forked = false;
+    for (size_t q : l) {
+      const HostIO& b = hio[q];
+      if (b.out_dev) continue;
+      if (!forked) {
+        cudaEventRecord(ev_pfork, cstream);
+        cudaStreamWaitEvent(pstream, ev_pfork, 0);
+        forked = true;
+      }
+      PackJobs one;
+      one.n = 1;
+      one.job[0] = job(b, b.stage);
+      launch_pack_fields(d_mems, one, pstream);
+      cudaEventRecord(ev_pk[q], pstream);
+      cudaStreamWaitEvent(cstream, ev_pk[q], 0);
+      cudaMemcpyAsync(b.out, b.stage, b.count * 4, cudaMemcpyDeviceToHost, cstream);
+      cudaEventRecord(ev_dn[q], cstream);
+    }
   }
   void io_dry_out() {
     if (!io_step) return;
@@ -348,12 +388,13 @@ struct Ensemble {
     cudaStreamWaitEvent(cstream, ev_ofork, 0);
     cudaStreamWaitEvent(ustream, ev_ofork, 0);
     std::vector<char> dn(hio.size(), 0);
+    std::vector<size_t> l;
     for (size_t q = 0; q < hio.size(); ++q)
       if (hio[q].out && early_out(hio[q])) {
-        copy_out(hio[q], cstream);
-        cudaEventRecord(ev_dn[q], cstream);
+        l.push_back(q);
         dn[q] = 1;
       }
+    copy_out(l);
     // the next step's inputs that no later download of this step can change,
     // on the other copy engine direction, each after the downloads it waits for
     if (io_prefetch)
@@ -362,6 +403,34 @@ struct Ensemble {
     cudaEventRecord(ev_ojoin, cstream);
     cudaEventRecord(ev_ojoin2, ustream);
     io_out_pending = true;
+  }
+  // A call's last step: the positive-definite transport in groups of pairs,
+  // each group's species swapped, their halos filled and downloaded while the
+  // next group is transported and calc_p_rho_phi runs.  Two or three groups where
+  // a group still fills the GPU (a launch passes over the other groups'
+  // blocks); one next to open boundaries, whose strips follow the transport.
+  // 512x512x80 with 11 species: the downloads left after the step went from
+  // 6.8 to 3 ms.
+  int io_pd_groups() const {
+    if (!io_step || io_prefetch) return 1;
+    return any_open ? 1 : nb_pr >= 3000 ? 3 : nb_pr >= 1200 ? 2 : 1;
+  }
+  void io_species_out(unsigned pairs) {
+    launch_swap_species(d_mems, nmem, stream, pairs);
+    JobList js;
+    for (int s = 0; s < nsp_max; ++s)
+      if ((pairs >> (s / 2)) & 1u) js.sp(s, 0, 'p');
+    fill(js);
+    std::vector<size_t> l;
+    for (size_t q = 0; q < hio.size(); ++q)
+      if (hio[q].out && hio[q].species >= 0 && ((pairs >> (hio[q].species / 2)) & 1u)) {
+        l.push_back(q);
+        io_moist_done[q] = 1;
+      }
+    if (l.empty()) return;
+    cudaEventRecord(ev_mfork, stream);
+    cudaStreamWaitEvent(cstream, ev_mfork, 0);
+    copy_out(l);
   }
   // An early input (the dry state, moist species) may be uploaded during the
   // previous step's last stage when its staging buffer is free then (no
@@ -429,6 +498,7 @@ struct Ensemble {
           cudaGetLastError();
           return WRFGPU_E_ARG;
         }
+        if (hp == b.out && b.count * 4 <= DIRECT_OUT_MAX) b.out_dev = (float*)at.devicePointer;
       }
       const int sid = b.id - WRFGPU_SPECIES_BASE;
       if (sid >= 0 && sid % 2 == 0) {
@@ -463,6 +533,8 @@ struct Ensemble {
       cudaEvent_t e;
       CK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
       ev_dn.push_back(e);
+      CK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+      ev_pk.push_back(e);
     }
     if (cstream) return WRFGPU_OK;
     // the copy streams' pack / unpack kernels take SM slots ahead of the
@@ -471,8 +543,9 @@ struct Ensemble {
     CK(cudaDeviceGetStreamPriorityRange(&least, &greatest));
     CK(cudaStreamCreateWithPriority(&cstream, cudaStreamNonBlocking, greatest));
     CK(cudaStreamCreateWithPriority(&ustream, cudaStreamNonBlocking, greatest));
+    CK(cudaStreamCreateWithPriority(&pstream, cudaStreamNonBlocking, greatest));
     for (cudaEvent_t* e : {&ev_fork, &ev_join, &ev_ofork, &ev_ojoin, &ev_dryin, &ev_head, &ev_ojoin2, &ev_tfork,
-                           &ev_tjoin, &ev_tjoin2, &ev_upA, &ev_mfork})
+                           &ev_tjoin, &ev_tjoin2, &ev_upA, &ev_mfork, &ev_pfork})
       CK(cudaEventCreateWithFlags(e, cudaEventDisableTiming));
     return WRFGPU_OK;
   }
@@ -483,9 +556,9 @@ struct Ensemble {
   // next input only after it).
   static bool deferrable(const HostIO& b) { return b.species >= 0 && b.late; }
   // One step with its copies, enqueued on `stream` and `cstream`.  head: the
-  // previous step's deferred downloads first; defer: this step's passive
-  // scalars left for the next step's head (or flush_deferred).
-  int enqueue_io_step(bool head, bool defer, bool pre) {
+  // previous step's deferred downloads first; pre: a step of the same call
+  // follows, this one's passive scalars are left for its head.
+  int enqueue_io_step(bool head, bool pre) {
     if (int rc = io_streams()) return rc;
     auto unpack = [&](const HostIO& b, cudaStream_t st) {
       if (b.species >= 0)
@@ -500,13 +573,15 @@ struct Ensemble {
     CK(cudaStreamWaitEvent(ustream, ev_fork, 0));
     // the previous step's deferred downloads on one copy direction ...
     std::vector<char> dn(hio.size(), 0);
-    if (head)
+    if (head) {
+      std::vector<size_t> l;
       for (size_t q = 0; q < hio.size(); ++q)
         if (hio[q].out && deferrable(hio[q])) {
-          copy_out(hio[q], cstream);
-          CK(cudaEventRecord(ev_dn[q], cstream));
+          l.push_back(q);
           dn[q] = 1;
         }
+      copy_out(l);
+    }
     CK(cudaEventRecord(ev_head, cstream));
     // ... the dry state and the moist species first on the other, at the
     // link's full rate (those prefetched during the previous step are across)
@@ -557,38 +632,29 @@ struct Ensemble {
       CK(cudaStreamWaitEvent(stream, ev_ojoin2, 0));
       io_out_pending = false;
     }
-    if (!pre) {
-      for (const HostIO& b : hio)
-        if (b.out && !early_out(b) && !(defer && deferrable(b))) copy_out(b, stream);
-    } else {
+    {
       // the final downloads on one link direction and, behind each, the next
       // step's inputs that wait for it on the other
       CK(cudaEventRecord(ev_tfork, stream));
       CK(cudaStreamWaitEvent(cstream, ev_tfork, 0));
       CK(cudaStreamWaitEvent(ustream, ev_tfork, 0));
       std::vector<char> tdn(hio.size(), 0);
+      std::vector<size_t> l;
       for (size_t q = 0; q < hio.size(); ++q) {
         const HostIO& b = hio[q];
-        if (!b.out || early_out(b) || (defer && deferrable(b))) continue;
+        if (!b.out || early_out(b) || (pre && deferrable(b))) continue;
         tdn[q] = 1;
-        if (io_moist_done[q]) continue;  // downloaded after the last transport
-        copy_out(b, cstream);
-        CK(cudaEventRecord(ev_dn[q], cstream));
-        tdn[q] = 1;
+        if (!io_moist_done[q]) l.push_back(q);  // else downloaded after the last transport
       }
-      for (size_t q = 0; q < hio.size(); ++q)
-        if (hio[q].tail) upload_after(q, tdn);
+      copy_out(l);
+      if (pre)
+        for (size_t q = 0; q < hio.size(); ++q)
+          if (hio[q].tail) upload_after(q, tdn);
       CK(cudaEventRecord(ev_tjoin, cstream));
       CK(cudaEventRecord(ev_tjoin2, ustream));
       CK(cudaStreamWaitEvent(stream, ev_tjoin, 0));
       CK(cudaStreamWaitEvent(stream, ev_tjoin2, 0));
     }
-    CK(cudaGetLastError());
-    return WRFGPU_OK;
-  }
-  int flush_deferred() {
-    for (const HostIO& b : hio)
-      if (b.out && deferrable(b)) copy_out(b, stream);
     CK(cudaGetLastError());
     return WRFGPU_OK;
   }
@@ -601,7 +667,7 @@ struct Ensemble {
     capturing = true;
     capture_swaps = 0;
     CK(cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal));
-    const int rc = enqueue_io_step(h == 1, true, v == 1);
+    const int rc = enqueue_io_step(h == 1, v == 1);
     capturing = false;
     io_swaps = capture_swaps;
     for (int q = 0; q < capture_swaps; ++q) host_flip();
@@ -621,7 +687,7 @@ struct Ensemble {
     if (nsteps == 0) return WRFGPU_OK;
     if (flags & WRFGPU_FLAG_NO_GRAPH) {
       for (int s = 0; s < nsteps; ++s) {
-        int rc = enqueue_io_step(s > 0, true, s + 1 < nsteps);
+        int rc = enqueue_io_step(s > 0, s + 1 < nsteps);
         if (rc) return rc;
       }
     } else {
@@ -639,7 +705,6 @@ struct Ensemble {
         for (int q = 0; q < io_swaps; ++q) host_flip();
       }
     }
-    if (int rc = flush_deferred()) return rc;
     CK(cudaStreamSynchronize(stream));
     return WRFGPU_OK;
   }
@@ -648,7 +713,10 @@ struct Ensemble {
     unbind_host();
     if (cstream) cudaStreamDestroy(cstream);
     if (ustream) cudaStreamDestroy(ustream);
+    if (pstream) cudaStreamDestroy(pstream);
     for (cudaEvent_t e : ev_dn) cudaEventDestroy(e);
+    for (cudaEvent_t e : ev_pk) cudaEventDestroy(e);
+    if (ev_pfork) cudaEventDestroy(ev_pfork);
     for (cudaEvent_t e : {ev_head, ev_ojoin2})
       if (e) cudaEventDestroy(e);
     for (cudaEvent_t e : {ev_fork, ev_join, ev_ofork, ev_ojoin, ev_dryin})
@@ -1053,13 +1121,21 @@ struct Ensemble {
       if (rk_step == 3 && any_pd) {
         mark(PH_PD);
         launch_pd_courant(l2, nb2, rk_step, stream);
-        launch_scalar_pd_update(LP(), nb_pr, nlev_max, rk_step, stream, tune[TU_PD]);
+        const int np = (nsp_max + 1) / 2, ng = std::min(np, io_pd_groups());
+        for (int g = 0, p0 = 0; g < ng; ++g) {
+          const int p1 = np * (g + 1) / ng;
+          const unsigned pairs = ng == 1 ? ~0u : ((1u << p1) - 1u) & ~((1u << p0) - 1u);
+          launch_scalar_pd_update(LP(), nb_pr, nlev_max, rk_step, stream, tune[TU_PD], pairs);
+          if (io_step && !io_prefetch && !any_open) io_species_out(pairs);
+          p0 = p1;
+        }
+        species_filled = io_step && !io_prefetch && !any_open;
       }
       if (any_open) {
         launch_strip_scalar(LS3(), nb_s3, rk_step, stream);
         if (rk_step == 3) launch_strip_pd(LS5(), nb_s5, LS4(), nb_s4, rk_step, nsp_max, d_pd_scratch, stream);
       }
-      swap_species();
+      swap_species(species_filled);
       // a host I/O step with a next step: the species' final halo values
       // (the end-of-step fill, issued here: calc_p_rho_phi reads qv at its
       // own points only) and the moist species' downloads, beside calc_p_rho_phi
@@ -1473,7 +1549,10 @@ int wrfgpu_get_field_f32(WrfGpuEnsemble* h, int member, int id, float* dst, long
     if (cudaMemcpyAsync(dst, p, cnt * 4, cudaMemcpyDeviceToHost, s) != cudaSuccess) return WRFGPU_E_CUDA;
   } else {
     if (int rc = h->e.ensure_stage(cnt)) return rc;
-    wrfgpu::launch_pack_rows(p, h->e.d_stage, (int)cols, (int)rows, (int)pitch, s);
+    wrfgpu::PackJobs one;
+    one.n = 1;
+    one.job[0] = wrfgpu::PackJob{p, h->e.d_stage, member, -1, (int)cols, (int)rows, (int)pitch};
+    wrfgpu::launch_pack_fields(h->e.d_mems, one, s);
     if (cudaMemcpyAsync(dst, h->e.d_stage, cnt * 4, cudaMemcpyDeviceToHost, s) != cudaSuccess) return WRFGPU_E_CUDA;
   }
   if (cudaStreamSynchronize(s) != cudaSuccess) return WRFGPU_E_CUDA;

@@ -195,9 +195,6 @@ __global__ void k_unpack_rows(const float* __restrict__ src, float* __restrict__
                               int cols, int rows, int pitch) {
   copy_rows(src, cols, dst, dst2, pitch, cols, rows);
 }
-__global__ void k_pack_rows(const float* __restrict__ src, float* __restrict__ dst, int cols, int rows, int pitch) {
-  copy_rows(src, pitch, dst, nullptr, cols, cols, rows);
-}
 // The same for species s of member `member`, whose current and spare buffers
 // are read from the device member table when the copy runs (the buffers
 // exchange roles at every scalar update, so a captured copy must not hold
@@ -206,9 +203,13 @@ __global__ void k_unpack_species(const Mem* __restrict__ mems, int member, int s
                                  int cols, int rows, int pitch) {
   copy_rows(src, cols, mems[member].q[s], mems[member].qa[s], pitch, cols, rows);
 }
-__global__ void k_pack_species(const Mem* __restrict__ mems, int member, int s, float* __restrict__ dst, int cols,
-                               int rows, int pitch) {
-  copy_rows(mems[member].q[s], pitch, dst, nullptr, cols, cols, rows);
+// Several fields into their contiguous buffers, one per blockIdx.y.  A buffer
+// may be page-locked host memory: the rows then cross the link as stores, with
+// no staging copy and no copy of its own.
+__global__ void k_pack_fields(const Mem* __restrict__ mems, const __grid_constant__ PackJobs jobs) {
+  const PackJob& J = jobs.job[blockIdx.y];
+  const float* src = J.species < 0 ? J.src : mems[J.member].q[J.species];
+  copy_rows(src, J.pitch, J.dst, nullptr, J.cols, J.cols, J.rows);
 }
 static int rows_grid(int rows) {  // 256-thread blocks of 8 row-warps, at most 8 blocks per SM of 152
   return rows / 8 + 1 < 8 * 152 ? rows / 8 + 1 : 8 * 152;
@@ -216,16 +217,17 @@ static int rows_grid(int rows) {  // 256-thread blocks of 8 row-warps, at most 8
 void launch_unpack_rows(const float* src, float* dst, float* dst2, int cols, int rows, int pitch, cudaStream_t s) {
   if (cols > 0 && rows > 0) k_unpack_rows<<<rows_grid(rows), 256, 0, s>>>(src, dst, dst2, cols, rows, pitch);
 }
-void launch_pack_rows(const float* src, float* dst, int cols, int rows, int pitch, cudaStream_t s) {
-  if (cols > 0 && rows > 0) k_pack_rows<<<rows_grid(rows), 256, 0, s>>>(src, dst, cols, rows, pitch);
-}
 void launch_unpack_species(const Mem* mems, int member, int s, const float* src, int cols, int rows, int pitch,
                            cudaStream_t st) {
   if (cols > 0 && rows > 0) k_unpack_species<<<rows_grid(rows), 256, 0, st>>>(mems, member, s, src, cols, rows, pitch);
 }
-void launch_pack_species(const Mem* mems, int member, int s, float* dst, int cols, int rows, int pitch,
-                         cudaStream_t st) {
-  if (cols > 0 && rows > 0) k_pack_species<<<rows_grid(rows), 256, 0, st>>>(mems, member, s, dst, cols, rows, pitch);
+void launch_pack_fields(const Mem* mems, const PackJobs& jobs, cudaStream_t st) {
+  if (jobs.n <= 0) return;
+  int rows = 0;
+  for (int q = 0; q < jobs.n; ++q) rows = jobs.job[q].rows > rows ? jobs.job[q].rows : rows;
+  const int per = 8 * 152 / jobs.n;
+  const int g = rows / 8 + 1 < per ? rows / 8 + 1 : per;
+  k_pack_fields<<<dim3(g, jobs.n), 256, 0, st>>>(mems, jobs);
 }
 
 void launch_fill_halo(const Mem* d_mems, int nmem, const HaloJobs& jobs, int blocks_per_job, cudaStream_t s) {

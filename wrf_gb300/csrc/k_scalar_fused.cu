@@ -342,12 +342,14 @@ __device__ __forceinline__ float lim1(float v, float sc) { return sc >= 0.f ? sc
 // Positive-definite transport of a pair of species (the lanes of packed
 // FP32 arithmetic, pair.cuh): species 2 p and 2 p + 1 of block (tile, p).
 // Where only one species of the pair uses the positive-definite scheme at
-// this stage, both lanes carry it and it is written once.
+// this stage, both lanes carry it and it is written once.  pairs: as for
+// k_scalar_adv_update.
 template <int MINB>
-__global__ void __launch_bounds__(PD_THREADS, MINB) k_scalar_pd_update(TileLaunch L, int rk_step) {
+__global__ void __launch_bounds__(PD_THREADS, MINB) k_scalar_pd_update(TileLaunch L, int rk_step, unsigned pairs) {
   using P = PDPlanes;
   extern __shared__ __align__(128) unsigned char smem[];
   const TilePos tp = tile_pos(L, TILE_PER_PAIR);
+  if (!((pairs >> tp.sub) & 1u)) return;  // block-uniform
   const Mem& m = block_member(L.mem, tp.m);
   const int sa = 2 * tp.sub, sb = 2 * tp.sub + 1;
   const bool va = sa < m.nsp && pd_scheme(m, sa, rk_step), vb = sb < m.nsp && pd_scheme(m, sb, rk_step);
@@ -656,11 +658,12 @@ __global__ void __launch_bounds__(PD_THREADS, MINB) k_scalar_pd_update(TileLaunc
 // ------------------------------------------------------------------ swap
 // After a fused update: the spare buffer holds the new scalar; exchange it
 // with the current one (pointers and tensor-map slots) in every member's table.
-__global__ void k_swap_species(Mem* mems, int nmem) {
+__global__ void k_swap_species(Mem* mems, int nmem, unsigned pairs) {
   const int m = blockIdx.x * blockDim.x + threadIdx.x;
   if (m >= nmem) return;
   Mem& M = mems[m];
   for (int s = 0; s < M.nsp; ++s) {
+    if (!((pairs >> (s / 2)) & 1u)) continue;
     float* t = M.q[s];
     M.q[s] = M.qa[s];
     M.qa[s] = t;
@@ -691,7 +694,8 @@ void launch_scalar_adv_update(const TileLaunch& L, int nblocks, int rk_step, cud
   else if (minb == 3) k_scalar_adv_update<3, false><<<grid, dim3(TX, TY), ADV_SMEM, s>>>(L, rk_step, pairs);
   else k_scalar_adv_update<4, false><<<grid, dim3(TX, TY), ADV_SMEM, s>>>(L, rk_step, pairs);
 }
-void launch_scalar_pd_update(const TileLaunch& L, int nblocks, int nlev_max, int rk_step, cudaStream_t s, int var) {
+void launch_scalar_pd_update(const TileLaunch& L, int nblocks, int nlev_max, int rk_step, cudaStream_t s, int var,
+                             unsigned pairs) {
   static size_t attr = 0;
   const size_t bytes = PD_SMEM + sizeof(LevelConst) * (size_t)nlev_max;
   if (bytes > attr) {
@@ -701,14 +705,14 @@ void launch_scalar_pd_update(const TileLaunch& L, int nblocks, int nlev_max, int
   }
   // a chunk computes two levels more than it writes
   const dim3 grid(nblocks, level_chunks(nblocks, L.nlev, 1, 6, 2 * 152));
-  if (TUNE_PARAM[TU_PD][var] == 1) k_scalar_pd_update<1><<<grid, PD_THREADS, bytes, s>>>(L, rk_step);
-  else k_scalar_pd_update<2><<<grid, PD_THREADS, bytes, s>>>(L, rk_step);
+  if (TUNE_PARAM[TU_PD][var] == 1) k_scalar_pd_update<1><<<grid, PD_THREADS, bytes, s>>>(L, rk_step, pairs);
+  else k_scalar_pd_update<2><<<grid, PD_THREADS, bytes, s>>>(L, rk_step, pairs);
 }
 void launch_pd_courant(const Launch& L2, int nblocks, int rk_step, cudaStream_t s) {
   k_pd_courant<<<dim3(nblocks, level_chunks(nblocks, L2.nlev, 1, 4, 8 * 152)), dim3(BX, BY), 0, s>>>(L2, rk_step);
 }
-void launch_swap_species(Mem* d_mems, int nmem, cudaStream_t s) {
-  k_swap_species<<<(nmem + 63) / 64, 64, 0, s>>>(d_mems, nmem);
+void launch_swap_species(Mem* d_mems, int nmem, cudaStream_t s, unsigned pairs) {
+  k_swap_species<<<(nmem + 63) / 64, 64, 0, s>>>(d_mems, nmem, pairs);
 }
 
 }  // namespace wrfgpu

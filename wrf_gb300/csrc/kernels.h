@@ -20,6 +20,21 @@ struct HaloJobs {
   HaloJob job[MAX_HALO_JOBS];
 };
 
+// Fields copied from their padded device rows into contiguous buffers by one
+// launch (k_pack_fields): a fixed device buffer, or the current buffer of
+// species `species` of member `member`.
+struct PackJob {
+  const float* src;
+  float* dst;
+  int member, species;
+  int cols, rows, pitch;
+};
+constexpr int MAX_PACK_JOBS = 32;
+struct PackJobs {
+  int n;
+  PackJob job[MAX_PACK_JOBS];
+};
+
 // Stage / iteration arguments shared by the step kernels.
 struct StepArgs {
   int rk_step;     // 1..3
@@ -120,11 +135,9 @@ void launch_update_scalar_routine(const Launch& L3, int nblocks, int rk_step, in
 void launch_calc_p_rho_phi(const Launch& L3, int nblocks, cudaStream_t s);
 // host <-> device field copies through a contiguous staging buffer
 void launch_unpack_rows(const float* src, float* dst, float* dst2, int cols, int rows, int pitch, cudaStream_t s);
-void launch_pack_rows(const float* src, float* dst, int cols, int rows, int pitch, cudaStream_t s);
 void launch_unpack_species(const Mem* mems, int member, int s, const float* src, int cols, int rows, int pitch,
                            cudaStream_t st);
-void launch_pack_species(const Mem* mems, int member, int s, float* dst, int cols, int rows, int pitch,
-                         cudaStream_t st);
+void launch_pack_fields(const Mem* mems, const PackJobs& jobs, cudaStream_t st);
 // mass tiles x level chunks; iteration 0: step 0 of the stage, else the acoustic step (halo images stored)
 void launch_calc_p_rho_col(const TileLaunch& L, int nblocks, StepArgs a, cudaStream_t s, int chunks = 4);
 // sct: some member stores the species' sixth-order diffusion tendency sc_tend
@@ -141,8 +154,9 @@ void launch_scalar_adv_update(const TileLaunch& L, int nblocks, int rk_step, cud
 void launch_pd_courant(const Launch& L2, int nblocks, int rk_step, cudaStream_t s);
 // nlev_max: the largest kme - kms + 1 of the members (sizes a per-level table in shared memory)
 void launch_scalar_pd_update(const TileLaunch& L, int nblocks, int nlev_max, int rk_step, cudaStream_t s,
-                             int var = TUNE_DEFAULT[TU_PD]);
-void launch_swap_species(Mem* d_mems, int nmem, cudaStream_t s);
+                             int var = TUNE_DEFAULT[TU_PD], unsigned pairs = ~0u);
+// pairs: as for the transport
+void launch_swap_species(Mem* d_mems, int nmem, cudaStream_t s, unsigned pairs = ~0u);
 
 // the acoustic step (k_acoustic_col.cu): one block per tile of the staggered
 // extents, then either one block per row segment of 32 mass columns
