@@ -1024,8 +1024,8 @@ struct Ensemble {
       if (cfl_check) { mark(PH_CFL); launch_cfl_check_col(LTM(), nb_tm, sw, tune[TU_CFL]); }
       mark(PH_TEND_T); launch_tend_t_col(LST(), nb_st, TF_ZERO | TF_ADV, sp);
       mark(PH_TEND_PH); launch_tend_ph_col(LST(), nb_st, TF_ZERO | TF_ADV, sp);
-      mark(PH_TEND_U); launch_tend_u_col(LST(), nb_st, TF_ALL, stream, tune[TU_TENDU]);
-      mark(PH_TEND_V); launch_tend_v_col(LST(), nb_st, TF_ALL, stream, tune[TU_TENDV]);
+      mark(PH_TEND_U); launch_tend_u_col(LST(), nb_st, stream, tune[TU_TENDU]);
+      mark(PH_TEND_V); launch_tend_v_col(LST(), nb_st, stream, tune[TU_TENDV]);
       join(0);
       join(1);
       // open boundaries: the lower-order fluxes and radiation terms next to them

@@ -3,7 +3,7 @@
 // for 5th/3rd order; horizontal_pressure_gradient, module_big_step_utilities_em.F:1585-1718;
 // coriolis :3106-3215; curvature :3234-3363).
 //
-// One thread per (i, j) column of a 32 x 8 tile of the staggered extents,
+// One thread per (i, j) column (u and v: two columns) of a 32 x 8 tile of the staggered extents,
 // levels kts..kte in order (or one chunk of them per block along y).  For u
 // and v, the advected field and the mass fluxes ru, rv of each level arrive
 // by TMA as halo planes, several levels ahead, and every horizontal face
@@ -21,6 +21,7 @@
 #include "common.cuh"
 #include "kernels.h"
 #include "open_adv.cuh"
+#include "pair.cuh"
 
 namespace wrfgpu {
 
@@ -58,396 +59,246 @@ __device__ __forceinline__ void tile_faces(const float* Q, float* FX, float* FY,
   if (ty == TY - 2) yface(TY, tx);
 }
 
-// ---------------------------------------------------------------- ru_tend
-// A level's point inputs of the u (v) tendency beyond the staged planes, with
-// the sums and differences of the two columns formed as the reference's
-// expressions form them (so every rounding is unchanged): the tendency so
-// far, the advected field three levels up, the omega sum of the face above,
-// rw, p and ph one level up, alt, al, pb, php and cqu (cqv) of the two
-// columns, and the two sums of the cross velocity for the curvature term.
-struct LevelIn {
-  float t, f3, romsum, rw_l1, rw_r1, p_l1, p_r1, ph_l1, ph_r1, altsum, alsum, pbd, phpd, cq, cs_r, cs_l;
-};
-// They are loaded together, right before the level's arithmetic, so their
-// latencies overlap one another (interleaved with the arithmetic that uses
-// them, the kernel took 1.63 instead of 1.31 ms per 512x512x80 step).
-template <int FL, int MINB>
-__global__ void __launch_bounds__(TX* TY, MINB) k_tend_u_col(TileLaunch L) {
-  static_assert(FL & TF_ADV, "the staged form includes advection");
-  extern __shared__ __align__(128) unsigned char smem[];
-  const TilePos tp = tile_pos(L, false, true);
-  const Mem& m = block_member(L.mem, tp.m);
-  const int tx = threadIdx.x, ty = threadIdx.y, tid = ty * TX + tx;
-  const int i = tp.i0 + tx, j = tp.j0 + ty;
-  const F3 tend = f3(m, WRFGPU_RU_TEND);
-  const int kts = m.kts, kte = m.kte, kde = m.kde, kme = m.kme, ktf = min(kte, kde - 1);
-  const int jacc = min(m.jte, m.jde - 1);
-  const bool inside = i <= m.ite && j <= m.jte;
-  const bool acc = inside && j <= jacc;
-  if ((FL & TF_ZERO) && inside && !acc && blockIdx.y == 0)
-    for (int k = kts; k <= kte; ++k) tend(i, k, j) = 0.f;
-  const Chunk ch = level_chunk_of(kts, ktf);
-  const int k0 = ch.k0, k1 = ch.k1;
-  if (tp.i0 <= m.ite && tp.j0 <= jacc && k0 <= k1) {  // block-uniform
-    const F3 u = f3(m, WRFGPU_U_2), rw = f3(m, WRFGPU_RW), rom = f3(m, WRFGPU_WW);
-    const F3 ph = f3(m, WRFGPU_PH_2), alt = f3(m, WRFGPU_ALT), p = f3(m, WRFGPU_P), pb = f3(m, WRFGPU_PB),
-             al = f3(m, WRFGPU_AL), php = f3(m, WRFGPU_PHP), cqu = f3(m, WRFGPU_CQU), v = f3(m, WRFGPU_V_2);
-    const F1 fzm = f1(m, WRFGPU_FNM), fzp = f1(m, WRFGPU_FNP), rdzw = f1(m, WRFGPU_RDNW), c1h = f1(m, WRFGPU_C1H),
-             c2h = f1(m, WRFGPU_C2H);
-    const float rdx = m.rdx, rdy = m.rdy;
-    HaloRing ring;
-    ring.init(smem, k0);
-    float* FXb = (float*)(smem + HaloRing::SMEM);
-    float* FYb = FXb + 2 * FXN;
-    const CUtensorMap* maps[3] = {tmap_of(m, WRFGPU_U_2, BOX_HALO), tmap_of(m, WRFGPU_RU, BOX_HALO),
-                                  tmap_of(m, WRFGPU_RV, BOX_HALO)};
-    const int x0 = tp.i0 - TMA_HALO - m.ims, z0 = tp.j0 - TMA_HALO - m.jms;
-    if (tid == 0) {
-      ring.init_barriers();
-      mbar_fence_init();
-    }
-    __syncthreads();
-    if (tid == 0)
-      for (int d = 0; d < TEND_RING - 1 && k0 + d <= k1; ++d) ring.issue(k0 + d, maps, x0, z0, m.kms);
-    // column constants
-    float mrdy = 0.f, mrdx = 0.f, ratio = 0.f, pgA = 0.f, pgB = 0.f;
-    float muu_c = 0.f, mu_l = 0.f, mu_r = 0.f, corA = 0.f, corB = 0.f;
-    float dvx_l = 0.f, dvx_r = 0.f, duy_l = 0.f, duy_r = 0.f;
-    // own-column window of u for the vertical flux u(k-1 .. k+2), the vertical
-    // flux of face k, and the pressure-gradient / rw carries (formed afresh at
-    // the chunk's first level k0, with the same expressions as one level down)
-    float um1 = 0.f, u0 = 0.f, up1 = 0.f, up2 = 0.f, vf_lo = 0.f;
-    float p_l = 0.f, p_r = 0.f, ph_l = 0.f, ph_r = 0.f, dpn_lo = 0.f, rw_l = 0.f, rw_r = 0.f;
-    if (acc) {
-      const F2 msfux = f2(m, WRFGPU_MSFUX), msfuy = f2(m, WRFGPU_MSFUY);
-      const float msfux_c = msfux(i, j), msfuy_c = msfuy(i, j);
-      mrdy = msfux_c * rdy; mrdx = msfux_c * rdx;
-      ratio = msfux_c / msfuy_c;
-      pgA = ratio * .5f * rdx; pgB = ratio * rdx;
-      if (FL & TF_PG) {
-        muu_c = f2(m, WRFGPU_MUU)(i, j);
-        mu_l = f2(m, WRFGPU_MU_2)(i - 1, j);
-        mu_r = f2(m, WRFGPU_MU_2)(i, j);
-      }
-      if (FL & TF_COR) {
-        const F2 f = f2(m, WRFGPU_F), e = f2(m, WRFGPU_E), cosa = f2(m, WRFGPU_COSA);
-        corA = ratio * 0.5f * (f(i, j) + f(i - 1, j)) * 0.25f;
-        corB = 0.5f * (e(i, j) + e(i - 1, j)) * 0.5f * (cosa(i, j) + cosa(i - 1, j)) * 0.25f;
-      }
-      if (FL & TF_CURV) {
-        const F2 msfvx = f2(m, WRFGPU_MSFVX);
-        dvx_r = msfvx(i, j + 1) - msfvx(i, j);
-        dvx_l = msfvx(i - 1, j + 1) - msfvx(i - 1, j);
-        duy_r = msfuy(i + 1, j) - msfuy(i, j);
-        duy_l = msfuy(i, j) - msfuy(i - 1, j);
-      }
-      um1 = (k0 - 1 >= kts) ? u(i, k0 - 1, j) : 0.f; u0 = u(i, k0, j); up1 = u(i, k0 + 1, j);
-      up2 = (k0 + 2 <= kme) ? u(i, k0 + 2, j) : 0.f;
-      {
-        const int kk = k0;
-        if (kk == kts || kk == kte) vf_lo = 0.f;
-        else if (kk == kts + 1 || kk == ktf)
-          vf_lo = 0.5f * (rom(i, kk, j) + rom(i - 1, kk, j)) * (fzm(kk) * u0 + fzp(kk) * um1);
-        else {
-          const float vel = 0.5f * (rom(i - 1, kk, j) + rom(i, kk, j));
-          vf_lo = vel * flux3(u(i, kk - 2, j), um1, u0, up1, -vel);
-        }
-      }
-      if (FL & TF_PG) {
-        p_l = p(i - 1, k0, j); p_r = p(i, k0, j);
-        ph_l = ph(i - 1, k0, j); ph_r = ph(i, k0, j);
-        if (k0 == 1)
-          dpn_lo = .5f * (m.cf1 * (p(i - 1, 1, j) + p(i, 1, j)) + m.cf2 * (p(i - 1, 2, j) + p(i, 2, j)) +
-                          m.cf3 * (p(i - 1, 3, j) + p(i, 3, j)));
-        else
-          dpn_lo = .5f * (fzm(k0) * (p_l + p_r) + fzp(k0) * (p(i - 1, k0 - 1, j) + p(i, k0 - 1, j)));
-      }
-      if (FL & (TF_COR | TF_CURV)) { rw_l = rw(i - 1, k0, j); rw_r = rw(i, k0, j); }
-    }
-    const int o = (ty + TMA_HALO) * HALO_W + tx + TMA_HALO;  // own point in the halo planes
-    auto load_in = [&](int k) {
-      LevelIn q;
-      q.t = (FL & TF_ZERO) ? 0.f : tend(i, k, j);
-      q.f3 = (k + 3 <= kme) ? u(i, k + 3, j) : 0.f;
-      const int kk = k + 1;
-      // rom(i) + rom(i-1) = rom(i-1) + rom(i) exactly: IEEE addition commutes
-      q.romsum = (kk == kts || kk == kte) ? 0.f : rom(i, kk, j) + rom(i - 1, kk, j);
-      q.rw_l1 = q.rw_r1 = 0.f;
-      if (FL & (TF_COR | TF_CURV)) { q.rw_l1 = rw(i - 1, k + 1, j); q.rw_r1 = rw(i, k + 1, j); }
-      q.p_l1 = q.p_r1 = q.ph_l1 = q.ph_r1 = q.altsum = q.alsum = q.pbd = q.phpd = q.cq = 0.f;
-      if (FL & TF_PG) {
-        if (kk != kde) { q.p_l1 = p(i - 1, kk, j); q.p_r1 = p(i, kk, j); }
-        q.ph_l1 = ph(i - 1, k + 1, j); q.ph_r1 = ph(i, k + 1, j);
-        q.altsum = alt(i, k, j) + alt(i - 1, k, j);
-        q.alsum = al(i, k, j) + al(i - 1, k, j);
-        q.pbd = pb(i, k, j) - pb(i - 1, k, j);
-        q.phpd = php(i, k, j) - php(i - 1, k, j);
-        q.cq = cqu(i, k, j);
-      }
-      q.cs_r = q.cs_l = 0.f;
-      if (FL & TF_CURV) { q.cs_r = v(i, k, j) + v(i, k, j + 1); q.cs_l = v(i - 1, k, j) + v(i - 1, k, j + 1); }
-      return q;
-    };
-    bool ok = true;
-    for (int k = k0; k <= k1; ++k) {
-      ok = ring.wait(k) && ok;
-      const float* U = ring.plane(k, 0);
-      const float* RU = ring.plane(k, 1);
-      const float* RV = ring.plane(k, 2);
-      float* FX = FXb + (k & 1) * FXN;
-      float* FY = FYb + (k & 1) * FYN;
-      tile_faces(U, FX, FY, [&](int q) { return 0.5f * (RU[q] + RU[q - 1]); },
-                 [&](int q) { return 0.5f * (RV[q] + RV[q - 1]); }, tx, ty);
-      __syncthreads();
-      // the slot of level k-1, which every thread has finished with
-      if (tid == 0 && k + TEND_RING - 1 <= k1) ring.issue(k + TEND_RING - 1, maps, x0, z0, m.kms);
-      if (!acc) continue;
-      if (k + 2 <= kme) {
-        prefetch_l2(&rom(i, k + 2, j)); prefetch_l2(&p(i, k + 2, j)); prefetch_l2(&ph(i, k + 2, j));
-        prefetch_l2(&alt(i, k + 2, j)); prefetch_l2(&al(i, k + 2, j)); prefetch_l2(&pb(i, k + 2, j));
-        prefetch_l2(&php(i, k + 2, j)); prefetch_l2(&cqu(i, k + 2, j)); prefetch_l2(&rw(i, k + 2, j));
-        prefetch_l2(&v(i, k + 2, j)); prefetch_l2(&tend(i, k + 2, j));
-      }
-      const LevelIn q = load_in(k);
-      float t = q.t;
-      t = t - mrdy * (FY[(ty + 1) * TX + tx] - FY[ty * TX + tx]);
-      t = t - mrdx * (FX[ty * (TX + 1) + tx + 1] - FX[ty * (TX + 1) + tx]);
-      {  // vertical flux of face k+1
-        const int kk = k + 1;
-        float vf_hi;
-        if (kk == kts || kk == kte) vf_hi = 0.f;
-        else if (kk == kts + 1 || kk == ktf)
-          vf_hi = 0.5f * q.romsum * (fzm(kk) * up1 + fzp(kk) * u0);
-        else {
-          const float vel = 0.5f * q.romsum;
-          vf_hi = vel * flux3(um1, u0, up1, up2, -vel);
-        }
-        t = t - rdzw(k) * (vf_hi - vf_lo);
-        vf_lo = vf_hi;
-      }
-      if (FL & TF_PG) {
-        const int kk = k + 1;
-        float dpn_hi;
-        if (kk == kde) {
-          if (m.cf.top_lid)
-            dpn_hi = .5f * (m.cfn * (p(i - 1, kde - 1, j) + p(i, kde - 1, j)) +
-                            m.cfn1 * (p(i - 1, kde - 2, j) + p(i, kde - 2, j)));
-          else dpn_hi = 0.f;
-        } else {
-          dpn_hi = .5f * (fzm(kk) * (q.p_l1 + q.p_r1) + fzp(kk) * (p_l + p_r));
-        }
-        float dpx = pgA * (c1h(k) * muu_c + c2h(k)) *
-                    ((q.ph_r1 - q.ph_l1 + ph_r - ph_l) + q.altsum * (p_r - p_l) + q.alsum * q.pbd);
-        dpx = dpx + pgB * q.phpd * (rdzw(k) * (dpn_hi - dpn_lo) - .5f * ((c1h(k) * mu_l) + (c1h(k) * mu_r)));
-        t = t - q.cq * dpx;
-        dpn_lo = dpn_hi;
-        p_l = q.p_l1; p_r = q.p_r1; ph_l = q.ph_l1; ph_r = q.ph_r1;
-      }
-      if (FL & (TF_COR | TF_CURV)) {
-        const float rvsum = RV[o + HALO_W - 1] + RV[o + HALO_W] + RV[o - 1] + RV[o];
-        const float rwsum = q.rw_l1 + rw_l + q.rw_r1 + rw_r;
-        if (FL & TF_COR) t = t + corA * rvsum - corB * rwsum;
-        if (FL & TF_CURV) {
-          const float vx_r = 0.5f * (u0 + U[o + 1]) * dvx_r * rdy - 0.5f * q.cs_r * duy_r * rdx;
-          const float vx_l = 0.5f * (U[o - 1] + u0) * dvx_l * rdy - 0.5f * q.cs_l * duy_l * rdx;
-          t = t + 0.5f * (vx_r + vx_l) * 0.25f * rvsum - u0 * RERADIUS * 0.25f * rwsum;
-        }
-      }
-      rw_l = q.rw_l1; rw_r = q.rw_r1;
-      tend(i, k, j) = t;
-      um1 = u0; u0 = up1; up1 = up2; up2 = q.f3;
-    }
-    if (!ok && tid == 0) raise_err(m, ERR_TIMEOUT);
-  }
-  if ((FL & TF_ZERO) && acc && blockIdx.y == gridDim.y - 1)
-    for (int k = ktf + 1; k <= kte; ++k) tend(i, k, j) = 0.f;
-}
+// ---------------------------------------------------------------- ru_tend, rv_tend
+// The two are one computation with the directions exchanged: DIR 0 is u (the
+// other column of every average is i - 1), DIR 1 v (row j - 1).
+//
+// Two adjacent columns per thread: the planes are read and the own-column
+// fields loaded in 8-byte pairs, the additions of both columns are packed
+// (pair.cuh), and a level's addresses, coefficients and loop cost one thread
+// instead of two.  One column per thread issued 600 instructions per column
+// and level, 67% of the issue slots at 30% of HBM; ms per large step against
+// two columns: rk_tend_u 5.54 / 4.31 and rk_tend_v 5.45 / 4.69 on 1024x1024x96,
+// 1.31 / 0.99 and 1.22 / 1.06 on 512x512x80.  Every face flux is still
+// formed once; a thread keeps its own cells' and takes the right and top
+// neighbours' from shared memory.
+constexpr int FX2 = TX + 2, FXN2 = TY * FX2;  // x faces of a tile, rows padded to an even length
+constexpr size_t TEND2_SMEM = HaloRing::SMEM + 2 * (FXN2 + FYN) * 4;
+constexpr int TEND2_THREADS = TX * TY / 2;
 
-// ---------------------------------------------------------------- rv_tend
-template <int FL, int MINB>
-__global__ void __launch_bounds__(TX* TY, MINB) k_tend_v_col(TileLaunch L) {
-  static_assert(FL & TF_ADV, "the staged form includes advection");
+template <int DIR, int MINB>
+__global__ void __launch_bounds__(TEND2_THREADS, MINB) k_tend_uv_col(TileLaunch L) {
   extern __shared__ __align__(128) unsigned char smem[];
   const TilePos tp = tile_pos(L, false, true);
   const Mem& m = block_member(L.mem, tp.m);
-  const int tx = threadIdx.x, ty = threadIdx.y, tid = ty * TX + tx;
-  const int i = tp.i0 + tx, j = tp.j0 + ty;
-  const F3 tend = f3(m, WRFGPU_RV_TEND);
+  const int tid = threadIdx.x, c = (tid & 15) * 2, ty = tid >> 4;
+  const int i = tp.i0 + c, j = tp.j0 + ty;
+  const F3 tend = f3(m, DIR ? WRFGPU_RV_TEND : WRFGPU_RU_TEND);
   const int kts = m.kts, kte = m.kte, kde = m.kde, kme = m.kme, ktf = min(kte, kde - 1);
-  const int iacc = min(m.ite, m.ide - 1);
-  const bool inside = i <= m.ite && j <= m.jte;
-  const bool acc = inside && i <= iacc;
-  if ((FL & TF_ZERO) && inside && !acc && blockIdx.y == 0)
-    for (int k = kts; k <= kte; ++k) tend(i, k, j) = 0.f;
+  // the points that take a tendency, and (of the staggered tile) those set to zero
+  const int iacc = DIR ? min(m.ite, m.ide - 1) : m.ite, jacc = DIR ? m.jte : min(m.jte, m.jde - 1);
+  const bool in0 = i <= m.ite && j <= m.jte, in1 = i + 1 <= m.ite && j <= m.jte;
+  const bool acc = i <= iacc && j <= jacc, acc1 = i + 1 <= iacc && j <= jacc;
+  auto zero = [&](int k) {
+    if (in0 && !acc) tend(i, k, j) = 0.f;
+    if (in1 && !acc1) tend(i + 1, k, j) = 0.f;
+  };
+  if (blockIdx.y == 0)
+    for (int k = kts; k <= kte; ++k) zero(k);
   const Chunk ch = level_chunk_of(kts, ktf);
   const int k0 = ch.k0, k1 = ch.k1;
-  if (tp.i0 <= iacc && tp.j0 <= m.jte && k0 <= k1) {  // block-uniform
-    const F3 v = f3(m, WRFGPU_V_2), rw = f3(m, WRFGPU_RW), rom = f3(m, WRFGPU_WW);
-    const F3 ph = f3(m, WRFGPU_PH_2), alt = f3(m, WRFGPU_ALT), p = f3(m, WRFGPU_P), pb = f3(m, WRFGPU_PB),
-             al = f3(m, WRFGPU_AL), php = f3(m, WRFGPU_PHP), cqv = f3(m, WRFGPU_CQV), u = f3(m, WRFGPU_U_2);
-    const F1 fzm = f1(m, WRFGPU_FNM), fzp = f1(m, WRFGPU_FNP), rdzw = f1(m, WRFGPU_RDNW), c1h = f1(m, WRFGPU_C1H),
-             c2h = f1(m, WRFGPU_C2H);
-    const float rdx = m.rdx, rdy = m.rdy;
-    HaloRing ring;
-    ring.init(smem, k0);
-    float* FXb = (float*)(smem + HaloRing::SMEM);
-    float* FYb = FXb + 2 * FXN;
-    const CUtensorMap* maps[3] = {tmap_of(m, WRFGPU_V_2, BOX_HALO), tmap_of(m, WRFGPU_RU, BOX_HALO),
-                                  tmap_of(m, WRFGPU_RV, BOX_HALO)};
-    const int x0 = tp.i0 - TMA_HALO - m.ims, z0 = tp.j0 - TMA_HALO - m.jms;
-    if (tid == 0) {
-      ring.init_barriers();
-      mbar_fence_init();
+  if (blockIdx.y == gridDim.y - 1)
+    for (int k = ktf + 1; k <= kte; ++k) {
+      if (acc) tend(i, k, j) = 0.f;
+      if (acc1) tend(i + 1, k, j) = 0.f;
     }
-    __syncthreads();
-    if (tid == 0)
-      for (int d = 0; d < TEND_RING - 1 && k0 + d <= k1; ++d) ring.issue(k0 + d, maps, x0, z0, m.kms);
-    float mrdy = 0.f, mrdx = 0.f, ratio = 0.f, pgA = 0.f, pgB = 0.f;
-    float muv_c = 0.f, mu_l = 0.f, mu_r = 0.f, corA = 0.f, corB = 0.f;
-    float dvx_l = 0.f, dvx_r = 0.f, duy_l = 0.f, duy_r = 0.f;
-    float vm1 = 0.f, v0 = 0.f, vp1 = 0.f, vp2 = 0.f, vf_lo = 0.f;
-    float p_l = 0.f, p_r = 0.f, ph_l = 0.f, ph_r = 0.f, dpn_lo = 0.f, rw_l = 0.f, rw_r = 0.f;
-    if (acc) {
-      const F2 msfvx = f2(m, WRFGPU_MSFVX), msfvy = f2(m, WRFGPU_MSFVY);
-      const float msfvy_c = msfvy(i, j), msfvx_c = msfvx(i, j);
-      mrdy = msfvy_c * rdy; mrdx = msfvy_c * rdx;
-      ratio = msfvy_c / msfvx_c;
-      pgA = ratio * .5f * rdy; pgB = ratio * rdy;
-      if (FL & TF_PG) {
-        muv_c = f2(m, WRFGPU_MUV)(i, j);
-        mu_l = f2(m, WRFGPU_MU_2)(i, j - 1);
-        mu_r = f2(m, WRFGPU_MU_2)(i, j);
-      }
-      if (FL & TF_COR) {
-        const F2 f = f2(m, WRFGPU_F), e = f2(m, WRFGPU_E), sina = f2(m, WRFGPU_SINA);
-        corA = ratio * 0.5f * (f(i, j) + f(i, j - 1)) * 0.25f;
-        corB = ratio * 0.5f * (e(i, j) + e(i, j - 1)) * 0.5f * (sina(i, j) + sina(i, j - 1)) * 0.25f;
-      }
-      if (FL & TF_CURV) {
-        const F2 msfuy = f2(m, WRFGPU_MSFUY);
-        dvx_r = msfvx(i, j + 1) - msfvx(i, j);
-        dvx_l = msfvx(i, j) - msfvx(i, j - 1);
-        duy_r = msfuy(i + 1, j) - msfuy(i, j);
-        duy_l = msfuy(i + 1, j - 1) - msfuy(i, j - 1);
-      }
-      vm1 = (k0 - 1 >= kts) ? v(i, k0 - 1, j) : 0.f; v0 = v(i, k0, j); vp1 = v(i, k0 + 1, j);
-      vp2 = (k0 + 2 <= kme) ? v(i, k0 + 2, j) : 0.f;
-      {
-        const int kk = k0;
-        if (kk == kts || kk == kte) vf_lo = 0.f;
-        else if (kk == kts + 1 || kk == ktf)
-          vf_lo = 0.5f * (rom(i, kk, j) + rom(i, kk, j - 1)) * (fzm(kk) * v0 + fzp(kk) * vm1);
-        else {
-          const float vel = 0.5f * (rom(i, kk, j) + rom(i, kk, j - 1));
-          vf_lo = vel * flux3(v(i, kk - 2, j), vm1, v0, vp1, -vel);
-        }
-      }
-      if (FL & TF_PG) {
-        p_l = p(i, k0, j - 1); p_r = p(i, k0, j);
-        ph_l = ph(i, k0, j - 1); ph_r = ph(i, k0, j);
-        if (k0 == 1)
-          dpn_lo = .5f * (m.cf1 * (p(i, 1, j - 1) + p(i, 1, j)) + m.cf2 * (p(i, 2, j - 1) + p(i, 2, j)) +
-                          m.cf3 * (p(i, 3, j - 1) + p(i, 3, j)));
-        else
-          dpn_lo = .5f * (fzm(k0) * (p_l + p_r) + fzp(k0) * (p(i, k0 - 1, j - 1) + p(i, k0 - 1, j)));
-      }
-      if (FL & (TF_COR | TF_CURV)) { rw_l = rw(i, k0, j - 1); rw_r = rw(i, k0, j); }
-    }
-    const int o = (ty + TMA_HALO) * HALO_W + tx + TMA_HALO;
-    auto load_in = [&](int k) {
-      LevelIn q;
-      q.t = (FL & TF_ZERO) ? 0.f : tend(i, k, j);
-      q.f3 = (k + 3 <= kme) ? v(i, k + 3, j) : 0.f;
-      const int kk = k + 1;
-      q.romsum = (kk == kts || kk == kte) ? 0.f : rom(i, kk, j) + rom(i, kk, j - 1);
-      q.rw_l1 = q.rw_r1 = 0.f;
-      if (FL & (TF_COR | TF_CURV)) { q.rw_l1 = rw(i, k + 1, j - 1); q.rw_r1 = rw(i, k + 1, j); }
-      q.p_l1 = q.p_r1 = q.ph_l1 = q.ph_r1 = q.altsum = q.alsum = q.pbd = q.phpd = q.cq = 0.f;
-      if (FL & TF_PG) {
-        if (kk != kde) { q.p_l1 = p(i, kk, j - 1); q.p_r1 = p(i, kk, j); }
-        q.ph_l1 = ph(i, k + 1, j - 1); q.ph_r1 = ph(i, k + 1, j);
-        q.altsum = alt(i, k, j) + alt(i, k, j - 1);
-        q.alsum = al(i, k, j) + al(i, k, j - 1);
-        q.pbd = pb(i, k, j) - pb(i, k, j - 1);
-        q.phpd = php(i, k, j) - php(i, k, j - 1);
-        q.cq = cqv(i, k, j);
-      }
-      q.cs_r = q.cs_l = 0.f;
-      if (FL & TF_CURV) { q.cs_r = u(i, k, j) + u(i + 1, k, j); q.cs_l = u(i, k, j - 1) + u(i + 1, k, j - 1); }
-      return q;
-    };
-    bool ok = true;
-    for (int k = k0; k <= k1; ++k) {
-      ok = ring.wait(k) && ok;
-      const float* V = ring.plane(k, 0);
-      const float* RU = ring.plane(k, 1);
-      const float* RV = ring.plane(k, 2);
-      float* FX = FXb + (k & 1) * FXN;
-      float* FY = FYb + (k & 1) * FYN;
-      tile_faces(V, FX, FY, [&](int q) { return 0.5f * (RU[q] + RU[q - HALO_W]); },
-                 [&](int q) { return 0.5f * (RV[q] + RV[q - HALO_W]); }, tx, ty);
-      __syncthreads();
-      if (tid == 0 && k + TEND_RING - 1 <= k1) ring.issue(k + TEND_RING - 1, maps, x0, z0, m.kms);
-      if (!acc) continue;
-      if (k + 2 <= kme) {
-        prefetch_l2(&rom(i, k + 2, j)); prefetch_l2(&p(i, k + 2, j)); prefetch_l2(&ph(i, k + 2, j));
-        prefetch_l2(&alt(i, k + 2, j)); prefetch_l2(&al(i, k + 2, j)); prefetch_l2(&pb(i, k + 2, j));
-        prefetch_l2(&php(i, k + 2, j)); prefetch_l2(&cqv(i, k + 2, j)); prefetch_l2(&rw(i, k + 2, j));
-        prefetch_l2(&u(i, k + 2, j)); prefetch_l2(&tend(i, k + 2, j));
-      }
-      const LevelIn q = load_in(k);
-      float t = q.t;
-      t = t - mrdy * (FY[(ty + 1) * TX + tx] - FY[ty * TX + tx]);
-      t = t - mrdx * (FX[ty * (TX + 1) + tx + 1] - FX[ty * (TX + 1) + tx]);
-      {
-        const int kk = k + 1;
-        float vf_hi;
-        if (kk == kts || kk == kte) vf_hi = 0.f;
-        else if (kk == kts + 1 || kk == ktf)
-          vf_hi = 0.5f * q.romsum * (fzm(kk) * vp1 + fzp(kk) * v0);
-        else {
-          const float vel = 0.5f * q.romsum;
-          vf_hi = vel * flux3(vm1, v0, vp1, vp2, -vel);
-        }
-        t = t - ratio * rdzw(k) * (vf_hi - vf_lo);
-        vf_lo = vf_hi;
-      }
-      if (FL & TF_PG) {
-        const int kk = k + 1;
-        float dpn_hi;
-        if (kk == kde) {
-          if (m.cf.top_lid)
-            dpn_hi = .5f * (m.cfn * (p(i, kde - 1, j - 1) + p(i, kde - 1, j)) +
-                            m.cfn1 * (p(i, kde - 2, j - 1) + p(i, kde - 2, j)));
-          else dpn_hi = 0.f;
-        } else {
-          dpn_hi = .5f * (fzm(kk) * (q.p_l1 + q.p_r1) + fzp(kk) * (p_l + p_r));
-        }
-        float dpy = pgA * (c1h(k) * muv_c + c2h(k)) *
-                    ((q.ph_r1 - q.ph_l1 + ph_r - ph_l) + q.altsum * (p_r - p_l) + q.alsum * q.pbd);
-        dpy = dpy + pgB * q.phpd * (rdzw(k) * (dpn_hi - dpn_lo) - .5f * ((c1h(k) * mu_l) + (c1h(k) * mu_r)));
-        t = t - q.cq * dpy;
-        dpn_lo = dpn_hi;
-        p_l = q.p_l1; p_r = q.p_r1; ph_l = q.ph_l1; ph_r = q.ph_r1;
-      }
-      if (FL & (TF_COR | TF_CURV)) {
-        const float rusum = RU[o] + RU[o + 1] + RU[o - HALO_W] + RU[o - HALO_W + 1];
-        const float rwsum = q.rw_l1 + rw_l + q.rw_r1 + rw_r;
-        if (FL & TF_COR) t = t - corA * rusum + corB * rwsum;
-        if (FL & TF_CURV) {
-          const float vx_r = 0.5f * q.cs_r * dvx_r * rdy - 0.5f * (v0 + V[o + HALO_W]) * duy_r * rdx;
-          const float vx_l = 0.5f * q.cs_l * dvx_l * rdy - 0.5f * (V[o - HALO_W] + v0) * duy_l * rdx;
-          t = t - 0.5f * (vx_r + vx_l) * 0.25f * rusum - ratio * v0 * RERADIUS * 0.25f * rwsum;
-        }
-      }
-      rw_l = q.rw_l1; rw_r = q.rw_r1;
-      tend(i, k, j) = t;
-      vm1 = v0; v0 = vp1; vp1 = vp2; vp2 = q.f3;
-    }
-    if (!ok && tid == 0) raise_err(m, ERR_TIMEOUT);
+  if (tp.i0 > iacc || tp.j0 > jacc || k0 > k1) return;  // block-uniform
+  const F3 fld = f3(m, DIR ? WRFGPU_V_2 : WRFGPU_U_2), crs = f3(m, DIR ? WRFGPU_U_2 : WRFGPU_V_2),
+           rw = f3(m, WRFGPU_RW), rom = f3(m, WRFGPU_WW);
+  const F3 ph = f3(m, WRFGPU_PH_2), alt = f3(m, WRFGPU_ALT), p = f3(m, WRFGPU_P), pb = f3(m, WRFGPU_PB),
+           al = f3(m, WRFGPU_AL), php = f3(m, WRFGPU_PHP), cq = f3(m, DIR ? WRFGPU_CQV : WRFGPU_CQU);
+  const F1 fzm = f1(m, WRFGPU_FNM), fzp = f1(m, WRFGPU_FNP), rdzw = f1(m, WRFGPU_RDNW), c1h = f1(m, WRFGPU_C1H),
+           c2h = f1(m, WRFGPU_C2H);
+  const float rdx = m.rdx, rdy = m.rdy, rd = DIR ? rdy : rdx;
+  HaloRing ring;
+  ring.init(smem, k0);
+  float* FXb = (float*)(smem + HaloRing::SMEM);
+  float* FYb = FXb + 2 * FXN2;
+  const CUtensorMap* maps[3] = {tmap_of(m, DIR ? WRFGPU_V_2 : WRFGPU_U_2, BOX_HALO), tmap_of(m, WRFGPU_RU, BOX_HALO),
+                                tmap_of(m, WRFGPU_RV, BOX_HALO)};
+  const int x0 = tp.i0 - TMA_HALO - m.ims, z0 = tp.j0 - TMA_HALO - m.jms;
+  if (tid == 0) {
+    ring.init_barriers();
+    mbar_fence_init();
   }
-  if ((FL & TF_ZERO) && acc && blockIdx.y == gridDim.y - 1)
-    for (int k = ktf + 1; k <= kte; ++k) tend(i, k, j) = 0.f;
+  __syncthreads();
+  if (tid == 0)
+    for (int d = 0; d < TEND_RING - 1 && k0 + d <= k1; ++d) ring.issue(k0 + d, maps, x0, z0, m.kms);
+  auto mul = [](float2 a, float2 b) { return make_float2(a.x * b.x, a.y * b.y); };
+  auto div = [](float2 a, float2 b) { return make_float2(a.x / b.x, a.y / b.y); };
+  auto at2 = [](const float* q) { return *reinterpret_cast<const float2*>(q); };
+  // the pair's own value, its first neighbours' (DIR) given the own one, and at another point
+  auto own = [&](const F3& a, int k) { return at2(a.p + a.off(i, k, j)); };
+  auto low = [&](const F3& a, int k, float2 o) {
+    return DIR ? at2(a.p + a.off(i, k, j - 1)) : make_float2(a(i - 1, k, j), o.x);
+  };
+  auto sum = [&](const F3& a, int k) { const float2 o = own(a, k); return add2(o, low(a, k, o)); };
+  auto dif = [&](const F3& a, int k) { const float2 o = own(a, k); return sub2(o, low(a, k, o)); };
+  auto g2 = [&](int f, int ii, int jj) { const F2 a = f2(m, f); return make_float2(a(ii, jj), a(ii + 1, jj)); };
+  // column constants, formed in the order of the per-level expressions
+  float2 mrdy, mrdx, ratio, pgA, pgB, mu_c, mu_l, mu_r, corA, corB, dvx_l, dvx_r, duy_l, duy_r;
+  // own-column window of the field (k-1 .. k+2), the vertical flux of face k,
+  // and the pressure-gradient / rw carries (formed afresh at the chunk's first
+  // level, with the same expressions as one level down)
+  float2 fm1 = bc2(0.f), f0, fp1, fp2 = bc2(0.f), vf_lo = bc2(0.f), p_l, p_r, ph_l, ph_r, dpn_lo, rw_l, rw_r;
+  if (acc) {
+    constexpr int il = DIR ? 0 : 1, jl = DIR ? 1 : 0;
+    const float2 ma = g2(DIR ? WRFGPU_MSFVY : WRFGPU_MSFUX, i, j);
+    mrdy = muls(rdy, ma); mrdx = muls(rdx, ma);
+    ratio = div(ma, g2(DIR ? WRFGPU_MSFVX : WRFGPU_MSFUY, i, j));
+    pgA = muls(rd, muls(.5f, ratio)); pgB = muls(rd, ratio);
+    mu_c = g2(DIR ? WRFGPU_MUV : WRFGPU_MUU, i, j);
+    mu_l = g2(WRFGPU_MU_2, i - il, j - jl);
+    mu_r = g2(WRFGPU_MU_2, i, j);
+    corA = muls(0.25f, mul(muls(0.5f, ratio), add2(g2(WRFGPU_F, i, j), g2(WRFGPU_F, i - il, j - jl))));
+    const float2 es = add2(g2(WRFGPU_E, i, j), g2(WRFGPU_E, i - il, j - jl));
+    const int cs = DIR ? WRFGPU_SINA : WRFGPU_COSA;
+    const float2 ca = add2(g2(cs, i, j), g2(cs, i - il, j - jl));
+    corB = muls(0.25f, mul(muls(0.5f, DIR ? mul(muls(0.5f, ratio), es) : muls(0.5f, es)), ca));
+    dvx_r = sub2(g2(WRFGPU_MSFVX, i, j + 1), g2(WRFGPU_MSFVX, i, j));
+    dvx_l = sub2(g2(WRFGPU_MSFVX, i - il, j + 1 - jl), g2(WRFGPU_MSFVX, i - il, j - jl));
+    duy_r = sub2(g2(WRFGPU_MSFUY, i + 1, j), g2(WRFGPU_MSFUY, i, j));
+    duy_l = sub2(g2(WRFGPU_MSFUY, i + 1 - il, j - jl), g2(WRFGPU_MSFUY, i - il, j - jl));
+    if (k0 - 1 >= kts) fm1 = own(fld, k0 - 1);
+    f0 = own(fld, k0); fp1 = own(fld, k0 + 1);
+    if (k0 + 2 <= kme) fp2 = own(fld, k0 + 2);
+    if (k0 != kts && k0 != kte) {
+      const float2 vel = muls(0.5f, sum(rom, k0));
+      if (k0 == kts + 1 || k0 == ktf) vf_lo = mul(vel, add2(muls(fzm(k0), f0), muls(fzp(k0), fm1)));
+      else vf_lo = mul(vel, flux3_c2(own(fld, k0 - 2), fm1, f0, fp1, make_float2(-vel.x, -vel.y)));
+    }
+    p_r = own(p, k0); p_l = low(p, k0, p_r);
+    ph_r = own(ph, k0); ph_l = low(ph, k0, ph_r);
+    if (k0 == 1) dpn_lo = muls(.5f, add2(add2(muls(m.cf1, sum(p, 1)), muls(m.cf2, sum(p, 2))), muls(m.cf3, sum(p, 3))));
+    else dpn_lo = muls(.5f, add2(muls(fzm(k0), add2(p_l, p_r)), muls(fzp(k0), sum(p, k0 - 1))));
+    rw_r = own(rw, k0); rw_l = low(rw, k0, rw_r);
+  }
+  const int o = (ty + TMA_HALO) * HALO_W + c + TMA_HALO;  // own first point in the halo planes
+  constexpr int W = HALO_W, d = DIR ? W : 1;
+  bool ok = true;
+  for (int k = k0; k <= k1; ++k) {
+    ok = ring.wait(k) && ok;
+    const float* Q = ring.plane(k, 0);
+    const float* RU = ring.plane(k, 1);
+    const float* RV = ring.plane(k, 2);
+    float* FX = FXb + (k & 1) * FXN2;
+    float* FY = FYb + (k & 1) * FYN;
+    // face velocities at the two columns from q on: 0.5 (r(q) + r(q - d))
+    auto vel2 = [&](const float* R, int q) {
+      const float2 a = at2(R + q);
+      return muls(0.5f, add2(a, DIR ? at2(R + q - W) : make_float2(R[q - 1], a.x)));
+    };
+    auto yfaces = [&](int q) {
+      const float2 vel = vel2(RV, q);
+      return mul(vel, flux5_c2(at2(Q + q - 3 * W), at2(Q + q - 2 * W), at2(Q + q - W), at2(Q + q), at2(Q + q + W),
+                               at2(Q + q + 2 * W), vel));
+    };
+    // own left faces (columns c, c + 1) and bottom faces
+    const float2 q2 = at2(Q + o), qm = at2(Q + o - 2), qp = at2(Q + o + 2);
+    float2 fx, fy;
+    {
+      const float2 vel = vel2(RU, o);
+      fx = mul(vel, flux5_c2(make_float2(Q[o - 3], qm.x), qm, make_float2(qm.y, q2.x), q2, make_float2(q2.y, qp.x), qp,
+                             vel));
+      fy = yfaces(o);
+    }
+    *reinterpret_cast<float2*>(FX + ty * FX2 + c) = fx;
+    *reinterpret_cast<float2*>(FY + ty * TX + c) = fy;
+    if (tid >= 96 && tid < 96 + TY) {  // the last column's right faces
+      const int r = tid - 96, q = (r + TMA_HALO) * W + TX + TMA_HALO;
+      const float vel = 0.5f * (RU[q] + RU[q - d]);
+      FX[r * FX2 + TX] = vel * flux5(Q[q - 3], Q[q - 2], Q[q - 1], Q[q], Q[q + 1], Q[q + 2], vel);
+    }
+    if (tid >= 64 && tid < 80)  // the last row's top faces
+      *reinterpret_cast<float2*>(FY + TY * TX + c) = yfaces((TY + TMA_HALO) * W + c + TMA_HALO);
+    __syncthreads();
+    // the slot of level k-1, which every thread has finished with
+    if (tid == 0 && k + TEND_RING - 1 <= k1) ring.issue(k + TEND_RING - 1, maps, x0, z0, m.kms);
+    if (!acc) continue;
+    if (k + 2 <= kme) {
+      prefetch_l2(&rom(i, k + 2, j)); prefetch_l2(&p(i, k + 2, j)); prefetch_l2(&ph(i, k + 2, j));
+      prefetch_l2(&alt(i, k + 2, j)); prefetch_l2(&al(i, k + 2, j)); prefetch_l2(&pb(i, k + 2, j));
+      prefetch_l2(&php(i, k + 2, j)); prefetch_l2(&cq(i, k + 2, j)); prefetch_l2(&rw(i, k + 2, j));
+      prefetch_l2(&crs(i, k + 2, j));
+    }
+    // the level's own-column inputs go out together
+    const int kk = k + 1;
+    const float2 fp3 = k + 3 <= kme ? own(fld, k + 3) : bc2(0.f);
+    const float2 romsum = (kk == kts || kk == kte) ? bc2(0.f) : sum(rom, kk);
+    const float2 rw_r1 = own(rw, kk), rw_l1 = low(rw, kk, rw_r1);
+    float2 p_r1 = bc2(0.f), p_l1 = bc2(0.f);
+    if (kk != kde) { p_r1 = own(p, kk); p_l1 = low(p, kk, p_r1); }
+    const float2 ph_r1 = own(ph, kk), ph_l1 = low(ph, kk, ph_r1);
+    const float2 altsum = sum(alt, k), alsum = sum(al, k), pbd = dif(pb, k), phpd = dif(php, k), cqk = own(cq, k);
+    // the two sums of the cross velocity: of the point and of its lower neighbour
+    float2 cs_r, cs_l;
+    {
+      const float2 a = own(crs, k);
+      if (DIR) {
+        const float2 b = at2(crs.p + crs.off(i, k, j - 1));
+        cs_r = make_float2(a.x + a.y, a.y + crs(i + 2, k, j));
+        cs_l = make_float2(b.x + b.y, b.y + crs(i + 2, k, j - 1));
+      } else {
+        cs_r = add2(a, at2(crs.p + crs.off(i, k, j + 1)));
+        cs_l = make_float2(crs(i - 1, k, j) + crs(i - 1, k, j + 1), cs_r.x);
+      }
+    }
+    float2 t = bc2(0.f);
+    t = sub2(t, mul(mrdy, sub2(at2(FY + (ty + 1) * TX + c), fy)));
+    t = sub2(t, mul(mrdx, sub2(make_float2(fx.y, FX[ty * FX2 + c + 2]), fx)));
+    const float rz = rdzw(k);
+    {  // vertical flux of face k+1
+      float2 vf_hi = bc2(0.f);
+      if (kk != kts && kk != kte) {
+        const float2 vel = muls(0.5f, romsum);
+        if (kk == kts + 1 || kk == ktf) vf_hi = mul(vel, add2(muls(fzm(kk), fp1), muls(fzp(kk), f0)));
+        else vf_hi = mul(vel, flux3_c2(fm1, f0, fp1, fp2, make_float2(-vel.x, -vel.y)));
+      }
+      t = sub2(t, mul(DIR ? muls(rz, ratio) : bc2(rz), sub2(vf_hi, vf_lo)));
+      vf_lo = vf_hi;
+    }
+    {  // horizontal_pressure_gradient
+      float2 dpn_hi = bc2(0.f);
+      if (kk == kde) {
+        if (m.cf.top_lid) dpn_hi = muls(.5f, add2(muls(m.cfn, sum(p, kde - 1)), muls(m.cfn1, sum(p, kde - 2))));
+      } else {
+        dpn_hi = muls(.5f, add2(muls(fzm(kk), add2(p_l1, p_r1)), muls(fzp(kk), add2(p_l, p_r))));
+      }
+      const float h1 = c1h(k), h2 = c2h(k);
+      float2 dp = mul(mul(pgA, add2(muls(h1, mu_c), bc2(h2))),
+                      add2(add2(sub2(add2(sub2(ph_r1, ph_l1), ph_r), ph_l), mul(altsum, sub2(p_r, p_l))), mul(alsum, pbd)));
+      dp = add2(dp, mul(mul(pgB, phpd),
+                        sub2(muls(rz, sub2(dpn_hi, dpn_lo)), muls(.5f, add2(muls(h1, mu_l), muls(h1, mu_r))))));
+      t = sub2(t, mul(cqk, dp));
+      dpn_lo = dpn_hi;
+      p_l = p_l1; p_r = p_r1; ph_l = ph_l1; ph_r = ph_r1;
+    }
+    {  // coriolis, curvature
+      const float2 rwsum = add2(add2(add2(rw_l1, rw_l), rw_r1), rw_r);
+      float2 rsum, vx_r, vx_l;
+      if (DIR) {
+        const float2 a = at2(RU + o), b = at2(RU + o - W);
+        rsum = add2(add2(add2(a, make_float2(a.y, RU[o + 2])), b), make_float2(b.y, RU[o - W + 2]));
+        t = add2(sub2(t, mul(corA, rsum)), mul(corB, rwsum));
+        vx_r = sub2(muls(rdy, mul(muls(0.5f, cs_r), dvx_r)), muls(rdx, mul(muls(0.5f, add2(f0, at2(Q + o + W))), duy_r)));
+        vx_l = sub2(muls(rdy, mul(muls(0.5f, cs_l), dvx_l)), muls(rdx, mul(muls(0.5f, add2(at2(Q + o - W), f0)), duy_l)));
+        t = sub2(sub2(t, mul(muls(0.25f, muls(0.5f, add2(vx_r, vx_l))), rsum)),
+                 mul(muls(0.25f, muls(RERADIUS, mul(ratio, f0))), rwsum));
+      } else {
+        const float2 a = at2(RV + o), b = at2(RV + o + W);
+        rsum = add2(add2(add2(make_float2(RV[o + W - 1], b.x), b), make_float2(RV[o - 1], a.x)), a);
+        t = sub2(add2(t, mul(corA, rsum)), mul(corB, rwsum));
+        vx_r = sub2(muls(rdy, mul(muls(0.5f, add2(f0, make_float2(q2.y, qp.x))), dvx_r)), muls(rdx, mul(muls(0.5f, cs_r), duy_r)));
+        vx_l = sub2(muls(rdy, mul(muls(0.5f, add2(make_float2(qm.y, q2.x), f0)), dvx_l)), muls(rdx, mul(muls(0.5f, cs_l), duy_l)));
+        t = sub2(add2(t, mul(muls(0.25f, muls(0.5f, add2(vx_r, vx_l))), rsum)), mul(muls(0.25f, muls(RERADIUS, f0)), rwsum));
+      }
+    }
+    rw_l = rw_l1; rw_r = rw_r1;
+    if (acc1) *reinterpret_cast<float2*>(tend.p + tend.off(i, k, j)) = t;
+    else tend(i, k, j) = t.x;
+    fm1 = f0; f0 = fp1; fp1 = fp2; fp2 = fp3;
+  }
+  if (!ok && tid == 0) raise_err(m, ERR_TIMEOUT);
 }
 
 // ---------------------------------------------------------------- rw_tend
@@ -899,20 +750,19 @@ __global__ void __launch_bounds__(TX* TY, 4) k_tend_ph_col(TileLaunch L) {
 // The shortest level chunk of the staged tendencies.
 constexpr int TEND_MINLEV = 4;
 
-// variant parameter: 10 x blocks per SM + level chunks
-void launch_tend_u_col(const TileLaunch& L, int nb, int flags, cudaStream_t s, int var) {
-  const int p = TUNE_PARAM[TU_TENDU][var];
+// variant parameter: 10 x blocks per SM + level chunks (4: as many registers
+// as 5 blocks of 128 threads leave, else 4)
+template <int DIR>
+static void launch_tend_uv(const TileLaunch& L, int nb, cudaStream_t s, int p) {
   const dim3 grid(nb, level_chunks(nb, L.nlev, p % 10, TEND_MINLEV));
-  if (flags != TF_ALL) return;
-  if (p / 10 == 4) k_tend_u_col<TF_ALL, 4><<<grid, dim3(TX, TY), TEND_SMEM, s>>>(L);
-  else k_tend_u_col<TF_ALL, 3><<<grid, dim3(TX, TY), TEND_SMEM, s>>>(L);
+  if (p / 10 == 4) k_tend_uv_col<DIR, 5><<<grid, TEND2_THREADS, TEND2_SMEM, s>>>(L);
+  else k_tend_uv_col<DIR, 4><<<grid, TEND2_THREADS, TEND2_SMEM, s>>>(L);
 }
-void launch_tend_v_col(const TileLaunch& L, int nb, int flags, cudaStream_t s, int var) {
-  const int p = TUNE_PARAM[TU_TENDV][var];
-  const dim3 grid(nb, level_chunks(nb, L.nlev, p % 10, TEND_MINLEV));
-  if (flags != TF_ALL) return;
-  if (p / 10 == 4) k_tend_v_col<TF_ALL, 4><<<grid, dim3(TX, TY), TEND_SMEM, s>>>(L);
-  else k_tend_v_col<TF_ALL, 3><<<grid, dim3(TX, TY), TEND_SMEM, s>>>(L);
+void launch_tend_u_col(const TileLaunch& L, int nb, cudaStream_t s, int var) {
+  launch_tend_uv<0>(L, nb, s, TUNE_PARAM[TU_TENDU][var]);
+}
+void launch_tend_v_col(const TileLaunch& L, int nb, cudaStream_t s, int var) {
+  launch_tend_uv<1>(L, nb, s, TUNE_PARAM[TU_TENDV][var]);
 }
 void launch_tend_w_col(const TileLaunch& L, int nb, int var, cudaStream_t s) {
   static bool attr = false;

@@ -64,7 +64,7 @@ constexpr int TUNE_NVAR[NTUNE] = {2, 3, 3, 4, 4, 2, 2, 4, 4, 3, 4, 4, 4, 4};
 // (defaults measured on 512x512x80 and up: advance_mu_t 278 us with four blocks
 // per SM against 393 with two, advance_w 340 against 388; the FP64 form of
 // advance_mu_t is best with three, 524 against 571 us on the 16-member ensemble)
-constexpr int TUNE_DEFAULT[NTUNE] = {1, 1, 2, 0, 2, 1, 0, 2, 2, 1, 3, 3, 2, 2};
+constexpr int TUNE_DEFAULT[NTUNE] = {1, 1, 2, 0, 2, 1, 0, 2, 2, 1, 3, 2, 2, 2};
 // the parameter each variant stands for: blocks per SM, level chunks
 // (sumflux: of calc_p_rho), or (advance_uv, rk_tend_u, rk_tend_v) 10 x blocks
 // per SM + level chunks
@@ -89,8 +89,8 @@ void launch_tend_w_col(const TileLaunch& L, int nblocks, int var, cudaStream_t s
 void launch_tend_t(const Launch& L3, int nblocks, int flags, cudaStream_t s);
 void launch_tend_ph(const Launch& L3, int nblocks, int flags, cudaStream_t s);
 // column forms over tiles of the staggered extents
-void launch_tend_u_col(const TileLaunch& L, int nblocks, int flags, cudaStream_t s, int var = 0);
-void launch_tend_v_col(const TileLaunch& L, int nblocks, int flags, cudaStream_t s, int var = 0);
+void launch_tend_u_col(const TileLaunch& L, int nblocks, cudaStream_t s, int var = 0);
+void launch_tend_v_col(const TileLaunch& L, int nblocks, cudaStream_t s, int var = 0);
 void launch_tend_t_col(const TileLaunch& L, int nblocks, int flags, cudaStream_t s);
 void launch_tend_ph_col(const TileLaunch& L, int nblocks, int flags, cudaStream_t s);
 // sixth-order diffusion of the dry state at stage 1, and rk_addtend_dry (k_diff.cu)

@@ -102,6 +102,19 @@ __device__ __forceinline__ float2 flux3_2(float2 qm2, float2 qm1, float2 q, floa
   return div_const_pair2(x, y, 1.0f, 12.0f, 1.0f / 12.0f);
 }
 
+// flux5 / flux3 of two adjacent columns in the lanes, each with its own face velocity
+__device__ __forceinline__ float2 flux5_c2(float2 qm3, float2 qm2, float2 qm1, float2 q, float2 qp1, float2 qp2,
+                                           float2 ua) {
+  const float2 x = add2(sub2(muls(37.f, add2(q, qm1)), muls(8.f, add2(qp1, qm2))), add2(qp2, qm3));
+  const float2 d = add2(sub2(sub2(qp2, qm3), muls(5.f, sub2(qp1, qm2))), muls(10.f, sub2(q, qm1)));
+  return div_const_pair2(x, make_float2(1.f * sgn1(ua.x) * d.x, 1.f * sgn1(ua.y) * d.y), -1.0f, 60.0f, 1.0f / 60.0f);
+}
+__device__ __forceinline__ float2 flux3_c2(float2 qm2, float2 qm1, float2 q, float2 qp1, float2 ua) {
+  const float2 x = sub2(muls(7.f, add2(q, qm1)), add2(qp1, qm2));
+  const float2 d = sub2(sub2(qp1, qm2), muls(3.f, sub2(q, qm1)));
+  return div_const_pair2(x, make_float2(1.f * sgn1(ua.x) * d.x, 1.f * sgn1(ua.y) * d.y), 1.0f, 12.0f, 1.0f / 12.0f);
+}
+
 __device__ __forceinline__ float2 max0_2(float2 x) { return make_float2(fmaxf_f(0.f, x.x), fmaxf_f(0.f, x.y)); }
 __device__ __forceinline__ float2 min0_2(float2 x) { return make_float2(fminf_f(0.f, x.x), fminf_f(0.f, x.y)); }
 
