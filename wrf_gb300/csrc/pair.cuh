@@ -69,37 +69,29 @@ __device__ __forceinline__ float2 flux_upwind_2(float2 qm1, float2 q, Upw w) {
   return add2(muls(w.a, qm1), muls(w.b, q));
 }
 
-// wrfgpu_div_const_pair (cdiv.h) of both lanes: x / c + s y / c with each
-// quotient rounded as IEEE division.  When every numerator of both lanes is
-// in the method's range the two lanes go through the packed fused
-// multiply-adds together (each lane the scalar method's operations);
-// otherwise each lane takes the scalar function.
-__device__ __forceinline__ bool div_range_ok(float x, float y) {
-  const float ax = fabsf(x), ay = fabsf(y);
-  const float lo = ax < ay ? ax : ay, hi = ax < ay ? ay : ax;
-  return lo >= 0x1p-110f && hi <= 3.40282347e38f;
-}
-__device__ __forceinline__ float2 div_const_pair2(float2 x, float2 y, float s, float c, float zh) {
-  if (div_range_ok(x.x, y.x) && div_range_ok(x.y, y.y)) {
-    const float2 z2 = bc2(zh), nc2 = bc2(-c);
-    const float2 qx = mul2(x, z2), qy = mul2(y, z2);
-    const float2 rx = fma2(qx, nc2, x), ry = fma2(qy, nc2, y);
-    const float2 a = fma2(rx, z2, qx), b = fma2(ry, z2, qy);
-    return s > 0.f ? add2(a, b) : sub2(a, b);
-  }
-  return make_float2(wrfgpu_div_const_pair(x.x, y.x, s, c, zh), wrfgpu_div_const_pair(x.y, y.y, s, c, zh));
+// wrfgpu_div_const_sub (cdiv.h) of both lanes: x / c - y / c with each quotient
+// rounded as IEEE division, one test for the four numerators and the two
+// results; where it fails each lane takes the scalar function.
+__device__ __forceinline__ float2 div_const_sub2(float2 x, float2 y, float c, float zh) {
+  const unsigned k = min(min(wrfgpu_div_key(x.x), wrfgpu_div_key(x.y)), min(wrfgpu_div_key(y.x), wrfgpu_div_key(y.y)));
+  const float2 nz = bc2(-zh), c2 = bc2(c);
+  const float2 qx = muls(-zh, x), qy = muls(-zh, y);
+  const float2 wx = fma2(fma2(qx, c2, x), nz, qx), wy = fma2(fma2(qy, c2, y), nz, qy);
+  const float2 z = sub2(wy, wx);
+  if (k >= WRFGPU_DIV_MIN && fabsf(z.x) <= 3.40282347e38f && fabsf(z.y) <= 3.40282347e38f) return z;
+  return make_float2(wrfgpu_div_const_sub(x.x, y.x, c, zh), wrfgpu_div_const_sub(x.y, y.y, c, zh));
 }
 // flux5 / flux3 (common.cuh) of both lanes
 __device__ __forceinline__ float2 flux5_2(float2 qm3, float2 qm2, float2 qm1, float2 q, float2 qp1, float2 qp2,
                                           float ua) {
   const float2 x = add2(sub2(muls(37.f, add2(q, qm1)), muls(8.f, add2(qp1, qm2))), add2(qp2, qm3));
   const float2 y = muls(1.f * sgn1(ua), add2(sub2(sub2(qp2, qm3), muls(5.f, sub2(qp1, qm2))), muls(10.f, sub2(q, qm1))));
-  return div_const_pair2(x, y, -1.0f, 60.0f, 1.0f / 60.0f);
+  return div_const_sub2(x, y, 60.0f, 1.0f / 60.0f);
 }
 __device__ __forceinline__ float2 flux3_2(float2 qm2, float2 qm1, float2 q, float2 qp1, float ua) {
   const float2 x = sub2(muls(7.f, add2(q, qm1)), add2(qp1, qm2));
-  const float2 y = muls(1.f * sgn1(ua), sub2(sub2(qp1, qm2), muls(3.f, sub2(q, qm1))));
-  return div_const_pair2(x, y, 1.0f, 12.0f, 1.0f / 12.0f);
+  const float2 y = muls(sgn1(-ua), sub2(sub2(qp1, qm2), muls(3.f, sub2(q, qm1))));  // minus the reference's
+  return div_const_sub2(x, y, 12.0f, 1.0f / 12.0f);
 }
 
 // flux5 / flux3 of two adjacent columns in the lanes, each with its own face velocity
@@ -107,12 +99,12 @@ __device__ __forceinline__ float2 flux5_c2(float2 qm3, float2 qm2, float2 qm1, f
                                            float2 ua) {
   const float2 x = add2(sub2(muls(37.f, add2(q, qm1)), muls(8.f, add2(qp1, qm2))), add2(qp2, qm3));
   const float2 d = add2(sub2(sub2(qp2, qm3), muls(5.f, sub2(qp1, qm2))), muls(10.f, sub2(q, qm1)));
-  return div_const_pair2(x, make_float2(1.f * sgn1(ua.x) * d.x, 1.f * sgn1(ua.y) * d.y), -1.0f, 60.0f, 1.0f / 60.0f);
+  return div_const_sub2(x, make_float2(sgn1(ua.x) * d.x, sgn1(ua.y) * d.y), 60.0f, 1.0f / 60.0f);
 }
 __device__ __forceinline__ float2 flux3_c2(float2 qm2, float2 qm1, float2 q, float2 qp1, float2 ua) {
   const float2 x = sub2(muls(7.f, add2(q, qm1)), add2(qp1, qm2));
   const float2 d = sub2(sub2(qp1, qm2), muls(3.f, sub2(q, qm1)));
-  return div_const_pair2(x, make_float2(1.f * sgn1(ua.x) * d.x, 1.f * sgn1(ua.y) * d.y), 1.0f, 12.0f, 1.0f / 12.0f);
+  return div_const_sub2(x, make_float2(sgn1(-ua.x) * d.x, sgn1(-ua.y) * d.y), 12.0f, 1.0f / 12.0f);
 }
 
 __device__ __forceinline__ float2 max0_2(float2 x) { return make_float2(fmaxf_f(0.f, x.x), fmaxf_f(0.f, x.y)); }
