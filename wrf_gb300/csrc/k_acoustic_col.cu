@@ -1008,26 +1008,33 @@ __global__ void __launch_bounds__(32 * COL_MAXW, 1) k_advance_col(TileLaunch L, 
       x_m = *reinterpret_cast<const float2*>(sX + (hw - 1) * 32 + c);
     }
     float2 r_m = bc2(0.f), ph_m = bc2(0.f);
-    for (int k = ka; k <= kb; ++k) {
-      c_c2a = gro(c2a, i, k, j);
-      const float2 ph_p = g(ph, k + 1), r_p = rdf(sR, k + 1);
-      const P xr = rd(sW, k);
-      const float2 x = make_float2((float)xr.x, (float)xr.y);
-      const float2 c_w = g(w, k), c_rwt = gro(rwt, i, k, j), c_cqw = gro(cqw, i, k, j);
-      const P ca = coef(0, k), cal = coef(1, k), cga = coef(2, k);
-      const float2 dz_k = dz(k, c_c2a, r_k, r_p, ph_k, ph_p);
-      if (k >= 2) {
-        const float rdnk = rdn(k);
-        const float2 wk = add2(add2(add2(c_w, muls(dts, c_rwt)),
-                                    mul(mul(msft_inv, c_cqw), muls(+.5f * dts * G * rdnk, sub2(dz_k, dz_m)))),
-                               mul(muls(dts * G, msft_inv), sub2(muls(rdnk, sub2(x, x_m)), muls(tA[k].z, mua))));
-        wr(sW, k, (RC)wk.x, (RC)wk.y);
-        wr(sA, k, ca.x, ca.y);
-        wr(sAL, k, cal.x, cal.y);
-        wr(sGA, k, cga.x, cga.y);
-      }
-      dz_m = dz_k; x_m = x; r_m = r_k; ph_m = ph_k; r_k = r_p; ph_k = ph_p;
-    }
+    // (the loads of two levels go out together)
+    struct L4 { float2 c2a, ph, w, rwt, cqw; P a, al, ga; };
+    chunked_levels<2, L4>(
+        ka, kb,
+        [&](int k, L4& d) {
+          d.c2a = gro(c2a, i, k, j); d.ph = g(ph, k + 1); d.w = g(w, k);
+          d.rwt = gro(rwt, i, k, j); d.cqw = gro(cqw, i, k, j);
+          d.a = coef(0, k); d.al = coef(1, k); d.ga = coef(2, k);
+        },
+        [&](int k, const L4& d) {
+          c_c2a = d.c2a;
+          const float2 ph_p = d.ph, r_p = rdf(sR, k + 1);
+          const P xr = rd(sW, k);
+          const float2 x = make_float2((float)xr.x, (float)xr.y);
+          const float2 dz_k = dz(k, c_c2a, r_k, r_p, ph_k, ph_p);
+          if (k >= 2) {
+            const float rdnk = rdn(k);
+            const float2 wk = add2(add2(add2(d.w, muls(dts, d.rwt)),
+                                        mul(mul(msft_inv, d.cqw), muls(+.5f * dts * G * rdnk, sub2(dz_k, dz_m)))),
+                                   mul(muls(dts * G, msft_inv), sub2(muls(rdnk, sub2(x, x_m)), muls(tA[k].z, mua))));
+            wr(sW, k, (RC)wk.x, (RC)wk.y);
+            wr(sA, k, d.a.x, d.a.y);
+            wr(sAL, k, d.al.x, d.al.y);
+            wr(sGA, k, d.ga.x, d.ga.y);
+          }
+          dz_m = dz_k; x_m = x; r_m = r_k; ph_m = ph_k; r_k = r_p; ph_k = ph_p;
+        });
     if (hw == 0) wr(sW, 1, (RC)w1.x, (RC)w1.y);
     if (top) {
       const int k = kde;
@@ -1151,23 +1158,25 @@ __global__ void __launch_bounds__(32 * COL_MAXW, 1) k_advance_col(TileLaunch L, 
     ph_k = new_ph(ka, wst);
     put_img(ph, ka, ph_k);
   }
-  for (int k = ka; k <= kb; ++k) {
-    const float2 a = gro(alt, i, k, j), c_c2a = gro(c2a, i, k, j), c_pm1 = g(pm1, k);
-    const int kn = k + 1;
-    const float2 wst = new_w(kn), ph_n = new_ph(kn, wst);
-    if (kn <= kb || kn == kde) {  // else the next half warp's own level
-      put(w, kn, wst);
-      put_img(ph, kn, ph_n);
-    }
-    const float4 ta = tA[k];
-    const float2 alv = mul(div(bc2(-1.f), lin(ta.x, mts, ta.y)),
-                           add2(mul(a, muls(ta.x, mu)), muls(tB[k].y, sub2(ph_n, ph_k))));
-    put_img(al, k, alv);
-    const float2 pn = mul(c_c2a, sub2(rdf(sQ, k), alv));
-    put(pm1, k, pn);
-    put_img(p, k, add2(pn, muls(smdiv, sub2(pn, c_pm1))));
-    ph_k = ph_n;
-  }
+  struct L6 { float2 a, c2a, pm1; };
+  chunked_levels<2, L6>(
+      ka, kb, [&](int k, L6& d) { d.a = gro(alt, i, k, j); d.c2a = gro(c2a, i, k, j); d.pm1 = g(pm1, k); },
+      [&](int k, const L6& d) {
+        const int kn = k + 1;
+        const float2 wst = new_w(kn), ph_n = new_ph(kn, wst);
+        if (kn <= kb || kn == kde) {  // else the next half warp's own level
+          put(w, kn, wst);
+          put_img(ph, kn, ph_n);
+        }
+        const float4 ta = tA[k];
+        const float2 alv = mul(div(bc2(-1.f), lin(ta.x, mts, ta.y)),
+                               add2(mul(d.a, muls(ta.x, mu)), muls(tB[k].y, sub2(ph_n, ph_k))));
+        put_img(al, k, alv);
+        const float2 pn = mul(d.c2a, sub2(rdf(sQ, k), alv));
+        put(pm1, k, pn);
+        put_img(p, k, add2(pn, muls(smdiv, sub2(pn, d.pm1))));
+        ph_k = ph_n;
+      });
 }
 
 void launch_advance_col(const TileLaunch& L, int nblocks, int nlev_max, int rk_step, int iteration, bool fp64,
