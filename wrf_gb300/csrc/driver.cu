@@ -1037,19 +1037,24 @@ struct Ensemble {
       }
       // small_step_prep, calc_p_rho(step 0), calc_coef_w (solve_em.F:1089-1140)
       mark(PH_SSP); launch_small_step_prep(l2, nb2, LST(), nb_st, a, stream, tune[TU_SSP]);
-      const cudaStream_t sc = fork(0);  // the acoustic steps' coefficients beside p and the halo fill
+      // the acoustic steps' coefficients, p and al (whose halos their kernel
+      // stores itself, but for open boundaries' copies) and the halo fill of
+      // solve_em.F:1176-1264 side by side
+      const cudaStream_t sc = fork(0), sq = any_open ? stream : fork(1);
       mark(PH_COEFW);
       if (!fp64 && nb_rw <= COEF_ROW_MAX) launch_calc_coef_w_row(LRW(), nb_rw, a, sc);
       else launch_calc_coef_w_col(LTM(), nb_tm, a, fp64, sc);
-      mark(PH_CPR0); launch_calc_p_rho_col(LTM(), nb_tm, StepArgs{rk_step, 0, 0, 0}, stream);
-      {  // solve_em.F:1176-1264
+      mark(PH_CPR0); launch_calc_p_rho_col(LTM(), nb_tm, StepArgs{rk_step, 0, 0, 0}, sq);
+      {
         JobList j;
-        j.f3(WRFGPU_RU_TEND, 'u'); j.f3(WRFGPU_RV_TEND, 'v'); j.f3(WRFGPU_PH_2, 'w'); j.f3(WRFGPU_AL, 'p');
-        j.f3(WRFGPU_P, 'p'); j.f3(WRFGPU_T_1, 'p'); j.f3(WRFGPU_T_SAVE, 't');
+        j.f3(WRFGPU_RU_TEND, 'u'); j.f3(WRFGPU_RV_TEND, 'v'); j.f3(WRFGPU_PH_2, 'w');
+        if (any_open) { j.f3(WRFGPU_AL, 'p'); j.f3(WRFGPU_P, 'p'); }
+        j.f3(WRFGPU_T_1, 'p'); j.f3(WRFGPU_T_SAVE, 't');
         j.f2(WRFGPU_MU_1, 't'); j.f2(WRFGPU_MU_2, 't'); j.f2(WRFGPU_MUDF, 't');
         fill(j);
       }
       join(0);
+      if (!any_open) join(1);
       int nsmall_max = 0;
       for (int m = 0; m < nmem; ++m) nsmall_max = std::max(nsmall_max, stage_of(hm[m], rk_step).nsmall);
       for (int it = 1; it <= nsmall_max; ++it) {
@@ -1146,13 +1151,15 @@ struct Ensemble {
         species_filled = true;
         io_moist_out();
       }
-      mark(PH_CPRP); launch_calc_p_rho_phi_col(LTM(), nb_tm, stream, tune[TU_CPRP]);
+      // beside the fills below, which touch no interior point of what it reads or writes
+      mark(PH_CPRP); launch_calc_p_rho_phi_col(LTM(), nb_tm, fork(0), tune[TU_CPRP]);
       if (rk_step < 3) {
         JobList j;  // rk_phys_bc_dry_2 + species (solve_em.F:3240-3330)
         j.f3(WRFGPU_U_2, 'u'); j.f3(WRFGPU_V_2, 'v'); j.f3(WRFGPU_W_2, 'w'); j.f3(WRFGPU_T_2, 'p');
         j.f3(WRFGPU_PH_2, 'w'); j.f2(WRFGPU_MU_2, 't');
         for (int s = 0; s < nsp_max; ++s) j.sp(s, 0, 'p');
         fill(j);
+        join(0);
       }
     }
     {  // set_phys_bc_dry_2 of the _1 state + species (solve_em.F:4439-4535); the
@@ -1163,6 +1170,7 @@ struct Ensemble {
       if (!species_filled)
         for (int s = 0; s < nsp_max; ++s) j.sp(s, 0, 'p');
       fill(j);
+      join(0);
     }
     mark(PH_END);
   }

@@ -54,9 +54,10 @@ __device__ __forceinline__ bool open_copy(char v, bool f3d) {
 // grid: (blocks per job, jobs, members).  Work units: for the x halo
 // (periodic x) one (level, row) segment of nxw <= 9 points per thread, for
 // the y halo one (level, halo row, 128 points of i) piece per warp, four
-// points per lane.  A unit's loads are all issued before its stores (a store
-// may alias a later load as far as the compiler knows, so copying point by
-// point would wait out one memory latency per point).  The points written by
+// points per lane.  The loads of a thread's x unit and its warp's y unit are all
+// issued before the stores of either (a store may alias a later load as far as
+// the compiler knows, so copying point by point would wait out one memory
+// latency per point).  The points written by
 // the two kinds of unit are disjoint and every source point is an interior
 // point (or, without periodic x, a point no unit writes), so the units need
 // no ordering.
@@ -110,61 +111,62 @@ __global__ void k_fill_halo(const Mem* __restrict__ mems, HaloJobs jobs) {
   const int sk = (int)m.sk, sj = f3d ? (int)m.sj : (int)m.s2;
   auto off = [&](int i, int k, int j) { return (i - m.ims) + (f3d ? (k - m.kms) * sk : 0) + (j - m.jms) * sj; };
   const int tid = blockIdx.x * blockDim.x + threadIdx.x, nthr = gridDim.x * blockDim.x;
-  if (px || ox) {
-    const int nunits = nk * nxj;
-    for (int u = tid; u < nunits; u += nthr) {
-      const int kk = u / nxj;
-      const int r = u - kk * nxj, k = kk + m.kts;
-      const int tj = r <= xj1 - xj0 ? xj0 + r : (r == xj1 - xj0 + 1 ? m.jds - WRFGPU_HALO : m.jde + jstag + WRFGPU_HALO);
-      bool negj = false;
+  constexpr int PER = 4;  // points per lane of a y unit
+  const int lane = threadIdx.x & 31, warp = tid >> 5, nwarps = nthr >> 5;
+  const int npiece = (nyi + 32 * PER - 1) / (32 * PER);
+  const int nux = (px || ox) ? nk * nxj : 0, nuy = (py || sy || oy) ? nk * nyrows * npiece : 0;
+  // one x and one y unit at a time, the loads of both before the stores of either
+  for (int u = tid, w = warp; u < nux || w < nuy; u += nthr, w += nwarps) {
+    const bool ux = u < nux, uy = w < nuy;
+    float val[NXW_MAX], vy[PER];
+    bool neg[PER], negj = false;
+    int k = 0, tj = 0, ky = 0, tjy = 0, pc = 0;
+    if (ux) {
+      const int kk = u / nxj, r = u - kk * nxj;
+      k = kk + m.kts;
+      tj = r <= xj1 - xj0 ? xj0 + r : (r == xj1 - xj0 + 1 ? m.jds - WRFGPU_HALO : m.jde + jstag + WRFGPU_HALO);
       const int sjj = (py || sy) ? bc_src(tj, m.jde, vs, py, var == 'v', &negj) : tj;
-      float val[NXW_MAX];
+      const int row = off(0, k, sjj);
 #pragma unroll
       for (int c = 0; c < NXW_MAX; ++c) {
         if (c < nxw) {
           const int ti = c < nxl ? m.ids - nxl + c : xr0 + (c - nxl);
-          bool neg = false;
-          const int si = xsrc(ti, &neg);
-          val[c] = base[off(si, k, sjj)];
-        }
-      }
-#pragma unroll
-      for (int c = 0; c < NXW_MAX; ++c) {
-        if (c < nxw) {
-          const int ti = c < nxl ? m.ids - nxl + c : xr0 + (c - nxl);
-          base[off(ti, k, tj)] = negj ? -val[c] : val[c];
+          bool n = false;
+          val[c] = base[row + xsrc(ti, &n)];
         }
       }
     }
-  }
-  if (py || sy || oy) {
-    constexpr int PER = 4;  // points per lane
-    const int lane = threadIdx.x & 31, warp = tid >> 5, nwarps = nthr >> 5;
-    const int npiece = (nyi + 32 * PER - 1) / (32 * PER);
-    const int nunits = nk * nyrows * npiece;
-    for (int w = warp; w < nunits; w += nwarps) {
-      const int row = w / npiece, pc = w - row * npiece;
-      const int kk = row / nyrows, r = row - kk * nyrows;
-      const int k = kk + m.kts;
-      const int tj = r < ynl ? m.jds - ynl + r : yr0 + (r - ynl);
-      bool negj = false;
-      const int sjj = oy ? open_src(tj, m.jde, vs) : bc_src(tj, m.jde, vs, py, var == 'v', &negj);
-      float val[PER];
-      bool neg[PER];
+    if (uy) {
+      const int row = w / npiece, kk = row / nyrows, r = row - kk * nyrows;
+      pc = w - row * npiece;
+      ky = kk + m.kts;
+      tjy = r < ynl ? m.jds - ynl + r : yr0 + (r - ynl);
+      bool nj = false;
+      const int sjj = oy ? open_src(tjy, m.jde, vs) : bc_src(tjy, m.jde, vs, py, var == 'v', &nj);
+      const int from = off(0, ky, sjj);
 #pragma unroll
       for (int q = 0; q < PER; ++q) {
         const int ii = pc * 32 * PER + q * 32 + lane;
-        neg[q] = negj;
-        if (ii < nyi) {
-          const int ti = yi0 + ii;
-          const int si = xsrc(ti, &neg[q]);
-          val[q] = base[off(si, k, sjj)];
+        neg[q] = nj;
+        if (ii < nyi) vy[q] = base[from + xsrc(yi0 + ii, &neg[q])];
+      }
+    }
+    if (ux) {
+      const int row = off(0, k, tj);
+#pragma unroll
+      for (int c = 0; c < NXW_MAX; ++c) {
+        if (c < nxw) {
+          const int ti = c < nxl ? m.ids - nxl + c : xr0 + (c - nxl);
+          base[row + ti] = negj ? -val[c] : val[c];
         }
       }
+    }
+    if (uy) {
+      const int row = off(yi0, ky, tjy);
 #pragma unroll
       for (int q = 0; q < PER; ++q) {
         const int ii = pc * 32 * PER + q * 32 + lane;
-        if (ii < nyi) base[off(yi0 + ii, k, tj)] = neg[q] ? -val[q] : val[q];
+        if (ii < nyi) base[row + ii] = neg[q] ? -vy[q] : vy[q];
       }
     }
   }

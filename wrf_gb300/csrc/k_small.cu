@@ -170,8 +170,8 @@ __global__ void __launch_bounds__(BX* BY) k_calc_p_rho(Launch L, int step) {
 
 // Column form over mass tiles x level chunks: the levels of a chunk are
 // independent, so their loads go out four levels at a time; the arithmetic
-// of each point is calc_p_rho_point's.  ACOUSTIC: an acoustic step's
-// (step >= 1), whose halo fill is this kernel's own stores (MassImages).
+// of each point is calc_p_rho_point's.  The halo fill of al and p is this
+// kernel's own stores (MassImages).  ACOUSTIC: an acoustic step's (step >= 1).
 template <bool ACOUSTIC>
 __global__ void __launch_bounds__(TX* TY, ACOUSTIC ? 4 : 1) k_calc_p_rho_col(TileLaunch L, int rk_step, int step) {
   const TilePos tp = tile_pos(L, false, false);
@@ -186,10 +186,9 @@ __global__ void __launch_bounds__(TX* TY, ACOUSTIC ? 4 : 1) k_calc_p_rho_col(Til
   F1 c1h = f1(m, WRFGPU_C1H), c2h = f1(m, WRFGPU_C2H), rdnw = f1(m, WRFGPU_RDNW);
   const float muij = f2(m, WRFGPU_MU_2).ro(i, j), mutij = f2(m, WRFGPU_MUTS).ro(i, j), smdiv = m.smdiv;
   MassImages img;
-  if (ACOUSTIC) img.init(m, i, j);
+  img.init(m, i, j);
   auto put = [&](const F3& a, int k, float v) {
-    if (ACOUSTIC) img.store([&](int ii, int jj) { a(ii, k, jj) = v; });
-    else a(i, k, j) = v;
+    img.store([&](int ii, int jj) { a(ii, k, jj) = v; });
   };
   struct LP { float a, t1, t2, c2a, ph0, ph1, pm1; };
   chunked_levels<4, LP>(
