@@ -182,9 +182,9 @@ struct Ensemble {
   // are used.  A narrow domain's kernels leave most SMs idle, so the step's
   // length is its longest chain of launches; a wide one gains only the tails.
   // Not while profiling (the phase marks time the main stream).
-  static constexpr int NSIDE = 3;
-  cudaStream_t side[NSIDE] = {nullptr, nullptr, nullptr};
-  cudaEvent_t ev_side[NSIDE] = {nullptr, nullptr, nullptr}, ev_sfork = nullptr;
+  static constexpr int NSIDE = 4;
+  cudaStream_t side[NSIDE] = {};
+  cudaEvent_t ev_side[NSIDE] = {}, ev_sfork = nullptr;
   // the stream of branch b from here on (the main one while profiling)
   cudaStream_t fork(int b) {
     if (prof) return stream;
@@ -1008,8 +1008,12 @@ struct Ensemble {
         j.f3(WRFGPU_AL, 'p'); j.f3(WRFGPU_PH_2, 'w');
         fill(j);
       }
-      // rk_tendency (module_em.F:370-781): five independent tendencies
-      const cudaStream_t sw = fork(0), sp = fork(1);
+      // rk_tendency (module_em.F:370-781): five independent tendencies; v beside u
+      // too where the tiles leave most SMs idle (us per step, v on the main
+      // stream / on a branch: 41x41x41 with 12 tiles 497 / 462, 100x70x30 with 36
+      // 697 / 659, 190x161x60 with 126 3173 / 3194, 24 small members 8806 / 8964)
+      const bool narrow = nb_st <= 76;
+      const cudaStream_t sw = fork(0), sp = fork(1), sv = narrow ? fork(3) : stream;
       const bool fdiff = rk_step == 1 && (diff6 || damp2);  // module_em.F:801-944 (stage 1), into arrays of its own
       if (fdiff) {
         const cudaStream_t sd = fork(2);
@@ -1025,9 +1029,10 @@ struct Ensemble {
       mark(PH_TEND_T); launch_tend_t_col(LST(), nb_st, TF_ZERO | TF_ADV, sp);
       mark(PH_TEND_PH); launch_tend_ph_col(LST(), nb_st, TF_ZERO | TF_ADV, sp);
       mark(PH_TEND_U); launch_tend_u_col(LST(), nb_st, stream, tune[TU_TENDU]);
-      mark(PH_TEND_V); launch_tend_v_col(LST(), nb_st, stream, tune[TU_TENDV]);
+      mark(PH_TEND_V); launch_tend_v_col(LST(), nb_st, sv, tune[TU_TENDV]);
       join(0);
       join(1);
+      if (narrow) join(3);
       // open boundaries: the lower-order fluxes and radiation terms next to them
       if (any_open) { mark(PH_TEND_PH); launch_strip_tend(LS3(), nb_s3, stream); }
       if (fdiff) join(2);
@@ -1037,24 +1042,26 @@ struct Ensemble {
       }
       // small_step_prep, calc_p_rho(step 0), calc_coef_w (solve_em.F:1089-1140)
       mark(PH_SSP); launch_small_step_prep(l2, nb2, LST(), nb_st, a, stream, tune[TU_SSP]);
-      // the acoustic steps' coefficients, p and al (whose halos their kernel
-      // stores itself, but for open boundaries' copies) and the halo fill of
-      // solve_em.F:1176-1264 side by side
-      const cudaStream_t sc = fork(0), sq = any_open ? stream : fork(1);
+      // the acoustic steps' coefficients beside p, al and the halo fill of
+      // solve_em.F:1176-1264; on a narrow domain p and al beside the fill too, their
+      // halos stored by their own kernel (which costs a wide one more, 1.8 against
+      // 2.4 ms per step of 1024x1024x96, than the fill's shorter job list gives)
+      const bool img0 = col_step && !any_open;
+      const cudaStream_t sc = fork(0), sq = img0 ? fork(1) : stream;
       mark(PH_COEFW);
       if (!fp64 && nb_rw <= COEF_ROW_MAX) launch_calc_coef_w_row(LRW(), nb_rw, a, sc);
       else launch_calc_coef_w_col(LTM(), nb_tm, a, fp64, sc);
-      mark(PH_CPR0); launch_calc_p_rho_col(LTM(), nb_tm, StepArgs{rk_step, 0, 0, 0}, sq);
+      mark(PH_CPR0); launch_calc_p_rho_col(LTM(), nb_tm, StepArgs{rk_step, 0, 0, 0}, sq, 4, img0);
       {
         JobList j;
         j.f3(WRFGPU_RU_TEND, 'u'); j.f3(WRFGPU_RV_TEND, 'v'); j.f3(WRFGPU_PH_2, 'w');
-        if (any_open) { j.f3(WRFGPU_AL, 'p'); j.f3(WRFGPU_P, 'p'); }
+        if (!img0) { j.f3(WRFGPU_AL, 'p'); j.f3(WRFGPU_P, 'p'); }
         j.f3(WRFGPU_T_1, 'p'); j.f3(WRFGPU_T_SAVE, 't');
         j.f2(WRFGPU_MU_1, 't'); j.f2(WRFGPU_MU_2, 't'); j.f2(WRFGPU_MUDF, 't');
         fill(j);
       }
       join(0);
-      if (!any_open) join(1);
+      if (img0) join(1);
       int nsmall_max = 0;
       for (int m = 0; m < nmem; ++m) nsmall_max = std::max(nsmall_max, stage_of(hm[m], rk_step).nsmall);
       for (int it = 1; it <= nsmall_max; ++it) {

@@ -704,7 +704,7 @@ void launch_scalar_pd_update(const TileLaunch& L, int nblocks, int nlev_max, int
     attr = bytes;
   }
   // a chunk computes two levels more than it writes
-  const dim3 grid(nblocks, level_chunks(nblocks, L.nlev, 1, 6, 2 * 152));
+  const dim3 grid(nblocks, level_chunks(nblocks, L.nlev, 1, 4, 2 * 152));
   if (TUNE_PARAM[TU_PD][var] == 1) k_scalar_pd_update<1><<<grid, PD_THREADS, bytes, s>>>(L, rk_step, pairs);
   else k_scalar_pd_update<2><<<grid, PD_THREADS, bytes, s>>>(L, rk_step, pairs);
 }

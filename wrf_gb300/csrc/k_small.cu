@@ -170,9 +170,9 @@ __global__ void __launch_bounds__(BX* BY) k_calc_p_rho(Launch L, int step) {
 
 // Column form over mass tiles x level chunks: the levels of a chunk are
 // independent, so their loads go out four levels at a time; the arithmetic
-// of each point is calc_p_rho_point's.  The halo fill of al and p is this
-// kernel's own stores (MassImages).  ACOUSTIC: an acoustic step's (step >= 1).
-template <bool ACOUSTIC>
+// of each point is calc_p_rho_point's.  ACOUSTIC: an acoustic step's (step >=
+// 1).  IMG: the halo fill of al and p is this kernel's own stores (MassImages).
+template <bool ACOUSTIC, bool IMG>
 __global__ void __launch_bounds__(TX* TY, ACOUSTIC ? 4 : 1) k_calc_p_rho_col(TileLaunch L, int rk_step, int step) {
   const TilePos tp = tile_pos(L, false, false);
   const Mem& m = block_member(L.mem, tp.m);
@@ -186,9 +186,10 @@ __global__ void __launch_bounds__(TX* TY, ACOUSTIC ? 4 : 1) k_calc_p_rho_col(Til
   F1 c1h = f1(m, WRFGPU_C1H), c2h = f1(m, WRFGPU_C2H), rdnw = f1(m, WRFGPU_RDNW);
   const float muij = f2(m, WRFGPU_MU_2).ro(i, j), mutij = f2(m, WRFGPU_MUTS).ro(i, j), smdiv = m.smdiv;
   MassImages img;
-  img.init(m, i, j);
+  if (IMG) img.init(m, i, j);
   auto put = [&](const F3& a, int k, float v) {
-    img.store([&](int ii, int jj) { a(ii, k, jj) = v; });
+    if (IMG) img.store([&](int ii, int jj) { a(ii, k, jj) = v; });
+    else a(i, k, j) = v;
   };
   struct LP { float a, t1, t2, c2a, ph0, ph1, pm1; };
   chunked_levels<4, LP>(
@@ -821,10 +822,11 @@ void launch_small_step_prep(const Launch& L2, int nb2, const TileLaunch& LST, in
 void launch_calc_p_rho(const Launch& L, int nb, StepArgs a, cudaStream_t s) {
   k_calc_p_rho<<<nb, dim3(BX, BY), 0, s>>>(L, a.iteration);
 }
-void launch_calc_p_rho_col(const TileLaunch& L, int nb, StepArgs a, cudaStream_t s, int chunks) {
+void launch_calc_p_rho_col(const TileLaunch& L, int nb, StepArgs a, cudaStream_t s, int chunks, bool img) {
   chunks = level_chunks(nb, L.nlev, chunks, 2);
-  if (a.iteration > 0) k_calc_p_rho_col<true><<<dim3(nb, chunks), dim3(TX, TY), 0, s>>>(L, a.rk_step, a.iteration);
-  else k_calc_p_rho_col<false><<<dim3(nb, chunks), dim3(TX, TY), 0, s>>>(L, a.rk_step, 0);
+  if (a.iteration > 0) k_calc_p_rho_col<true, true><<<dim3(nb, chunks), dim3(TX, TY), 0, s>>>(L, a.rk_step, a.iteration);
+  else if (img) k_calc_p_rho_col<false, true><<<dim3(nb, chunks), dim3(TX, TY), 0, s>>>(L, a.rk_step, 0);
+  else k_calc_p_rho_col<false, false><<<dim3(nb, chunks), dim3(TX, TY), 0, s>>>(L, a.rk_step, 0);
 }
 void launch_calc_coef_w_col(const TileLaunch& L, int nb, StepArgs a, bool fp64, cudaStream_t s) {
   if (fp64) k_calc_coef_w_col<double><<<nb, dim3(TX, TY), 0, s>>>(L, a.rk_step);

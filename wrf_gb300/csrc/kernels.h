@@ -138,8 +138,10 @@ void launch_unpack_rows(const float* src, float* dst, float* dst2, int cols, int
 void launch_unpack_species(const Mem* mems, int member, int s, const float* src, int cols, int rows, int pitch,
                            cudaStream_t st);
 void launch_pack_fields(const Mem* mems, const PackJobs& jobs, cudaStream_t st);
-// mass tiles x level chunks; iteration 0: step 0 of the stage, else the acoustic step (halo images stored)
-void launch_calc_p_rho_col(const TileLaunch& L, int nblocks, StepArgs a, cudaStream_t s, int chunks = 4);
+// mass tiles x level chunks; iteration 0: step 0 of the stage, else the acoustic step (img: halo images stored; the
+// acoustic step always does)
+void launch_calc_p_rho_col(const TileLaunch& L, int nblocks, StepArgs a, cudaStream_t s, int chunks = 4,
+                           bool img = false);
 // sct: some member stores the species' sixth-order diffusion tendency sc_tend
 void launch_update_scalar_pd_col(const TileLaunch& L, int nblocks, StepArgs a, cudaStream_t s, bool sct = false);  // mass tiles
 void launch_calc_p_rho_phi_col(const TileLaunch& L, int nblocks, cudaStream_t s, int var = TUNE_DEFAULT[TU_CPRP]);  // mass tiles
