@@ -751,6 +751,10 @@ struct Ensemble {
   }
 
   static size_t al256(size_t b) { return (b + 255) & ~size_t(255); }
+  // bytes of a member's limiter factors, every species of the widest strip
+  static size_t strip_scratch(const WrfGpuDomainDesc& d, int nsp) {
+    return al256((size_t)strip_cols(d.ide, d.jde, d.config.open_xs, d.config.open_ys, STRIP_W_PD + 1, 1) * d.kde * nsp * 4);
+  }
 
   int init(const WrfGpuDomainDesc* ds, int n, int fl) {
     nmem = n; flags = fl; fp64 = (fl & WRFGPU_FLAG_MIXED) != 0;
@@ -786,7 +790,7 @@ struct Ensemble {
       b += (size_t)3 * nsp * al256(n3[m] * 4);  // current, old, spare
       b += (size_t)WRFGPU_N2D * al256(n2[m] * 4);
       b += (size_t)WRFGPU_N1D * al256(n1[m] * 4);
-      b += al256(n3[m] * 4);  // limiter scratch
+      b += strip_scratch(d, nsp);  // limiter factors next to open boundaries
       b += 6 * al256(n3[m] * 4);  // face Courant numbers and low-order factors of the PD transport
       if (fp64) b += 3 * al256(n3[m] * 8);
       const bool sct = d.config.diff_6th_opt != 0 || d.config.diff_opt == 1;  // stored diffusion tendencies
@@ -826,7 +830,7 @@ struct Ensemble {
       }
       for (int f = 0; f < WRFGPU_N2D; ++f) { M.f2[f] = (float*)p; p += al256(n2[m] * 4); }
       for (int f = 0; f < WRFGPU_N1D; ++f) { M.f1[f] = (float*)p; p += al256(n1[m] * 4); }
-      scr[m] = (float*)p; p += al256(n3[m] * 4);
+      scr[m] = (float*)p; p += strip_scratch(d, M.nsp);
       for (int q = 0; q < 6; ++q) { M.pdc[q] = (float*)p; p += al256(n3[m] * 4); }
       if (fp64) for (int q = 0; q < 3; ++q) { M.wd[q] = (double*)p; p += al256(n3[m] * 8); }
       const bool sct = d.config.diff_6th_opt != 0 || d.config.diff_opt == 1;
@@ -1018,7 +1022,7 @@ struct Ensemble {
       if (fdiff) {
         const cudaStream_t sd = fork(2);
         mark(PH_DIFF);
-        if (diff6) launch_forward_diff(l3, nb3, 0, sd);
+        if (diff6) launch_forward_diff(LST(), nb_st, 0, sd);
         if (damp2) launch_rayleigh_damp(l2, nb2, sd);
       }
       mark(PH_TEND_W);
@@ -1038,7 +1042,7 @@ struct Ensemble {
       if (fdiff) join(2);
       if (diff6 || damp2) {  // rk_addtend_dry (solve_em.F:967)
         mark(PH_DIFF);
-        launch_addtend_dry(l3, nb3, stream);
+        launch_addtend_dry(LST(), nb_st, stream);
       }
       // small_step_prep, calc_p_rho(step 0), calc_coef_w (solve_em.F:1089-1140)
       mark(PH_SSP); launch_small_step_prep(l2, nb2, LST(), nb_st, a, stream, tune[TU_SSP]);
@@ -1125,7 +1129,7 @@ struct Ensemble {
         launch_scalar_adv_update(LP(), nb_pr, rk_step, stream, tune[TU_ADV], diff6, ~io_pairs_early);
       } else {
         io_join();  // passive scalars copied in by a host I/O step are read from here on
-        if (diff6 && rk_step == 1) { mark(PH_DIFF); launch_forward_diff(l3, nb3, 1, stream); }  // module_em.F:1378-1435
+        if (diff6 && rk_step == 1) { mark(PH_DIFF); launch_forward_diff(LST(), nb_st, 1, stream, nsp_max); }  // module_em.F:1378-1435
         if (rk_step < 3 || !all_pd) {
           mark(PH_ADVS); launch_scalar_adv_update(LP(), nb_pr, rk_step, stream, tune[TU_ADV], diff6);
         }
@@ -1144,7 +1148,7 @@ struct Ensemble {
         species_filled = io_step && !io_prefetch && !any_open;
       }
       if (any_open) {
-        launch_strip_scalar(LS3(), nb_s3, rk_step, stream);
+        launch_strip_scalar(LS3(), nb_s3, rk_step, nsp_max, stream);
         if (rk_step == 3) launch_strip_pd(LS5(), nb_s5, LS4(), nb_s4, rk_step, nsp_max, d_pd_scratch, stream);
       }
       swap_species(species_filled);
@@ -1304,7 +1308,7 @@ struct Ensemble {
       case 131: launch_update_scalar_routine(l3, nb3, rk_step, 1, stream); break;
       case 132: launch_species_diff_routine(l3, nb3, iteration, stream); break;
       // rk_tendency's forward terms at stage 1 added to the caller's *_tendf
-      case 133: launch_forward_diff(l3, nb3, 2, stream); launch_rayleigh_damp(l2, nb2, stream, true); break;
+      case 133: launch_forward_diff(LST(), nb_st, 2, stream); launch_rayleigh_damp(l2, nb2, stream, true); break;
       case 134: launch_addtend_dry_routine(l3, nb3, rk_step, stream); break;  // rk_addtend_dry
       case 24: launch_calc_p_rho_phi(l3, nb3, stream); break;
       case 25: launch_set_w_surface(l2, nb2, stream); break;

@@ -31,8 +31,12 @@ __device__ __forceinline__ float flux6(float fm3, float fm2, float fm1, float f0
   return 10.0f * (f0 - fm1) - 5.0f * (fp1 - fm2) + (fp2 - fm3);
 }
 
+// x / d; a zero numerator over a positive divisor is x itself and skips the
+// division, which takes its slow path for zeros (flat ground, undamped levels).
+__device__ __forceinline__ float div_z(float x, float d) { return x == 0.f && d > 0.f ? x : x / d; }
+
 // max(1 - dzmax / dzthresh, 0): the terrain-slope taper (:6481-6497).
-__device__ __forceinline__ float taper(float dzmax, float thresh) { return fmaxf(1.f - (dzmax / thresh), 0.f); }
+__device__ __forceinline__ float taper(float dzmax, float thresh) { return fmaxf(1.f - div_z(dzmax, thresh), 0.f); }
 
 // One point of sixth_order_diffusion for variable kind V at (i, k, j), with
 // the column constants c1, c2 of level k: returns t0 + tendency_x +
@@ -241,22 +245,31 @@ __device__ __forceinline__ float vflux_at(const Mem& m, const F3& f, const F1& b
   return a * (df - b3->ro(i, kk + 1, j) + b3->ro(i, kk, j));
 }
 
-// The term vertical diffusion of kind V adds to the tendency at level k,
-// with the column mass c1 mass + c2 of that level: the divergence of the
-// fluxes vflux(k) - vflux(k-1), vflux(kts-1) = vflux(kts), vflux(ktf) = 0.
+// The fluxes whose difference over level k the term is: vflux(kts-1) =
+// vflux(kts), vflux(ktf) = 0.
 template <int V>
-__device__ float vdiff_point(const Mem& m, const F3& f, const F1& b1, const F3* b3, float mass, float c1, float c2,
-                             int i, int k, int j, float kvdif) {
+__device__ __forceinline__ float vflux_of(const Mem& m, const F3& f, const F1& b1, const F3* b3, int i, int kk, int j,
+                                          float kvdif) {
   const F3 alt = f3(m, WRFGPU_ALT);
-  const int kts = m.kts, ktf = min(m.kte, m.kde - 1);
-  auto vf = [&](int kk) { return kk >= ktf ? 0.f : vflux_at<V>(m, f, b1, b3, alt, i, max(kk, kts), j, kvdif); };
-  const float dv = vf(k) - vf(k - 1);
+  return kk >= min(m.kte, m.kde - 1) ? 0.f : vflux_at<V>(m, f, b1, b3, alt, i, max(kk, m.kts), j, kvdif);
+}
+// The term vertical diffusion of kind V adds to the tendency at level k,
+// with the column mass c1 mass + c2 of that level and dv = vflux(k) - vflux(k-1).
+template <int V>
+__device__ __forceinline__ float vdiff_term(const Mem& m, float dv, float mass, float c1, float c2, int i, int k, int j) {
+  const F3 alt = f3(m, WRFGPU_ALT);
   const float g2 = G * G;
   if (V == VD_U) return g2 * f1(m, WRFGPU_RDNW)(k) / (c1 * mass + c2) / (0.5f * (alt.ro(i - 1, k, j) + alt.ro(i, k, j))) * dv;
   if (V == VD_V) return g2 * f1(m, WRFGPU_RDNW)(k) / (c1 * mass + c2) / (0.5f * (alt.ro(i, k, j - 1) + alt.ro(i, k, j))) * dv;
   if (V == VD_W)
     return f1(m, WRFGPU_RDN)(k) * G * G / (c1 * mass + c2) / (0.5f * (alt.ro(i, k, j) + alt.ro(i, k - 1, j))) * dv;
   return g2 / (c1 * mass + c2) / alt.ro(i, k, j) * f1(m, WRFGPU_RDNW)(k) * dv;
+}
+template <int V>
+__device__ float vdiff_point(const Mem& m, const F3& f, const F1& b1, const F3* b3, float mass, float c1, float c2,
+                             int i, int k, int j, float kvdif) {
+  const float dv = vflux_of<V>(m, f, b1, b3, i, k, j, kvdif) - vflux_of<V>(m, f, b1, b3, i, k - 1, j, kvdif);
+  return vdiff_term<V>(m, dv, mass, c1, c2, i, k, j);
 }
 
 // Point ranges of the diffusion terms next to open boundaries (a periodic x
@@ -283,6 +296,41 @@ __device__ __forceinline__ bool diff6_open_in(const Mem& m, int V, int i, int j)
   return (!oxs || i >= ids + 3) && (!oxe || i <= xe) && (!oys || j >= jds + 3) && (!oye || j <= ye);
 }
 
+// The forward terms of one field in column (i, j), levels k0..k1: horizontal
+// diffusion where `hor`, vertical at levels up to kv (none: kv < k0), sixth
+// order where `six`, in the reference's order onto 0 (acc: onto the stored
+// value).  The flux below a level is the one formed above the level before.  ALL:
+// every term, as on all points but those next to open boundaries; without the
+// conditions the compiler keeps the map-factor quotients, which do not
+// change with the level, over the loop.
+template <int V, int VD, bool ALL>
+__device__ __forceinline__ void forward_levels(const Mem& m, const F3& f, const F3* base, const F1& b1, const F1& c1v,
+                                            const F1& c2v, const F2& mu, float mass, const F3& out, int i, int j, int k0,
+                                            int k1, bool hor, int kv, bool six, float xkh, float xkv, float coef, bool acc) {
+  float vbelow = k0 <= min(kv, k1) ? vflux_of<VD>(m, f, b1, base, i, k0 - 1, j, xkv) : 0.f;
+  for (int k = k0; k <= k1; ++k) {
+    const float c1 = c1v(k), c2 = c2v(k);
+    float t = acc ? out(i, k, j) : 0.f;
+    if (ALL || hor) t = t + hdiff_point<V>(m, f, base, mu, c1, c2, i, k, j, xkh);
+    if (k <= kv) {
+      const float v = vflux_of<VD>(m, f, b1, base, i, k, j, xkv);
+      t = t + vdiff_term<VD>(m, v - vbelow, mass, c1, c2, i, k, j);
+      vbelow = v;
+    }
+    if (ALL || six) t = diff6_point<V>(m, f, mu, i, k, j, c1, c2, coef, t);
+    out(i, k, j) = t;
+  }
+}
+template <int V, int VD>
+__device__ __forceinline__ void forward_col(const Mem& m, const F3& f, const F3* base, const F1& b1, const F1& c1v,
+                                            const F1& c2v, const F2& mu, float mass, const F3& out, int i, int j, int k0,
+                                            int k1, bool hor, int kv, bool six, float xkh, float xkv, float coef, bool acc) {
+  if (hor && six)
+    forward_levels<V, VD, true>(m, f, base, b1, c1v, c2v, mu, mass, out, i, j, k0, k1, hor, kv, six, xkh, xkv, coef, acc);
+  else
+    forward_levels<V, VD, false>(m, f, base, b1, c1v, c2v, mu, mass, out, i, j, k0, k1, hor, kv, six, xkh, xkv, coef, acc);
+}
+
 // Stage 1, mode 0 (rk_tendency): the forward-in-time tendencies ru_tendf,
 // rv_tendf, rw_tendf and t_tendf of u_2, v_2, w_2 and t_2: the explicit
 // diffusion (diff_opt = 1; mut, khdif, kvdif), then the sixth-order diffusion
@@ -294,88 +342,66 @@ __device__ __forceinline__ bool diff6_open_in(const Mem& m, int V, int i, int j)
 // points outside them get no term.  Mode 2 is mode 0 added
 // onto the stored tendencies' values (the routine-level rk_tendency, whose
 // *_tendf arrays arrive holding the physics tendencies).
-__global__ void __launch_bounds__(BX* BY) k_forward_diff(Launch L, int mode) {
-  BlockPos bp = block_pos(L);
-  const Mem& m = block_member(L.mem, bp.m);
+// blockIdx.y: level chunk, blockIdx.z: the field (u, v, w, theta; mode 1: the
+// species).  About 480 instructions a point and 24 reads with a 92% L1 hit rate:
+// bound by their latency (issue 36% at 16 warps per SM), so by the warps an SM
+// holds: us of modes 0 / 1 at 160x144x64 with 2 species and 1, 2, 3, 4, 5, 6 blocks
+// per SM 251/111, 188/90, 173/70, 127/61, 133/75, 170/73 (spills from 5 on); a
+// thread per point, each vertical flux formed twice, 214/107.
+__global__ void __launch_bounds__(TX* TY, 4) k_forward_diff(TileLaunch L, int mode) {
+  const TilePos tp = tile_pos(L, TILE_ONE, true);
+  const Mem& m = block_member(L.mem, tp.m);
   const bool d1 = m.cf.diff_opt == 1, d6 = m.cf.diff_6th_opt != 0;
-  if (!bp.valid || m.tendf[0] == nullptr || !(d1 || d6)) return;
-  const int i = bp.i, j = bp.j, k = bp.k;
+  if (m.tendf[0] == nullptr || !(d1 || d6)) return;
+  const int i = tp.i0 + (int)threadIdx.x, j = tp.j0 + (int)threadIdx.y;
   const int ktf = min(m.kte, m.kde - 1);
-  if (i < m.its || j < m.jts || k < m.kts || k > ktf) return;
+  const Chunk ch = level_chunk_of(m.kts, ktf);
   const int i_end = min(m.ide - 1, m.ite), j_end = min(m.jde - 1, m.jte);
   const F1 c1h = f1(m, WRFGPU_C1H), c2h = f1(m, WRFGPU_C2H);
-  const float c1 = c1h(k), c2 = c2h(k);
+  const int fld = blockIdx.z;
   if (mode == 1) {
-    if (i > i_end || j > j_end) return;
+    float* sc = fld < m.nsp ? sc_tend_of(m, fld) : nullptr;
+    if (!sc || i > i_end || j > j_end) return;
     const float coef = m.cf.diff_6th_factor * 0.015625f / (2.0f * stage_of(m, 1).dt_rk);
     const float khdq = m.cf.khdif / PRANDTL, kvdq = m.cf.kvdif / PRANDTL;
     const F2 muts = f2(m, WRFGPU_MUTS);
+    const F3 q = f3p(m, m.q[fld]), out = f3p(m, sc);
+    const bool mix2 = mix2_on(m, fld), hor = mix2 && hdiff_open_in(m, DV_M, i, j);
+    const bool six = mix6_on(m, fld) && diff6_open_in(m, DV_M, i, j);
+    const int kv = mix2 ? ktf : m.kts - 1;
     const F1 qvb = f1(m, WRFGPU_QV_BASE);
-    for (int s = 0; s < m.nsp; ++s) {
-      float* sc = sc_tend_of(m, s);
-      if (!sc) continue;
-      const F3 q = f3p(m, m.q[s]);
-      float t = 0.f;
-      if (mix2_on(m, s)) {
-        if (hdiff_open_in(m, DV_M, i, j)) t = t + hdiff_point<DV_M>(m, q, nullptr, muts, c1, c2, i, k, j, khdq);
-        const float mu = muts.ro(i, j);
-        t = t + (s == 0 ? vdiff_point<VD_MP>(m, q, qvb, nullptr, mu, c1, c2, i, k, j, kvdq)
-                        : vdiff_point<VD_M>(m, q, qvb, nullptr, mu, c1, c2, i, k, j, kvdq));
-      }
-      if (mix6_on(m, s) && diff6_open_in(m, DV_M, i, j)) t = diff6_point<DV_M>(m, q, muts, i, k, j, c1, c2, coef, t);
-      f3p(m, sc)(i, k, j) = t;
-    }
+    if (fld == 0)
+      forward_col<DV_M, VD_MP>(m, q, nullptr, qvb, c1h, c2h, muts, muts.ro(i, j), out, i, j, ch.k0, ch.k1, hor, kv, six,
+                               khdq, kvdq, coef, false);
+    else
+      forward_col<DV_M, VD_M>(m, q, nullptr, qvb, c1h, c2h, muts, muts.ro(i, j), out, i, j, ch.k0, ch.k1, hor, kv, six,
+                              khdq, kvdq, coef, false);
     return;
   }
   const float coef = m.cf.diff_6th_factor * 0.015625f / (2.0f * m.dt);
   const float xkmh = m.cf.khdif, xkhh = m.cf.khdif / PRANDTL, kvdif = m.cf.kvdif;
   const F2 mut = f2(m, WRFGPU_MUT);
   const bool acc = mode == 2;  // onto the stored values (the routine-level form: physics tendencies)
-  if (i <= m.ite && j <= j_end) {
-    const F3 u = f3(m, WRFGPU_U_2);
-    float t = acc ? f3p(m, m.tendf[0])(i, k, j) : 0.f;
-    if (d1) {
-      if (hdiff_open_in(m, DV_U, i, j)) t = t + hdiff_point<DV_U>(m, u, nullptr, mut, c1, c2, i, k, j, xkmh);
-      if (k <= ktf - 1 && vdiff_open_in(m, VD_U, i, j))
-        t = t + vdiff_point<VD_U>(m, u, f1(m, WRFGPU_U_BASE), nullptr, f2(m, WRFGPU_MUU).ro(i, j), c1, c2, i, k, j,
-                                  kvdif);
-    }
-    if (d6 && diff6_open_in(m, DV_U, i, j)) t = diff6_point<DV_U>(m, u, mut, i, k, j, c1, c2, coef, t);
-    f3p(m, m.tendf[0])(i, k, j) = t;
-  }
-  if (i <= i_end && j <= m.jte) {
-    const F3 v = f3(m, WRFGPU_V_2);
-    float t = acc ? f3p(m, m.tendf[1])(i, k, j) : 0.f;
-    if (d1) {
-      if (hdiff_open_in(m, DV_V, i, j)) t = t + hdiff_point<DV_V>(m, v, nullptr, mut, c1, c2, i, k, j, xkmh);
-      if (k <= ktf - 1 && j <= j_end && vdiff_open_in(m, VD_V, i, j))
-        t = t + vdiff_point<VD_V>(m, v, f1(m, WRFGPU_V_BASE), nullptr, f2(m, WRFGPU_MUV).ro(i, j), c1, c2, i, k, j,
-                                  kvdif);
-    }
-    if (d6 && diff6_open_in(m, DV_V, i, j)) t = diff6_point<DV_V>(m, v, mut, i, k, j, c1, c2, coef, t);
-    f3p(m, m.tendf[1])(i, k, j) = t;
-  }
-  if (i <= i_end && j <= j_end) {
-    const float mt = mut.ro(i, j);
-    if (k >= m.kts + 1) {
-      const F3 w = f3(m, WRFGPU_W_2);
-      const float c1w = f1(m, WRFGPU_C1F)(k), c2w = f1(m, WRFGPU_C2F)(k);
-      float t = acc ? f3p(m, m.tendf[2])(i, k, j) : 0.f;
-      if (d1) {
-        if (hdiff_open_in(m, DV_W, i, j)) t = t + hdiff_point<DV_W>(m, w, nullptr, mut, c1w, c2w, i, k, j, xkmh);
-        t = t + vdiff_point<VD_W>(m, w, c1h, nullptr, mt, c1w, c2w, i, k, j, kvdif);
-      }
-      if (d6 && diff6_open_in(m, DV_W, i, j)) t = diff6_point<DV_W>(m, w, mut, i, k, j, c1w, c2w, coef, t);
-      f3p(m, m.tendf[2])(i, k, j) = t;
-    }
-    const F3 th = f3(m, WRFGPU_T_2), tb = f3(m, WRFGPU_T_INIT);
-    float t = acc ? f3p(m, m.tendf[3])(i, k, j) : 0.f;
-    if (d1) {
-      if (hdiff_open_in(m, DV_M, i, j)) t = t + hdiff_point<DV_M>(m, th, &tb, mut, c1, c2, i, k, j, xkhh);
-      t = t + vdiff_point<VD_3DMP>(m, th, c1h, &tb, mt, c1, c2, i, k, j, 3.f * kvdif);
-    }
-    if (d6 && diff6_open_in(m, DV_M, i, j)) t = diff6_point<DV_M>(m, th, mut, i, k, j, c1, c2, coef, t);
-    f3p(m, m.tendf[3])(i, k, j) = t;
+  if (fld == 0 && i <= m.ite && j <= j_end)
+    forward_col<DV_U, VD_U>(m, f3(m, WRFGPU_U_2), nullptr, f1(m, WRFGPU_U_BASE), c1h, c2h, mut,
+                            f2(m, WRFGPU_MUU).ro(i, j), f3p(m, m.tendf[0]), i, j, ch.k0, ch.k1,
+                            d1 && hdiff_open_in(m, DV_U, i, j), d1 && vdiff_open_in(m, VD_U, i, j) ? ktf - 1 : m.kts - 1,
+                            d6 && diff6_open_in(m, DV_U, i, j), xkmh, kvdif, coef, acc);
+  if (fld == 1 && i <= i_end && j <= m.jte)
+    forward_col<DV_V, VD_V>(m, f3(m, WRFGPU_V_2), nullptr, f1(m, WRFGPU_V_BASE), c1h, c2h, mut,
+                            f2(m, WRFGPU_MUV).ro(i, j), f3p(m, m.tendf[1]), i, j, ch.k0, ch.k1,
+                            d1 && hdiff_open_in(m, DV_V, i, j),
+                            d1 && j <= j_end && vdiff_open_in(m, VD_V, i, j) ? ktf - 1 : m.kts - 1,
+                            d6 && diff6_open_in(m, DV_V, i, j), xkmh, kvdif, coef, acc);
+  if (fld == 2 && i <= i_end && j <= j_end)
+    forward_col<DV_W, VD_W>(m, f3(m, WRFGPU_W_2), nullptr, c1h, f1(m, WRFGPU_C1F), f1(m, WRFGPU_C2F), mut, mut.ro(i, j),
+                            f3p(m, m.tendf[2]), i, j, max(ch.k0, m.kts + 1), ch.k1, d1 && hdiff_open_in(m, DV_W, i, j),
+                            d1 ? ktf : m.kts - 1, d6 && diff6_open_in(m, DV_W, i, j), xkmh, kvdif, coef, acc);
+  if (fld == 3 && i <= i_end && j <= j_end) {
+    const F3 tb = f3(m, WRFGPU_T_INIT);
+    forward_col<DV_M, VD_3DMP>(m, f3(m, WRFGPU_T_2), &tb, c1h, c1h, c2h, mut, mut.ro(i, j), f3p(m, m.tendf[3]), i, j,
+                               ch.k0, ch.k1, d1 && hdiff_open_in(m, DV_M, i, j), d1 ? ktf : m.kts - 1,
+                               d6 && diff6_open_in(m, DV_M, i, j), xkhh, 3.f * kvdif, coef, acc);
   }
 }
 
@@ -415,8 +441,8 @@ __global__ void __launch_bounds__(BX* BY) k_species_diff_routine(Launch L, int q
 // Stage 1, damp_opt = 2: rk_rayleigh_damp (module_big_step_utilities_em.F:
 // 5836-6110), relaxation of u, v, w and theta toward the base-state
 // profiles in the top zdamp metres, into ru_tendf .. t_tendf.  One thread per
-// column (i, j) of the memory extent, handling u, v, w and theta of that
-// column; the top layer's level heights are formed again where they are
+// column (i, j) of the memory extent and field (blockIdx.y: u, v, w, theta; all
+// four in one thread took 68 us at 190x161x60, now 46); the top layer's level heights are formed again where they are
 // used (the same expressions, so the same bits) instead of being stored.
 // A member that also stores the explicit or sixth-order diffusion
 // accumulates onto it (written earlier in the same stage), as does the
@@ -458,7 +484,8 @@ __global__ void __launch_bounds__(BX* BY) k_rayleigh_damp(Launch L, bool acc_all
   const F1 c1h = f1(m, WRFGPU_C1H), c2h = f1(m, WRFGPU_C2H), c1f = f1(m, WRFGPU_C1F), c2f = f1(m, WRFGPU_C2F);
   const F1 zb = f1(m, WRFGPU_Z_BASE);
   // u (:5897-5945)
-  if (i <= min(m.ite, m.ide) && j <= min(m.jte, m.jde - 1)) {
+  const int fld = blockIdx.y;
+  if (fld == 0 && i <= min(m.ite, m.ide) && j <= min(m.jte, m.jde - 1)) {
     const F3 u = f3(m, WRFGPU_U_2), tend = f3p(m, m.tendf[0]);
     const F1 prof = f1(m, WRFGPU_U_BASE);
     const float mu = f2(m, WRFGPU_MUU)(i, j);
@@ -479,7 +506,7 @@ __global__ void __launch_bounds__(BX* BY) k_rayleigh_damp(Launch L, bool acc_all
     }
   }
   // v (:5947-5995)
-  if (i <= min(m.ite, m.ide - 1) && j <= min(m.jte, m.jde)) {
+  if (fld == 1 && i <= min(m.ite, m.ide - 1) && j <= min(m.jte, m.jde)) {
     const F3 v = f3(m, WRFGPU_V_2), tend = f3p(m, m.tendf[1]);
     const F1 prof = f1(m, WRFGPU_V_BASE);
     const float mv = f2(m, WRFGPU_MUV)(i, j);
@@ -500,19 +527,20 @@ __global__ void __launch_bounds__(BX* BY) k_rayleigh_damp(Launch L, bool acc_all
     }
   }
   // w (:5997-6013) and theta (:6015-6062)
-  if (i <= min(m.ite, m.ide - 1) && j <= min(m.jte, m.jde - 1)) {
+  if (fld >= 2 && i <= min(m.ite, m.ide - 1) && j <= min(m.jte, m.jde - 1)) {
     const F3 w = f3(m, WRFGPU_W_2), t3 = f3(m, WRFGPU_T_2);
     const F3 tw = f3p(m, m.tendf[2]), tt = f3p(m, m.tendf[3]);
     const F1 prof = f1(m, WRFGPU_T_BASE);
     const float mt = f2(m, WRFGPU_MUT)(i, j);
     const float ztop = (phb(i, kde, j) + ph(i, kde, j)) / G;
-    for (int k = kts; k <= min(m.kte, kde); ++k) {
+    for (int k = kts; fld == 2 && k <= min(m.kte, kde); ++k) {
       float t = acc ? tw(i, k, j) : 0.f;
       const float z = (phb(i, k, j) + ph(i, k, j)) / G;
       if (z >= ztop - zdamp)
         t = t - (c1f(k) * mt + c2f(k)) * (rayleigh_weight(ztop, z, zdamp) * dampcoef) * w(i, k, j);
       tw(i, k, j) = t;
     }
+    if (fld == 2) return;
     auto height = [&](int k) { return 0.5f * (phb(i, k, j) + phb(i, k + 1, j) + ph(i, k, j) + ph(i, k + 1, j)) / G; };
     const int k1 = rayleigh_top_level(ztop, zdamp, kts, ktf, height);
     for (int k = kts; k <= ktf; ++k) {
@@ -532,32 +560,48 @@ __global__ void __launch_bounds__(BX* BY) k_rayleigh_damp(Launch L, bool acc_all
 // stage-1 "tendf + save * msf" steps add +0 to a tendency that is never -0
 // and the ph / mu additions are left out; theta keeps its h_diabatic term,
 // which can turn a -0 sum into +0.
-__global__ void __launch_bounds__(BX* BY) k_addtend_dry(Launch L) {
-  BlockPos bp = block_pos(L);
-  const Mem& m = block_member(L.mem, bp.m);
-  if (!bp.valid || m.tendf[0] == nullptr) return;
-  const int i = bp.i, j = bp.j, k = bp.k;
-  if (i < m.its || j < m.jts || k < m.kts || k > m.kte) return;
-  const int i_end = min(m.ite, m.ide - 1), j_end = min(m.jte, m.jde - 1);
-  if (k <= m.kte - 1) {
-    if (i <= m.ite && j <= j_end) {
-      F3 t = f3(m, WRFGPU_RU_TEND);
-      t(i, k, j) = t(i, k, j) + f3p(m, m.tendf[0]).ro(i, k, j) / f2(m, WRFGPU_MSFUY).ro(i, j);
+// Twelve memory streams and no arithmetic to speak of: a thread takes a column
+// of a level chunk, its 2-D factors loaded once and the loads of ADD_LEV levels of
+// all four fields issued together (a thread per point, each block with its own
+// copy of the member descriptor: 39 us at 190x161x60; now 26.  Batches of 4 levels and
+// 3 blocks per SM 24 us at 160x144x64, 2 and 5 19 us).
+constexpr int ADD_LEV = 2;
+__global__ void __launch_bounds__(TX* TY, 5) k_addtend_dry(TileLaunch L) {
+  const TilePos tp = tile_pos(L, TILE_ONE, true);
+  const Mem& m = block_member(L.mem, tp.m);
+  if (m.tendf[0] == nullptr) return;
+  const int i = tp.i0 + (int)threadIdx.x, j = tp.j0 + (int)threadIdx.y;
+  if (i > m.ite || j > m.jte) return;
+  const bool bu = j <= min(m.jte, m.jde - 1), bv = i <= min(m.ite, m.ide - 1), bm = bu && bv;
+  const Chunk ch = level_chunk_of(m.kts, m.kte);
+  const F3 ut = f3(m, WRFGPU_RU_TEND), vt = f3(m, WRFGPU_RV_TEND), tt = f3(m, WRFGPU_T_TEND), wt = f3(m, WRFGPU_RW_TEND);
+  const F3 uf = f3p(m, m.tendf[0]), vf = f3p(m, m.tendf[1]), wf = f3p(m, m.tendf[2]), tf = f3p(m, m.tendf[3]);
+  const F1 c1h = f1(m, WRFGPU_C1H), c2h = f1(m, WRFGPU_C2H);
+  const float msfuy = bu ? f2(m, WRFGPU_MSFUY).ro(i, j) : 1.f, msfvx_inv = bv ? f2(m, WRFGPU_MSFVX_INV).ro(i, j) : 1.f;
+  const float msfty = bm ? f2(m, WRFGPU_MSFTY).ro(i, j) : 1.f, mut = bm ? f2(m, WRFGPU_MUT).ro(i, j) : 0.f;
+  for (int kb = ch.k0; kb <= ch.k1; kb += ADD_LEV) {
+    float a[4][ADD_LEV], b[4][ADD_LEV];
+#pragma unroll
+    for (int q = 0; q < ADD_LEV; ++q) {
+      const int k = kb + q;
+      const bool half = k <= min(ch.k1, m.kte - 1);
+      if (bu && half) { a[0][q] = ut(i, k, j); b[0][q] = uf.ro(i, k, j); }
+      if (bv && half) { a[1][q] = vt(i, k, j); b[1][q] = vf.ro(i, k, j); }
+      if (bm && half) { a[2][q] = tt(i, k, j); b[2][q] = tf.ro(i, k, j); }
+      if (bm && k <= ch.k1) { a[3][q] = wt(i, k, j); b[3][q] = wf.ro(i, k, j); }
     }
-    if (i <= i_end && j <= m.jte) {
-      F3 t = f3(m, WRFGPU_RV_TEND);
-      t(i, k, j) = t(i, k, j) + f3p(m, m.tendf[1]).ro(i, k, j) * f2(m, WRFGPU_MSFVX_INV).ro(i, j);
+#pragma unroll
+    for (int q = 0; q < ADD_LEV; ++q) {
+      const int k = kb + q;
+      const bool half = k <= min(ch.k1, m.kte - 1);
+      if (bu && half) ut(i, k, j) = a[0][q] + div_z(b[0][q], msfuy);
+      if (bv && half) vt(i, k, j) = a[1][q] + b[1][q] * msfvx_inv;
+      if (bm && half) {
+        const float mass = c1h(k) * mut + c2h(k);
+        tt(i, k, j) = a[2][q] + div_z(b[2][q], msfty) + div_z(mass * 0.f, msfty);
+      }
+      if (bm && k <= ch.k1) wt(i, k, j) = a[3][q] + div_z(b[3][q], msfty);
     }
-    if (i <= i_end && j <= j_end) {
-      F3 t = f3(m, WRFGPU_T_TEND);
-      const float msfty = f2(m, WRFGPU_MSFTY).ro(i, j);
-      const float mass = f1(m, WRFGPU_C1H)(k) * f2(m, WRFGPU_MUT).ro(i, j) + f1(m, WRFGPU_C2H)(k);
-      t(i, k, j) = t(i, k, j) + f3p(m, m.tendf[3]).ro(i, k, j) / msfty + mass * 0.f / msfty;
-    }
-  }
-  if (i <= i_end && j <= j_end) {
-    F3 t = f3(m, WRFGPU_RW_TEND);
-    t(i, k, j) = t(i, k, j) + f3p(m, m.tendf[2]).ro(i, k, j) / f2(m, WRFGPU_MSFTY).ro(i, j);
   }
 }
 
@@ -613,8 +657,10 @@ void launch_addtend_dry_routine(const Launch& L, int nblocks, int rk_step, cudaS
   k_addtend_dry_routine<<<nblocks, dim3(BX, BY), 0, s>>>(L, rk_step);
 }
 
-void launch_forward_diff(const Launch& L, int nblocks, int mode, cudaStream_t s) {
-  k_forward_diff<<<nblocks, dim3(BX, BY), 0, s>>>(L, mode);
+void launch_forward_diff(const TileLaunch& L, int nblocks, int mode, cudaStream_t s, int nsp) {
+  if (mode == 1 && nsp <= 0) return;
+  const int nf = mode == 1 ? nsp : 4;
+  k_forward_diff<<<dim3(nblocks, level_chunks(nblocks * nf, L.nlev, 1, 4), nf), dim3(TX, TY), 0, s>>>(L, mode);
 }
 
 void launch_species_diff_routine(const Launch& L, int nblocks, int qv, cudaStream_t s) {
@@ -622,11 +668,11 @@ void launch_species_diff_routine(const Launch& L, int nblocks, int qv, cudaStrea
 }
 
 void launch_rayleigh_damp(const Launch& L2, int nblocks, cudaStream_t s, bool acc_all) {
-  k_rayleigh_damp<<<nblocks, dim3(BX, BY), 0, s>>>(L2, acc_all);
+  k_rayleigh_damp<<<dim3(nblocks, 4), dim3(BX, BY), 0, s>>>(L2, acc_all);
 }
 
-void launch_addtend_dry(const Launch& L, int nblocks, cudaStream_t s) {
-  k_addtend_dry<<<nblocks, dim3(BX, BY), 0, s>>>(L);
+void launch_addtend_dry(const TileLaunch& L, int nblocks, cudaStream_t s) {
+  k_addtend_dry<<<dim3(nblocks, level_chunks(nblocks, L.nlev, 1, 4, 5 * 152)), dim3(TX, TY), 0, s>>>(L);
 }
 
 }  // namespace wrfgpu

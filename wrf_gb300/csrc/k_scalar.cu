@@ -400,7 +400,9 @@ __device__ __forceinline__ void strip_update(const Mem& m, int s, int rk_step, i
   qa(i, k, j) = ((c1(k) * muold + c2(k)) * q1 + st.dt_rk * tendency) / (c1(k) * munew + c2(k));
 }
 // advect_scalar species (every species at stages 1 and 2, the others at the
-// last): the tendency plus the stored sc_tend of the species' diffusion
+// last): the tendency plus the stored sc_tend of the species' diffusion.  A
+// strip is a few hundred blocks of dependent loads: one species per blockIdx.y
+// keeps more loads in flight (190x161x60, 4 species: 33 -> 26 us).
 __global__ void __launch_bounds__(STRIP_THREADS) k_strip_scalar(StripLaunch L, int rk_step) {
   const StripPos sp = strip_pos(L);
   const Mem& m = block_member(L.mem, sp.m);
@@ -408,55 +410,60 @@ __global__ void __launch_bounds__(STRIP_THREADS) k_strip_scalar(StripLaunch L, i
   const int i = sp.i, j = sp.j, k = sp.k;
   if (!mass_pt(m, i, j) || k < m.kts || k > min(m.kte, m.kde - 1)) return;
   const F2 msfty = f2(m, WRFGPU_MSFTY);
-  for (int s = 0; s < m.nsp; ++s) {
-    if (pd_applies(m, s, rk_step)) continue;
-    const F3 fld = f3p(m, m.q[s]);
-    const ScalarAdv a{fld, fld, f3(m, WRFGPU_RU_M), f3(m, WRFGPU_RV_M), f3(m, WRFGPU_WW_M), f2(m, WRFGPU_MSFTX),
-                      f1(m, WRFGPU_FNM), f1(m, WRFGPU_FNP), f1(m, WRFGPU_RDNW)};
-    float tendency = msfty(i, j) * adv_scalar_point(m, a, 0.f, i, j, k);
-    const F3 sct = f3p(m, sc_tend_of(m, s));
-    if (sct.p) tendency = tendency + sct(i, k, j);
-    strip_update(m, s, rk_step, i, j, k, tendency);
-  }
+  const int s = blockIdx.y;
+  if (s >= m.nsp || pd_applies(m, s, rk_step)) return;
+  const F3 fld = f3p(m, m.q[s]);
+  const ScalarAdv a{fld, fld, f3(m, WRFGPU_RU_M), f3(m, WRFGPU_RV_M), f3(m, WRFGPU_WW_M), f2(m, WRFGPU_MSFTX),
+                    f1(m, WRFGPU_FNM), f1(m, WRFGPU_FNP), f1(m, WRFGPU_RDNW)};
+  float tendency = msfty(i, j) * adv_scalar_point(m, a, 0.f, i, j, k);
+  const F3 sct = f3p(m, sc_tend_of(m, s));
+  if (sct.p) tendency = tendency + sct(i, k, j);
+  strip_update(m, s, rk_step, i, j, k, tendency);
 }
-// advect_scalar_pd species s at the last stage, in two passes: the limiter
-// factors of the strip cells and their neighbours (the strip one wider, halo
-// row / column included) into the member's PD scratch, then the limited
-// divergence and the update at the strip cells
-__global__ void __launch_bounds__(STRIP_THREADS) k_strip_pd_scale(StripLaunch L, int rk_step, int s,
-                                                                 float* const* scratch) {
+// advect_scalar_pd species at the last stage, in two passes over every species
+// (blockIdx.y): the limiter factors of the strip cells and their neighbours (the
+// strip one wider, halo row / column included) into the member's scratch,
+// [species][level][strip column], then the limited divergence and the update at
+// the strip cells.  190x161x60, 4 species: a pass per species 16 and 19 us each,
+// all species at once 56 and 66.
+__global__ void __launch_bounds__(STRIP_THREADS) k_strip_pd_scale(StripLaunch L, int rk_step, float* const* scratch) {
   const StripPos sp = strip_pos(L);
   const Mem& m = block_member(L.mem, sp.m);
+  const int s = blockIdx.y;
   if (!sp.valid || s >= m.nsp || !pd_applies(m, s, rk_step)) return;
   const int i = sp.i, j = sp.j, k = sp.k;
   if (k < m.kts || k > min(m.kte, m.kde - 1)) return;
   const Stage st = stage_of(m, rk_step);
   const PDCtx c = pd_ctx(m, s, st.dt_rk, true);
-  f3p(m, scratch[sp.m])(i, k, j) = pd_scale_cell(m, c, i, k, j);
+  const long long plane = (long long)strip_cols(m.ide, m.jde, m.cf.open_xs, m.cf.open_ys, L.w, L.h) * (m.kme - m.kms + 1);
+  scratch[sp.m][s * plane + sp.p] = pd_scale_cell(m, c, i, k, j);
 }
-__global__ void __launch_bounds__(STRIP_THREADS) k_strip_pd_tend(StripLaunch L, int rk_step, int s,
+// ww, wh: the strip width and halo rows the factors were stored for
+__global__ void __launch_bounds__(STRIP_THREADS) k_strip_pd_tend(StripLaunch L, int rk_step, int ww, int wh,
                                                                 float* const* scratch) {
   const StripPos sp = strip_pos(L);
   const Mem& m = block_member(L.mem, sp.m);
+  const int s = blockIdx.y;
   if (!sp.valid || s >= m.nsp || !pd_applies(m, s, rk_step)) return;
   const int i = sp.i, j = sp.j, k = sp.k;
   if (!mass_pt(m, i, j) || k < m.kts || k > min(m.kte, m.kde - 1)) return;
   const Stage st = stage_of(m, rk_step);
   const PDCtx c = pd_ctx(m, s, st.dt_rk, true);
-  const F3 sc = f3p(m, scratch[sp.m]);
-  const float t = pd_tend_cell(m, c, i, k, j, 0.f, [&](int ci, int ck, int cj) { return sc(ci, ck, cj); });
+  const int nc = strip_cols(m.ide, m.jde, m.cf.open_xs, m.cf.open_ys, ww, wh);
+  const float* sc = scratch[sp.m] + (long long)s * nc * (m.kme - m.kms + 1);
+  const float t = pd_tend_cell(m, c, i, k, j, 0.f, [&](int ci, int ck, int cj) {
+    return sc[(ck - m.kms) * nc + strip_index(m.ide, m.jde, m.cf.open_xs, ci, cj, ww, wh)];
+  });
   strip_update(m, s, rk_step, i, j, k, f2(m, WRFGPU_MSFTY)(i, j) * t);
 }
-void launch_strip_scalar(const StripLaunch& L, int nb, int rk_step, cudaStream_t s) {
-  if (nb > 0) k_strip_scalar<<<nb, STRIP_THREADS, 0, s>>>(L, rk_step);
+void launch_strip_scalar(const StripLaunch& L, int nb, int rk_step, int nsp_max, cudaStream_t s) {
+  if (nb > 0 && nsp_max > 0) k_strip_scalar<<<dim3(nb, nsp_max), STRIP_THREADS, 0, s>>>(L, rk_step);
 }
 void launch_strip_pd(const StripLaunch& wide, int nb_wide, const StripLaunch& L, int nb, int rk_step, int nsp_max,
                      float* const* d_scratch, cudaStream_t s) {
-  if (nb <= 0) return;
-  for (int sp = 0; sp < nsp_max; ++sp) {
-    k_strip_pd_scale<<<nb_wide, STRIP_THREADS, 0, s>>>(wide, rk_step, sp, d_scratch);
-    k_strip_pd_tend<<<nb, STRIP_THREADS, 0, s>>>(L, rk_step, sp, d_scratch);
-  }
+  if (nb <= 0 || nsp_max <= 0) return;
+  k_strip_pd_scale<<<dim3(nb_wide, nsp_max), STRIP_THREADS, 0, s>>>(wide, rk_step, d_scratch);
+  k_strip_pd_tend<<<dim3(nb, nsp_max), STRIP_THREADS, 0, s>>>(L, rk_step, wide.w, wide.h, d_scratch);
 }
 
 // ------------------------------------------------------------ rk_update_scalar

@@ -94,12 +94,12 @@ void launch_tend_v_col(const TileLaunch& L, int nblocks, cudaStream_t s, int var
 void launch_tend_t_col(const TileLaunch& L, int nblocks, int flags, cudaStream_t s);
 void launch_tend_ph_col(const TileLaunch& L, int nblocks, int flags, cudaStream_t s);
 // sixth-order diffusion of the dry state at stage 1, and rk_addtend_dry (k_diff.cu)
-// mode 0: u, v, w, theta into ru_tendf .. t_tendf; 1: the species into sc_tend
-void launch_forward_diff(const Launch& L, int nblocks, int mode, cudaStream_t s);
+// mode 0: u, v, w, theta into ru_tendf .. t_tendf; 1: nsp species into sc_tend
+void launch_forward_diff(const TileLaunch& L, int nblocks, int mode, cudaStream_t s, int nsp = 0);
 void launch_species_diff_routine(const Launch& L, int nblocks, int qv, cudaStream_t s);
 void launch_addtend_dry_routine(const Launch& L, int nblocks, int rk_step, cudaStream_t s);
 void launch_rayleigh_damp(const Launch& L2, int nblocks, cudaStream_t s, bool acc_all = false);
-void launch_addtend_dry(const Launch& L, int nblocks, cudaStream_t s);
+void launch_addtend_dry(const TileLaunch& L, int nblocks, cudaStream_t s);  // staggered tiles
 
 // acoustic steps
 // 2-D part over column blocks, then the 3-D part over staggered tiles x level chunks
@@ -191,10 +191,10 @@ void launch_advance_w_col(const TileLaunch& L, int nblocks, int rk_step, int ite
 // tile kernels (k_scalar.cu)
 void launch_strip_tend(const StripLaunch& L, int nblocks, cudaStream_t s);
 void launch_strip_tend_w(const StripLaunch& L, int nblocks, cudaStream_t s);
-void launch_strip_scalar(const StripLaunch& L, int nblocks, int rk_step, cudaStream_t s);
-// the positive-definite species at the last stage, one species at a time
-// through the member's PD scratch: limiter factors over `wide`, then the
-// limited divergence and update over L
+void launch_strip_scalar(const StripLaunch& L, int nblocks, int rk_step, int nsp_max, cudaStream_t s);
+// the positive-definite species at the last stage, through the member's
+// scratch (strip_cols of `wide` x levels x species floats): limiter factors over
+// `wide`, then the limited divergence and update over L
 void launch_strip_pd(const StripLaunch& wide, int nb_wide, const StripLaunch& L, int nb, int rk_step, int nsp_max,
                      float* const* d_scratch, cudaStream_t s);
 

@@ -148,14 +148,21 @@ __device__ __forceinline__ void strip_col(const Mem& m, int c, int w, int h, int
   *i = i0 + c % ni;
   *j = r < w ? 1 + r : m.jde - w + (r - w);
 }
+// The inverse: the index of column (i, j) of the strip (it must lie in it).
+__host__ __device__ inline int strip_index(int ide, int jde, bool ox, int i, int j, int w, int h) {
+  const int nw = 2 * w + 1;
+  if (ox && (i <= w || i >= ide - w)) return (j - 1 + h) * nw + (i <= w ? i - 1 : i - (ide - w) + w);
+  const int i0 = ox ? 1 + w : 1 - h, ni = ox ? ide - nw : ide + h;
+  return (ox ? nw * (jde + h) : 0) + (j <= w ? j - 1 : j - (jde - w) + w) * ni + (i - i0);
+}
 __device__ __forceinline__ bool in_open_strip(const Mem& m, int i, int j, int w) {
   return (m.cf.open_xs && (i <= m.ids + w - 1 || i >= m.ide - w)) ||
          (m.cf.open_ys && (j <= m.jds + w - 1 || j >= m.jde - w));
 }
 // Position of a thread of a strip launch: blocks of STRIP_THREADS over each
-// member's strip columns x levels kms..kme.
+// member's strip columns x levels kms..kme (p: strip index + level x columns).
 struct StripPos {
-  int m, i, j, k;
+  int m, i, j, k, p;
   bool valid;
 };
 __device__ __forceinline__ StripPos strip_pos(const StripLaunch& L) {
@@ -163,7 +170,7 @@ __device__ __forceinline__ StripPos strip_pos(const StripLaunch& L) {
   const int b = blockIdx.x;
   sp.m = find_member(L.block_start, L.nmem, b);
   const Mem& m = L.mem[sp.m];
-  const int p = (b - __ldg(L.block_start + sp.m)) * STRIP_THREADS + (int)threadIdx.x;
+  const int p = sp.p = (b - __ldg(L.block_start + sp.m)) * STRIP_THREADS + (int)threadIdx.x;
   const int nc = strip_cols(m.ide, m.jde, m.cf.open_xs, m.cf.open_ys, L.w, L.h);
   const int nk = m.kme - m.kms + 1;
   sp.valid = nc > 0 && p < nc * nk;
