@@ -665,11 +665,15 @@ constexpr int COL_MAXW = 16;  // warps per block
 
 template <typename RC> struct alignas(2 * sizeof(RC)) Pair { RC x, y; };
 
-// Shared memory: level tables, then columns [kde + 1][32] of type RC (four:
-// the sum's terms, then c2a alt t_2ave, then w; and a, alpha, gamma, before
-// them the omega recursion's) and float (two: dv, then rhs; theta's part of p).
+// Shared memory: level tables, then columns [kde + 1][32] of type RC (sW: the
+// sum's terms, then c2a alt t_2ave, then w; FP32 three more: a, alpha, gamma,
+// before them the omega recursion's terms; FP64 one more: the omega recursion's
+// terms, then omega, then gamma, a and alpha read from global memory by the
+// elimination) and float (two: dv, then rhs; theta's part of p).  With all
+// four in FP64, 128 levels took 170 KB, one block per SM, and 270 segments two
+// waves; with two they take 106 KB and two blocks (75x90x128: 2.39 and 2.18 ms per step).
 template <typename RC> constexpr size_t col_smem(int nlev) {
-  return (size_t)(nlev + 2) * (2 * sizeof(float4) + 32 * (2 * sizeof(float) + 4 * sizeof(RC))) +
+  return (size_t)(nlev + 2) * (2 * sizeof(float4) + 32 * (2 * sizeof(float) + (sizeof(RC) == 8 ? 2 : 4) * sizeof(RC))) +
          2 * COL_MAXW * 32 * sizeof(float);
 }
 
@@ -706,10 +710,11 @@ __global__ void __launch_bounds__(32 * COL_MAXW, 1) k_advance_col(TileLaunch L, 
   float4* tB = tA + nlev + 2;
   RC* sW = reinterpret_cast<RC*>(tB + nlev + 2);
   RC* sA = sW + NC;
-  RC* sAL = sA + NC;
-  RC* sGA = sAL + NC;
+  RC* sAL = fp64 ? nullptr : sA + NC;
+  RC* sGA = fp64 ? sA : sAL + NC;
   float* sR = reinterpret_cast<float*>(sGA + NC);
   float* sQ = sR + NC;
+  RC* sS = reinterpret_cast<RC*>(sQ);  // FP64, before sQ is in use: the divergence sum, omega of level 1
   float* sX = sQ + NC;  // c2a alt t_2ave of each half warp's last level
   auto at = [&](int k) { return k * 32 + c; };
   auto rd = [&](const RC* s, int k) -> P { return *reinterpret_cast<const P*>(s + at(k)); };
@@ -785,10 +790,10 @@ __global__ void __launch_bounds__(32 * COL_MAXW, 1) k_advance_col(TileLaunch L, 
       RC s = RC(0.);
 #pragma unroll 8
       for (int k = 1; k <= k_end; ++k) s = s + sW[k * 32 + tid];
-      sGA[32 + tid] = s;
+      sS[tid] = s;
     }
     __syncthreads();
-    dmdt = rd(sGA, 1);
+    dmdt = rd(sS, 0);
     const P rmy{rcp_rc<RC>((RC)my.x), rcp_rc<RC>((RC)my.y)};
     const P dm{dmdt.x + (RC)mu_tend.x, dmdt.y + (RC)mu_tend.y};
     for (int k = ka; k <= kb; ++k) {
@@ -797,14 +802,14 @@ __global__ void __launch_bounds__(32 * COL_MAXW, 1) k_advance_col(TileLaunch L, 
       wr(sA, k, -fma(c1, dm.x, (RC)dv.x), -fma(c1, dm.y, (RC)dv.y));
       wr(sW, k, dn * rmy.x, dn * rmy.y);
     }
-    if (hw == 0) wr(sAL, 1, (RC)ww_bot.x, (RC)ww_bot.y);
+    if (hw == 0) wr(sS, 1, (RC)ww_bot.x, (RC)ww_bot.y);
     __syncthreads();
-    if (tid < 32) {
-      RC wwk = sAL[32 + tid];
+    if (tid < 32) {  // omega of level k + 1 over the term it took
+      RC wwk = sS[32 + tid];
 #pragma unroll 4
       for (int k = 1; k < k_end; ++k) {
         wwk = fma(sA[k * 32 + tid], sW[k * 32 + tid], wwk);
-        sAL[(k + 1) * 32 + tid] = wwk;
+        sA[k * 32 + tid] = wwk;
       }
     }
   } else {
@@ -866,9 +871,13 @@ __global__ void __launch_bounds__(32 * COL_MAXW, 1) k_advance_col(TileLaunch L, 
     // omega before the linear part is taken off, at levels ka - 1 and ka
     float2 wr_m = bc2(0.f), wrr = ww_bot;
     if constexpr (fp64) {
-      const P a = rd(sAL, max(ka - 1, 1)), b = rd(sAL, ka);
-      wr_m = make_float2((float)a.x, (float)a.y);
-      wrr = make_float2((float)b.x, (float)b.y);
+      auto om = [&](int k) {  // of level k
+        if (k <= 1) return ww_bot;
+        const P b = rd(sA, k - 1);
+        return make_float2((float)b.x, (float)b.y);
+      };
+      wr_m = om(ka - 1);
+      wrr = om(ka);
     } else {
 #pragma unroll 8
       for (int k = 2; k <= ka; ++k) { wr_m = wrr; wrr = sub2(wrr, rdf(sAL, k - 1)); }
@@ -904,7 +913,7 @@ __global__ void __launch_bounds__(32 * COL_MAXW, 1) k_advance_col(TileLaunch L, 
       float2 wwf_n = bc2(0.f), ww_n = ww_top;
       if (in) {
         if constexpr (fp64) {
-          const P b = rd(sAL, k + 1);
+          const P b = rd(sA, k);
           wrr = make_float2((float)b.x, (float)b.y);
         } else {
           wrr = sub2(wrr, rdf(sAL, k));
@@ -1015,7 +1024,8 @@ __global__ void __launch_bounds__(32 * COL_MAXW, 1) k_advance_col(TileLaunch L, 
         [&](int k, L4& d) {
           d.c2a = gro(c2a, i, k, j); d.ph = g(ph, k + 1); d.w = g(w, k);
           d.rwt = gro(rwt, i, k, j); d.cqw = gro(cqw, i, k, j);
-          d.a = coef(0, k); d.al = coef(1, k); d.ga = coef(2, k);
+          if constexpr (!fp64) { d.a = coef(0, k); d.al = coef(1, k); }
+          d.ga = coef(2, k);
         },
         [&](int k, const L4& d) {
           c_c2a = d.c2a;
@@ -1029,8 +1039,10 @@ __global__ void __launch_bounds__(32 * COL_MAXW, 1) k_advance_col(TileLaunch L, 
                                         mul(mul(msft_inv, d.cqw), muls(+.5f * dts * G * rdnk, sub2(dz_k, dz_m)))),
                                    mul(muls(dts * G, msft_inv), sub2(muls(rdnk, sub2(x, x_m)), muls(tA[k].z, mua))));
             wr(sW, k, (RC)wk.x, (RC)wk.y);
-            wr(sA, k, d.a.x, d.a.y);
-            wr(sAL, k, d.al.x, d.al.y);
+            if constexpr (!fp64) {
+              wr(sA, k, d.a.x, d.a.y);
+              wr(sAL, k, d.al.x, d.al.y);
+            }
             wr(sGA, k, d.ga.x, d.ga.y);
           }
           dz_m = dz_k; x_m = x; r_m = r_k; ph_m = ph_k; r_k = r_p; ph_k = ph_p;
@@ -1046,23 +1058,31 @@ __global__ void __launch_bounds__(32 * COL_MAXW, 1) k_advance_col(TileLaunch L, 
       float2 wk = add2(add2(g(w, k), muls(dts, gro(rwt, i, k, j))),
                        mul(msft_inv, sub2(a, muls(dts * G, add2(x_top, muls(tA[k].z, mua))))));
       if (m.cf.top_lid) wk = bc2(0.f);
-      const P ca = coef(0, k), cal = coef(1, k);
       wr(sW, k, (RC)wk.x, (RC)wk.y);
-      wr(sA, k, ca.x, ca.y);
-      wr(sAL, k, cal.x, cal.y);
+      if constexpr (!fp64) {
+        const P ca = coef(0, k), cal = coef(1, k);
+        wr(sA, k, ca.x, ca.y);
+        wr(sAL, k, cal.x, cal.y);
+      }
     }
   }
   __syncthreads();
   // ---- the tridiagonal solve, one lane per column; a batch of levels is read
   // ahead of its recursion
   if (tid < 32) {
-    constexpr int Q = fp64 ? 4 : 8;
+    constexpr int Q = 8;  // FP64, whose a and alpha come from global memory: 4 / 6 / 8 2.23 / 2.19 / 2.18 ms per step
     RC wk = sW[32 + tid], b[Q], a[Q], al[Q];
+    const int ic = i0 + tid <= i_end ? i0 + tid : i0;  // a lane past the domain takes the first column
     auto up = [&](int kq) {
 #pragma unroll
       for (int q = 0; q < Q; ++q) {
-        const int o = min(kq + q, kde) * 32 + tid;
-        b[q] = sW[o]; a[q] = sA[o]; al[q] = sAL[o];
+        const int k = min(kq + q, kde), o = k * 32 + tid;
+        b[q] = sW[o];
+        if constexpr (fp64) {
+          a[q] = __ldg(&d3(m, m.wd[0])(ic, k, j)); al[q] = __ldg(&d3(m, m.wd[1])(ic, k, j));
+        } else {
+          a[q] = sA[o]; al[q] = sAL[o];
+        }
       }
     };
     up(2);
