@@ -309,7 +309,7 @@ template <typename RC>
 __global__ void __launch_bounds__(TX* TY) k_calc_coef_w_col(TileLaunch L, int rk_step) {
   const TilePos tp = tile_pos(L, false, false);
   const Mem& m = block_member(L.mem, tp.m);
-  const int i = tp.i0 + threadIdx.x, j = tp.j0 + threadIdx.y;
+  const int i = tp.i0 + threadIdx.x, j = tp.j0 + blockIdx.y * blockDim.y + threadIdx.y;
   if (i > min(m.ite, m.ide - 1) || j > min(m.jte, m.jde - 1)) return;
   coef_w_column<RC>(m, i, j, rk_step);
 }
@@ -829,8 +829,13 @@ void launch_calc_p_rho_col(const TileLaunch& L, int nb, StepArgs a, cudaStream_t
   else k_calc_p_rho_col<false, false><<<dim3(nb, chunks), dim3(TX, TY), 0, s>>>(L, a.rk_step, 0);
 }
 void launch_calc_coef_w_col(const TileLaunch& L, int nb, StepArgs a, bool fp64, cudaStream_t s) {
-  if (fp64) k_calc_coef_w_col<double><<<nb, dim3(TX, TY), 0, s>>>(L, a.rk_step);
-  else k_calc_coef_w_col<float><<<nb, dim3(TX, TY), 0, s>>>(L, a.rk_step);
+  // a tile's rows over two blocks where the recursion, not the memory, bounds
+  // (a few warps per SM, or FP64): ms per step of 8 / 4 / 1 rows per block, FP64
+  // 75x90x128 0.403 / 0.357 / 0.361, 16 members 1.73 / 1.64 / 1.73; FP32 24 small members (363
+  // tiles) 0.210 / 0.189 / 0.186, 512x512x80 (1024 tiles) 0.485 / 0.491 / 0.497
+  const int rows = fp64 || nb <= 4 * 152 ? TY / 2 : TY;
+  if (fp64) k_calc_coef_w_col<double><<<dim3(nb, TY / rows), dim3(TX, rows), 0, s>>>(L, a.rk_step);
+  else k_calc_coef_w_col<float><<<dim3(nb, TY / rows), dim3(TX, rows), 0, s>>>(L, a.rk_step);
 }
 void launch_calc_coef_w(const Launch& L, int nb, StepArgs a, bool fp64, cudaStream_t s) {
   if (fp64) k_calc_coef_w<double><<<nb, dim3(BX, BY), 0, s>>>(L, a.rk_step);
