@@ -2,7 +2,7 @@
 columns; one thread per column above col_max_segments) bit for bit with the
 FP32 oracle at the sizes where their index arithmetic can go wrong: row
 segments of one column, one short of full, full and one over, the shortest
-and the tallest column, odd widths (whose last pair of columns is half
+and the tallest column, the smallest domain accepted, odd widths (whose last pair of columns is half
 inside), and a domain on each side of the size rule.  The FP64 column form
 is compared between the two: a member alone takes one of them, in an ensemble
 above the rule the other, and the fields agree bit for bit.
@@ -25,7 +25,8 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("nx,ny,kde", [(31, 9, 14), (32, 8, 15), (33, 10, 17), (64, 9, 33), (65, 8, 128),
-                                       (12, 3011, 14), (33, 1510, 16), (31, 950, 14), (40, 1255, 15)])
+                                       (12, 3011, 14), (33, 1510, 16), (31, 950, 14), (40, 1255, 15),
+                                       (7, 7, 6), (33, 7, 7)])
 def test_column_forms_bitwise(gpulib, nx, ny, kde):
     case = cases.small_case(nx=nx, ny=ny, kde=kde, n_scalar=1, seed=nx + kde)
     od = OracleDomain(case, "f32")

@@ -310,8 +310,9 @@ FFM_HD ff ff_sin_t(float x) {
 // float-float series with Ziv's rounding test (FP64 runs at 1/64 of the FP32
 // rate here, and at the damping layer's top the sine's distance to 1 sent every
 // column through the double-double series: the damped column kernel of the
-// acoustic step took 1.88 ms per large step of 160x144x64, now 0.76).  Then the FP64 sine (libm on the host, CUDA's double sin on
-// the device; both within 2 ulp of FP64) rounded once, accepted when it lies
+// acoustic step took 1.88 ms per large step of 160x144x64, now 0.76).  Then the
+// FP64 sine (libm on the host, CUDA's double sin on the device; both within 2 ulp
+// of FP64) rounded once, accepted when it lies
 // farther than 2^-45 of its value from a float rounding boundary; otherwise
 // the double-double series decides (the same code on host and device).  Used
 // by the w Rayleigh damping of advance_w (damp_opt = 3), whose argument lies

@@ -174,7 +174,7 @@ void launch_advance_uv_col(const TileLaunch& L, int nblocks, int rk_step, int it
 // 190x161x60 (966) 0.77 / 1.33, 256x256x80 (2048) 1.70 / 1.99, 24 small members
 // (about 2900) 2.23 / 2.30, 512x512x80 (8192) 6.30 / 5.67, 1024x1024x96 (32768)
 // 29.0 / 24.9; FP64 columns (whose chains wait about 110 cycles per operation)
-// 75x90x128 (270) 1.12 / 3.11, 16 members of up to 256x256x80 (about 14000)
+// 75x90x128 (270) 0.81 / 3.11, 16 members of up to 256x256x80 (about 14000)
 // 17.5 / 9.3; with damp_opt = 3 160x144x64 (720) 0.76 / 1.39.
 constexpr int col_max_segments(bool fp64) { return fp64 ? 1000 : 3000; }
 // damp: some member uses damp_opt = 3 (compiles the damping into the kernel)
