@@ -60,8 +60,8 @@ def alg_bytes_per_cell_step(phase, s_pd, s_all, n_acoustic=7):
         "calc_p_rho_0": 3 * (7 + 3),
         "calc_coef_w": 3 * (2 + 3),
         "advance_uv": n_acoustic * (14 + 4),         # with sumflux's ru_m, rv_m
-        "advance_mu_t": n_acoustic * (10 + 4),       # with sumflux's ww_m
-        "advance_w": n_acoustic * (17 + 3),
+        "advance_mu_t": n_acoustic * (10 + 5),       # with sumflux's ww_m and t_2ave
+        "advance_w": n_acoustic * (14 + 2),
         "sumflux_calc_p_rho": n_acoustic * (6 + 3),  # calc_p_rho alone
         "small_step_finish": 3 * (13 + 6),
         "rk_update_scalar_pd": 2 * s_pd,
@@ -90,12 +90,10 @@ def contract_bytes_per_cell_step(n_moist, n_species, mixed=False):
 # DRAM bytes (read + write) per mass cell of one launch, from the ncu
 # captures summarised in profiles/ (256x256x80 case, inputs far larger than
 # L2; traffic grows with the cells processed, so it scales to other sizes):
-# the capture of k_scalar_pd_update, of k_scalar_adv_update (stage 1) and of
-# the acoustic column kernels.
+# the captures of k_scalar_pd_update and of k_scalar_adv_update (stage 1).
 NCU_DRAM_BYTES_PER_CELL = {
     "scalar_pd_update": 1032.8e6 / 5177344,
     "scalar_adv_update": 780.6e6 / 5177344,
-    "advance_w": 451.3e6 / 5177344,
 }
 
 PHASE_NAMES = ["step_prep", "rk_tend_u", "rk_tend_v", "rk_tend_w", "rk_tend_t", "rk_tend_ph", "cfl_check",
