@@ -266,7 +266,8 @@ __device__ __forceinline__ void pd_tile(const Mem& m, int species, int rk_step, 
     }
   }
   float sc_m1 = -1.f, sc_0 = -1.f, sc_p1 = -1.f;  // own column's factors at levels L-2, L-1, L
-  auto lim = [](float h, float sc) { return sc >= 0.f ? sc * h : h; };
+  // (selections, no branches: a warp's faces have either sign)
+  auto lim = [](float h, float sc) { return sc >= 0.f && h != 0.f ? sc * h : h; };
   cp_async_wait<2>();
   __syncthreads();  // level L0 staged
   for (int L = L0; L <= k1 + 1; ++L) {
@@ -339,19 +340,21 @@ __device__ __forceinline__ void pd_tile(const Mem& m, int species, int rk_step, 
       const float* SC = sSC + (k & 1) * P::SN;
       t = scalar_radiation(m, f, fo, ru, rv, t, i, j, k);
       float h0 = hzm, h1 = hz0;
-      if (k > 1) { if (h0 < 0.f) h0 = lim(h0, sc_m1); else if (h0 > 0.f) h0 = lim(h0, sc_0); }
-      if (k + 1 < kde) { if (h1 < 0.f) h1 = lim(h1, sc_0); else if (h1 > 0.f) h1 = lim(h1, sc_p1); }
+      if (k > 1) h0 = lim(h0, h0 < 0.f ? sc_m1 : sc_0);
+      if (k + 1 < kde) h1 = lim(h1, h1 < 0.f ? sc_0 : sc_p1);
       t = t - sLV[k - kts].a.z * (h1 - h0 + lz0 - lzm);
       if (xdiv) {
         float g0 = kXH[xq], g1 = kXH[xq + 1];
-        if (g0 > 0.f) g0 = lim(g0, SC[so - 1]); else if (g0 < 0.f) g0 = lim(g0, sc_0);
-        if (g1 > 0.f) g1 = lim(g1, sc_0); else if (g1 < 0.f) g1 = lim(g1, SC[so + 1]);
+        const float sm = SC[so - 1], sp = SC[so + 1];
+        g0 = lim(g0, g0 > 0.f ? sm : sc_0);
+        g1 = lim(g1, g1 > 0.f ? sc_0 : sp);
         t = t - mx * (rdx * (g1 - g0 + kXL[xq + 1] - kXL[xq]));
       }
       if (ydiv) {
         float g0 = kYH[yq], g1 = kYH[yq + P::YW];
-        if (g0 > 0.f) g0 = lim(g0, SC[so - P::SW]); else if (g0 < 0.f) g0 = lim(g0, sc_0);
-        if (g1 > 0.f) g1 = lim(g1, sc_0); else if (g1 < 0.f) g1 = lim(g1, SC[so + P::SW]);
+        const float sm = SC[so - P::SW], sp = SC[so + P::SW];
+        g0 = lim(g0, g0 > 0.f ? sm : sc_0);
+        g1 = lim(g1, g1 > 0.f ? sc_0 : sp);
         t = t - mx * (rdy * (g1 - g0 + kYL[yq + P::YW] - kYL[yq]));
       }
       tend(i, k, j) = t;
