@@ -5,6 +5,8 @@ cut into many level chunks, periodic and open on all sides; and, on device
 arrays whose rows are neither 16-byte aligned nor a multiple of 16 bytes,
 equal to the host-array entry point (test_zz_no_alloc's calls).
 """
+import ctypes as C
+
 import numpy as np
 import pytest
 
@@ -12,6 +14,8 @@ from wrf_gb300 import abi, cases
 from wrf_gb300 import gpu as G
 
 from _harness import OracleDomain, interior, max_abs
+from test_fortran_abi import _fid, _scalars, _state
+from test_zz_no_alloc import NAMES, _Args, _dims
 
 pytestmark = pytest.mark.gpu
 
@@ -35,3 +39,66 @@ def test_routine_pd_bitwise(gpulib, nx, ny, kde, open_sides):
         a, b = interior(case, fid, ge.get(0, fid)), interior(case, fid, od.get(fid))
         assert float(np.max(np.abs(b))) > 0.0
         assert max_abs(a, b) == 0.0
+
+def _device_call(lib, case, dev, tend, scal, stream):
+    """wrfgpu_advect_scalar_pd_noalloc's argument list on `stream`: (function, arguments, what they point to)."""
+    a = _Args()
+    a.ptr(dev["qv"].data_ptr()); a.ptr(dev["qv_old"].data_ptr()); a.ptr(tend.data_ptr())
+    for nm in ("ru_m", "rv_m", "ww_m", "c1h", "c2h", "muts", "mub", "mu_1"):
+        a.ptr(dev[nm].data_ptr())
+    a.cfg(case.desc.config)
+    for nm in ("msftx", "msfty", "fnm", "fnp"):
+        a.ptr(dev[nm].data_ptr())
+    a.f32(scal["rdx"]); a.f32(scal["rdy"]); a.ptr(dev["rdnw"].data_ptr()); a.f32(scal["dtrk"])
+    for d in _dims(case):
+        a.i32(d)
+    a.args.append(C.c_void_p(stream))
+    fn = lib.wrfgpu_advect_scalar_pd_noalloc
+    fn.restype = C.c_int
+    fn.argtypes = [C.c_void_p] * len(a.args)
+    return fn, a.args, a
+
+
+def test_device_calls_of_two_threads(gpulib):
+    """Two host threads, each on its own stream, over columns of 14 and of 128 levels: the kernel's shared
+    memory depends on the height, and neither thread's calls may be refused or changed by the other's.  Every
+    call accumulates onto the thread's tendency, whose end state equals the same calls made alone."""
+    import threading
+
+    torch = pytest.importorskip("torch")
+    ncall = 2000
+    jobs = []
+    for kde in (14, 128):
+        case = cases.small_case(nx=16, ny=12, kde=kde, n_scalar=0, seed=kde)
+        od = _state(case)
+        dev = {nm: torch.from_numpy(np.ascontiguousarray(od.get(_fid(nm)), dtype=np.float32)).cuda() for nm in NAMES}
+        n = np.asarray(od.get(abi.FIELD_ID["advect_tend"])).size
+        tends = [torch.zeros(n, device="cuda") for _ in range(2)]
+        stream = torch.cuda.Stream()
+        calls = [_device_call(gpulib, case, dev, t, _scalars(case, 3, 1), stream.cuda_stream) for t in tends]
+        jobs.append((dev, tends, calls))
+    torch.cuda.synchronize()
+
+    def many(call):
+        fn, args, _ = call
+        return [rc for rc in (fn(*args) for _ in range(ncall)) if rc != 0]
+
+    for _, _, calls in jobs:  # alone, one thread after the other
+        assert many(calls[0]) == []
+    refused = {}
+    ready = threading.Barrier(2)
+
+    def work(q):
+        ready.wait()
+        refused[q] = many(jobs[q][2][1])
+
+    threads = [threading.Thread(target=work, args=(q,)) for q in range(2)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    torch.cuda.synchronize()
+    assert refused == {0: [], 1: []}
+    for _, tends, _ in jobs:
+        assert float(tends[0].abs().max()) > 0.0
+        assert torch.equal(tends[0], tends[1])

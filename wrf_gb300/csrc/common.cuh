@@ -25,6 +25,7 @@
 namespace wrfgpu {
 
 constexpr int NSPMAX = 16;           // species per member (moist + passive)
+constexpr int KDE_MAX = 128;         // tallest column accepted (check_desc)
 constexpr int TMA_HALO = 4;          // halo of the staged planes
 constexpr int BX = 32, BY = 4;       // thread block: 32 (i) x 4 (j)
 constexpr float G = 9.81f;
@@ -476,6 +477,16 @@ struct TileLaunch {
   int nmem;
   int nlev = 0;            // levels of the tallest member (host: the launchers' level chunks)
 };
+
+// Allows a kernel more than 48 KB of dynamic shared memory.  The allowance is
+// one value per kernel and device, shared by every thread that launches it, so
+// every caller gives the kernel's largest size, that of the tallest column, and
+// never the size of its own launch: a call for a short column would lower the
+// allowance under another thread's launch of a taller one, which is then refused.
+template <typename K>
+inline void allow_smem(K kernel, size_t largest) {
+  cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)largest);
+}
 
 // Level chunks (gridDim.y) of a column kernel of nblocks tiles, `resident` of
 // whose blocks the GPU holds at a time: the count from `base` on with the

@@ -58,7 +58,7 @@ static const char* PHASE_NAMES[NPHASE] = {
 
 int check_desc(const WrfGpuDomainDesc& d) {
   const WrfDynConfig& c = d.config;
-  if (d.ide < 8 || d.jde < 8 || d.kde < 6 || d.kde > 128) return WRFGPU_E_ARG;
+  if (d.ide < 8 || d.jde < 8 || d.kde < 6 || d.kde > KDE_MAX) return WRFGPU_E_ARG;
   if (d.n_moist != 1 || d.n_scalar < 0 || d.n_moist + d.n_scalar > NSPMAX) return WRFGPU_E_ARG;
   if (c.rk_ord != 3 || c.h_mom_adv_order != 5 || c.h_sca_adv_order != 5 || c.v_mom_adv_order != 3 ||
       c.v_sca_adv_order != 3)

@@ -709,23 +709,19 @@ void launch_update_scalar_pd_col(const TileLaunch& L, int nb, StepArgs a, cudaSt
 void launch_advect_scalar(const Launch& L, int nb, StepArgs a, cudaStream_t s) {
   k_advect_scalar<<<nb, dim3(BX, BY), 0, s>>>(L, a.species, a.rk_step, a.flags);
 }
-// Shared memory of pd_tile; the attribute belongs to the current device's
-// context, so it is set at every launch (a table lookup).
-template <typename K>
-static size_t pdr_smem(K kernel, int nlev) {
-  const size_t n = PdrPlanes::FLOATS * 4 + (size_t)nlev * sizeof(PdrLevel);
-  cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)n);
-  return n;
-}
+// Shared memory of pd_tile for columns of nlev levels.
+constexpr size_t pdr_bytes(int nlev) { return PdrPlanes::FLOATS * 4 + (size_t)nlev * sizeof(PdrLevel); }
 // a chunk computes two levels more than it writes; two blocks per SM
 void launch_advect_scalar_pd(const TileLaunch& L, int nb, int species, int rk_step, bool accum, cudaStream_t s) {
   const dim3 grid(nb, level_chunks(nb, L.nlev, 1, 6, 2 * 152));
-  k_pd_tend<<<grid, PdrPlanes::THREADS, pdr_smem(k_pd_tend, L.nlev), s>>>(L, species, rk_step, accum);
+  allow_smem(k_pd_tend, pdr_bytes(KDE_MAX));
+  k_pd_tend<<<grid, PdrPlanes::THREADS, pdr_bytes(L.nlev), s>>>(L, species, rk_step, accum);
 }
 void launch_advect_scalar_pd_member(const Mem& m, int rk_step, bool accum, cudaStream_t s) {
   const int nb = tiles_x(m) * tiles_y(m), nlev = m.kme - m.kms + 1;
   const dim3 grid(nb, level_chunks(nb, nlev, 1, 6, 2 * 152));
-  k_pd_tend_member<<<grid, PdrPlanes::THREADS, pdr_smem(k_pd_tend_member, nlev), s>>>(m, rk_step, accum);
+  allow_smem(k_pd_tend_member, pdr_bytes(KDE_MAX));
+  k_pd_tend_member<<<grid, PdrPlanes::THREADS, pdr_bytes(nlev), s>>>(m, rk_step, accum);
 }
 void launch_update_scalar_routine(const Launch& L, int nb, int rk_step, int pd, cudaStream_t s) {
   k_update_scalar_routine<<<nb, dim3(BX, BY), 0, s>>>(L, rk_step, pd);

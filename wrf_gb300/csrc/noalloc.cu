@@ -52,7 +52,7 @@ extern "C" int wrfgpu_advect_scalar_pd_noalloc(
       *jme != *jde + WRFGPU_HALO || *kms != 1 || *kme != *kde)
     return WRFGPU_E_ARG;
   if (*its != 1 || *ite != *ide || *jts != 1 || *jte != *jde || *kts != 1 || *kte != *kde) return WRFGPU_E_ARG;
-  if (*ide < 8 || *jde < 8 || *kde < 6 || *kde > 128) return WRFGPU_E_ARG;  // the limits of a member
+  if (*ide < 8 || *jde < 8 || *kde < 6 || *kde > KDE_MAX) return WRFGPU_E_ARG;  // the limits of a member
   const long long ni = *ime - *ims + 1, nk = *kme - *kms + 1, nj = *jme - *jms + 1;
   if (ni * nk * nj > NOALLOC_MAX_POINTS) return WRFGPU_E_SIZE;
   if (!(*dt > 0.f) || !(*rdx > 0.f) || !(*rdy > 0.f)) return WRFGPU_E_ARG;
