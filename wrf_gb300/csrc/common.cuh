@@ -480,9 +480,11 @@ struct TileLaunch {
 
 // Allows a kernel more than 48 KB of dynamic shared memory.  The allowance is
 // one value per kernel and device, shared by every thread that launches it, so
-// every caller gives the kernel's largest size, that of the tallest column, and
-// never the size of its own launch: a call for a short column would lower the
-// allowance under another thread's launch of a taller one, which is then refused.
+// every launch sets it (the device may be another than the last launch's; a
+// captured step pays once), and every caller gives the kernel's largest size,
+// that of the tallest column, and never the size of its own launch: a call for
+// a short column would lower the allowance under another thread's launch of a
+// taller one, which is then refused.
 template <typename K>
 inline void allow_smem(K kernel, size_t largest) {
   cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)largest);

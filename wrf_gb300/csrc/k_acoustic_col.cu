@@ -612,25 +612,19 @@ void launch_advance_mu_t_col(const TileLaunch& L, int nblocks, int rk_step, int 
 template <bool DAMP>
 static void launch_advance_w_var(const TileLaunch& L, int nblocks, int rk_step, int iteration, bool fp64,
                                  cudaStream_t s, int minb) {
-  static bool attr = false;
   constexpr size_t S32 = AwCfg<float>::Ring::SMEM, S64 = AwCfg<double>::Ring::SMEM;
-  if (!attr) {
-    cudaFuncSetAttribute(k_advance_w_col<float, 2, DAMP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S32);
-    cudaFuncSetAttribute(k_advance_w_col<float, 3, DAMP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S32);
-    cudaFuncSetAttribute(k_advance_w_col<float, 4, DAMP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S32);
-    cudaFuncSetAttribute(k_advance_w_col<double, 2, DAMP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S64);
-    cudaFuncSetAttribute(k_advance_w_col<double, 3, DAMP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S64);
-    cudaFuncSetAttribute(k_advance_w_col<double, 4, DAMP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S64);
-    attr = true;
-  }
+  auto run = [&](auto kernel, size_t smem) {
+    allow_smem(kernel, smem);
+    kernel<<<nblocks, dim3(TX, TY), smem, s>>>(L, rk_step, iteration);
+  };
   if (fp64) {
-    if (minb == 2) k_advance_w_col<double, 2, DAMP><<<nblocks, dim3(TX, TY), S64, s>>>(L, rk_step, iteration);
-    else if (minb == 3) k_advance_w_col<double, 3, DAMP><<<nblocks, dim3(TX, TY), S64, s>>>(L, rk_step, iteration);
-    else k_advance_w_col<double, 4, DAMP><<<nblocks, dim3(TX, TY), S64, s>>>(L, rk_step, iteration);
+    if (minb == 2) run(k_advance_w_col<double, 2, DAMP>, S64);
+    else if (minb == 3) run(k_advance_w_col<double, 3, DAMP>, S64);
+    else run(k_advance_w_col<double, 4, DAMP>, S64);
   } else {
-    if (minb == 2) k_advance_w_col<float, 2, DAMP><<<nblocks, dim3(TX, TY), S32, s>>>(L, rk_step, iteration);
-    else if (minb == 3) k_advance_w_col<float, 3, DAMP><<<nblocks, dim3(TX, TY), S32, s>>>(L, rk_step, iteration);
-    else k_advance_w_col<float, 4, DAMP><<<nblocks, dim3(TX, TY), S32, s>>>(L, rk_step, iteration);
+    if (minb == 2) run(k_advance_w_col<float, 2, DAMP>, S32);
+    else if (minb == 3) run(k_advance_w_col<float, 3, DAMP>, S32);
+    else run(k_advance_w_col<float, 4, DAMP>, S32);
   }
 }
 void launch_advance_w_col(const TileLaunch& L, int nblocks, int rk_step, int iteration, bool fp64, cudaStream_t s,
@@ -1201,23 +1195,18 @@ __global__ void __launch_bounds__(32 * COL_MAXW, 1) k_advance_col(TileLaunch L, 
 
 void launch_advance_col(const TileLaunch& L, int nblocks, int nlev_max, int rk_step, int iteration, bool fp64,
                         cudaStream_t s, bool damp) {
-  static bool attr = false;
-  if (!attr) {
-    const int f = (int)col_smem<float>(128), d = (int)col_smem<double>(128);
-    cudaFuncSetAttribute(k_advance_col<float, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, f);
-    cudaFuncSetAttribute(k_advance_col<float, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, f);
-    cudaFuncSetAttribute(k_advance_col<double, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, d);
-    cudaFuncSetAttribute(k_advance_col<double, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, d);
-    attr = true;
-  }
   const size_t sm = fp64 ? col_smem<double>(nlev_max) : col_smem<float>(nlev_max);
   // two blocks of 8 warps per SM; 16 warps where shared memory or the domain
   // leaves an SM one block (41x41x41: 0.131 against 0.145 ms per step)
   const int threads = 32 * (sm > 113 * 1024 || nblocks <= 152 ? COL_MAXW : COL_MAXW / 2);
-  if (fp64 && damp) k_advance_col<double, true><<<nblocks, threads, sm, s>>>(L, rk_step, iteration);
-  else if (fp64) k_advance_col<double, false><<<nblocks, threads, sm, s>>>(L, rk_step, iteration);
-  else if (damp) k_advance_col<float, true><<<nblocks, threads, sm, s>>>(L, rk_step, iteration);
-  else k_advance_col<float, false><<<nblocks, threads, sm, s>>>(L, rk_step, iteration);
+  auto run = [&](auto kernel, size_t largest) {
+    allow_smem(kernel, largest);
+    kernel<<<nblocks, threads, sm, s>>>(L, rk_step, iteration);
+  };
+  if (fp64 && damp) run(k_advance_col<double, true>, col_smem<double>(KDE_MAX));
+  else if (fp64) run(k_advance_col<double, false>, col_smem<double>(KDE_MAX));
+  else if (damp) run(k_advance_col<float, true>, col_smem<float>(KDE_MAX));
+  else run(k_advance_col<float, false>, col_smem<float>(KDE_MAX));
 }
 
 }  // namespace wrfgpu

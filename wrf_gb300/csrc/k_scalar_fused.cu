@@ -676,40 +676,30 @@ __global__ void k_swap_species(Mem* mems, int nmem, unsigned pairs) {
   }
 }
 
-template <typename K>
-static void set_smem(K kernel, size_t bytes) {
-  cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
-}
 void launch_scalar_adv_update(const TileLaunch& L, int nblocks, int rk_step, cudaStream_t s, int var, bool sct,
                               unsigned pairs) {
-  static bool attr = false;
-  if (!attr) {
-    set_smem(k_scalar_adv_update<2, false>, ADV_SMEM);
-    set_smem(k_scalar_adv_update<3, false>, ADV_SMEM);
-    set_smem(k_scalar_adv_update<4, false>, ADV_SMEM);
-    set_smem(k_scalar_adv_update<3, true>, ADV_SMEM);
-    attr = true;
-  }
   const int minb = TUNE_PARAM[TU_ADV][var];
   const dim3 grid(nblocks, level_chunks(nblocks, L.nlev, 1, 4, 3 * 152));
-  if (sct) k_scalar_adv_update<3, true><<<grid, dim3(TX, TY), ADV_SMEM, s>>>(L, rk_step, pairs);
-  else if (minb == 2) k_scalar_adv_update<2, false><<<grid, dim3(TX, TY), ADV_SMEM, s>>>(L, rk_step, pairs);
-  else if (minb == 3) k_scalar_adv_update<3, false><<<grid, dim3(TX, TY), ADV_SMEM, s>>>(L, rk_step, pairs);
-  else k_scalar_adv_update<4, false><<<grid, dim3(TX, TY), ADV_SMEM, s>>>(L, rk_step, pairs);
+  auto run = [&](auto kernel) {
+    allow_smem(kernel, ADV_SMEM);
+    kernel<<<grid, dim3(TX, TY), ADV_SMEM, s>>>(L, rk_step, pairs);
+  };
+  if (sct) run(k_scalar_adv_update<3, true>);
+  else if (minb == 2) run(k_scalar_adv_update<2, false>);
+  else if (minb == 3) run(k_scalar_adv_update<3, false>);
+  else run(k_scalar_adv_update<4, false>);
 }
 void launch_scalar_pd_update(const TileLaunch& L, int nblocks, int nlev_max, int rk_step, cudaStream_t s, int var,
                              unsigned pairs) {
-  static size_t attr = 0;
-  const size_t bytes = PD_SMEM + sizeof(LevelConst) * (size_t)nlev_max;
-  if (bytes > attr) {
-    set_smem(k_scalar_pd_update<1>, bytes);
-    set_smem(k_scalar_pd_update<2>, bytes);
-    attr = bytes;
-  }
+  auto smem = [](int nlev) { return PD_SMEM + sizeof(LevelConst) * (size_t)nlev; };
   // a chunk computes two levels more than it writes
   const dim3 grid(nblocks, level_chunks(nblocks, L.nlev, 1, 4, 2 * 152));
-  if (TUNE_PARAM[TU_PD][var] == 1) k_scalar_pd_update<1><<<grid, PD_THREADS, bytes, s>>>(L, rk_step, pairs);
-  else k_scalar_pd_update<2><<<grid, PD_THREADS, bytes, s>>>(L, rk_step, pairs);
+  auto run = [&](auto kernel) {
+    allow_smem(kernel, smem(KDE_MAX));
+    kernel<<<grid, PD_THREADS, smem(nlev_max), s>>>(L, rk_step, pairs);
+  };
+  if (TUNE_PARAM[TU_PD][var] == 1) run(k_scalar_pd_update<1>);
+  else run(k_scalar_pd_update<2>);
 }
 void launch_pd_courant(const Launch& L2, int nblocks, int rk_step, cudaStream_t s) {
   k_pd_courant<<<dim3(nblocks, level_chunks(nblocks, L2.nlev, 1, 4, 8 * 152)), dim3(BX, BY), 0, s>>>(L2, rk_step);

@@ -381,12 +381,9 @@ __global__ void __launch_bounds__(32 * COEF_WARPS) k_calc_coef_w_row(TileLaunch 
   }
 }
 void launch_calc_coef_w_row(const TileLaunch& L, int nb, StepArgs a, cudaStream_t s) {
-  static bool attr = false;
-  if (!attr) {
-    cudaFuncSetAttribute(k_calc_coef_w_row, cudaFuncAttributeMaxDynamicSharedMemorySize, 129 * 32 * 20);
-    attr = true;
-  }
-  k_calc_coef_w_row<<<nb, 32 * COEF_WARPS, (size_t)(L.nlev + 1) * 32 * 20, s>>>(L, a.rk_step);
+  auto bytes = [](int nlev) { return (size_t)(nlev + 1) * 32 * 20; };
+  allow_smem(k_calc_coef_w_row, bytes(KDE_MAX));
+  k_calc_coef_w_row<<<nb, 32 * COEF_WARPS, bytes(L.nlev), s>>>(L, a.rk_step);
 }
 
 // ------------------------------------------------------------ advance_uv

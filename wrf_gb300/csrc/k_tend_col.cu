@@ -765,18 +765,15 @@ void launch_tend_v_col(const TileLaunch& L, int nb, cudaStream_t s, int var) {
   launch_tend_uv<1>(L, nb, s, TUNE_PARAM[TU_TENDV][var]);
 }
 void launch_tend_w_col(const TileLaunch& L, int nb, int var, cudaStream_t s) {
-  static bool attr = false;
-  if (!attr) {
-    cudaFuncSetAttribute(k_tend_w_col<TF_ALL, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TENDW_SMEM);
-    cudaFuncSetAttribute(k_tend_w_col<TF_ALL, 3>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TENDW_SMEM);
-    cudaFuncSetAttribute(k_tend_w_col<TF_ALL, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TENDW_SMEM);
-    attr = true;
-  }
   const int minb = TUNE_PARAM[TU_TENDW][var];
   const dim3 grid(nb, level_chunks(nb, L.nlev, 1, TEND_MINLEV));
-  if (minb == 2) k_tend_w_col<TF_ALL, 2><<<grid, dim3(TX, TY), TENDW_SMEM, s>>>(L);
-  else if (minb == 3) k_tend_w_col<TF_ALL, 3><<<grid, dim3(TX, TY), TENDW_SMEM, s>>>(L);
-  else k_tend_w_col<TF_ALL, 4><<<grid, dim3(TX, TY), TENDW_SMEM, s>>>(L);
+  auto run = [&](auto kernel) {
+    allow_smem(kernel, TENDW_SMEM);
+    kernel<<<grid, dim3(TX, TY), TENDW_SMEM, s>>>(L);
+  };
+  if (minb == 2) run(k_tend_w_col<TF_ALL, 2>);
+  else if (minb == 3) run(k_tend_w_col<TF_ALL, 3>);
+  else run(k_tend_w_col<TF_ALL, 4>);
 }
 void launch_tend_t_col(const TileLaunch& L, int nb, int flags, cudaStream_t s) {
   if (flags == (TF_ZERO | TF_ADV)) k_tend_t_col<TF_ZERO | TF_ADV, 4><<<dim3(nb, level_chunks(nb, L.nlev, 1, TEND_MINLEV)), dim3(TX, TY), TEND_SMEM, s>>>(L);
