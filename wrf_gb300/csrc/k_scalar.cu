@@ -127,7 +127,8 @@ __global__ void __launch_bounds__(BX* BY) k_advect_scalar(Launch L, int species,
 // (the face's two cells) times, with its two divisions, from global memory:
 // a call on 231 x 180 x 64 took 384 us, with this form 137 us.  Issue-bound.
 //
-// The arithmetic is open_adv.cuh's point functions', term for term.
+// The arithmetic is that of open_adv.cuh's point functions, term for term, with each
+// face's Courant number and low-order factor formed here as k_pd_courant forms them.
 struct PdrPlanes {
   static constexpr int HW = TX + 8, HH = TY + 8, HN = HW * HH;  // staged plane, origin (i0 - 4, j0 - 4)
   static constexpr int SW = TX + 2, SH = TY + 2, SN = SW * SH;  // limiter region
@@ -437,7 +438,7 @@ __global__ void __launch_bounds__(STRIP_THREADS) k_strip_pd_scale(StripLaunch L,
   const int i = sp.i, j = sp.j, k = sp.k;
   if (k < m.kts || k > min(m.kte, m.kde - 1)) return;
   const Stage st = stage_of(m, rk_step);
-  const PDCtx c = pd_ctx(m, s, st.dt_rk, true);
+  const PDCtx c = pd_ctx(m, s, st.dt_rk);
   const long long plane = (long long)strip_cols(m.ide, m.jde, m.cf.open_xs, m.cf.open_ys, L.w, L.h) * (m.kme - m.kms + 1);
   scratch[sp.m][s * plane + sp.p] = pd_scale_cell(m, c, i, k, j);
 }
@@ -451,7 +452,7 @@ __global__ void __launch_bounds__(STRIP_THREADS) k_strip_pd_tend(StripLaunch L, 
   const int i = sp.i, j = sp.j, k = sp.k;
   if (!mass_pt(m, i, j) || k < m.kts || k > min(m.kte, m.kde - 1)) return;
   const Stage st = stage_of(m, rk_step);
-  const PDCtx c = pd_ctx(m, s, st.dt_rk, true);
+  const PDCtx c = pd_ctx(m, s, st.dt_rk);
   const int nc = strip_cols(m.ide, m.jde, m.cf.open_xs, m.cf.open_ys, ww, wh);
   const float* sc = scratch[sp.m] + (long long)s * nc * (m.kme - m.kms + 1);
   const float t = pd_tend_cell(m, c, i, k, j, 0.f, [&](int ci, int ck, int cj) {
