@@ -242,15 +242,21 @@ int wrfgpu_profile_phases(WrfGpuEnsemble* h, int nsteps, double* ms_out, int* la
  * families its launch variants — blocks per SM of the column and
  * scalar-transport kernels, level chunks of the split column kernels — and
  * keeps the fastest per family for the captured step.  Every variant
- * computes the same bits.  Family order: scalar_pd_update,
+ * computes the same bits.  The families are timed one after another on one
+ * stream (the step itself runs several side by side).  Where the step takes a
+ * row-segment kernel (narrow domains) the variants of advance_mu_t, advance_w
+ * and sumflux_calc_p_rho, and of step_prep, select nothing and their times
+ * differ by noise only.  Family order: scalar_pd_update,
  * scalar_adv_update, advance_w, advance_uv, sumflux_calc_p_rho, step_prep,
  * small_step_finish, small_step_prep, cfl_check, rk_tend_w, rk_tend_u,
  * rk_tend_v, calc_p_rho_phi, advance_mu_t. */
 #define WRFGPU_NTUNE 14
 int wrfgpu_autotune(WrfGpuEnsemble* h, int rounds);
 /* The chosen variant of each family, the parameter it stands for (blocks per
- * SM, level chunks, or 10 x blocks per SM + level chunks for advance_uv,
- * rk_tend_u and rk_tend_v), and the measured ms per step of every variant
+ * SM, level chunks, or 10 b + level chunks for advance_uv, rk_tend_u and
+ * rk_tend_v, b = 3 for four and b = 4 for five of their 128-thread blocks per
+ * SM; the level chunks are the fewest, a launch adds to them where the tiles
+ * leave SMs idle), and the measured ms per step of every variant
  * (ms[f * 4 + v], -1 when not timed).  Returns WRFGPU_NTUNE. */
 int wrfgpu_tuning(WrfGpuEnsemble* h, int* variant, int* param, float* ms, int nfamily);
 const char* wrfgpu_phase_name(int phase);

@@ -1,10 +1,10 @@
-"""wrfgpu_advect_scalar_pd_noalloc: the PD advection on device arrays with
-the limiter-factor scratch in a static device array (no allocation).
+"""wrfgpu_advect_scalar_pd_noalloc: the PD advection on device arrays, one
+launch that keeps the limiter factors in shared memory (no allocation).
 
 Checked against the routine-level entry point wrfgpu_advect_scalar_pd (host
 arrays, its own device domain) on the same developed state: two calls in a
 row, the tendency accumulating from the same seeded start.  The two run the
-same kernels on the same member layout, so the tendency must agree bit for
+same tile code on the same values, so the tendency must agree bit for
 bit.  This file is collected last and passes alone as well."""
 import ctypes as C
 

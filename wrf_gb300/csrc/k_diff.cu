@@ -346,8 +346,8 @@ __device__ __forceinline__ void forward_col(const Mem& m, const F3& f, const F3*
 // species).  About 480 instructions a point and 24 reads with a 92% L1 hit rate:
 // bound by their latency (issue 36% at 16 warps per SM), so by the warps an SM
 // holds: us of modes 0 / 1 at 160x144x64 with 2 species and 1, 2, 3, 4, 5, 6 blocks
-// per SM 251/111, 188/90, 173/70, 127/61, 133/75, 170/73 (spills from 5 on); a
-// thread per point, each vertical flux formed twice, 214/107.
+// per SM 251/111, 188/90, 173/70, 127/61, 133/75, 170/73 (bytes of spill stores
+// and loads per thread 0 up to 3 blocks, 92 and 224 at 4, 640 and 1196 at 5); a thread per point, each vertical flux formed twice, 214/107.
 __global__ void __launch_bounds__(TX* TY, 4) k_forward_diff(TileLaunch L, int mode) {
   const TilePos tp = tile_pos(L, TILE_ONE, true);
   const Mem& m = block_member(L.mem, tp.m);

@@ -2,16 +2,16 @@
 //   rk_update_scalar_pd  dyn_em/module_em.F:1803-1916 (physics tendency 0)
 //   advect_scalar        dyn_em/module_advect_em.F:3394-3650, :4306-4333
 //   advect_scalar_pd     dyn_em/module_advect_em.F:6505-6779, :7595-7645, limiter :7681-7781,
-//                        divergence :7783-7883 — two passes: (1) per-cell limiter scale of
-//                        every cell of the tile and its 1-cell halo into a scratch array,
-//                        (2) per-cell divergence of the face fluxes, each face scaled by its
-//                        upwind cell's factor (a face is only ever modified by its upwind
-//                        cell, so the result does not depend on the reference's loop order)
+//                        divergence :7783-7883 — routine-level calls: pd_tile, one launch, the
+//                        face fluxes and limiter factors of a tile in shared memory; edge
+//                        strips of the large step: the factors into a scratch, then the
+//                        divergence of the limited fluxes (a face is only ever modified by its
+//                        upwind cell, so the result does not depend on the reference's loop order)
 //   rk_update_scalar     dyn_em/module_em.F:1587-1799
 //   calc_p_rho_phi       dyn_em/module_big_step_utilities_em.F:953-1226 (non-hydrostatic)
 //   set_w_surface        dyn_em/module_bc_em.F:1196-1295
-// Roofline: HBM-bound; the limiter pass reads the 5 transport arrays twice
-// (scale pass and divergence pass) plus the scale scratch.
+// Roofline: calc_p_rho_phi and rk_update_scalar are HBM-bound; pd_tile and the
+// strips are bound by instructions and latency (measured beside each).
 #include "common.cuh"
 #include "kernels.h"
 #include "ffmath.h"
@@ -125,7 +125,7 @@ __global__ void __launch_bounds__(BX* BY) k_advect_scalar(Launch L, int species,
 // k_scalar_pd_update, k_scalar_fused.cu, which documents their reuse).  Two
 // passes over points formed each flux two (limiter, divergence) times two
 // (the face's two cells) times, with its two divisions, from global memory:
-// a call on 231 x 180 x 64 took 384 us, with this form 137 us.  Issue-bound.
+// a call on 231 x 180 x 64 took 384 us, with this form 130 us.  Issue-bound.
 //
 // The arithmetic is that of open_adv.cuh's point functions, term for term, with each
 // face's Courant number and low-order factor formed here as k_pd_courant forms them.

@@ -66,8 +66,9 @@ constexpr int TUNE_NVAR[NTUNE] = {2, 3, 3, 4, 4, 2, 2, 4, 4, 3, 4, 4, 4, 4};
 // advance_mu_t is best with three, 524 against 571 us on the 16-member ensemble)
 constexpr int TUNE_DEFAULT[NTUNE] = {1, 1, 2, 0, 2, 1, 0, 2, 2, 1, 3, 2, 2, 2};
 // the parameter each variant stands for: blocks per SM, level chunks
-// (sumflux: of calc_p_rho), or (advance_uv, rk_tend_u, rk_tend_v) 10 x blocks
-// per SM + level chunks
+// (sumflux: of calc_p_rho), or (advance_uv, rk_tend_u, rk_tend_v) 10 b + level
+// chunks, b = 3: four 128-thread blocks per SM, b = 4: five.  Level chunks are the
+// fewest: level_chunks adds to them.
 constexpr int TUNE_PARAM[NTUNE][TUNE_MAXVAR] = {{1, 2, 0, 0}, {2, 3, 4, 0}, {2, 3, 4, 0}, {32, 42, 34, 44}, {1, 2, 4, 8},
                                                 {3, 8, 0, 0}, {4, 8, 0, 0}, {1, 2, 4, 8}, {2, 4, 8, 16}, {2, 3, 4, 0},
                                                 {32, 42, 34, 44}, {32, 42, 34, 44}, {1, 2, 4, 8}, {2, 3, 4, 5}};
@@ -109,9 +110,13 @@ void launch_calc_p_rho(const Launch& L3, int nblocks, StepArgs a, cudaStream_t s
 void launch_calc_coef_w(const Launch& L2, int nblocks, StepArgs a, bool fp64, cudaStream_t s);
 void launch_calc_coef_w_col(const TileLaunch& L, int nblocks, StepArgs a, bool fp64, cudaStream_t s);  // mass tiles
 // mass row segments, FP32, up to COEF_ROW_MAX of them (its recursion runs in one
-// warp of a block): 41x41x41 (82) 0.037 / 0.083, 160x144x64 (720) 0.099 / 0.139,
-// 190x161x60 (966) 0.129 / 0.132, 256x256x80 (2048) 0.27 / 0.19; FP64 75x90x128
-// (270) 0.43 / 0.40
+// warp of a block): ms per step, this form / the column march, 41x41x41 (82 segments)
+// 0.037 / 0.083, 160x144x64 (720) 0.099 / 0.139, 190x161x60 (966) 0.129 / 0.136,
+// 224x192x64 (1344) 0.141 / 0.151, 256x210x80 (1680) 0.221 / 0.184, 256x256x80 (2048)
+// 0.270 / 0.196; FP64 75x90x128 (270) 0.43 / 0.40.  Timed alone the forms are level near
+// 1500 segments, but in the step, beside the halo fill, this one's blocks cost more than
+// it gains from 966 on (whole step 2.578 / 2.515, at 1344 3.536 / 3.448): the line is
+// below that
 constexpr int COEF_ROW_MAX = 900;
 void launch_calc_coef_w_row(const TileLaunch& L, int nblocks, StepArgs a, cudaStream_t s);
 void launch_advance_uv(const Launch& L3, int nblocks, StepArgs a, cudaStream_t s);
@@ -174,8 +179,11 @@ void launch_advance_uv_col(const TileLaunch& L, int nblocks, int rk_step, int it
 // 190x161x60 (966) 0.77 / 1.33, 256x256x80 (2048) 1.70 / 1.99, 24 small members
 // (about 2900) 2.23 / 2.30, 512x512x80 (8192) 6.30 / 5.67, 1024x1024x96 (32768)
 // 29.0 / 24.9; FP64 columns (whose chains wait about 110 cycles per operation)
-// 75x90x128 (270) 0.81 / 3.11, 16 members of up to 256x256x80 (about 14000)
-// 17.5 / 9.3; with damp_opt = 3 160x144x64 (720) 0.76 / 1.39.
+// 75x90x128 (270) 0.81 / 3.11, 200x170x80 (1190) 1.75 / 2.21, 256x256x80 (2048)
+// 3.01 / 2.48, 384x320x80 (3840) 5.46 / 4.12, 512x384x80 (6144) 8.62 / 6.10, 16 members
+// of up to 256x256x80 (about 14000) 17.5 / 9.3; with damp_opt = 3 160x144x64 (720)
+// 0.76 / 1.39.  The FP64 forms cross between 1190 and 2048 segments; 1000 is on the
+// column kernel's side, short of the crossing.
 constexpr int col_max_segments(bool fp64) { return fp64 ? 1000 : 3000; }
 // damp: some member uses damp_opt = 3 (compiles the damping into the kernel)
 void launch_advance_col(const TileLaunch& L, int nblocks, int nlev_max, int rk_step, int iteration, bool fp64,
