@@ -319,10 +319,10 @@ struct Ensemble {
     cudaStreamWaitEvent(stream, ev_head, 0);
     io_pending = false;
   }
-  // Upload of field q on ustream after the downloads of this phase that use
-  // its staging buffer or write its host input (dn[g]: g's download is in
-  // this phase).
-  void upload_after(size_t q, const std::vector<char>& dn) {
+  // Upload of field q on `st` after the downloads of this phase that use its
+  // staging buffer or write its host input (dn[g]: g's download is in this
+  // phase).
+  void upload_after(size_t q, const std::vector<char>& dn, cudaStream_t st) {
     const HostIO& b = hio[q];
     const char* lo = (const char*)b.in;
     const char* hi = lo + b.count * 4;
@@ -330,9 +330,9 @@ struct Ensemble {
       if (!dn[g]) continue;
       const char* glo = (const char*)hio[g].out;
       const char* ghi = glo + hio[g].count * 4;
-      if (g == q || (lo < ghi && glo < hi)) cudaStreamWaitEvent(ustream, ev_dn[g], 0);
+      if (g == q || (lo < ghi && glo < hi)) cudaStreamWaitEvent(st, ev_dn[g], 0);
     }
-    cudaMemcpyAsync(b.stage, b.in, b.count * 4, cudaMemcpyHostToDevice, ustream);
+    cudaMemcpyAsync(b.stage, b.in, b.count * 4, cudaMemcpyHostToDevice, st);
   }
   // the _2 dry state is final once the last stage's fills and set_w_surface
   // are done (enqueue_step): its bound outputs cross the link on the copy
@@ -399,7 +399,7 @@ struct Ensemble {
     // on the other copy engine direction, each after the downloads it waits for
     if (io_prefetch)
       for (size_t q = 0; q < hio.size(); ++q)
-        if (hio[q].prefetch) upload_after(q, dn);
+        if (hio[q].prefetch) upload_after(q, dn, ustream);
     cudaEventRecord(ev_ojoin, cstream);
     cudaEventRecord(ev_ojoin2, ustream);
     io_out_pending = true;
@@ -584,10 +584,10 @@ struct Ensemble {
     }
     CK(cudaEventRecord(ev_head, cstream));
     // ... the dry state and the moist species first on the other, at the
-    // link's full rate (those prefetched during the previous step are across)
-    for (const HostIO& b : hio)
-      if (b.in && !b.late && !(head && (b.prefetch || b.tail)))
-        CK(cudaMemcpyAsync(b.stage, b.in, b.count * 4, cudaMemcpyHostToDevice, stream));
+    // link's full rate (those prefetched during the previous step are across;
+    // one whose host input a deferred download writes comes behind it)
+    for (size_t q = 0; q < hio.size(); ++q)
+      if (hio[q].in && !hio[q].late && !(head && (hio[q].prefetch || hio[q].tail))) upload_after(q, dn, stream);
     CK(cudaEventRecord(ev_dryin, stream));
     for (const HostIO& b : hio)
       if (b.in && !b.late) unpack(b, stream);
@@ -612,7 +612,7 @@ struct Ensemble {
       io_split = late_b != 0 && na > 0;
     }
     for (size_t r = 0; r < lq.size(); ++r) {
-      upload_after(lq[r], dn);
+      upload_after(lq[r], dn, ustream);
       unpack(hio[lq[r]], ustream);
       if (io_split && r + 1 == na) CK(cudaEventRecord(ev_upA, ustream));
     }
@@ -649,7 +649,7 @@ struct Ensemble {
       copy_out(l);
       if (pre)
         for (size_t q = 0; q < hio.size(); ++q)
-          if (hio[q].tail) upload_after(q, tdn);
+          if (hio[q].tail) upload_after(q, tdn, ustream);
       CK(cudaEventRecord(ev_tjoin, cstream));
       CK(cudaEventRecord(ev_tjoin2, ustream));
       CK(cudaStreamWaitEvent(stream, ev_tjoin, 0));
